@@ -54,6 +54,7 @@ struct Params {
     double bl_exp;                       // 1/7
     double inv_cv;                       // 1/CV
     double cp_pr, cp_prt;                // CP/PRANDTL, CP/PRANDTLT
+    double inv_cmu_suth;                 // 1/(CMU*SUTH_COEF*DSQRT(AMOL))
 };
 
 // Static per-face geometry of the viscous flux (viscous.f90:130-217), [FG_N][nfaces]
@@ -111,40 +112,73 @@ TNS_HD double powi(double x, int n) {
     return n < 0 ? 1.0 / r : r;
 }
 
-// T**0.6 for T > 0, as T * w with w = T^(-2/5) = (T^2)^(-1/5): a single-precision
-// estimate exp2(-0.4 log2 T) (about 1e-7 relative) refined by two Newton steps for the
-// inverse fifth root of a = T^2, which need no division:
-//   w <- w + w (1 - a w^5) / 5,
-// whose error goes as e' ~ 3 e^2: 3e-14 after one step, FP64 rounding after two.
-// Within a few ulp of pow.
-TNS_HD double pow06(double T) {
+// 1/x and sqrt(x) by Newton's method on the hardware's reciprocal and reciprocal-square-root
+// estimates (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64: 20 bits or more), two quadratic steps
+// each, the last one rounding the final sum: within one ulp for normal arguments.  They have no
+// slow path (a call with its register and branch cost), which the arguments here -- densities,
+// temperatures, squared speeds -- never need.  The kernels are bound by instruction issue and
+// dependent FP64 latency: with these, the cubic T**-1/5 step, the shorter expm1 and the skipped
+// denominators below, a FP64 iteration of the 1024 x 384 nozzle-plume went 0.180 -> 0.160 ms
+// (0.041 -> 0.0375 ms on the 115 x 50 nozzle), its error against a FP64 restatement unchanged.  recip(0), recip(inf) and root(inf) are NaN: a
+// state that holds them is non-finite either way.  root() takes a subnormal for zero.
+TNS_HD double recip(double x) {
 #ifdef __CUDA_ARCH__
-    double w = (double)exp2f(-0.4f * __log2f((float)T));
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
 #else
-    double w = (double)exp2f(-0.4f * log2f((float)T));
+    return 1.0 / x;
 #endif
-    const double a = T * T;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const double w2 = w * w;
-        const double t = 1.0 - a * (w2 * w2 * w);
-        w = w + 0.2 * w * t;
-    }
-    return T * w;
+}
+TNS_HD double root(double x) {
+#ifdef __CUDA_ARCH__
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    double g = x * r, h = 0.5 * r;
+    const double e = fma(-g, h, 0.5);
+    g = fma(g, e, g);
+    h = fma(h, e, h);
+    g = fma(h, fma(-g, g, x), g);
+    return fabs(x) < 2.2250738585072014e-308 ? 0.0 : g;
+#else
+    return sqrt(x);
+#endif
+}
+
+// T**(-1/5) for T > 0: a single-precision estimate exp2(-0.2 log2 T) (about 1e-7 relative)
+// refined by one cubically convergent step for the inverse fifth root,
+//   t = 1 - T y^5,  y <- y (1 + t/5 + 3 t^2/25),
+// whose truncation error is below 1e-19.  T**0.6 is T y^2 and T**-0.6 is y^3, so the
+// viscosity and its reciprocal come from one evaluation without a division.
+TNS_HD double inv_fifth_root(double T) {
+#ifdef __CUDA_ARCH__
+    const double y = (double)exp2f(-0.2f * __log2f((float)T));
+#else
+    const double y = (double)exp2f(-0.2f * log2f((float)T));
+#endif
+    const double y2 = y * y;
+    const double t = fma(-T, (y2 * y2) * y, 1.0);
+    return fma(y, t * fma(0.12, t, 0.2), y);
+}
+
+// T**0.6, within a few ulp of pow.
+TNS_HD double pow06(double T) {
+    const double y = inv_fifth_root(T);
+    return T * (y * y);
 }
 
 // expm1(x) for 0 <= x <= 40 (device; libm on the host), by the classical additive
-// argument reduction and a truncated series (Cody & Waite; the structure of Tang's
-// expm1, ACM TOMS 18(2), 1992, without its table):
+// argument reduction (Cody & Waite; the structure of Tang's expm1, ACM TOMS 18(2), 1992,
+// without its table):
 //   x = k ln2 + r, k = rint(x / ln2), |r| <= ln2 / 2, with ln2 = LN2_HI + LN2_LO and
 //   LN2_HI carrying 32 significant bits, so k LN2_HI is exact and r has no cancellation
 //   error;
-//   expm1(r) = r + r^2 (1/2! + r/3! + ... + r^11/13!), the Taylor series of e^r - 1 to
-//   r^13/13!: the first omitted term, r^14/14!, is below 5e-18 for |r| <= ln2 / 2;
+//   expm1(r) = r + r^2 q(r), q the degree-9 interpolant of (e^r - 1 - r)/r^2 at the
+//   Chebyshev points of [-ln2/2, ln2/2] (error of the whole below 4.1e-17 relative),
+//   its even and odd powers summed apart so that the dependent chain is half as long;
 //   expm1(x) = 2^k expm1(r) + (2^k - 1) in one fused multiply-add (2^k - 1 is exact
 //   for k <= 53, and k <= 58 here).
-// Measured on B200 over 4M points of [0, 40]: within 2.7e-16 relative of libm (the CUDA
-// function: 2.2e-16), at 1.4x its throughput.
 TNS_HD double expm1_nonneg(double x) {
 #ifdef __CUDA_ARCH__
     constexpr double INV_LN2 = 1.4426950408889634;
@@ -152,32 +186,45 @@ TNS_HD double expm1_nonneg(double x) {
     constexpr double LN2_LO = 7.440617110012397e-11;  // ln 2 - LN2_HI
     const double k = rint(x * INV_LN2);
     const double r = fma(-k, LN2_LO, fma(-k, LN2_HI, x));
-    double q = 1.6059043836821613e-10;  // 1/13!
-    q = fma(q, r, 2.08767569878681e-09);   // 1/12!
-    q = fma(q, r, 2.505210838544172e-08);  // 1/11!
-    q = fma(q, r, 2.755731922398589e-07);  // 1/10!
-    q = fma(q, r, 2.7557319223985893e-06); // 1/9!
-    q = fma(q, r, 2.48015873015873e-05);   // 1/8!
-    q = fma(q, r, 0.0001984126984126984);  // 1/7!
-    q = fma(q, r, 0.001388888888888889);   // 1/6!
-    q = fma(q, r, 0.008333333333333333);   // 1/5!
-    q = fma(q, r, 0.041666666666666664);   // 1/4!
-    q = fma(q, r, 0.16666666666666666);    // 1/3!
-    q = fma(q, r, 0.5);                    // 1/2!
-    const double p = fma(r * r, q, r);
-    const double s = __longlong_as_double((long long)((int)k + 1023) << 52);  // 2^k
-    return fma(s, p, s - 1.0);
+    const double s = r * r;
+    double a = 2.7620138719733994e-07, b = 2.5100424157005067e-08;
+    a = fma(a, s, 2.480152119021773e-05);
+    b = fma(b, s, 2.7557268378684192e-06);
+    a = fma(a, s, 0.0013888888917281794);
+    b = fma(b, s, 0.00019841269863105968);
+    a = fma(a, s, 0.04166666666662399);
+    b = fma(b, s, 0.008333333333330051);
+    a = fma(a, s, 0.5000000000000001);
+    b = fma(b, s, 0.16666666666666669);
+    const double p = fma(s, fma(b, r, a), r);
+    const double w = __longlong_as_double((long long)((int)k + 1023) << 52);  // 2^k
+    return fma(w, p, w - 1.0);
 #else
     return expm1(x);
 #endif
 }
 
-// tanh(a) / tanh(b) for a, b >= 0, from tanh(x) = E / (E + 2) with E = expm1(2x):
-// Ea (Eb + 2) / (Eb (Ea + 2)), one division instead of three.  Arguments are capped at
-// 20, where tanh is 1 to double precision, so E stays finite.
+// tanh(a) / tanh(b) for a, b >= 0, from tanh(x) = E / (E + 2) with E = expm1(2x), as
+// num / den = Ea (Eb + 2) / (Eb (Ea + 2)).  Arguments are capped at 20, where tanh is 1 to
+// double precision, so E stays finite; a denominator's tanh(b) that is 1 (b >= 20: the
+// damping of a cell whose eddy viscosity is ten times the molecular one or more) is left
+// out, expm1 and all.
+struct Ratio {
+    double num, den;
+};
+TNS_HD Ratio tanh_ratio_parts(double a, double b) {
+    const double ea = expm1_nonneg(2.0 * fmin(a, 20.0));
+    Ratio r{ea, ea + 2.0};
+    if (!(b >= 20.0)) {
+        const double eb = expm1_nonneg(2.0 * b);
+        r.num = ea * (eb + 2.0);
+        r.den = eb * (ea + 2.0);
+    }
+    return r;
+}
 TNS_HD double tanh_ratio(double a, double b) {
-    const double ea = expm1_nonneg(2.0 * fmin(a, 20.0)), eb = expm1_nonneg(2.0 * fmin(b, 20.0));
-    return (ea * (eb + 2.0)) / (eb * (ea + 2.0));
+    const Ratio r = tanh_ratio_parts(a, b);
+    return r.num / r.den;
 }
 
 // Sutherland-type molecular viscosity SUTH_COEF*DSQRT(AMOL)*T**0.6 (viscous.f90:188).
@@ -220,7 +267,7 @@ struct Prim {
 TNS_HD void primitive(const Params& P, double c1, double c2, double c3,
                                           double c4, double c5, Prim& s) {
     const double RHO = c1;
-    const double rr = 1.0 / RHO;  // one reciprocal instead of four divisions
+    const double rr = recip(RHO);  // one reciprocal instead of four divisions
     s.rho = RHO;
     s.u = c2 * rr;
     s.v = c3 * rr;
@@ -240,7 +287,7 @@ TNS_HD void primitive(const Params& P, double c1, double c2, double c3,
     s.g[4] = RHO * RT * s.v;
     s.ri = RT;
     s.c5 = c5;
-    s.qm = sqrt(s.u * s.u + s.v * s.v);
+    s.qm = root(s.u * s.u + s.v * s.v);
 }
 
 // The mixed path's reference state of a stage tile: a FP64 state of the tile (its first
@@ -456,10 +503,18 @@ __device__ __forceinline__ void source_terms(const Params& P, const SrcIn& s, do
     const double DRX = drac * s.ga + drbd * s.gb, DRY = drac * s.gc + drbd * s.gd;
     const double DUX = duac * s.ga + dubd * s.gb, DUY = duac * s.gc + dubd * s.gd;
     const double DVX = dvac * s.ga + dvbd * s.gb, DVY = dvac * s.gc + dvbd * s.gd;
-    const double AMU = amu_of(P, TI);
-    const double CHI = RHO * RI / (CMU * AMU);
-    const double FMU = tanh_ratio(ALPHA_T * CHI * CHI, BETA_T * CHI * CHI);
-    const double FR2 = tanh_ratio(sqrt(CHI), CHI * P.fr2k);
+    // AMU = SUTH T^0.6, CHI = RHO RI / (CMU AMU) with T^-0.6, and both damping ratios by one
+    // reciprocal
+    const double y = inv_fifth_root(TI);
+    const double y2 = y * y;
+    const double AMU = P.suth_amol * (TI * y2);
+    const double CHI = RHO * RI * (P.inv_cmu_suth * (y2 * y));
+    const double chi2 = CHI * CHI;
+    const Ratio fm = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
+    const Ratio fr = tanh_ratio_parts(root(CHI), CHI * P.fr2k);
+    const double inv = recip(fm.den * fr.den);
+    const double FMU = fm.num * fr.den * inv;
+    const double FR2 = fr.num * fm.den * inv;
     const double AMUT = FMU * RHO * RI;
     const double PHI = DQX * DRX + DQY * DRY;
     double DEE = 0.0;
@@ -472,20 +527,20 @@ __device__ __forceinline__ void source_terms(const Params& P, const SrcIn& s, do
     if (P.iaxis == 1) {
         const double VBYY = (YCCI < YAXIS_THRESH) ? DVY : VI * RYCC;
         const double DIVVEL = DUX + DVY + VBYY;
-        PK = AMUT / RHO *
+        PK = FMU * RI *  // AMUT / RHO
              (DUX * DUX + DVY * DVY + VBYY * VBYY + DUX * DUX + DVY * DVY + VBYY * VBYY +
               (DUY + DVX) * (DUY + DVX) - DIV23 * DIVVEL * DIVVEL);
         PK = dmax1(PK, 0.0);
-        src5 = (RHO * (CONST1 - CONST2 * FR2) * sqrt(RI * PK) - RHO * CONST3 * DEE) * pw;
+        src5 = (RHO * (CONST1 - CONST2 * FR2) * root(RI * PK) - RHO * CONST3 * DEE) * pw;
         const double TTT = (AMU + AMUT) * (VBYY + VBYY - DIV23 * DIVVEL);
         src3 = (PI - TTT) * RYCC;
     } else {
         const double DIVVEL = DUX + DVY;
-        PK = AMUT / RHO *
+        PK = FMU * RI *
              (DUX * DUX + DVY * DVY + DUX * DUX + DVY * DVY + (DUY + DVX) * (DUY + DVX) -
               DIV23 * DIVVEL * DIVVEL);
         PK = dmax1(PK, 0.0);
-        src5 = (RHO * (CONST1 - CONST2 * FR2) * sqrt(RI * PK) - RHO * CONST3 * DEE) * pw;
+        src5 = (RHO * (CONST1 - CONST2 * FR2) * root(RI * PK) - RHO * CONST3 * DEE) * pw;
         src3 = 0.0;
     }
 }
@@ -551,10 +606,14 @@ __device__ __forceinline__ void viscous_face(const Params& P, const FaceVals& f,
     } else {
         DIVVEL = DUX + DVY;
     }
-    const double AMU = amu_of(P, TAVG);
+    const double y = inv_fifth_root(TAVG);
+    const double y2 = y * y;
+    const double AMU = P.suth_amol * (TAVG * y2);
     const double AK = AMU * P.cp_pr;
-    const double CHI = RHOAVG * RAVG / (AMU * CMU);
-    const double FMU = tanh_ratio(ALPHA_T * CHI * CHI, BETA_T * CHI * CHI);
+    const double CHI = RHOAVG * RAVG * (P.inv_cmu_suth * (y2 * y));
+    const double chi2 = CHI * CHI;
+    const Ratio fm = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
+    const double FMU = fm.num * recip(fm.den);
     const double AMUT = RHOAVG * RAVG * FMU;
     const double AKT = AMUT * P.cp_prt;
     const double AMUEFF = AMU + AMUT;

@@ -36,6 +36,7 @@ inline Params make_params(const tns_params& p) {
     P.inv_cv = 1.0 / P.cv;
     P.cp_pr = P.cp / p.prandtl;
     P.cp_prt = P.cp / p.prandtlt;
+    P.inv_cmu_suth = 1.0 / (CMU * P.suth_amol);
     return P;
 }
 
