@@ -217,8 +217,6 @@ long long sens_size(long long n, long long npad, long long nnode) {
     return 8 * n + 2 * n + 2 * npad + 2 * nnode + n + nnode + 2 * n;
 }
 
-const double kAlpha[4] = {0.25, 1.0 / 3.0, 0.5, 1.0};  // constants.f90:30-33
-
 // Forward values of the state in set `set` (its q0), on stream st: the iteration with the
 // solver's kernels (stages 1-3 keep their outputs), then every pass of the reverse that
 // depends on the state alone.  Returns the number of kernels launched.
@@ -249,7 +247,7 @@ long long enqueue_forward_primal(tns_handle* h, tns_adjoint_state* s, int set, c
     tns::launch_viscous(P, Ms[0], f.q0.p, f.vis, st);
     for (int k = 0; k < 3; k++) {
         if (k) gport(k);
-        tns::launch_stage(P, Ms[k], qs[k], f.q0.p, qs[k + 1], f.d, f.vis, f.dt, f.dtmin, kAlpha[k], nullptr,
+        tns::launch_stage(P, Ms[k], qs[k], f.q0.p, qs[k + 1], f.d, f.vis, f.dt, f.dtmin, k, h->e.p, nullptr,
                           nullptr, h->status.p, st);
     }
     gport(3);
@@ -300,7 +298,7 @@ long long enqueue_reverse(tns_handle* h, tns_adjoint_state* s, int set, int geo,
     double* lam_stage[5] = {nullptr, s->lamA.p, s->lamB.p, s->lamA.p, s->lam.p};
     for (int k = 3; k >= 0; k--) {
         a.qin = qs[k];
-        a.alpha = kAlpha[k];
+        a.alpha = tns::RK_ALPHA[k];
         a.first = k == 3;
         a.stage1 = k == 0;
         a.lam_in = lam_stage[k + 1];
@@ -599,7 +597,7 @@ int tns_adjoint_record(tns_handle* h, const double* d_q, double* d_q_next, doubl
     s->launches += enqueue_forward_primal(h, s, set, st, &r);
     Mesh M3 = h->M;
     M3.gport = r.gport + 3 * (size_t)h->M.nghosts();
-    tns::launch_stage(h->P, M3, r.q3, r.q0.p, d_q_next, r.d, r.vis, r.dt, r.dtmin, kAlpha[3], nullptr, nullptr,
+    tns::launch_stage(h->P, M3, r.q3, r.q0.p, d_q_next, r.d, r.vis, r.dt, r.dtmin, 3, h->e.p, nullptr, nullptr,
                       h->status.p, st);
     s->launches++;
     r.q0.p = nullptr;  // borrowed: not released by the DevBuf

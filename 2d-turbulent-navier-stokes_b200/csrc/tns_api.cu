@@ -347,6 +347,25 @@ int upload_mesh(tns_handle* h) {
         (rc = up(h->fgj.p, h->hfgj.data(), h->hfgj.size() * 8)))
         return rc;
     // the host copies are not read again
+    // static ghost records
+    {
+        const int ni = h->ni, nj = h->nj;
+        std::vector<tns::GhostRec> rec(ngs);
+        for (int g = 0; g < (int)ngs; g++) {
+            const int side = g < ni ? 1 : g < ni + nj ? 2 : g < 2 * ni + nj ? 3 : 4;
+            const int along = side == 1 ? g : side == 2 ? g - ni : side == 3 ? g - ni - nj : g - 2 * ni - nj;
+            const int ip = side == 2 ? ni - 1 : side == 4 ? 0 : along, jp = side == 1 ? 0 : side == 3 ? nj - 1 : along;
+            const size_t n1 = (size_t)ip * (nj + 1) + jp;
+            const double X[4] = {h->hX[n1], h->hX[n1 + nj + 1], h->hX[n1 + nj + 2], h->hX[n1 + 1]};
+            const double Y[4] = {h->hY[n1], h->hY[n1 + nj + 1], h->hY[n1 + nj + 2], h->hY[n1 + 1]};
+            tns::face_vector(h->P.iaxis, side, X, Y, rec[g].psx, rec[g].psy);
+            rec[g].ycg = h->hgyc[g];
+            rec[g].ycp = (Y[0] + Y[1] + Y[2] + Y[3]) * 0.25;
+        }
+        if ((rc = h->cuda(h->grec.alloc(ngs), "cudaMalloc")) ||
+            (rc = up(h->grec.p, rec.data(), ngs * sizeof(tns::GhostRec))))
+            return rc;
+    }
     std::vector<double>().swap(h->hcvol);
     std::vector<double>().swap(h->hstile);
     std::vector<double>().swap(h->hfgi);
@@ -355,6 +374,7 @@ int upload_mesh(tns_handle* h) {
     M.ni = h->ni; M.nj = h->nj; M.x = h->x.p; M.y = h->y.p; M.cfldl = h->cfldl.p; M.gtype = h->gtype.p;
     M.grank = h->grank.p; M.gxc = h->gxc.p; M.gyc = h->gyc.p; M.ginj = h->ginj.p;
     M.gport = h->gport.p;
+    M.grec = h->grec.p;
     M.cvol = h->cvol.p;
     M.stile = h->stile.p;
     M.fgi = h->fgi.p;
@@ -383,7 +403,8 @@ int alloc_state(tns_handle* h) {
         if (h->unstructured && (rc = h->cuda(h->dt.alloc(nc), "cudaMalloc"))) return rc;
     } else if ((rc = h->cuda(h->qa.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->qb.alloc(5 * nc), "cudaMalloc")) ||
                (rc = h->cuda(h->qc.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->d.alloc(5 * nc), "cudaMalloc")) ||
-               (rc = h->cuda(h->vis.alloc(4 * nc), "cudaMalloc")) || (rc = h->cuda(h->dt.alloc(nc), "cudaMalloc"))) {
+               (rc = h->cuda(h->vis.alloc(4 * nc), "cudaMalloc")) || (rc = h->cuda(h->dt.alloc(nc), "cudaMalloc")) ||
+               (!h->unstructured && (rc = h->cuda(h->e.alloc(5 * nc), "cudaMalloc")))) {
         return rc;
     }
     if ((rc = h->cuda(h->dtmin.alloc(1), "cudaMalloc")) ||
@@ -474,7 +495,6 @@ void enqueue_iteration_f64(tns_handle* h, bool monitor) {
     const Mesh& M = h->M;
     double *A = h->qa.p, *B = h->qb.p, *Cq = h->qc.p;
     const int np = (int)h->port_ghosts.size();
-    static const double alpha[4] = {0.25, 1.0 / 3.0, 0.5, 1.0};  // constants.f90:30-33
     const double* in[4] = {A, B, Cq, B};
     double* out[4] = {B, Cq, B, A};
     prepass(
@@ -495,8 +515,8 @@ void enqueue_iteration_f64(tns_handle* h, bool monitor) {
         if (np && st > 0)
             launch(h, K_GPORT, [&] { tns::launch_gport(P, M, in[st], h->ports.p, np, h->gport.p, s); });
         launch(h, K_STAGE, [&] {
-            tns::launch_stage(P, M, in[st], A, out[st], h->d.p, h->vis.p, h->dt.p, h->dtmin.p,
-                              alpha[st], (monitor && st == 3) ? h->cdiff.p : nullptr,
+            tns::launch_stage(P, M, in[st], A, out[st], h->d.p, h->vis.p, h->dt.p, h->dtmin.p, st, h->e.p,
+                              (monitor && st == 3) ? h->cdiff.p : nullptr,
                               st == 3 ? h->status.p : nullptr, h->status.p, s);
         });
     }
@@ -1137,10 +1157,10 @@ void tns_destroy(tns_handle* h) {
     h->qa2.release(); h->dqb.release(); h->dqc.release(); h->df.release(); h->visf.release();
     h->dtf.release(); h->tref.release();
     for (auto* b : {&h->x, &h->y, &h->cfldl, &h->gxc, &h->gyc, &h->ginj, &h->gport, &h->qa, &h->qb,
-                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol,
+                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->e,
                     &h->stile, &h->fgi, &h->fgj})
         b->release();
-    h->gtype.release(); h->grank.release(); h->ports.release();
+    h->grec.release(); h->gtype.release(); h->grank.release(); h->ports.release();
     h->counter.release(); h->status.release(); h->cdiff.release();
     if (h->pinned) cudaFreeHost(h->pinned);
     if (h->status_host) cudaFreeHost(h->status_host);

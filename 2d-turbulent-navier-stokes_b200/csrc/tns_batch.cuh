@@ -18,11 +18,15 @@ struct StageArgs {
     const double* qin;   // stage input state [5][ncell]
     const double* qold;  // state at the start of the iteration [5][ncell]
     double* qout;        // stage output [5][ncell] (may alias qold: own-cell reads only)
-    const double* d;     // dissipation [5][ncell]
-    const double* vis;   // viscous flux [4][ncell]
+    const double* d;     // dissipation [5][ncell] (stage 1)
+    const double* vis;   // viscous flux [4][ncell] (stage 1)
     const double* dt;    // per-cell DT (LOCAL=1)
     const double* dtmin; // DTMIN (LOCAL=0)
     double alpha;
+    // the frozen terms VIS + D of the iteration, [5][ncell]: stage 1 (e null) forms them and
+    // writes them to eout, stages 2-4 read them from e instead of the nine D and VIS arrays
+    const double* e;
+    double* eout;
     unsigned long long* cdiff;  // 5 slots, ordered bits of max|Q_old-Q_new| (or null)
     unsigned int* status;       // bit 0: non-finite state (checked where non-null)
     unsigned int* error;        // bit 1: a tile's static-block copy did not complete

@@ -116,14 +116,14 @@ BatchCase describe(tns_batch* b, int k) {
         c.diss = tns::DissArgs<double>{A, h->d.p, h->dt.p, h->dtmin.p};
         c.q = A;
         c.vis = h->vis.p;
-        const double alpha[4] = {0.25, 1.0 / 3.0, 0.5, 1.0};  // constants.f90:30-33
         const double* in[4] = {A, B, Cq, B};
         double* out[4] = {B, Cq, B, A};
         for (int mon = 0; mon < 2; mon++)
             for (int st = 0; st < 4; st++)
                 c.stage[mon][st] = tns::StageArgs{in[st], A, out[st], h->d.p, h->vis.p, h->dt.p, h->dtmin.p,
-                                                  alpha[st], (mon && st == 3) ? cdiff : nullptr,
-                                                  st == 3 ? status : nullptr, status};
+                                                  tns::RK_ALPHA[st], st ? h->e.p : nullptr, st ? nullptr : h->e.p,
+                                                  (mon && st == 3) ? cdiff : nullptr, st == 3 ? status : nullptr,
+                                                  status};
     } else {
         double* q[2] = {h->state(), h->other_state()};
         c.qmx[0] = q[0];

@@ -35,6 +35,7 @@ constexpr double YAXIS_THRESH = 0.001;
 constexpr double AMU_THRESH = 0.001;
 constexpr double GTH = 35.0;
 constexpr double CONVKSC = 1.0 / 98066.5;
+constexpr double RK_ALPHA[4] = {0.25, 1.0 / 3.0, 0.5, 1.0};  // constants.f90:30-33
 
 // Scalar inputs plus every constant the Fortran folds left to right (computed once on
 // the host with the same operation order, so device values equal the reference's).
@@ -55,6 +56,8 @@ struct Params {
     double inv_cv;                       // 1/CV
     double cp_pr, cp_prt;                // CP/PRANDTL, CP/PRANDTLT
     double inv_cmu_suth;                 // 1/(CMU*SUTH_COEF*DSQRT(AMOL))
+    double inv_cp, inv_t0;               // 1/CP, 1/T0
+    double rho0, inv_gm1;                // P0/(RR*T0), 1/(GAMA-1)
 };
 
 // Static per-face geometry of the viscous flux (viscous.f90:130-217), [FG_N][nfaces]
@@ -72,6 +75,12 @@ enum FaceGeo { FG_SX, FG_SY, FG_GA, FG_GB, FG_GC, FG_GD, FG_RYAVG, FG_N };
 // and 4 (i=-1) by j; the four runs are stored back to back.
 struct TileRefMx;
 
+// Static geometry of one ghost: its parent's face vector on the ghost's side, the mirrored
+// centroid's y and the parent's.
+struct alignas(16) GhostRec {
+    double psx, psy, ycg, ycp;
+};
+
 struct Mesh {
     int ni, nj;             // cells in i and j
     const double* x;        // node x [(ni+1)*(nj+1)], node (i,j) at i*(nj+1)+j
@@ -81,6 +90,7 @@ struct Mesh {
     const int* grank;       // bc.in line of each ghost (node-average order)
     const double* gxc;      // mirrored ghost centroids (geometry.f90:114-142)
     const double* gyc;
+    const GhostRec* grec;   // static geometry per ghost
     const double* ginj;     // type-6 burn-rate multiplier
     const double* gport;    // type-6 port mass flux of the current stage
     const double* cvol;     // VOL per cell (geometry.f90:87,98,101)
@@ -146,27 +156,30 @@ TNS_HD double root(double x) {
 #endif
 }
 
-// T**(-1/5) for T > 0: a single-precision estimate exp2(-0.2 log2 T) (about 1e-7 relative)
-// refined by one cubically convergent step for the inverse fifth root,
-//   t = 1 - T y^5,  y <- y (1 + t/5 + 3 t^2/25),
-// whose truncation error is below 1e-19.  T**0.6 is T y^2 and T**-0.6 is y^3, so the
-// viscosity and its reciprocal come from one evaluation without a division.
-TNS_HD double inv_fifth_root(double T) {
+// T**-0.4 and T**-0.6 for T > 0: a single-precision estimate y = exp2(-0.2 log2 T) of
+// T**(-1/5) (about 1e-7 relative) and one cubically convergent step for the inverse fifth
+// root,
+//   t = 1 - T y^5,  y (1 + c),  c = t/5 + 3 t^2/25,
+// whose truncation error is below 1e-19; (1 + c)^2 and (1 + c)^3 then correct y^2 (exact: y
+// has 24 bits) and y^3 in one rounding each.  The viscosity, T**0.6 = T T**-0.4, and its
+// reciprocal thus come from one evaluation without a division (T**0.6 within 1.5 ulp).
+struct FifthRoots {
+    double m04, m06;
+};
+TNS_HD FifthRoots fifth_roots(double T) {
 #ifdef __CUDA_ARCH__
     const double y = (double)exp2f(-0.2f * __log2f((float)T));
 #else
     const double y = (double)exp2f(-0.2f * log2f((float)T));
 #endif
-    const double y2 = y * y;
-    const double t = fma(-T, (y2 * y2) * y, 1.0);
-    return fma(y, t * fma(0.12, t, 0.2), y);
+    const double y2 = y * y, y3 = y2 * y;
+    const double t = fma(-T, y2 * y3, 1.0);
+    const double c = t * fma(0.12, t, 0.2);
+    return FifthRoots{fma(y2, fma(c, c, 2.0 * c), y2), fma(y3, c * fma(3.0, c, 3.0), y3)};
 }
 
 // T**0.6, within a few ulp of pow.
-TNS_HD double pow06(double T) {
-    const double y = inv_fifth_root(T);
-    return T * (y * y);
-}
+TNS_HD double pow06(double T) { return T * fifth_roots(T).m04; }
 
 // expm1(x) for 0 <= x <= 40 (device; libm on the host), by the classical additive
 // argument reduction (Cody & Waite; the structure of Tang's expm1, ACM TOMS 18(2), 1992,
@@ -359,6 +372,32 @@ TNS_HD double cell_volume(int iaxis, const double X[4], const double Y[4],
     return v;
 }
 
+// Density of the type-2 inlet at temperature T, (S0/(RR T))**(1/(1-GAMA)): the isentrope
+// through (P0, T0), RHO0 (T/T0)**(1/(GAMA-1)).  With z = 1 - T/T0 = (GAMA-1)/2 M^2 T/T0 small
+// (M < 1.29 at GAMA = 1.4), log(1 - z) = -2 atanh(z/(2-z)) by its series to the 19th power
+// (the next term is below 4e-18), so the exponent carries no rounding of a large logarithm;
+// pow elsewhere.  A third of pow's instructions on the path a boundary tile waits for.
+TNS_HD double inlet_density(const Params& P, double T) {
+#ifdef __CUDA_ARCH__
+    const double z = (P.t0 - T) * P.inv_t0;
+    if (z >= 0.0 && z < 0.25) {
+        const double w = z * recip(2.0 - z), w2 = w * w;
+        double a = 1.0 / 19.0;
+        a = fma(a, w2, 1.0 / 17.0);
+        a = fma(a, w2, 1.0 / 15.0);
+        a = fma(a, w2, 1.0 / 13.0);
+        a = fma(a, w2, 1.0 / 11.0);
+        a = fma(a, w2, 1.0 / 9.0);
+        a = fma(a, w2, 1.0 / 7.0);
+        a = fma(a, w2, 0.2);
+        a = fma(a, w2, 1.0 / 3.0);
+        a = fma(a, w2, 1.0);
+        return P.rho0 * exp(-2.0 * P.inv_gm1 * (w * a));
+    }
+#endif
+    return pow(P.s0 / (P.rr * T), P.inv1mg);
+}
+
 // Ghost state from its parent (and the parent's opposite neighbour) for BC types 2..7
 // (boundary.f90:53-327; type 6 with the port flux supplied by the caller).
 // par: parent cell, opp: parent's neighbour across the face opposite the ghost.
@@ -368,18 +407,16 @@ TNS_HD void boundary_ghost(const Params& P, int type, const Prim& par,
                                                const Prim& opp, double psx, double psy,
                                                double ycc_g, double ycc_p, double gport,
                                                double inj, Prim& g) {
-    double RHO, AMU, RT, C5;
+    double RHO, AMU, C5;
     switch (type) {
         case 2: {  // subsonic inlet :53-71
             g.u = fabs(par.u);
             g.v = -par.v;
-            g.t = P.t0 - 0.5 * (g.u * g.u + g.v * g.v) / P.cp;
-            RHO = pow(P.s0 / (P.rr * g.t), P.inv1mg);
+            g.t = P.t0 - 0.5 * (g.u * g.u + g.v * g.v) * P.inv_cp;
+            RHO = inlet_density(P, g.t);
             g.p = RHO * P.rr * g.t;
-            AMU = amu_of(P, g.t);
-            RT = AMU / RHO;
             ghost_tail(P, RHO, g);
-            C5 = RHO * RT;
+            C5 = amu_of(P, g.t);  // RHO * (AMU / RHO)
             g.f[4] = C5 * g.u;
             g.g[4] = C5 * g.v;
             break;
@@ -390,7 +427,7 @@ TNS_HD void boundary_ghost(const Params& P, int type, const Prim& par,
             g.t = 2.0 * par.t - opp.t;
             g.p = 2.0 * par.p - opp.p;
             if (P.pamb >= 0.0) g.p = P.pamb;
-            RHO = g.p / (P.rr * g.t);
+            RHO = g.p * recip(P.rr * g.t);
             ghost_tail(P, RHO, g);
             C5 = par.c5;
             g.f[4] = par.f[4];
@@ -441,7 +478,7 @@ TNS_HD void boundary_ghost(const Params& P, int type, const Prim& par,
             g.p = par.p;
             g.u = VEL * ENX + VEL * ENX - par.u;
             g.v = VEL * ENY + VEL * ENY - par.v;
-            g.t = P.tflame - 0.5 * (g.u * g.u + g.v * g.v) / P.cp;
+            g.t = P.tflame - 0.5 * (g.u * g.u + g.v * g.v) * P.inv_cp;
             AMU = amu_of(P, g.t);
             const double GVAL =
                 (GP / (P.rhoprop * RDOT)) * pow(P.rhoprop * RDOT * DHYD / AMU, -0.125);
@@ -449,11 +486,9 @@ TNS_HD void boundary_ghost(const Params& P, int type, const Prim& par,
             VEL = P.rhoprop / RHO * RDOTEB;
             g.u = VEL * ENX + VEL * ENX - par.u;
             g.v = VEL * ENY + VEL * ENY - par.v;
-            g.t = P.tflame - 0.5 * (g.u * g.u + g.v * g.v) / P.cp;
-            RHO = g.p / (P.rr * g.t);
-            AMU = amu_of(P, g.t);
-            RT = AMU / RHO;
-            C5 = RHO * RT;
+            g.t = P.tflame - 0.5 * (g.u * g.u + g.v * g.v) * P.inv_cp;
+            RHO = g.p * recip(P.rr * g.t);
+            C5 = amu_of(P, g.t);
             ghost_tail(P, RHO, g);
             g.f[4] = C5 * g.u;
             g.g[4] = C5 * g.v;
@@ -463,23 +498,21 @@ TNS_HD void boundary_ghost(const Params& P, int type, const Prim& par,
             g.p = P.pinf;
             g.t = P.tinf;
             g.v = -par.v;
-            RHO = g.p / (P.rr * g.t);
+            RHO = g.p * recip(P.rr * g.t);
             if (ycc_g <= P.deltabl)
                 g.u = P.bl_u * pow(ycc_g / P.deltabl, P.bl_exp) - par.u;
             else
                 g.u = P.bl_u - par.u;
-            AMU = amu_of(P, g.t);
-            RT = AMU / RHO;
             ghost_tail(P, RHO, g);
-            C5 = RHO * RT;
+            C5 = amu_of(P, g.t);
             g.f[4] = C5 * g.u;
             g.g[4] = C5 * g.v;
             break;
         }
     }
     g.c5 = C5;
-    g.ri = C5 / g.rho;
-    g.qm = sqrt(g.u * g.u + g.v * g.v);
+    g.ri = C5 * recip(g.rho);
+    g.qm = root(g.u * g.u + g.v * g.v);
 }
 
 // Turbulence / radial sources of one cell (source_terms.f90:24-104).  Neighbours
@@ -505,10 +538,9 @@ __device__ __forceinline__ void source_terms(const Params& P, const SrcIn& s, do
     const double DVX = dvac * s.ga + dvbd * s.gb, DVY = dvac * s.gc + dvbd * s.gd;
     // AMU = SUTH T^0.6, CHI = RHO RI / (CMU AMU) with T^-0.6, and both damping ratios by one
     // reciprocal
-    const double y = inv_fifth_root(TI);
-    const double y2 = y * y;
-    const double AMU = P.suth_amol * (TI * y2);
-    const double CHI = RHO * RI * (P.inv_cmu_suth * (y2 * y));
+    const FifthRoots tr = fifth_roots(TI);
+    const double AMU = P.suth_amol * (TI * tr.m04);
+    const double CHI = RHO * RI * (P.inv_cmu_suth * tr.m06);
     const double chi2 = CHI * CHI;
     const Ratio fm = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
     const Ratio fr = tanh_ratio_parts(root(CHI), CHI * P.fr2k);
@@ -606,11 +638,10 @@ __device__ __forceinline__ void viscous_face(const Params& P, const FaceVals& f,
     } else {
         DIVVEL = DUX + DVY;
     }
-    const double y = inv_fifth_root(TAVG);
-    const double y2 = y * y;
-    const double AMU = P.suth_amol * (TAVG * y2);
+    const FifthRoots tr = fifth_roots(TAVG);
+    const double AMU = P.suth_amol * (TAVG * tr.m04);
     const double AK = AMU * P.cp_pr;
-    const double CHI = RHOAVG * RAVG * (P.inv_cmu_suth * (y2 * y));
+    const double CHI = RHOAVG * RAVG * (P.inv_cmu_suth * tr.m06);
     const double chi2 = CHI * CHI;
     const Ratio fm = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
     const double FMU = fm.num * recip(fm.den);

@@ -60,7 +60,8 @@ struct tns_handle {
     // second branch of an iteration: the dissipation pre-pass runs beside the viscous flux
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    DevBuf<double> x, y, cfldl, gxc, gyc, ginj, gport, qa, qb, qc, d, vis, dt, dtmin, partial,
+    // e: the iteration's frozen terms VIS + D, formed by stage 1 (FP64, structured meshes)
+    DevBuf<double> x, y, cfldl, gxc, gyc, ginj, gport, qa, qb, qc, d, vis, e, dt, dtmin, partial,
         primout, cvol, stile, fgi, fgj;
     // mixed FP32/FP64 path: FP64 state ping-pong (qa, qa2) and FP32 scratch
     int precision = 0;
@@ -72,6 +73,7 @@ struct tns_handle {
     // monitored iteration (CDIFF reduction in stage 4): FP64, mixed per parity
     cudaGraphExec_t graph_mon = nullptr;
     cudaGraphExec_t graph_mon_mx[2] = {nullptr, nullptr};
+    DevBuf<tns::GhostRec> grec;
     DevBuf<int> gtype, grank, ports;
     DevBuf<unsigned int> counter, status;
     DevBuf<unsigned long long> cdiff;

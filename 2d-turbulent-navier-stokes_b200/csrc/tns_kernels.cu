@@ -14,7 +14,6 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <cstring>
 
 #include "tns_device.cuh"
 #include "tns_kernels.h"
@@ -25,129 +24,250 @@ namespace tns {
 
 // ------------------------------------------------------------------ stage kernel
 
-// Shared-memory fields of the stage tile, paired for 16-byte loads; the tile's static
-// block (nodes, gradient coefficients, 1/VOL, 1/YCC) arrives by one bulk copy.  The TMA
-// variant also receives the five Q planes of the tile's halo box by one tiled tensor
-// copy: rows i0-1 .. i0+TI, columns j0-2 .. j0+TJ+1 (the box starts one column early so
-// that its first column is a multiple of 16 bytes; out-of-mesh positions arrive as
-// zeros), and evaluates its slots from there.
-// Off by default: measured on 1024 x 384 (B200, FP64), the TMA variant took 157-159 us
-// for a RK4 iteration's four stage launches against 145 us with plain loads (same
-// results bit for bit).  A block waits for its whole box before its first slot, where
-// plain loads let each warp start as its own rows arrive.
-#ifndef TNS_STAGE_TMA
-#define TNS_STAGE_TMA 0
-#endif
-// Three blocks of the TMA variant fit an SM at TI >= 8 (at TI = 4 its box would cost the
-// sixth block).
-#define TNS_STAGE_TMA_ON (TNS_STAGE_TMA && TNS_TI >= 8)
-constexpr int QH = TI + 2, QW = TJ + 4;
-static_assert(QW % 2 == 0, "the Q box rows must be a multiple of 16 bytes");
-
-// Slot order: each thread first evaluates the slot of its own cell and keeps that cell's
-// T, P and RHO in registers (the only slot values read for the cell alone), then the
-// first NRING threads evaluate the halo ring's slots (tns_tile.cuh).
+// Shared-memory fields of the stage tile: per slot the six values its neighbours' face
+// fluxes are formed from and |V|, paired for 16-byte loads; the tile's static block (nodes,
+// gradient coefficients, 1/VOL, 1/YCC) arrives by one bulk copy.  A cell's flux through a
+// face needs its mass flux m = RHO (U SX + V SY) alone: (m, m U + P SX, m V + P SY,
+// (C4 + P)(U SX + V SY), m C5/C1), ten operations a neighbour from seven stored values
+// instead of ten stored flux components (a tile's slots take 19 KB, not 38).  A ghost keeps
+// its own flux through its face (a wall's components are mirrored, an outflow's fifth is the
+// parent's), by the tile cell it borders.
+// What bounds it: instruction issue and memory latency (735 instructions a cell, a third of
+// them FP64).  On a small mesh every tile borders the boundary and one tile's latency is the
+// kernel's: the ghosts' static data is loaded before the previous kernel has ended and every
+// state a slot needs is asked for at once, which took a boundary tile from 10,200 to 7,200
+// cycles (115 x 50 nozzle, a FP64 iteration: 37.6 -> 27.4 us).
+// Slot order: each thread first evaluates the slot of its own cell, then the first threads
+// evaluate the ring of slots around the tile's cells (tns_tile.cuh).
 static_assert(NRING <= NTHREADS, "one ring slot per thread at most");
+constexpr int NGF = 2 * (TI + TJ);  // ghosts bordering a tile: sides 1, 3 by row, 4, 2 by column
 
-template <bool TMA>
-struct StageSmemT {
-    double qs[TMA ? 5 * QH * QW : 2];  // (TMA) Q planes [5][QH][QW], 128-byte aligned
-    double st[STILE];                  // static block (tns_tile.cuh)
-    double2 fg[5][NSLOT];              // (F_m, G_m)
-    double2 uv[NSLOT];                 // (U, V)
-    double2 rq[NSLOT];                 // (C5/C1, |V|)
-    unsigned long long bar;   // completion of the static block's copy
-    unsigned long long qbar;  // (TMA) completion of the Q box
+// The slots of one tile.
+struct StageSlots {
+    double2 uv[NSLOT];     // (U, V)
+    double2 rp[NSLOT];     // (RHO, P)
+    double2 hr[NSLOT];     // (C4 + P, C5/C1)
+    double qm[NSLOT];      // |V|
+    double gf[5][NGF];     // the ghosts' fluxes through the faces they border
 };
-using StageSmem = StageSmemT<false>;
-static_assert(sizeof(double) * 5 * QH * QW % 16 == 0, "the static block follows the Q box at 16 bytes");
+
+struct StageSmem {
+    double st[STILE];      // static block (tns_tile.cuh)
+    StageSlots w;
+    unsigned long long bar;  // completion of the static block's copy
+};
 
 size_t stage_smem_bytes() { return sizeof(StageSmem); }
-#if TNS_STAGE_TMA_ON
-// (+128: the kernel aligns the Q box to 128 bytes inside its dynamic shared memory)
-static size_t stage_tma_smem_bytes() { return sizeof(StageSmemT<true>) + 128; }
-#endif
 
-template <bool TMA>
-__device__ __forceinline__ void put_slot(StageSmemT<TMA>& S, int s, const Prim& p) {
-#pragma unroll
-    for (int m = 0; m < 5; m++) S.fg[m][s] = make_double2(p.f[m], p.g[m]);
+__device__ __forceinline__ void put_slot(StageSlots& S, int s, const Prim& p, double h) {
     S.uv[s] = make_double2(p.u, p.v);
-    S.rq[s] = make_double2(p.ri, p.qm);
+    S.rp[s] = make_double2(p.rho, p.p);
+    S.hr[s] = make_double2(h, p.ri);
+    S.qm[s] = p.qm;
+}
+
+// A cell's slot from its state; returns the cell's T (read for the cell alone).
+__device__ __forceinline__ double put_cell_slot(const Params& P, StageSlots& S, int s, const double q[5]) {
+    Prim p;
+    primitive(P, q[0], q[1], q[2], q[3], q[4], p);
+    put_slot(S, s, p, q[3] + p.p);
+    return kept(p.t);
+}
+
+// The slot of halo position h: a cell's from its state q, a ghost's (and, where it borders a
+// cell of the tile, its flux through their face) from its parent's state q; opp(double[5])
+// gives the state of the parent's opposite neighbour.
+template <class Opp>
+__device__ __forceinline__ void put_halo_slot(const Params& P, const Mesh& M, StageSlots& S, const HaloPos& h,
+                                              const GhostSite& site, const double q[5], Opp opp) {
+    Prim p;
+    primitive(P, q[0], q[1], q[2], q[3], q[4], p);
+    if (h.kind == 0) {
+        put_slot(S, h.li * SW + h.lj, p, q[3] + p.p);
+        return;
+    }
+    Prim gh;
+    ghost_prim(P, M, site, h.g, p,
+               [&](Prim& o) {
+                   double c[5];
+                   opp(c);
+                   primitive(P, c[0], c[1], c[2], c[3], c[4], o);
+               }, gh);
+    put_slot(S, h.li * SW + h.lj, gh, 0.0);
+    const bool row = h.kind == 1 || h.kind == 3;  // ghosts beside the tile's rows
+    const int at = (row ? h.li : h.lj) - 1;
+    if (at >= 0 && at < (row ? TI : TJ)) {
+        const int f = (h.kind == 1 ? 0 : h.kind == 3 ? TI : h.kind == 4 ? 2 * TI : 2 * TI + TJ) + at;
+#pragma unroll
+        for (int m = 0; m < 5; m++) S.gf[m][f] = gh.f[m] * site.psx + gh.g[m] * site.psy;
+    }
+}
+
+// The update operands of one cell: Q_old, the frozen terms VIS + D and DT.
+struct StageOps {
+    double qold[5], e[5], dt;
+};
+
+// Residual, source and update of the thread's cell (i, j) of a tile from the tile's slots,
+// its nodes, the cells' static coefficients and `ops(StageOps&)`, which is called last and
+// may wait for the update operands.
+template <class Ops>
+__device__ __forceinline__ void stage_cell(const Params& P, const Mesh& M, const StageArgs& A, const StageSlots& S,
+                                           const double* nodes, const double* coef, bool inner, int i, int j,
+                                           double own_t, Ops ops, double dv[5]) {
+    const size_t ncell = (size_t)M.ni * M.nj;
+    const int tj = threadIdx.x, ti = threadIdx.y, tid = ti * TJ + tj;
+    const size_t cell = (size_t)i * M.nj + j;
+    const int c = (ti + 1) * SW + (tj + 1);
+    const int nb[4] = {c - 1, c + SW, c + 1, c - SW};  // NC1..NC4
+    const double* X0 = nodes + ti * SNW + tj;  // node 1 of the cell
+    const double* Y0 = X0 + SNN;
+    const double X[4] = {X0[0], X0[SNW], X0[SNW + 1], X0[1]};
+    const double Y[4] = {Y0[0], Y0[SNW], Y0[SNW + 1], Y0[1]};
+
+    // inviscid residual (residual.f90:23-62): half the sum over the faces of the cell's own
+    // flux and the neighbour's; the own flux meets the sum of the face vectors
+    double R[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    {
+        double SX[4], SY[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) face_vector(P.iaxis, k + 1, X, Y, SX[k], SY[k]);
+        auto add = [&](int s, double sx, double sy) {
+            const double2 uv = S.uv[s], rp = S.rp[s], hr = S.hr[s];
+            const double vn = uv.x * sx + uv.y * sy;
+            const double m = rp.x * vn;
+            R[0] = R[0] + m;
+            R[1] = fma(m, uv.x, fma(rp.y, sx, R[1]));
+            R[2] = fma(m, uv.y, fma(rp.y, sy, R[2]));
+            R[3] = fma(hr.x, vn, R[3]);
+            R[4] = fma(m, hr.y, R[4]);
+        };
+        add(c, (SX[0] + SX[2]) + (SX[1] + SX[3]), (SY[0] + SY[2]) + (SY[1] + SY[3]));
+        const bool gh[4] = {j == 0, i == M.ni - 1, j == M.nj - 1, i == 0};
+        const int gs[4] = {ti, 2 * TI + TJ + tj, TI + ti, 2 * TI + tj};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (!inner && gh[k]) {
+#pragma unroll
+                for (int m = 0; m < 5; m++) R[m] = R[m] + S.gf[m][gs[k]];
+            } else {
+                add(nb[k], SX[k], SY[k]);
+            }
+        }
+    }
+
+    // source terms (source_terms.f90:24-104)
+    double src3, src5;
+    {
+        const double* G = coef + tid;
+        SrcIn s;
+        s.ga = G[ST_GA * NTHREADS]; s.gb = G[ST_GB * NTHREADS];
+        s.gc = G[ST_GC * NTHREADS]; s.gd = G[ST_GD * NTHREADS];
+        const double2 ua = S.uv[nb[0]], ub = S.uv[nb[1]], uc = S.uv[nb[2]], ud = S.uv[nb[3]];
+        s.ua = ua.x; s.ub = ub.x; s.uc = uc.x; s.ud = ud.x;
+        s.va = ua.y; s.vb = ub.y; s.vc = uc.y; s.vd = ud.y;
+        s.ra = S.hr[nb[0]].y; s.rb = S.hr[nb[1]].y; s.rc = S.hr[nb[2]].y; s.rd = S.hr[nb[3]].y;
+        s.qa = S.qm[nb[0]]; s.qb = S.qm[nb[1]]; s.qc = S.qm[nb[2]]; s.qd = S.qm[nb[3]];
+        const double YCCI = (Y[0] + Y[1] + Y[2] + Y[3]) * 0.25;
+        source_terms(P, s, S.rp[c].x, S.hr[c].y, own_t, S.rp[c].y, S.uv[c].y, YCCI, G[ST_RYCC * NTHREADS], src3, src5);
+    }
+
+    // update (residual.f90:67-83), the sources per volume
+    const double RVOL = coef[ST_RVOL * NTHREADS + tid];
+    StageOps o;
+    ops(o);
+    const double aDT = A.alpha * o.dt;
+    double Cn[5];
+    const double* Co = o.qold;
+    Cn[0] = Co[0] - aDT * (RVOL * (HALF * R[0] - o.e[0]));
+    Cn[1] = Co[1] - aDT * (RVOL * (HALF * R[1] - o.e[1]));
+    Cn[2] = Co[2] - aDT * fma(RVOL, HALF * R[2] - o.e[2], -src3);
+    Cn[3] = Co[3] - aDT * (RVOL * (HALF * R[3] - o.e[3]));
+    Cn[4] = Co[4] - aDT * CFLTURB * fma(RVOL, HALF * R[4] - o.e[4], -src5);
+    Cn[4] = Cn[0] * dmax1(P.rtol, Cn[4] * recip(Cn[0]));
+#pragma unroll
+    for (int m = 0; m < 5; m++) A.qout[m * ncell + cell] = Cn[m];
+    if (A.status) {
+        bool bad = false;
+#pragma unroll
+        for (int m = 0; m < 5; m++) bad |= !isfinite(Cn[m]);
+        if (bad) atomicOr(A.status, 1u);
+    }
+#pragma unroll
+    for (int m = 0; m < 5; m++) dv[m] = fabs(Co[m] - Cn[m]);
+}
+
+// The frozen terms VIS + D of a cell, by stage 1.
+__device__ __forceinline__ void frozen_terms(const StageArgs& A, size_t ncell, size_t cell, double e[5]) {
+    double d[5], v[4];
+#pragma unroll
+    for (int m = 0; m < 5; m++) d[m] = A.d[m * ncell + cell];
+#pragma unroll
+    for (int m = 0; m < 4; m++) v[m] = A.vis[m * ncell + cell];
+    e[0] = d[0];
+#pragma unroll
+    for (int m = 1; m < 5; m++) e[m] = v[m - 1] + d[m];
+    if (A.eout) {
+#pragma unroll
+        for (int m = 0; m < 5; m++) A.eout[m * ncell + cell] = e[m];
+    }
+}
+
+// max |COLD - C| per component: warp max, then one atomic per warp on the ordered bit
+// pattern (non-negative doubles order like their bits)
+__device__ __forceinline__ void stage_cdiff(const StageArgs& A, const double dv[5]) {
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        double v = dv[m];
+        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if ((threadIdx.x & 31) == 0) atomicMax(&A.cdiff[m], (unsigned long long)__double_as_longlong(v));
+    }
 }
 
 // One RK stage (turbnstwod.f90:204-227, boundary.f90:24-48, source_terms.f90:24-104,
 // residual.f90:23-83) on a TI x TJ tile with its halo staged in shared memory.
-// TMA: qmap is the tensor map of A.qin ([5][NI][NJ] doubles, box [5][QH][QW]).
-template <bool TMA>
-__device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const StageArgs& A, int bx, int by,
-                                           const CUtensorMap* qmap = nullptr) {
+__device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const StageArgs& A, int bx, int by) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned char* base = smem_raw;
-    if (TMA) base += (128u - ((unsigned)__cvta_generic_to_shared(smem_raw) & 127u)) & 127u;
-    StageSmemT<TMA>& S = *reinterpret_cast<StageSmemT<TMA>*>(base);
+    StageSmem& S = *reinterpret_cast<StageSmem*>(smem_raw);
     const size_t ncell = (size_t)M.ni * M.nj;
     const int j0 = bx * TJ, i0 = by * TI;
-    const int tid = threadIdx.y * TJ + threadIdx.x;
+    const int tj = threadIdx.x, ti = threadIdx.y;
+    const int tid = ti * TJ + tj;
     pdl_trigger();
     // the static block is written by nothing: its copy overlaps the previous kernel's tail
     if (tid == 0) {
         bulk_barrier_init(&S.bar);
-        if (TMA) bulk_barrier_init(&S.qbar);
         const size_t tile = (size_t)by * ((M.nj + TJ - 1) / TJ) + bx;
         bulk_copy_start(S.st, M.stile + tile * STILE, STILE * sizeof(double), &S.bar);
     }
-    pdl_wait();
-    if (TMA && tid == 0)
-        tensor_copy_3d_start(S.qs, qmap, j0 - 2, i0 - 1, 0, (unsigned)(sizeof(double) * 5 * QH * QW), &S.qbar);
-    __syncthreads();
-    if (TMA) {
-        // a block-uniform decision: every thread leaves, or none
-        const bool ok = bulk_wait(&S.qbar);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) atomicOr(A.error, 2u);
-            bulk_wait(&S.qbar);
-            bulk_wait(&S.bar);
-            return;
-        }
-    }
-    // primitives of a cell of the Q box, by mesh position
-    auto box_prim = [&](int ci, int cj, Prim& q) {
-        const double* b = S.qs + (ci - i0 + 1) * QW + (cj - j0 + 2);
-        primitive(P, b[0], b[QH * QW], b[2 * QH * QW], b[3 * QH * QW], b[4 * QH * QW], q);
-    };
-    // the slot at (li, lj): false where the position is neither a cell nor a ghost
-    auto slot_prim = [&](int li, int lj, Prim& p) -> bool {
-        int along = 0;
-        const int kind = classify(M, i0 - 1 + li, j0 - 1 + lj, along);
-        if (kind < 0) return false;
-        if (TMA) {
-            if (kind == 0) box_prim(i0 - 1 + li, j0 - 1 + lj, p);
-            else ghost_state_at(P, M, kind, along, box_prim, p);
-        } else if (kind == 0) {
-            cell_prim(P, A.qin, ncell, (size_t)(i0 - 1 + li) * M.nj + (j0 - 1 + lj), p);
-        } else {
-            ghost_state(P, M, A.qin, ncell, kind, along, p);
-        }
-        return true;
-    };
-    // own cell first (its T, P, RHO kept), then the ring
-    double own_t = 0.0, own_p = 0.0, own_rho = 0.0;
-    {
-        Prim p;
-        if (slot_prim(threadIdx.y + 1, threadIdx.x + 1, p)) {
-            put_slot(S, (threadIdx.y + 1) * SW + threadIdx.x + 1, p);
-            own_t = kept(p.t);
-            own_p = kept(p.p);
-            own_rho = kept(p.rho);
-        }
-    }
-    if (tid < NRING) {
+    // a tile whose halo holds no ghost (and which is full) needs no classification
+    const bool inner = i0 > 0 && j0 > 0 && i0 + TI < M.ni && j0 + TJ < M.nj;
+    const int i = i0 + ti, j = j0 + tj;
+    const bool valid = i < M.ni && j < M.nj;
+    // the ring around the tile's cells; a ghost's type and geometry are static too
+    const int ri = inner ? TI : min(TI, M.ni - i0), rj = inner ? TJ : min(TJ, M.nj - j0);
+    HaloPos h;
+    h.kind = -1;
+    GhostSite site{0, 0.0, 0.0, 0.0, 0.0};
+    if (tid < 2 * (ri + rj + 2)) {
         int li, lj;
-        ring_slot(tid, li, lj);
-        Prim p;
-        if (slot_prim(li, lj, p)) put_slot(S, li * SW + lj, p);
+        ring_slot(tid, ri, rj, li, lj);
+        h = halo_pos(M, inner, i0, j0, li, lj);
+        if (h.kind > 0) site = ghost_site(M, h.g);
     }
+    pdl_wait();
+    __syncthreads();
+    auto load = [&](int ci, int cj, double q[5]) {
+        const double* p = A.qin + ((size_t)ci * M.nj + cj);
+#pragma unroll
+        for (int m = 0; m < 5; m++) q[m] = p[m * ncell];
+    };
+    // own cell (its T kept) and ring slot, both states on their way first
+    double qo[5], qr[5], own_t = 0.0;
+    if (valid) load(i, j, qo);
+    if (h.kind >= 0) load(h.ci, h.cj, qr);
+    if (valid) own_t = put_cell_slot(P, S.w, (ti + 1) * SW + tj + 1, qo);
+    if (h.kind >= 0) put_halo_slot(P, M, S.w, h, site, qr, [&](double c[5]) { load(h.ci + h.oi, h.cj + h.oj, c); });
     __syncthreads();
     if (!bulk_wait(&S.bar)) {
         // the copy did not complete: report it, give it one more bounded wait (it writes
@@ -156,109 +276,186 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
         bulk_wait(&S.bar);
         return;
     }
-
-    const int tj = threadIdx.x, ti = threadIdx.y;
-    const int i = i0 + ti, j = j0 + tj;
-    const bool valid = i < M.ni && j < M.nj;
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid) {
         const size_t cell = (size_t)i * M.nj + j;
-        const int c = (ti + 1) * SW + (tj + 1);
-        const int nb[4] = {c - 1, c + SW, c + 1, c - SW};  // NC1..NC4
-        const int n1 = ti * SNW + tj;  // node 1 of the cell in the static block
-        const int gc = 2 * SNN + ti * TJ + tj;
-        const double* X0 = S.st;
-        const double* Y0 = S.st + SNN;
-
-        // source terms first (source_terms.f90:24-104): only src3 / src5 stay live into
-        // the residual
-        double src3, src5;
-        {
-            SrcIn s;
-            s.ga = S.st[gc + ST_GA * NTHREADS]; s.gb = S.st[gc + ST_GB * NTHREADS];
-            s.gc = S.st[gc + ST_GC * NTHREADS]; s.gd = S.st[gc + ST_GD * NTHREADS];
-            const double2 ua = S.uv[nb[0]], ub = S.uv[nb[1]], uc = S.uv[nb[2]], ud = S.uv[nb[3]];
-            const double2 ra = S.rq[nb[0]], rb = S.rq[nb[1]], rc = S.rq[nb[2]], rd = S.rq[nb[3]];
-            s.ua = ua.x; s.ub = ub.x; s.uc = uc.x; s.ud = ud.x;
-            s.va = ua.y; s.vb = ub.y; s.vc = uc.y; s.vd = ud.y;
-            s.ra = ra.x; s.rb = rb.x; s.rc = rc.x; s.rd = rd.x;
-            s.qa = ra.y; s.qb = rb.y; s.qc = rc.y; s.qd = rd.y;
-            const double2 tp = make_double2(own_t, own_p);
-            const double RHOC = own_rho;
-            const double YCCI = (Y0[n1] + Y0[n1 + SNW] + Y0[n1 + SNW + 1] + Y0[n1 + 1]) * 0.25;
-            source_terms(P, s, RHOC, S.rq[c].x, tp.x, tp.y, S.uv[c].y, YCCI,
-                         S.st[gc + ST_RYCC * NTHREADS], src3, src5);
-        }
-
-        // inviscid residual (residual.f90:23-62) with the sources (residual.f90:54,58)
-        const double X[4] = {X0[n1], X0[n1 + SNW], X0[n1 + SNW + 1], X0[n1 + 1]};
-        const double Y[4] = {Y0[n1], Y0[n1 + SNW], Y0[n1 + SNW + 1], Y0[n1 + 1]};
-        double SX[4], SY[4];
+        stage_cell(P, M, A, S.w, S.st, S.st + 2 * SNN, inner, i, j, own_t,
+                   [&](StageOps& o) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) face_vector(P.iaxis, k + 1, X, Y, SX[k], SY[k]);
-        double R[5];
+                       for (int m = 0; m < 5; m++) o.qold[m] = A.qold[m * ncell + cell];
+                       o.dt = P.local ? A.dt[cell] : *A.dtmin;
+                       if (A.e) {
 #pragma unroll
-        for (int m = 0; m < 5; m++) {
-            const double2 I = S.fg[m][c], a = S.fg[m][nb[0]], b = S.fg[m][nb[1]],
-                          e = S.fg[m][nb[2]], d = S.fg[m][nb[3]];
-            R[m] = HALF * ((I.x + a.x) * SX[0] + (I.y + a.y) * SY[0] + (I.x + b.x) * SX[1] +
-                           (I.y + b.y) * SY[1] + (I.x + e.x) * SX[2] + (I.y + e.y) * SY[2] +
-                           (I.x + d.x) * SX[3] + (I.y + d.y) * SY[3]);
-        }
-        const double VOL = M.cvol[cell];
-        R[4] = R[4] - VOL * src5;
-        if (P.iaxis == 1) R[2] = R[2] - VOL * src3;
-
-        // update (residual.f90:67-83)
-        const double DT = P.local ? A.dt[cell] : *A.dtmin;
-        const double DTBYVOL = DT * S.st[gc + ST_RVOL * NTHREADS];
-        const double al = A.alpha;
-        double Cn[5], Co[5], vis[4], dd[5];
-#pragma unroll
-        for (int m = 0; m < 5; m++) {
-            Co[m] = A.qold[m * ncell + cell];
-            dd[m] = A.d[m * ncell + cell];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; k++) vis[k] = A.vis[k * ncell + cell];
-        Cn[0] = Co[0] - al * DTBYVOL * (R[0] - dd[0]);
-        Cn[1] = Co[1] - al * DTBYVOL * (R[1] - vis[0] - dd[1]);
-        Cn[2] = Co[2] - al * DTBYVOL * (R[2] - vis[1] - dd[2]);
-        Cn[3] = Co[3] - al * DTBYVOL * (R[3] - vis[2] - dd[3]);
-        Cn[4] = Co[4] - al * DTBYVOL * CFLTURB * (R[4] - vis[3] - dd[4]);
-        Cn[4] = Cn[0] * dmax1(P.rtol, Cn[4] / Cn[0]);
-#pragma unroll
-        for (int m = 0; m < 5; m++) A.qout[m * ncell + cell] = Cn[m];
-        if (A.status) {
-            bool bad = false;
-#pragma unroll
-            for (int m = 0; m < 5; m++) bad |= !isfinite(Cn[m]);
-            if (bad) atomicOr(A.status, 1u);
-        }
-#pragma unroll
-        for (int m = 0; m < 5; m++) dv[m] = fabs(Co[m] - Cn[m]);
+                           for (int m = 0; m < 5; m++) o.e[m] = A.e[m * ncell + cell];
+                       } else {
+                           frozen_terms(A, ncell, cell, o.e);
+                       }
+                   }, dv);
     }
-    if (A.cdiff) {
-        // max |COLD - C| per component: warp max, then one atomic per warp on the ordered
-        // bit pattern (non-negative doubles order like their bits)
-#pragma unroll
-        for (int m = 0; m < 5; m++) {
-            double v = dv[m];
-            for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-            if ((threadIdx.x & 31) == 0)
-                atomicMax(&A.cdiff[m], (unsigned long long)__double_as_longlong(v));
-        }
-    }
+    if (A.cdiff) stage_cdiff(A, dv);
 }
 
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
 // runs.
-template <int MONITOR, bool TMA>
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MINB))
-k_stage(Params P, Mesh M, StageArgs A, const __grid_constant__ CUtensorMap qmap) {
+template <int MONITOR>
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MINB)) k_stage(Params P, Mesh M, StageArgs A) {
     StageArgs Ac = A;
     if (!MONITOR) Ac.cdiff = nullptr;
-    stage_tile<TMA>(P, M, Ac, blockIdx.x, blockIdx.y, &qmap);
+    stage_tile(P, M, Ac, blockIdx.x, blockIdx.y);
+}
+
+// Stages 2-4 of a large mesh, by resident blocks that walk its tiles (tile t, t + grid, ...)
+// with the data of the next tile on its way through the TMA engine while they compute:
+//   a: the stage input's halo box (rows i0-1 .. i0+TI, columns j0-2 .. j0+TJ+1: one column
+//      early so that the box starts at a multiple of 16 bytes; positions outside the mesh
+//      arrive as zeros), asked for as soon as the tile before has formed its slots;
+//   b: the tile's static block, and
+//   c: Q_old, the frozen terms and DT of its cells, asked for when the tile before is done
+//      and needed when this one's slots are formed, and at its very end.
+// The copies take the global-load latency (4.7 of 11.6 stall cycles an instruction in the
+// kernel above, half of its time) out of the warps; a tile's buffers fit three times into an
+// SM because VIS + D is one array, so 24 warps stay resident at 80 registers (with D and VIS
+// apart and two blocks a SM it was no faster than the plain kernel).  What bounds it now:
+// issue (0.5 an SM quarter a cycle under 24 warps) and the launch.  1024 x 384 nozzle-plume,
+// a FP64 iteration: 0.153 ms with the plain kernel in all stages, 0.138 ms with this one;
+// 2048 x 768 port 0.647 -> 0.565 ms.  It needs more tiles than the plain kernel has resident
+// blocks (at 384 tiles the two take the same 42 us an iteration) and rows and arrays that
+// TMA can address.
+constexpr int QH = TI + 2, QW = TJ + 4;  // halo box
+static_assert(QW % 2 == 0 && STILE % 2 == 0, "box rows and static blocks are multiples of 16 bytes");
+
+// Planes of the update operands
+enum StageOp { SO_QOLD, SO_E = 5, SO_DT = 10, SO_N };
+
+struct StagePipeSmem {
+    // (128-byte aligned destinations first)
+    double q[(5 * QH * QW + 15) / 16 * 16];
+    double op[SO_N][NTHREADS];
+    double st[STILE];
+    StageSlots w;
+    unsigned long long bar_a, bar_b, bar_c;
+};
+
+struct StageMaps {
+    CUtensorMap q, qold, e, dt;
+};
+
+template <int MONITOR>
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MINB))
+k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ StageMaps maps) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    StagePipeSmem& W =
+        *reinterpret_cast<StagePipeSmem*>(smem_raw + ((128u - ((unsigned)__cvta_generic_to_shared(smem_raw) & 127u)) & 127u));
+    StageSlots& S = W.w;
+    const int ntj = (M.nj + TJ - 1) / TJ;
+    const int tj = threadIdx.x, ti = threadIdx.y, tid = ti * TJ + tj;
+    // tile t: row t / ntj, its column shifted by the row so that a block whose stride is a
+    // multiple of ntj does not meet the same (boundary) column every time
+    auto row_of = [&](int t) { return t / ntj; };
+    auto col_of = [&](int t) { return (t % ntj + t / ntj) % ntj; };
+    auto fetch_a = [&](int t) {
+        barrier_expect(&W.bar_a, sizeof(double) * 5 * QH * QW);
+        tensor_copy_3d(W.q, &maps.q, col_of(t) * TJ - 2, row_of(t) * TI - 1, 0, &W.bar_a);
+    };
+    auto fetch_b = [&](int t) {
+        bulk_copy_start(W.st, M.stile + ((size_t)row_of(t) * ntj + col_of(t)) * STILE, sizeof(double) * STILE, &W.bar_b);
+    };
+    auto fetch_c = [&](int t) {
+        const int j0 = col_of(t) * TJ, i0 = row_of(t) * TI;
+        barrier_expect(&W.bar_c, sizeof(double) * (P.local ? SO_N : SO_DT) * NTHREADS);
+        tensor_copy_3d(W.op[SO_E], &maps.e, j0, i0, 0, &W.bar_c);
+        tensor_copy_3d(W.op[SO_QOLD], &maps.qold, j0, i0, 0, &W.bar_c);
+        if (P.local) tensor_copy_3d(W.op[SO_DT], &maps.dt, j0, i0, 0, &W.bar_c);
+    };
+    pdl_trigger();
+    if (tid == 0) {
+        bulk_barrier_init(&W.bar_a);
+        bulk_barrier_init(&W.bar_b);
+        bulk_barrier_init(&W.bar_c);
+        fetch_b(blockIdx.x);  // static: before the previous kernel is done
+    }
+    pdl_wait();
+    if (tid == 0) {
+        fetch_a(blockIdx.x);
+        fetch_c(blockIdx.x);
+    }
+    __syncthreads();  // the barriers are set up
+    unsigned parity = 0;
+    bool ok = true;
+    double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, parity ^= 1) {
+        const int i0 = row_of(t) * TI, j0 = col_of(t) * TJ;
+        const int i = i0 + ti, j = j0 + tj;
+        const bool valid = i < M.ni && j < M.nj;
+        const bool inner = i0 > 0 && j0 > 0 && i0 + TI < M.ni && j0 + TJ < M.nj;
+        auto box = [&](int ci, int cj, double q[5]) {
+            const double* b = W.q + (ci - i0 + 1) * QW + (cj - j0 + 2);
+#pragma unroll
+            for (int m = 0; m < 5; m++) q[m] = b[m * QH * QW];
+        };
+        ok = bulk_wait(&W.bar_a, parity) && ok;
+        double own_t = 0.0;
+        if (valid) {
+            double q[5];
+            box(i, j, q);
+            own_t = put_cell_slot(P, S, (ti + 1) * SW + tj + 1, q);
+        }
+        const int ri = inner ? TI : min(TI, M.ni - i0), rj = inner ? TJ : min(TJ, M.nj - j0);
+        if (tid < 2 * (ri + rj + 2)) {
+            int li, lj;
+            ring_slot(tid, ri, rj, li, lj);
+            const HaloPos h = halo_pos(M, inner, i0, j0, li, lj);
+            if (h.kind >= 0) {
+                double q[5];
+                box(h.ci, h.cj, q);
+                GhostSite site{0, 0.0, 0.0, 0.0, 0.0};
+                if (h.kind > 0) site = ghost_site(M, h.g);
+                put_halo_slot(P, M, S, h, site, q, [&](double c[5]) { box(h.ci + h.oi, h.cj + h.oj, c); });
+            }
+        }
+        ok = bulk_wait(&W.bar_b, parity) && ok;
+        if (!__syncthreads_and(ok)) {
+            // a copy did not complete: report it, give the copies in flight one more bounded
+            // wait (they write this block's shared memory) and leave
+            if (tid == 0) {
+                atomicOr(A.error, 2u);
+                bulk_wait(&W.bar_a, parity);
+                bulk_wait(&W.bar_b, parity);
+                bulk_wait(&W.bar_c, parity);
+            }
+            return;
+        }
+        const int next = t + gridDim.x;
+        if (tid == 0 && next < ntiles) fetch_a(next);
+        if (valid) {
+            double d[5];
+            stage_cell(P, M, A, S, W.st, W.st + 2 * SNN, inner, i, j, own_t,
+                       [&](StageOps& o) {
+                           ok = bulk_wait(&W.bar_c, parity) && ok;
+#pragma unroll
+                           for (int m = 0; m < 5; m++) {
+                               o.qold[m] = W.op[SO_QOLD + m][tid];
+                               o.e[m] = W.op[SO_E + m][tid];
+                           }
+                           o.dt = P.local ? W.op[SO_DT][tid] : *A.dtmin;
+                       }, d);
+            if (MONITOR) {
+#pragma unroll
+                for (int m = 0; m < 5; m++) dv[m] = fmax(dv[m], d[m]);
+            }
+        }
+        ok = bulk_wait(&W.bar_c, parity) && ok;  // (threads without a cell, too)
+        __syncthreads();
+        if (tid == 0 && next < ntiles) {
+            fetch_b(next);
+            fetch_c(next);
+        }
+    }
+    if (!ok) {  // the last tile's operands
+        atomicOr(A.error, 2u);
+        bulk_wait(&W.bar_c, parity ^ 1);
+    }
+    if (MONITOR && A.cdiff) stage_cdiff(A, dv);
 }
 
 // ---------------------------------------------------------------- viscous kernel
@@ -893,9 +1090,9 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_BATCH_MINB)) k_
         copy_words(&sA, &c.stage[monitor][stage], sizeof(StageArgs), tid);
         __syncthreads();
     }
-    stage_tile<false>(sP, sM, sA, t.y, t.z);
+    stage_tile(sP, sM, sA, t.y, t.z);
 #else
-    stage_tile<false>(c.P, c.M, c.stage[monitor][stage], t.y, t.z);
+    stage_tile(c.P, c.M, c.stage[monitor][stage], t.y, t.z);
 #endif
 }
 
@@ -923,7 +1120,7 @@ k_batch_persistent(const BatchCase* __restrict__ cases, const int4* __restrict__
                     const BatchCase& c = cases[t.x];
                     if (ph == 0 && w < ntiles) dissipation_tile<double>(c.P, c.M, c.diss, t.y, t.z);
                     else if (ph == 0) viscous_tile(c.P, c.M, c.q, c.vis, t.y, t.z);
-                    else stage_tile<false>(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
+                    else stage_tile(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
                 }
                 __syncthreads();
             }
@@ -955,7 +1152,21 @@ void launch_debug_math(int fn, long long n, const double* a, const double* b, do
 
 static dim3 tile_grid(const Mesh& M) { return dim3((M.nj + TJ - 1) / TJ, (M.ni + TI - 1) / TI); }
 
-#if TNS_STAGE_TMA_ON
+// SMs of the current device, and the pipelined stage's resident blocks on all of them.
+static int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 148;
+    return n;
+}
+constexpr size_t PIPE_SMEM = sizeof(StagePipeSmem) + 128;  // (the kernel aligns its boxes to 128 bytes)
+static int pipe_grid() {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pipe<0>, NTHREADS, PIPE_SMEM) != cudaSuccess)
+        return 0;
+    return per_sm * sm_count();
+}
+
 // The driver's tensor-map encoder, looked up once through the runtime.
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
@@ -969,39 +1180,39 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// Tensor map of a state array [5][NI][NJ] for the stage's Q box; false (the caller takes
-// the plain-load kernel) where TMA cannot address it: NJ odd (rows not a multiple of 16
-// bytes) or the array not 16-byte aligned.
-static bool stage_q_map(const Mesh& M, const double* q, CUtensorMap* map) {
-    if (M.nj % 2 != 0 || (reinterpret_cast<uintptr_t>(q) & 15) != 0) return false;
+// Tensor map of an array [planes][NI][NJ] with boxes [planes][rows][cols]; false where TMA
+// cannot address it: NJ odd (rows not a multiple of 16 bytes) or the array not 16-byte
+// aligned.
+static bool plane_map(const Mesh& M, const double* a, int planes, int rows, int cols, CUtensorMap* map) {
     const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (!enc) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)M.nj, (cuuint64_t)M.ni, 5};
+    if (!enc || M.nj % 2 != 0 || (reinterpret_cast<uintptr_t>(a) & 15) != 0) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)M.nj, (cuuint64_t)M.ni, (cuuint64_t)planes};
     const cuuint64_t strides[2] = {(cuuint64_t)M.nj * sizeof(double), (cuuint64_t)M.ni * M.nj * sizeof(double)};
-    const cuuint32_t box[3] = {(cuuint32_t)QW, (cuuint32_t)QH, 5};
+    const cuuint32_t box[3] = {(cuuint32_t)cols, (cuuint32_t)rows, (cuuint32_t)planes};
     const cuuint32_t elem[3] = {1, 1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(q), dims, strides, box, elem,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(a), dims, strides, box, elem,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-#endif
+static bool stage_maps(const Params& P, const Mesh& M, const StageArgs& A, StageMaps* m) {
+    return plane_map(M, A.qin, 5, QH, QW, &m->q) && plane_map(M, A.qold, 5, TI, TJ, &m->qold) &&
+           plane_map(M, A.e, 5, TI, TJ, &m->e) && plane_map(M, P.local ? A.dt : A.e, 1, TI, TJ, &m->dt);
+}
 
 cudaError_t configure_kernels() {
     cudaError_t e;
-    e = cudaFuncSetAttribute(k_stage<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_stage<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)stage_smem_bytes());
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_stage<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_stage<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)stage_smem_bytes());
     if (e != cudaSuccess) return e;
-#if TNS_STAGE_TMA_ON
-    e = cudaFuncSetAttribute(k_stage<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)stage_tma_smem_bytes());
+    e = cudaFuncSetAttribute(k_stage_pipe<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)PIPE_SMEM);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_stage<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)stage_tma_smem_bytes());
+    e = cudaFuncSetAttribute(k_stage_pipe<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)PIPE_SMEM);
     if (e != cudaSuccess) return e;
-#endif
     e = cudaFuncSetAttribute(k_viscous, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)visc_smem_bytes());
     if (e != cudaSuccess) return e;
@@ -1079,20 +1290,20 @@ void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis
 
 void launch_stage(const Params& P, const Mesh& M, const double* qin, const double* qold,
                   double* qout, const double* d, const double* vis, const double* dt,
-                  const double* dtmin, double alpha, unsigned long long* cdiff,
+                  const double* dtmin, int stage, double* e, unsigned long long* cdiff,
                   unsigned int* status, unsigned int* error, cudaStream_t s) {
-    StageArgs A{qin, qold, qout, d, vis, dt, dtmin, alpha, cdiff, status, error};
-    CUtensorMap qmap;
-#if TNS_STAGE_TMA_ON
-    if (stage_q_map(M, qin, &qmap)) {
-        launch_tile(cdiff ? k_stage<1, true> : k_stage<0, true>, tile_grid(M), dim3(TJ, TI),
-                    stage_tma_smem_bytes(), s, P, M, A, qmap);
+    const StageArgs A{qin, qold, qout, d, vis, dt, dtmin, RK_ALPHA[stage], stage ? e : nullptr, stage ? nullptr : e,
+                      cdiff, status, error};
+    const dim3 grid = tile_grid(M);
+    const int ntiles = grid.x * grid.y;
+    StageMaps maps;
+    const int pipe = A.e && ntiles > TNS_PER_SM(TNS_STAGE_MINB) * sm_count() ? pipe_grid() : 0;
+    if (pipe > 0 && pipe <= ntiles && stage_maps(P, M, A, &maps)) {
+        launch_tile(cdiff ? k_stage_pipe<1> : k_stage_pipe<0>, dim3(pipe), dim3(TJ, TI), PIPE_SMEM, s, P, M, A, ntiles,
+                    maps);
         return;
     }
-#endif
-    memset(&qmap, 0, sizeof(qmap));
-    launch_tile(cdiff ? k_stage<1, false> : k_stage<0, false>, tile_grid(M), dim3(TJ, TI), stage_smem_bytes(), s,
-                P, M, A, qmap);
+    launch_tile(cdiff ? k_stage<1> : k_stage<0>, grid, dim3(TJ, TI), stage_smem_bytes(), s, P, M, A);
 }
 
 int dtmin_blocks(const Mesh& M) {

@@ -36,6 +36,10 @@ inline Params make_params(const tns_params& p) {
     P.inv_cv = 1.0 / P.cv;
     P.cp_pr = P.cp / p.prandtl;
     P.cp_prt = P.cp / p.prandtlt;
+    P.inv_cp = 1.0 / P.cp;
+    P.inv_t0 = 1.0 / p.t0;
+    P.rho0 = rho0;
+    P.inv_gm1 = 1.0 / (p.gama - 1.0);
     P.inv_cmu_suth = 1.0 / (CMU * P.suth_amol);
     return P;
 }

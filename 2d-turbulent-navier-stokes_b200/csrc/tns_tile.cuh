@@ -55,6 +55,15 @@ __device__ __forceinline__ void ring_slot(int r, int& li, int& lj) {
     else if (r < 2 * SW + TI) { li = 1 + r - 2 * SW; lj = 0; }
     else { li = 1 + r - 2 * SW - TI; lj = SW - 1; }
 }
+// The same around the first ri x rj cells of a tile that the mesh's edge cuts short,
+// 2 (ri + rj + 2) positions.
+__device__ __forceinline__ void ring_slot(int r, int ri, int rj, int& li, int& lj) {
+    const int w = rj + 2;
+    if (r < w) { li = 0; lj = r; }
+    else if (r < 2 * w) { li = ri + 1; lj = r - w; }
+    else if (r < 2 * w + ri) { li = 1 + r - 2 * w; lj = 0; }
+    else { li = 1 + r - 2 * w - ri; lj = w - 1; }
+}
 constexpr int AW = TJ + 1;  // node-average grid (TI+1) x (TJ+1)
 constexpr int NAVG = (TI + 1) * AW;
 
@@ -97,41 +106,45 @@ __device__ __forceinline__ void bulk_barrier_init(unsigned long long* bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void bulk_copy_start(void* dst, const void* src, unsigned bytes,
-                                                unsigned long long* bar) {
+// barrier_expect: the phase completes when `bytes` of copies have arrived.
+__device__ __forceinline__ void barrier_expect(unsigned long long* bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;"
+                 ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
     const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;"
-                 ::"r"(b), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(d), "l"(src), "r"(bytes), "r"(b) : "memory");
 }
-// One-shot tiled tensor copy global -> shared (cp.async.bulk.tensor, 3-D, no multicast):
-// the box of `map` at element coordinates (x, y, z), x the innermost; x * element size a
-// multiple of 16 bytes; the shared destination 128-byte aligned; `bytes` the whole box
-// (out-of-range elements arrive as zeros and count).  `map` is the address of a
-// __grid_constant__ kernel parameter.  One thread, after bulk_barrier_init.
-__device__ __forceinline__ void tensor_copy_3d_start(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                                     unsigned bytes, unsigned long long* bar) {
+__device__ __forceinline__ void bulk_copy_start(void* dst, const void* src, unsigned bytes,
+                                                unsigned long long* bar) {
+    barrier_expect(bar, bytes);
+    bulk_copy(dst, src, bytes, bar);
+}
+// Tiled tensor copy global -> shared (cp.async.bulk.tensor, 3-D, no multicast): the box of
+// `map` at element coordinates (x, y, z), x the innermost; x * element size a multiple of 16
+// bytes; the shared destination 128-byte aligned; out-of-range elements arrive as zeros and
+// count.  `map` is the address of a __grid_constant__ kernel parameter.
+__device__ __forceinline__ void tensor_copy_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
+                                               unsigned long long* bar) {
     const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;"
-                 ::"r"(b), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
                  " [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(d), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(b)
                  : "memory");
 }
-// Waits for phase 0 of the barrier with a bounded number of polls; false if the copy did
-// not complete in that many (the caller reports it and skips the tile).
-__device__ __forceinline__ bool bulk_wait(unsigned long long* bar, int max_polls = 1 << 20) {
+// Waits for the barrier's phase of the given parity with a bounded number of polls; false if
+// the copy did not complete in that many (the caller reports it and skips the tile).
+__device__ __forceinline__ bool bulk_wait(unsigned long long* bar, unsigned parity = 0, int max_polls = 1 << 20) {
     const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
     for (int k = 0; k < max_polls; k++) {
         unsigned done;
         asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(b) : "memory");
+                     : "=r"(done) : "r"(b), "r"(parity) : "memory");
         if (done) return true;
     }
     return false;
@@ -228,39 +241,64 @@ __device__ __forceinline__ int classify(const Mesh& M, int i, int j, int& along)
     return -1;
 }
 
-// BC state of the ghost on `side` at `along`, from the parent and the parent's opposite
-// neighbour, whose primitives cell(i, j, Prim&) evaluates (bit-identical to their
-// PRIMITIVE_VARS).
-template <class CellPrim>
-__device__ void ghost_state_at(const Params& P, const Mesh& M, int side, int along, CellPrim cell,
-                               Prim& gh) {
-    int ip, jp, io, jo;
-    if (side == 1) { ip = along; jp = 0; io = along; jo = 1; }
-    else if (side == 2) { ip = M.ni - 1; jp = along; io = M.ni - 2; jo = along; }
-    else if (side == 3) { ip = along; jp = M.nj - 1; io = along; jo = M.nj - 2; }
-    else { ip = 0; jp = along; io = 1; jo = along; }
-    const int g = M.ghost_index(side, along);
-    const int type = M.gtype[g];
-    Prim par, opp;
-    cell(ip, jp, par);
-    if (type == 3) cell(io, jo, opp);
-    else opp = par;
-    const size_t n1 = (size_t)ip * (M.nj + 1) + jp;
-    const double X[4] = {M.x[n1], M.x[n1 + M.nj + 1], M.x[n1 + M.nj + 2], M.x[n1 + 1]};
-    const double Y[4] = {M.y[n1], M.y[n1 + M.nj + 1], M.y[n1 + M.nj + 2], M.y[n1 + 1]};
-    double psx = 0.0, psy = 0.0;
-    if (type == 6) face_vector(P.iaxis, side, X, Y, psx, psy);
-    const double ycc_p = (Y[0] + Y[1] + Y[2] + Y[3]) * 0.25;
-    boundary_ghost(P, type, par, opp, psx, psy, M.gyc[g], ycc_p, type == 6 ? M.gport[g] : 0.0,
-                   M.ginj[g], gh);
+// What a ghost's state depends on besides its parent: its BC type and static geometry
+// (written by nothing while kernels run), loaded ahead of the states.
+struct GhostSite {
+    int type;
+    double psx, psy, ycg, ycp;
+};
+__device__ __forceinline__ GhostSite ghost_site(const Mesh& M, int g) {
+    const GhostRec r = M.grec[g];
+    return GhostSite{M.gtype[g], r.psx, r.psy, r.ycg, r.ycp};
 }
 
-// The same, with both cells read straight from the state array.
+// A halo position (li, lj) of a tile: what is there (classify), for a ghost its index, and
+// the cell its state comes from: the cell itself or the ghost's parent, whose neighbour
+// opposite the ghost is at (ci + oi, cj + oj).
+struct HaloPos {
+    int li, lj, kind, g, ci, cj, oi, oj;
+};
+__device__ __forceinline__ HaloPos halo_pos(const Mesh& M, bool inner, int i0, int j0, int li, int lj) {
+    HaloPos h{li, lj, 0, 0, i0 - 1 + li, j0 - 1 + lj, 0, 0};
+    if (inner) return h;
+    int along = 0;
+    h.kind = classify(M, h.ci, h.cj, along);
+    if (h.kind > 0) {
+        h.g = M.ghost_index(h.kind, along);
+        h.oi = h.kind == 2 ? -1 : h.kind == 4 ? 1 : 0;
+        h.oj = h.kind == 3 ? -1 : h.kind == 1 ? 1 : 0;
+        h.ci += h.oi;  // the parent lies where the opposite neighbour is seen from the ghost
+        h.cj += h.oj;
+    }
+    return h;
+}
+
+// BC state of a ghost from its parent's primitives; opp(Prim&) gives those of the parent's
+// opposite neighbour (type 3 alone reads them).
+template <class Opp>
+__device__ __forceinline__ void ghost_prim(const Params& P, const Mesh& M, const GhostSite& s, int g, const Prim& par,
+                                           Opp opp, Prim& gh) {
+    Prim o = par;
+    if (s.type == 3) opp(o);
+    double gport = 0.0, inj = 1.0;
+    if (s.type == 6) {
+        gport = M.gport[g];
+        inj = M.ginj[g];
+    }
+    boundary_ghost(P, s.type, par, o, s.psx, s.psy, s.ycg, s.ycp, gport, inj, gh);
+}
+
+// The same, with both cells read from the state `st`.
 template <class St>
 __device__ __forceinline__ void ghost_state(const Params& P, const Mesh& M, const St& st, int side, int along,
                                             Prim& gh) {
-    ghost_state_at(P, M, side, along,
-                   [&](int i, int j, Prim& p) { cell_prim(P, st, (size_t)i * M.nj + j, p); }, gh);
+    const int g = M.ghost_index(side, along);
+    const GhostSite s = ghost_site(M, g);
+    const int ip = side == 2 ? M.ni - 1 : side == 4 ? 0 : along, jp = side == 1 ? 0 : side == 3 ? M.nj - 1 : along;
+    const int oi = side == 2 ? -1 : side == 4 ? 1 : 0, oj = side == 3 ? -1 : side == 1 ? 1 : 0;
+    Prim par;
+    cell_prim(P, st, (size_t)ip * M.nj + jp, par);
+    ghost_prim(P, M, s, g, par, [&](Prim& o) { cell_prim(P, st, (size_t)(ip + oi) * M.nj + jp + oj, o); }, gh);
 }
 
 __device__ __forceinline__ void ghost_state(const Params& P, const Mesh& M, const double* __restrict__ q,
