@@ -244,7 +244,7 @@ long long enqueue_forward_primal(tns_handle* h, tns_adjoint_state* s, int set, c
     };
     tns::launch_dissipation(P, M, f.q0.p, f.d, f.dt, f.dtmin, st);
     gport(0);
-    tns::launch_viscous(P, Ms[0], f.q0.p, f.vis, st);
+    tns::launch_viscous(P, Ms[0], f.q0.p, f.vis, h->status.p, st);
     for (int k = 0; k < 3; k++) {
         if (k) gport(k);
         tns::launch_stage(P, Ms[k], qs[k], f.q0.p, qs[k + 1], f.d, f.vis, f.dt, f.dtmin, k, h->e.p, nullptr,

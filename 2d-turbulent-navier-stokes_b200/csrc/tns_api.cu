@@ -204,8 +204,8 @@ int build_mesh(tns_handle* h, const tns_mesh* m) {
 
 // Static geometry of the tile kernels, from the device-order node and ghost-centroid
 // arrays with the reference's formulas (geometry.f90:55-149; the gradients of
-// source_terms.f90:24-60 and viscous.f90:130-180): VOL per cell, the stage tiles' static
-// blocks (tns_tile.cuh) and the viscous face rows (tns_device.cuh FaceGeo).
+// source_terms.f90:24-60 and viscous.f90:130-180): VOL per cell, the tiles' static blocks of
+// the stage and viscous kernels (tns_tile.cuh) and the boundary nodes' codes.
 void build_geometry(tns_handle* h) {
     using namespace tns;
     const int ni = h->ni, nj = h->nj, iaxis = h->P.iaxis;
@@ -272,43 +272,67 @@ void build_geometry(tns_handle* h) {
                     node(a, b, blk[la * SNW + lb], blk[SNN + la * SNW + lb]);
                 }
     // one face: A = the evaluating cell, C = the neighbour, B, D = the face's nodes
-    auto face = [&](std::vector<double>& fg, size_t nf, size_t f, int ia, int ja, int ic, int jc,
-                    int ib, int jb, int id, int jd) {
+    auto face = [&](double* fg, int ia, int ja, int ic, int jc, int ib, int jb, int id, int jd) {
         double xa, ya, xc, yc, xb, yb, xd, yd;
         centroid(ia, ja, xa, ya);
         centroid(ic, jc, xc, yc);
         node(ib, jb, xb, yb);
         node(id, jd, xd, yd);
         if (iaxis == 1) {
-            fg[FG_SX * nf + f] = (yd - yb) * (yb + yd) * HALF;
-            fg[FG_SY * nf + f] = -(xd - xb) * (yb + yd) * HALF;
+            fg[FG_SX] = (yd - yb) * (yb + yd) * HALF;
+            fg[FG_SY] = -(xd - xb) * (yb + yd) * HALF;
         } else {
-            fg[FG_SX * nf + f] = (yd - yb);
-            fg[FG_SY * nf + f] = -(xd - xb);
+            fg[FG_SX] = (yd - yb);
+            fg[FG_SY] = -(xd - xb);
         }
-        grad(xa, ya, xb, yb, xc, yc, xd, yd, &fg[FG_GA * nf + f], nf);
+        grad(xa, ya, xb, yb, xc, yc, xd, yd, &fg[FG_GA], 1);
         const double yavg = HALF * (yb + yd);
-        fg[FG_RYAVG * nf + f] = (iaxis == 1 && !(yavg < YAXIS_THRESH)) ? 1.0 / yavg : 0.0;
+        fg[FG_RYAVG] = (iaxis == 1 && !(yavg < YAXIS_THRESH)) ? 1.0 / yavg : 0.0;
     };
-    const size_t nfi = (size_t)(ni + 1) * nj, nfj = (size_t)ni * (nj + 1);
-    h->hfgi.assign((size_t)FG_N * nfi, 0.0);
-    h->hfgj.assign((size_t)FG_N * nfj, 0.0);
+    h->hvtile.assign((size_t)ntj * nti * VTILE, 0.0);
+    auto store = [&](const double* fg, int bi, int bj, int f) {
+        double* blk = &h->hvtile[((size_t)bi * ntj + bj) * VTILE + f];
+        for (int k = 0; k < FG_N; k++) blk[(size_t)k * NVF] = fg[k];
+    };
+    double fg[FG_N];
     for (int i = 0; i <= ni; i++)
         for (int j = 0; j < nj; j++) {
-            const size_t f = (size_t)i * nj + j;
             if (i == 0)  // face 4 of cell (0, j): B = node (0, j+1), D = node (0, j)
-                face(h->hfgi, nfi, f, 0, j, -1, j, 0, j + 1, 0, j);
+                face(fg, 0, j, -1, j, 0, j + 1, 0, j);
             else  // face 2 of cell (i-1, j): B = node (i, j), D = node (i, j+1)
-                face(h->hfgi, nfi, f, i - 1, j, i, j, i, j, i, j + 1);
+                face(fg, i - 1, j, i, j, i, j, i, j + 1);
+            const int lb = j % TJ;
+            if (i < ni) store(fg, i / TI, j / TJ, i % TI * TJ + lb);
+            // the first row of a tile is also the last of the one before it
+            if (i > 0 && (i % TI == 0 || i == ni)) store(fg, (i - 1) / TI, j / TJ, ((i - 1) % TI + 1) * TJ + lb);
         }
     for (int i = 0; i < ni; i++)
         for (int j = 0; j <= nj; j++) {
-            const size_t f = (size_t)i * (nj + 1) + j;
             if (j == 0)  // face 1 of cell (i, 0): B = node (i, 0), D = node (i+1, 0)
-                face(h->hfgj, nfj, f, i, 0, i, -1, i, 0, i + 1, 0);
+                face(fg, i, 0, i, -1, i, 0, i + 1, 0);
             else  // face 3 of cell (i, j-1): B = node (i+1, j), D = node (i, j)
-                face(h->hfgj, nfj, f, i, j - 1, i, j, i + 1, j, i, j);
+                face(fg, i, j - 1, i, j, i + 1, j, i, j);
+            const int la = NIF + i % TI * (TJ + 1);
+            if (j < nj) store(fg, i / TI, j / TJ, la + j % TJ);
+            if (j > 0 && (j % TJ == 0 || j == nj)) store(fg, i / TI, (j - 1) / TJ, la + (j - 1) % TJ + 1);
         }
+    // the boundary nodes' ghosts (Mesh::bnode)
+    auto code = [&](int a, int b) {
+        int g[2] = {0, 0}, n = 0;
+        for (int k = 0; k < 4; k++) {
+            const int pi = a - 1 + (k >> 1), pj = b - 1 + (k & 1);
+            const bool in_i = pi >= 0 && pi < ni, in_j = pj >= 0 && pj < nj;
+            if (in_i == in_j) continue;  // a cell, or no position
+            g[n++] = in_i ? h->M.ghost_index(pj < 0 ? 1 : 3, pi) : h->M.ghost_index(pi < 0 ? 4 : 2, pj);
+        }
+        const bool swap = h->hgrank[g[1]] < h->hgrank[g[0]];
+        return h->hgtype[g[swap ? 1 : 0]] | h->hgtype[g[swap ? 0 : 1]] << 3 | (swap ? 1 << 6 : 0);
+    };
+    h->hbnode.clear();
+    for (int a = 0; a <= ni; a++) h->hbnode.push_back(code(a, 0));
+    for (int a = 0; a <= ni; a++) h->hbnode.push_back(code(a, nj));
+    for (int b = 0; b <= nj; b++) h->hbnode.push_back(code(0, b));
+    for (int b = 0; b <= nj; b++) h->hbnode.push_back(code(ni, b));
 }
 
 // Device copy of the layout built by build_mesh.
@@ -339,12 +363,12 @@ int upload_mesh(tns_handle* h) {
     build_geometry(h);
     if ((rc = h->cuda(h->cvol.alloc(h->hcvol.size()), "cudaMalloc")) ||
         (rc = h->cuda(h->stile.alloc(h->hstile.size()), "cudaMalloc")) ||
-        (rc = h->cuda(h->fgi.alloc(h->hfgi.size()), "cudaMalloc")) ||
-        (rc = h->cuda(h->fgj.alloc(h->hfgj.size()), "cudaMalloc")) ||
+        (rc = h->cuda(h->vtile.alloc(h->hvtile.size()), "cudaMalloc")) ||
+        (rc = h->cuda(h->bnode.alloc(h->hbnode.size()), "cudaMalloc")) ||
         (rc = up(h->cvol.p, h->hcvol.data(), h->hcvol.size() * 8)) ||
         (rc = up(h->stile.p, h->hstile.data(), h->hstile.size() * 8)) ||
-        (rc = up(h->fgi.p, h->hfgi.data(), h->hfgi.size() * 8)) ||
-        (rc = up(h->fgj.p, h->hfgj.data(), h->hfgj.size() * 8)))
+        (rc = up(h->vtile.p, h->hvtile.data(), h->hvtile.size() * 8)) ||
+        (rc = up(h->bnode.p, h->hbnode.data(), h->hbnode.size() * 4)))
         return rc;
     // the host copies are not read again
     // static ghost records
@@ -368,8 +392,7 @@ int upload_mesh(tns_handle* h) {
     }
     std::vector<double>().swap(h->hcvol);
     std::vector<double>().swap(h->hstile);
-    std::vector<double>().swap(h->hfgi);
-    std::vector<double>().swap(h->hfgj);
+    std::vector<double>().swap(h->hvtile);
     Mesh& M = h->M;
     M.ni = h->ni; M.nj = h->nj; M.x = h->x.p; M.y = h->y.p; M.cfldl = h->cfldl.p; M.gtype = h->gtype.p;
     M.grank = h->grank.p; M.gxc = h->gxc.p; M.gyc = h->gyc.p; M.ginj = h->ginj.p;
@@ -377,8 +400,8 @@ int upload_mesh(tns_handle* h) {
     M.grec = h->grec.p;
     M.cvol = h->cvol.p;
     M.stile = h->stile.p;
-    M.fgi = h->fgi.p;
-    M.fgj = h->fgj.p;
+    M.vtile = h->vtile.p;
+    M.bnode = h->bnode.p;
     return TNS_OK;
 }
 
@@ -469,7 +492,7 @@ void enqueue_iteration_mx(tns_handle* h, bool monitor, double* A, double* Aout) 
         },
         [&](cudaStream_t s) {
             if (np) launch(h, K_GPORT, [&] { tns::launch_gport_mx(P, M, A, in[0], h->ports.p, np, h->gport.p, s); });
-            launch(h, K_VISC, [&] { tns::launch_viscous_mx(P, M, A, h->visf.p, s); });
+            launch(h, K_VISC, [&] { tns::launch_viscous_mx(P, M, A, h->visf.p, h->status.p, s); });
         });
     cudaStream_t s = h->stream;
     if (monitor) cudaMemsetAsync(h->cdiff.p, 0, 5 * sizeof(unsigned long long), s);
@@ -507,7 +530,7 @@ void enqueue_iteration_f64(tns_handle* h, bool monitor) {
         [&](cudaStream_t s) {
             // the frozen viscous flux of Q_old uses stage 1's boundary state (viscous.f90:29)
             if (np) launch(h, K_GPORT, [&] { tns::launch_gport(P, M, in[0], h->ports.p, np, h->gport.p, s); });
-            launch(h, K_VISC, [&] { tns::launch_viscous(P, M, A, h->vis.p, s); });
+            launch(h, K_VISC, [&] { tns::launch_viscous(P, M, A, h->vis.p, h->status.p, s); });
         });
     cudaStream_t s = h->stream;
     if (monitor) cudaMemsetAsync(h->cdiff.p, 0, 5 * sizeof(unsigned long long), s);
@@ -1158,9 +1181,9 @@ void tns_destroy(tns_handle* h) {
     h->dtf.release(); h->tref.release();
     for (auto* b : {&h->x, &h->y, &h->cfldl, &h->gxc, &h->gyc, &h->ginj, &h->gport, &h->qa, &h->qb,
                     &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->e,
-                    &h->stile, &h->fgi, &h->fgj})
+                    &h->stile, &h->vtile})
         b->release();
-    h->grec.release(); h->gtype.release(); h->grank.release(); h->ports.release();
+    h->grec.release(); h->bnode.release(); h->gtype.release(); h->grank.release(); h->ports.release();
     h->counter.release(); h->status.release(); h->cdiff.release();
     if (h->pinned) cudaFreeHost(h->pinned);
     if (h->status_host) cudaFreeHost(h->status_host);

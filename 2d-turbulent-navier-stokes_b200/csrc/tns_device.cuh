@@ -60,11 +60,11 @@ struct Params {
     double rho0, inv_gm1;                // P0/(RR*T0), 1/(GAMA-1)
 };
 
-// Static per-face geometry of the viscous flux (viscous.f90:130-217), [FG_N][nfaces]
-// for the i-faces (index i*NJ + j, between cells (i-1, j) and (i, j), i = 0..NI) and the
-// j-faces (index i*(NJ+1) + j, between (i, j-1) and (i, j), j = 0..NJ), each in the
-// orientation of the cell that evaluates it (that of cell (i-1, j) as its face 2, or of
-// (0, j) as its face 4; that of (i, j-1) as its face 3, or of (i, 0) as its face 1):
+// Static per-face geometry of the viscous flux (viscous.f90:130-217), stored per tile
+// (tns_tile.cuh), each face in the orientation of the cell that evaluates it (an i-face
+// between cells (i-1, j) and (i, j) in that of (i-1, j) as its face 2, or of (0, j) as its
+// face 4; a j-face between (i, j-1) and (i, j) in that of (i, j-1) as its face 3, or of
+// (i, 0) as its face 1):
 //   FG_SX, FG_SY  face vector; FG_GA..FG_GD diamond-gradient coefficients (A = the cell,
 //   C = the neighbour, B, D = the face's nodes: dF/dx = (F_A - F_C) GA + (F_B - F_D) GB,
 //   dF/dy = (F_A - F_C) GC + (F_B - F_D) GD); FG_RYAVG 1/YAVG of the axisymmetric v/y
@@ -95,8 +95,11 @@ struct Mesh {
     const double* gport;    // type-6 port mass flux of the current stage
     const double* cvol;     // VOL per cell (geometry.f90:87,98,101)
     const double* stile;    // static data of the stage tiles, one block per tile (tns_tile.cuh)
-    const double* fgi;      // [FG_N][(ni+1)*nj] static i-face geometry
-    const double* fgj;      // [FG_N][ni*(nj+1)] static j-face geometry
+    const double* vtile;    // static face geometry of the viscous tiles (tns_tile.cuh)
+    // per boundary node (rows b = 0 and b = nj along a, then a = 0 and a = ni along b): the
+    // BC types of its two ghosts in bc.in order (bits 0-2, 3-5) and whether that order is the
+    // reverse of their ascending position order (bit 6)
+    const int* bnode;
     // (mixed precision) each stage tile's reference state for the current iteration,
     // written by the dissipation kernel from Q_old, read by the four stages
     TileRefMx* tref = nullptr;

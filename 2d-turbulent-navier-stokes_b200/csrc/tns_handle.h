@@ -53,7 +53,8 @@ struct tns_handle {
     std::vector<int> ghost_id;    // bc.in line -> Fortran ghost id
     std::vector<int> port_ghosts;
     std::vector<double> hX, hY, hcfldl, hgxc, hgyc, hginj;  // host layout (device order)
-    std::vector<double> hcvol, hstile, hfgi, hfgj;  // static geometry (VOL, stage tiles, faces)
+    std::vector<double> hcvol, hstile, hvtile;  // static geometry (VOL, stage tiles, viscous tiles)
+    std::vector<int> hbnode;                    // boundary nodes' codes
     std::vector<int> hgtype, hgrank;
     std::vector<int> node_of;   // structured node index -> 1-based node id
     cudaStream_t own = nullptr, stream = nullptr;
@@ -62,7 +63,7 @@ struct tns_handle {
     cudaEvent_t fork = nullptr, join = nullptr;
     // e: the iteration's frozen terms VIS + D, formed by stage 1 (FP64, structured meshes)
     DevBuf<double> x, y, cfldl, gxc, gyc, ginj, gport, qa, qb, qc, d, vis, e, dt, dtmin, partial,
-        primout, cvol, stile, fgi, fgj;
+        primout, cvol, stile, vtile;
     // mixed FP32/FP64 path: FP64 state ping-pong (qa, qa2) and FP32 scratch
     int precision = 0;
     int cur = 0;  // mixed: which of qa / qa2 holds the state
@@ -74,7 +75,7 @@ struct tns_handle {
     cudaGraphExec_t graph_mon = nullptr;
     cudaGraphExec_t graph_mon_mx[2] = {nullptr, nullptr};
     DevBuf<tns::GhostRec> grec;
-    DevBuf<int> gtype, grank, ports;
+    DevBuf<int> gtype, grank, ports, bnode;
     DevBuf<unsigned int> counter, status;
     DevBuf<unsigned long long> cdiff;
     double* pinned = nullptr;  // 5*ncell staging

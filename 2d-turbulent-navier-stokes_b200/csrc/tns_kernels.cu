@@ -19,6 +19,7 @@
 #include "tns_kernels.h"
 #include "tns_tile.cuh"
 #include "tns_batch.cuh"
+#include "tns_visc.cuh"
 
 namespace tns {
 
@@ -460,174 +461,18 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
 
 // ---------------------------------------------------------------- viscous kernel
 
-// Faces owned by a tile: i-faces (between cells (i-1,j) and (i,j)) for i in i0..i0+TI,
-// j-faces (between (i,j-1) and (i,j)) for j in j0..j0+TJ.
-constexpr int NIF = (TI + 1) * TJ;
-constexpr int NJF = TI * (TJ + 1);
-
-struct ViscSmem {
-    double u[NSLOT], v[NSLOT], t[NSLOT], rho[NSLOT], ri[NSLOT];
-    double au[NAVG], av[NAVG], at[NAVG], arho[NAVG], ar[NAVG];
-    double fi[4][NIF], fj[4][NJF];
-};
-
 size_t visc_smem_bytes() { return sizeof(ViscSmem); }
 
-// One face flux (viscous.f90:130-217) in the orientation of cell A (slot sa): C = slot
-// sc, B/D = the face's nodes in node-average coordinates, geometry from the face's
-// stored row fg[k * nf] (FG_*).
-__device__ __forceinline__ void face_flux(const Params& P, const ViscSmem& S, int sa, int sc,
-                                          int ab, int ad, const double* __restrict__ fg,
-                                          size_t nf, double out[4]) {
-    FaceVals f;
-    f.ua = S.u[sa]; f.va = S.v[sa]; f.ta = S.t[sa];
-    f.uc = S.u[sc]; f.vc = S.v[sc]; f.tc = S.t[sc];
-    f.ub = S.au[ab]; f.vb = S.av[ab]; f.tb = S.at[ab];
-    f.ud = S.au[ad]; f.vd = S.av[ad]; f.td = S.at[ad];
-    f.rhoa = S.rho[sa]; f.rhoc = S.rho[sc]; f.rhob = S.arho[ab]; f.rhod = S.arho[ad];
-    f.ra = S.ri[sa]; f.rc = S.ri[sc]; f.rb = S.ar[ab]; f.rd = S.ar[ad];
-    viscous_face(P, f, fg[FG_SX * nf], fg[FG_SY * nf], fg[FG_GA * nf], fg[FG_GB * nf],
-                 fg[FG_GC * nf], fg[FG_GD * nf], P.iaxis == 1 ? fg[FG_RYAVG * nf] : 0.0, out);
+__device__ __forceinline__ void viscous_tile_f64(const Params& P, const Mesh& M, const double* __restrict__ q,
+                                                 double* __restrict__ vis, unsigned int* error, int bx, int by) {
+    viscous_tile(P, M, q, vis, error, bx, by,
+                 [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
+                     double out[4]) { viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
 
-// Frozen viscous flux VIS of Q_old (viscous.f90:29-217): nodal averages, then each face
-// of the tile once; a cell adds its four faces in order 1..4, negating the faces that
-// were evaluated in the neighbour's orientation.
-__device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
-                                             double* __restrict__ vis, int bx, int by) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ViscSmem& S = *reinterpret_cast<ViscSmem*>(smem_raw);
-    const size_t ncell = (size_t)M.ni * M.nj;
-    const int j0 = bx * TJ, i0 = by * TI;
-    const int tid = threadIdx.y * TJ + threadIdx.x;
-    pdl_trigger();
-    pdl_wait();
-    for (int s = tid; s < NSLOT; s += VNT) {
-        const int li = s / SW, lj = s % SW;
-        int along = 0;
-        const int kind = classify(M, i0 - 1 + li, j0 - 1 + lj, along);
-        if (kind < 0) continue;
-        Prim p;
-        if (kind == 0)
-            cell_prim(P, q, ncell, (size_t)(i0 - 1 + li) * M.nj + (j0 - 1 + lj), p);
-        else
-            ghost_state(P, M, q, ncell, kind, along, p);
-        S.u[s] = p.u; S.v[s] = p.v; S.t[s] = p.t; S.rho[s] = p.rho; S.ri[s] = p.ri;
-    }
-    __syncthreads();
-    // nodal averages (viscous.f90:40-59,77-124) of nodes (i0..i0+TI, j0..j0+TJ)
-    for (int s = tid; s < NAVG; s += VNT) {
-        const int la = s / AW, lb = s % AW;
-        const int a = i0 + la, b = j0 + lb;
-        if (a > M.ni || b > M.nj) continue;
-        double un = 0.0, vn = 0.0, tn = 0.0, rhon = 0.0, rn = 0.0;
-        int cnt = 0, ng = 0, gs[2] = {0, 0}, gr[2] = {0, 0};
-        // the four surrounding positions in ascending cell-id order
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int pi = a - 1 + (k >> 1), pj = b - 1 + (k & 1);
-            const int sl = (la + (k >> 1)) * SW + lb + (k & 1);
-            int along = 0;
-            const int kind = classify(M, pi, pj, along);
-            if (kind == 0) {
-                un = un + S.u[sl]; vn = vn + S.v[sl]; tn = tn + S.t[sl];
-                rhon = rhon + S.rho[sl]; rn = rn + S.ri[sl];
-                cnt++;
-            } else if (kind > 0) {
-                gs[ng] = sl;
-                gr[ng] = M.ghost_index(kind, along);
-                ng++;
-            }
-        }
-        if (ng == 2 && M.grank[gr[1]] < M.grank[gr[0]]) {
-            int t = gs[0]; gs[0] = gs[1]; gs[1] = t;
-            t = gr[0]; gr[0] = gr[1]; gr[1] = t;
-        }
-        for (int k = 0; k < ng; k++) {
-            const int sl = gs[k];
-            un = un + S.u[sl]; vn = vn + S.v[sl]; tn = tn + S.t[sl];
-            rhon = rhon + S.rho[sl]; rn = rn + S.ri[sl];
-            const int type = M.gtype[gr[k]];
-            if (type == 4) {
-                vn = 0.0;
-            } else if (type == 5) {
-                un = 0.0; vn = 0.0; rn = P.rtol_rtred;
-            }
-            cnt++;
-        }
-        const double idf = cnt == 4 ? 0.25 : 1.0 / (double)cnt;
-        S.au[s] = un * idf; S.av[s] = vn * idf; S.at[s] = tn * idf; S.arho[s] = rhon * idf;
-        S.ar[s] = dmax1(P.rtol, rn * idf);
-    }
-    __syncthreads();
-    // all faces of the tile in one loop (i-faces first): at most three faces per thread,
-    // one inlined copy of the face flux
-    const size_t nfi = (size_t)(M.ni + 1) * M.nj, nfj = (size_t)M.ni * (M.nj + 1);
-    for (int f = tid; f < NIF + NJF; f += VNT) {
-        int sa, sc, ab, ad;
-        const double* fg;
-        size_t nf;
-        if (f < NIF) {
-            // i-face: orientation of cell (i-1, j) as its face 2, or of (0, j) as its face 4
-            const int ii = f / TJ, jj = f % TJ;
-            const int i = i0 + ii, j = j0 + jj;
-            if (i > M.ni || j >= M.nj) continue;
-            const int sL = ii * SW + jj + 1, sR = sL + SW;  // cells (i-1, j), (i, j)
-            const int aLo = ii * AW + jj, aHi = aLo + 1;    // nodes (i, j), (i, j+1)
-            if (i == 0) {  // face 4: B=N4, D=N1
-                sa = sR; sc = sL; ab = aHi; ad = aLo;
-            } else {  // face 2: B=N2, D=N3
-                sa = sL; sc = sR; ab = aLo; ad = aHi;
-            }
-            fg = M.fgi + ((size_t)i * M.nj + j);
-            nf = nfi;
-        } else {
-            // j-face: orientation of cell (i, j-1) as its face 3, or of (i, 0) as its face 1
-            const int g = f - NIF;
-            const int ii = g / AW, jj = g % AW;
-            const int i = i0 + ii, j = j0 + jj;
-            if (i >= M.ni || j > M.nj) continue;
-            const int sB = (ii + 1) * SW + jj, sT = sB + 1;  // cells (i, j-1), (i, j)
-            const int aL = ii * AW + jj, aR = aL + AW;       // nodes (i, j), (i+1, j)
-            if (j == 0) {  // face 1: B=N1, D=N2
-                sa = sT; sc = sB; ab = aL; ad = aR;
-            } else {  // face 3: B=N3, D=N4
-                sa = sB; sc = sT; ab = aR; ad = aL;
-            }
-            fg = M.fgj + ((size_t)i * (M.nj + 1) + j);
-            nf = nfj;
-        }
-        double out[4];
-        face_flux(P, S, sa, sc, ab, ad, fg, nf, out);
-        if (f < NIF) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) S.fi[k][f] = out[k];
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++) S.fj[k][f - NIF] = out[k];
-        }
-    }
-    __syncthreads();
-    const int tj = threadIdx.x, ti = threadIdx.y;
-    const int i = i0 + ti, j = j0 + tj;
-    if (ti >= TI || i >= M.ni || j >= M.nj) return;
-    const size_t cell = (size_t)i * M.nj + j;
-    const int f1 = ti * AW + tj, f3 = f1 + 1;          // j-faces j, j+1
-    const int f4 = ti * TJ + tj, f2 = f4 + TJ;         // i-faces i, i+1
-    const double s1 = (j == 0) ? 1.0 : -1.0, s4 = (i == 0) ? 1.0 : -1.0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        double acc = s1 * S.fj[k][f1];
-        acc = acc + S.fi[k][f2];
-        acc = acc + S.fj[k][f3];
-        acc = acc + s4 * S.fi[k][f4];
-        vis[k * ncell + cell] = acc;
-    }
-}
-
-__global__ void __launch_bounds__(VNT, TNS_PER_SM(TNS_VISC_MINB)) k_viscous(Params P, Mesh M, const double* __restrict__ q,
-                                                      double* __restrict__ vis) {
-    viscous_tile(P, M, q, vis, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_MINB))
+k_viscous(Params P, Mesh M, const double* __restrict__ q, double* __restrict__ vis, unsigned int* error) {
+    viscous_tile_f64(P, M, q, vis, error, blockIdx.x, blockIdx.y);
 }
 
 // --------------------------------------------------------- dissipation kernel
@@ -1060,13 +905,13 @@ __global__ void __launch_bounds__(NTHREADS) k_dissipation_batch(const BatchCase*
     dissipation_tile<double>(c.P, c.M, c.diss, t.y, t.z);
 }
 
-__global__ void __launch_bounds__(VNT, TNS_PER_SM(TNS_VISC_BATCH_MINB)) k_viscous_batch(const BatchCase* __restrict__ cases,
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_BATCH_MINB)) k_viscous_batch(const BatchCase* __restrict__ cases,
                                                                           const int4* __restrict__ tiles,
                                                                           const int* __restrict__ active) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;
     const BatchCase& c = cases[t.x];
-    viscous_tile(c.P, c.M, c.q, c.vis, t.y, t.z);
+    viscous_tile_f64(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
 }
 
 __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_BATCH_MINB)) k_stage_batch(const BatchCase* __restrict__ cases,
@@ -1119,9 +964,10 @@ k_batch_persistent(const BatchCase* __restrict__ cases, const int4* __restrict__
                 if (active[t.x]) {
                     const BatchCase& c = cases[t.x];
                     if (ph == 0 && w < ntiles) dissipation_tile<double>(c.P, c.M, c.diss, t.y, t.z);
-                    else if (ph == 0) viscous_tile(c.P, c.M, c.q, c.vis, t.y, t.z);
+                    else if (ph == 0) viscous_tile_f64(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
                     else stage_tile(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
                 }
+                async_proxy_fence();
                 __syncthreads();
             }
             if (!grid_barrier(bar, bar + 1)) {
@@ -1267,7 +1113,7 @@ void launch_batch_f64(const BatchCase* cases, const int4* tiles, const int* acti
     if (kernel == 0)
         launch_tile(k_dissipation_batch, dim3(ntiles), blk, diss_smem_bytes(), s, cases, tiles, active);
     else if (kernel == 1)
-        launch_tile(k_viscous_batch, dim3(ntiles), dim3(TJ, VROWS), visc_smem_bytes(), s, cases, tiles, active);
+        launch_tile(k_viscous_batch, dim3(ntiles), dim3(TJ, TI), visc_smem_bytes(), s, cases, tiles, active);
     else
         launch_tile(k_stage_batch, dim3(ntiles), blk, stage_smem_bytes(), s, cases, tiles, active, stage, monitor);
 }
@@ -1284,8 +1130,9 @@ void launch_dissipation_mx(const Params& P, const Mesh& M, const double* q, floa
     launch_tile(k_dissipation<float>, tile_grid(M), dim3(TJ, TI), diss_smem_bytes(), s, P, M, A);
 }
 
-void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, cudaStream_t s) {
-    launch_tile(k_viscous, tile_grid(M), dim3(TJ, VROWS), visc_smem_bytes(), s, P, M, q, vis);
+void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, unsigned int* error,
+                    cudaStream_t s) {
+    launch_tile(k_viscous, tile_grid(M), dim3(TJ, TI), visc_smem_bytes(), s, P, M, q, vis, error);
 }
 
 void launch_stage(const Params& P, const Mesh& M, const double* qin, const double* qold,

@@ -17,7 +17,8 @@ int dtmin_blocks(const Mesh& M);
 
 void launch_dissipation(const Params& P, const Mesh& M, const double* q, double* d, double* dt,
                         const double* dtmin, cudaStream_t s);
-void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, cudaStream_t s);
+void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, unsigned int* error,
+                    cudaStream_t s);
 // RK stage 0..3 of the iteration; e: [5][ncell] scratch that stage 0 fills with VIS + D and
 // the others read; error: bit 1 is set when a tile's copies did not complete (must not be
 // null)
@@ -74,7 +75,8 @@ void launch_dissipation_mx(const Params& P, const Mesh& M, const double* q, floa
                            const double* dtmin, cudaStream_t s);
 void launch_dissipation_mx2(const Params& P, const Mesh& M, const double* q, float* d, float* dt,
                             const double* dtmin, cudaStream_t s);
-void launch_viscous_mx(const Params& P, const Mesh& M, const double* q, float* vis, cudaStream_t s);
+void launch_viscous_mx(const Params& P, const Mesh& M, const double* q, float* vis, unsigned int* error,
+                       cudaStream_t s);
 void launch_stage_mx(const Params& P, const Mesh& M, const double* cold, const float* dqin,
                      float* dqout, double* qout, const float* d, const float* vis, const float* dt,
                      const double* dtmin, double alpha, unsigned long long* cdiff,

@@ -19,6 +19,7 @@
 #include "tns_mx.cuh"
 #include "tns_tile.cuh"
 #include "tns_batch.cuh"
+#include "tns_visc.cuh"
 
 namespace tns {
 
@@ -324,45 +325,30 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MX_MINB)) k_sta
 
 // ---------------------------------------------------------------- viscous kernel
 
-constexpr int NIFM = (TI + 1) * TJ;
-constexpr int NJFM = TI * (TJ + 1);
+size_t visc_mx_smem_bytes() { return sizeof(ViscSmem); }
 
-struct ViscSmemMx {
-    double u[NSLOT], v[NSLOT], t[NSLOT], rho[NSLOT], ri[NSLOT];
-    double au[NAVG], av[NAVG], at[NAVG], arho[NAVG], ar[NAVG];
-    float fi[4][NIFM], fj[4][NJFM];
-};
-
-size_t visc_mx_smem_bytes() { return sizeof(ViscSmemMx); }
-
-// One face of viscous.f90:130-217: FP64 stencil differences, FP32 rest; the face vector
-// and diamond-gradient coefficients from the face's stored row fg[k * nf] (FG_*).
-__device__ __forceinline__ void face_flux_mx(const Params& P, const ViscSmemMx& S, int sa, int sc,
-                                             int ab, int ad, const double* __restrict__ fg, size_t nf,
-                                             float out[4]) {
-    const float sx = (float)fg[FG_SX * nf], sy = (float)fg[FG_SY * nf];
-    const float ga = (float)fg[FG_GA * nf], gb = (float)fg[FG_GB * nf];
-    const float gc = (float)fg[FG_GC * nf], gd = (float)fg[FG_GD * nf];
-    const double ua = S.u[sa], va = S.v[sa], ta = S.t[sa], uc = S.u[sc], vc = S.v[sc], tc = S.t[sc];
-    const double ub = S.au[ab], vb = S.av[ab], tb = S.at[ab], ud = S.au[ad], vd = S.av[ad], td = S.at[ad];
-    const double ra = S.ri[sa], rc = S.ri[sc], rb = S.ar[ab], rd = S.ar[ad];
-    const float duac = (float)(ua - uc), dubd = (float)(ub - ud);
-    const float dvac = (float)(va - vc), dvbd = (float)(vb - vd);
-    const float dtac = (float)(ta - tc), dtbd = (float)(tb - td);
-    const float drac = (float)(ra - rc), drbd = (float)(rb - rd);
+// One face of viscous.f90:130-217: FP64 stencil differences, FP32 rest.
+__device__ __forceinline__ void viscous_face_mx(const Params& P, const FaceVals& f, double dsx, double dsy, double dga,
+                                                double dgb, double dgc, double dgd, double ryavg, double out[4]) {
+    const float sx = (float)dsx, sy = (float)dsy;
+    const float ga = (float)dga, gb = (float)dgb, gc = (float)dgc, gd = (float)dgd;
+    const float duac = (float)(f.ua - f.uc), dubd = (float)(f.ub - f.ud);
+    const float dvac = (float)(f.va - f.vc), dvbd = (float)(f.vb - f.vd);
+    const float dtac = (float)(f.ta - f.tc), dtbd = (float)(f.tb - f.td);
+    const float drac = (float)(f.ra - f.rc), drbd = (float)(f.rb - f.rd);
     const float DUX = duac * ga + dubd * gb, DUY = duac * gc + dubd * gd;
     const float DVX = dvac * ga + dvbd * gb, DVY = dvac * gc + dvbd * gd;
     const float DTX = dtac * ga + dtbd * gb, DTY = dtac * gc + dtbd * gd;
     const float DRX = drac * ga + drbd * gb, DRY = drac * gc + drbd * gd;
-    const float UAVG = (float)(QUARTER * (ua + ub + uc + ud));
-    const float VAVG = (float)(QUARTER * (va + vb + vc + vd));
-    const float TAVG = (float)(QUARTER * (ta + tb + tc + td));
-    const float RHOAVG = (float)(QUARTER * (S.rho[sa] + S.arho[ab] + S.rho[sc] + S.arho[ad]));
-    const float RAVG = (float)(QUARTER * (ra + rb + rc + rd));
+    const double vsum = f.va + f.vb + f.vc + f.vd;
+    const float UAVG = (float)(QUARTER * (f.ua + f.ub + f.uc + f.ud));
+    const float VAVG = (float)(QUARTER * vsum);
+    const float TAVG = (float)(QUARTER * (f.ta + f.tb + f.tc + f.td));
+    const float RHOAVG = (float)(QUARTER * (f.rhoa + f.rhob + f.rhoc + f.rhod));
+    const float RAVG = (float)(QUARTER * (f.ra + f.rb + f.rc + f.rd));
     float DIVVEL;
     if (P.iaxis == 1) {
-        const double ryavg = fg[FG_RYAVG * nf];
-        const float VBYY = (ryavg == 0.0) ? DVY : (float)(QUARTER * (va + vb + vc + vd) * ryavg);
+        const float VBYY = (ryavg == 0.0) ? DVY : (float)(QUARTER * vsum * ryavg);
         DIVVEL = DUX + DVY + VBYY;
     } else {
         DIVVEL = DUX + DVY;
@@ -389,133 +375,15 @@ __device__ __forceinline__ void face_flux_mx(const Params& P, const ViscSmemMx& 
 }
 
 __device__ __forceinline__ void viscous_mx_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
-                                                float* __restrict__ vis, int bx, int by) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ViscSmemMx& S = *reinterpret_cast<ViscSmemMx*>(smem_raw);
-    const size_t ncell = (size_t)M.ni * M.nj;
-    const int j0 = bx * TJ, i0 = by * TI;
-    const int tid = threadIdx.y * TJ + threadIdx.x;
-    pdl_trigger();
-    pdl_wait();
-    for (int s = tid; s < NSLOT; s += VNT) {
-        const int li = s / SW, lj = s % SW;
-        int along = 0;
-        const int kind = classify(M, i0 - 1 + li, j0 - 1 + lj, along);
-        if (kind < 0) continue;
-        Prim p;
-        if (kind == 0)
-            cell_prim(P, q, ncell, (size_t)(i0 - 1 + li) * M.nj + (j0 - 1 + lj), p);
-        else
-            ghost_state(P, M, q, ncell, kind, along, p);
-        S.u[s] = p.u; S.v[s] = p.v; S.t[s] = p.t; S.rho[s] = p.rho; S.ri[s] = p.ri;
-    }
-    __syncthreads();
-    for (int s = tid; s < NAVG; s += VNT) {
-        const int la = s / AW, lb = s % AW;
-        const int a = i0 + la, b = j0 + lb;
-        if (a > M.ni || b > M.nj) continue;
-        double un = 0.0, vn = 0.0, tn = 0.0, rhon = 0.0, rn = 0.0;
-        int cnt = 0, ng = 0, gs[2] = {0, 0}, gr[2] = {0, 0};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int pi = a - 1 + (k >> 1), pj = b - 1 + (k & 1);
-            const int sl = (la + (k >> 1)) * SW + lb + (k & 1);
-            int along = 0;
-            const int kind = classify(M, pi, pj, along);
-            if (kind == 0) {
-                un = un + S.u[sl]; vn = vn + S.v[sl]; tn = tn + S.t[sl];
-                rhon = rhon + S.rho[sl]; rn = rn + S.ri[sl];
-                cnt++;
-            } else if (kind > 0) {
-                gs[ng] = sl;
-                gr[ng] = M.ghost_index(kind, along);
-                ng++;
-            }
-        }
-        if (ng == 2 && M.grank[gr[1]] < M.grank[gr[0]]) {
-            int t = gs[0]; gs[0] = gs[1]; gs[1] = t;
-            t = gr[0]; gr[0] = gr[1]; gr[1] = t;
-        }
-        for (int k = 0; k < ng; k++) {
-            const int sl = gs[k];
-            un = un + S.u[sl]; vn = vn + S.v[sl]; tn = tn + S.t[sl];
-            rhon = rhon + S.rho[sl]; rn = rn + S.ri[sl];
-            const int type = M.gtype[gr[k]];
-            if (type == 4) {
-                vn = 0.0;
-            } else if (type == 5) {
-                un = 0.0; vn = 0.0; rn = P.rtol_rtred;
-            }
-            cnt++;
-        }
-        const double idf = cnt == 4 ? 0.25 : 1.0 / (double)cnt;
-        S.au[s] = un * idf; S.av[s] = vn * idf; S.at[s] = tn * idf; S.arho[s] = rhon * idf;
-        S.ar[s] = dmax1(P.rtol, rn * idf);
-    }
-    __syncthreads();
-    // all faces of the tile in one loop (i-faces first): at most three faces per thread,
-    // one inlined copy of the face flux
-    const size_t nfi = (size_t)(M.ni + 1) * M.nj, nfj = (size_t)M.ni * (M.nj + 1);
-    for (int f = tid; f < NIFM + NJFM; f += VNT) {
-        int sa, sc, ab, ad;
-        const double* fg;
-        size_t nf;
-        if (f < NIFM) {
-            // i-face: orientation of cell (i-1, j) as its face 2, or of (0, j) as its face 4
-            const int ii = f / TJ, jj = f % TJ;
-            const int i = i0 + ii, j = j0 + jj;
-            if (i > M.ni || j >= M.nj) continue;
-            const int sL = ii * SW + jj + 1, sR = sL + SW;  // cells (i-1, j), (i, j)
-            const int aLo = ii * AW + jj, aHi = aLo + 1;    // nodes (i, j), (i, j+1)
-            if (i == 0) {  // face 4: B=N4, D=N1
-                sa = sR; sc = sL; ab = aHi; ad = aLo;
-            } else {  // face 2: B=N2, D=N3
-                sa = sL; sc = sR; ab = aLo; ad = aHi;
-            }
-            fg = M.fgi + ((size_t)i * M.nj + j);
-            nf = nfi;
-        } else {
-            // j-face: orientation of cell (i, j-1) as its face 3, or of (i, 0) as its face 1
-            const int g = f - NIFM;
-            const int ii = g / AW, jj = g % AW;
-            const int i = i0 + ii, j = j0 + jj;
-            if (i >= M.ni || j > M.nj) continue;
-            const int sB = (ii + 1) * SW + jj, sT = sB + 1;  // cells (i, j-1), (i, j)
-            const int aL = ii * AW + jj, aR = aL + AW;       // nodes (i, j), (i+1, j)
-            if (j == 0) {  // face 1: B=N1, D=N2
-                sa = sT; sc = sB; ab = aL; ad = aR;
-            } else {  // face 3: B=N3, D=N4
-                sa = sB; sc = sT; ab = aR; ad = aL;
-            }
-            fg = M.fgj + ((size_t)i * (M.nj + 1) + j);
-            nf = nfj;
-        }
-        float out[4];
-        face_flux_mx(P, S, sa, sc, ab, ad, fg, nf, out);
-        if (f < NIFM) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) S.fi[k][f] = out[k];
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++) S.fj[k][f - NIFM] = out[k];
-        }
-    }
-    __syncthreads();
-    const int tj = threadIdx.x, ti = threadIdx.y;
-    const int i = i0 + ti, j = j0 + tj;
-    if (ti >= TI || i >= M.ni || j >= M.nj) return;
-    const size_t cell = (size_t)i * M.nj + j;
-    const int f1 = ti * AW + tj, f3 = f1 + 1;
-    const int f4 = ti * TJ + tj, f2 = f4 + TJ;
-    const float s1 = (j == 0) ? 1.0f : -1.0f, s4 = (i == 0) ? 1.0f : -1.0f;
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        vis[k * ncell + cell] = ((s1 * S.fj[k][f1] + S.fi[k][f2]) + S.fj[k][f3]) + s4 * S.fi[k][f4];
+                                                float* __restrict__ vis, unsigned int* error, int bx, int by) {
+    viscous_tile(P, M, q, vis, error, bx, by,
+                 [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
+                     double out[4]) { viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
 
-__global__ void __launch_bounds__(VNT, TNS_PER_SM(TNS_VISC_MX_MINB)) k_viscous_mx(Params P, Mesh M, const double* __restrict__ q,
-                                                         float* __restrict__ vis) {
-    viscous_mx_tile(P, M, q, vis, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_MX_MINB))
+k_viscous_mx(Params P, Mesh M, const double* __restrict__ q, float* __restrict__ vis, unsigned int* error) {
+    viscous_mx_tile(P, M, q, vis, error, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------ dissipation kernel
@@ -747,14 +615,14 @@ __global__ void __launch_bounds__(NTHREADS) k_dissipation_mx_batch(const BatchCa
     dissipation_mx_tile(c.P, c.M, c.qmx[parity], c.df, c.dtf, c.dtmin, t.y, t.z);
 }
 
-__global__ void __launch_bounds__(VNT, TNS_PER_SM(TNS_VISC_MX_BATCH_MINB)) k_viscous_mx_batch(const BatchCase* __restrict__ cases,
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_MX_BATCH_MINB)) k_viscous_mx_batch(const BatchCase* __restrict__ cases,
                                                                                 const int4* __restrict__ tiles,
                                                                                 const int* __restrict__ active,
                                                                                 int parity) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;
     const BatchCase& c = cases[t.x];
-    viscous_mx_tile(c.P, c.M, c.qmx[parity], c.visf, t.y, t.z);
+    viscous_mx_tile(c.P, c.M, c.qmx[parity], c.visf, c.stage_mx[0][0][0].error, t.y, t.z);
 }
 
 __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MX_BATCH_MINB)) k_stage_mx_batch(const BatchCase* __restrict__ cases,
@@ -805,10 +673,11 @@ k_batch_persistent_mx(const BatchCase* __restrict__ cases, const int4* __restric
                     if (ph == 0 && w < ntiles)
                         dissipation_mx_tile(c.P, c.M, c.qmx[parity], c.df, c.dtf, c.dtmin, t.y, t.z);
                     else if (ph == 0)
-                        viscous_mx_tile(c.P, c.M, c.qmx[parity], c.visf, t.y, t.z);
+                        viscous_mx_tile(c.P, c.M, c.qmx[parity], c.visf, c.stage_mx[0][0][0].error, t.y, t.z);
                     else
                         stage_mx_tile(c.P, c.M, c.stage_mx[parity][0][ph - 1], t.y, t.z);
                 }
+                async_proxy_fence();
                 __syncthreads();
             }
             if (!grid_barrier(bar, bar + 1)) {
@@ -866,7 +735,7 @@ void launch_batch_mx(const BatchCase* cases, const int4* tiles, const int* activ
     if (kernel == 0)
         launch_tile(k_dissipation_mx_batch, dim3(ntiles), blk, diss_mx_smem_bytes(), s, cases, tiles, active, parity);
     else if (kernel == 1)
-        launch_tile(k_viscous_mx_batch, dim3(ntiles), dim3(TJ, VROWS), visc_mx_smem_bytes(), s, cases, tiles, active,
+        launch_tile(k_viscous_mx_batch, dim3(ntiles), dim3(TJ, TI), visc_mx_smem_bytes(), s, cases, tiles, active,
                     parity);
     else
         launch_tile(k_stage_mx_batch, dim3(ntiles), blk, stage_mx_smem_bytes(), s, cases, tiles, active, parity, stage,
@@ -878,8 +747,9 @@ void launch_dissipation_mx2(const Params& P, const Mesh& M, const double* q, flo
     launch_tile(k_dissipation_mx, tile_grid_mx(M), dim3(TJ, TI), diss_mx_smem_bytes(), s, P, M, q, d, dt, dtmin);
 }
 
-void launch_viscous_mx(const Params& P, const Mesh& M, const double* q, float* vis, cudaStream_t s) {
-    launch_tile(k_viscous_mx, tile_grid_mx(M), dim3(TJ, VROWS), visc_mx_smem_bytes(), s, P, M, q, vis);
+void launch_viscous_mx(const Params& P, const Mesh& M, const double* q, float* vis, unsigned int* error,
+                       cudaStream_t s) {
+    launch_tile(k_viscous_mx, tile_grid_mx(M), dim3(TJ, TI), visc_mx_smem_bytes(), s, P, M, q, vis, error);
 }
 
 void launch_stage_mx(const Params& P, const Mesh& M, const double* cold, const float* dqin,

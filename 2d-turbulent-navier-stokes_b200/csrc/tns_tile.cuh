@@ -33,15 +33,6 @@ constexpr int TJ = 32;      // tile extent along j (contiguous in memory)
 constexpr int GP_THREADS = 128;  // threads per port line of the type-6 port-flux kernels
 constexpr int TI = TNS_TI;  // tile extent along i
 constexpr int NTHREADS = TJ * TI;
-// The viscous kernels may run one extra row of threads: a tile has (TI+1)*TJ + TI*(TJ+1)
-// faces, which TI+1 rows of threads cover in two rounds.
-#ifndef TNS_VISC_EXTRA_ROW
-#define TNS_VISC_EXTRA_ROW 0
-#endif
-constexpr int VROWS = TI + TNS_VISC_EXTRA_ROW;
-constexpr int VNT = TJ * VROWS;
-
-
 // Halo-1 slot grid (TI+2) x (TJ+2).
 constexpr int SW = TJ + 2;
 constexpr int NSLOT = (TI + 2) * SW;
@@ -77,6 +68,16 @@ constexpr int SNN = (TI + 1) * SNW;
 enum StageTileField { ST_GA, ST_GB, ST_GC, ST_GD, ST_RVOL, ST_RYCC, ST_NF };
 constexpr int STILE = 2 * SNN + ST_NF * TI * TJ;
 static_assert(STILE % 2 == 0, "a stage tile block must be a multiple of 16 bytes");
+
+// Faces of a tile: i-faces (between cells (i-1, j) and (i, j)) for i in i0..i0+TI, j-faces
+// (between (i, j-1) and (i, j)) for j in j0..j0+TJ; and the tile's static face geometry
+// (tile (bx, by) at M.vtile + (by * ntiles_j + bx) * VTILE), [FG_N][NVF], i-face (la, lb) at
+// la * TJ + lb, j-face (la, lb) at NIF + la * (TJ + 1) + lb.
+constexpr int NIF = (TI + 1) * TJ;
+constexpr int NJF = TI * (TJ + 1);
+constexpr int NVF = NIF + NJF;
+constexpr int VTILE = FG_N * NVF;
+static_assert(NVF % 2 == 0, "rows of the face geometry are multiples of 16 bytes");
 
 // Programmatic dependent launch: a tile kernel lets the next kernel in the stream start
 // as soon as all its blocks are running (pdl_trigger), and waits for the previous one
@@ -149,6 +150,10 @@ __device__ __forceinline__ bool bulk_wait(unsigned long long* bar, unsigned pari
     }
     return false;
 }
+
+// Orders this thread's shared-memory accesses before later bulk copies into them (issued after
+// a block barrier), for kernels whose tiles reuse one buffer.
+__device__ __forceinline__ void async_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Grid-wide barrier of a cooperative launch (every block resident): an arrival counter
 // and a generation word in global memory, both zero before the launch.  The last block
@@ -239,6 +244,15 @@ __device__ __forceinline__ int classify(const Mesh& M, int i, int j, int& along)
     if (in_i && j == M.nj) { along = i; return 3; }
     if (in_j && i == -1) { along = j; return 4; }
     return -1;
+}
+
+// The boundary code of node (a, b), 0 inside the mesh (see Mesh::bnode).
+__device__ __forceinline__ int node_code(const Mesh& M, int a, int b) {
+    if (b == 0 && a <= M.ni) return M.bnode[a];
+    if (b == M.nj && a <= M.ni) return M.bnode[M.ni + 1 + a];
+    if (a == 0 && b < M.nj) return M.bnode[2 * (M.ni + 1) + b];
+    if (a == M.ni && b < M.nj) return M.bnode[2 * (M.ni + 1) + M.nj + 1 + b];
+    return 0;
 }
 
 // What a ghost's state depends on besides its parent: its BC type and static geometry
