@@ -106,6 +106,9 @@ __device__ __forceinline__ void bulk_barrier_init(unsigned long long* bar) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // without this fence the copy engine may complete a copy on a barrier it does not see
+    // initialised yet, and the wait never ends
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 // barrier_expect: the phase completes when `bytes` of copies have arrived.
 __device__ __forceinline__ void barrier_expect(unsigned long long* bar, unsigned bytes) {
