@@ -361,7 +361,10 @@ int upload_mesh(tns_handle* h) {
         return rc;
     if ((rc = h->cuda(cudaMemset(h->gport.p, 0, ngs * 8), "cudaMemset"))) return rc;
     build_geometry(h);
+    std::vector<double> vcfl(ncell);
+    for (size_t k = 0; k < ncell; k++) vcfl[k] = h->hcvol[k] / h->hcfldl[k];
     if ((rc = h->cuda(h->cvol.alloc(h->hcvol.size()), "cudaMalloc")) ||
+        (rc = h->cuda(h->vcfl.alloc(ncell), "cudaMalloc")) || (rc = up(h->vcfl.p, vcfl.data(), ncell * 8)) ||
         (rc = h->cuda(h->stile.alloc(h->hstile.size()), "cudaMalloc")) ||
         (rc = h->cuda(h->vtile.alloc(h->hvtile.size()), "cudaMalloc")) ||
         (rc = h->cuda(h->bnode.alloc(h->hbnode.size()), "cudaMalloc")) ||
@@ -399,6 +402,7 @@ int upload_mesh(tns_handle* h) {
     M.gport = h->gport.p;
     M.grec = h->grec.p;
     M.cvol = h->cvol.p;
+    M.vcfl = h->vcfl.p;
     M.stile = h->stile.p;
     M.vtile = h->vtile.p;
     M.bnode = h->bnode.p;
@@ -488,7 +492,7 @@ void enqueue_iteration_mx(tns_handle* h, bool monitor, double* A, double* Aout) 
         [&](cudaStream_t s) {
             if (!P.local)
                 launch(h, K_DTMIN, [&] { tns::launch_dtmin(P, M, A, h->partial.p, h->counter.p, h->dtmin.p, s); });
-            launch(h, K_DISS, [&] { tns::launch_dissipation_mx2(P, M, A, h->df.p, h->dtf.p, h->dtmin.p, s); });
+            launch(h, K_DISS, [&] { tns::launch_dissipation_mx(P, M, A, h->df.p, h->dtf.p, h->dtmin.p, s); });
         },
         [&](cudaStream_t s) {
             if (np) launch(h, K_GPORT, [&] { tns::launch_gport_mx(P, M, A, in[0], h->ports.p, np, h->gport.p, s); });
@@ -1180,7 +1184,7 @@ void tns_destroy(tns_handle* h) {
     h->qa2.release(); h->dqb.release(); h->dqc.release(); h->df.release(); h->visf.release();
     h->dtf.release(); h->tref.release();
     for (auto* b : {&h->x, &h->y, &h->cfldl, &h->gxc, &h->gyc, &h->ginj, &h->gport, &h->qa, &h->qb,
-                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->e,
+                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->vcfl, &h->e,
                     &h->stile, &h->vtile})
         b->release();
     h->grec.release(); h->bnode.release(); h->gtype.release(); h->grank.release(); h->ports.release();

@@ -94,6 +94,7 @@ struct Mesh {
     const double* ginj;     // type-6 burn-rate multiplier
     const double* gport;    // type-6 port mass flux of the current stage
     const double* cvol;     // VOL per cell (geometry.f90:87,98,101)
+    const double* vcfl;     // VOL / (CFL*DL) per cell
     const double* stile;    // static data of the stage tiles, one block per tile (tns_tile.cuh)
     const double* vtile;    // static face geometry of the viscous tiles (tns_tile.cuh)
     // per boundary node (rows b = 0 and b = nj along a, then a = 0 and a = ni along b): the

@@ -19,6 +19,7 @@
 #include "tns_kernels.h"
 #include "tns_tile.cuh"
 #include "tns_batch.cuh"
+#include "tns_diss.cuh"
 #include "tns_visc.cuh"
 
 namespace tns {
@@ -477,16 +478,7 @@ k_viscous(Params P, Mesh M, const double* __restrict__ q, double* __restrict__ v
 
 // --------------------------------------------------------- dissipation kernel
 
-constexpr int DW = TJ + 4;             // halo-2 slot grid (TI+4) x (TJ+4)
-constexpr int NDSLOT = (TI + 4) * DW;
-constexpr int RW = TJ + 2;             // ring-1 grid (TI+2) x (TJ+2)
-constexpr int NRSLOT = (TI + 2) * RW;
-enum DField { DC0, DC1, DC2, DC3, DC4, DP, NDF };
-enum RField { RVBD, RANU, RANURT, RQ0, RQ1, RQ2, RQ3, RQ4, NRF };
-
-size_t diss_smem_bytes() {
-    return sizeof(double) * ((size_t)NDF * NDSLOT + (size_t)NRF * NRSLOT);
-}
+size_t diss_smem_bytes() { return sizeof(DissSmem<double>); }
 
 __device__ __forceinline__ double local_dt(const Params& P, double c1, double c2, double c3,
                                            double c4, double cfldl) {
@@ -500,128 +492,13 @@ __device__ __forceinline__ double local_dt(const Params& P, double c1, double c2
     return cfldl / (fabs(VEL) + sqrt(P.gamrr * T));
 }
 
-template <class OutT>
-__device__ __forceinline__ void dissipation_tile(const Params& P, const Mesh& M, const DissArgs<OutT>& A,
-                                                 int bx, int by) {
-    extern __shared__ double smem[];
-    double* sd = smem;                  // NDF x NDSLOT
-    double* sr = sd + NDF * NDSLOT;     // NRF x NRSLOT
-    const size_t ncell = (size_t)M.ni * M.nj;
-    const int j0 = bx * TJ, i0 = by * TI;
-    const int tid = threadIdx.y * TJ + threadIdx.x;
-
-    pdl_trigger();
-    pdl_wait();
-    for (int s = tid; s < NDSLOT; s += NTHREADS) {
-        const int i = i0 - 2 + s / DW, j = j0 - 2 + s % DW;
-        if (i >= 0 && i < M.ni && j >= 0 && j < M.nj) {
-            const size_t c = (size_t)i * M.nj + j;
-            double C[5];
-#pragma unroll
-            for (int m = 0; m < 5; m++) {
-                C[m] = A.q[m * ncell + c];
-                sd[(DC0 + m) * NDSLOT + s] = C[m];
-            }
-            // P as in the DT loop (turbnstwod.f90:98-104)
-            const double RHO = C[0];
-            const double rr = 1.0 / RHO;
-            const double U = C[1] * rr, V = C[2] * rr;
-            const double E = C[3] * rr;
-            const double T = (E - 0.5 * (U * U + V * V)) * P.inv_cv;
-            sd[DP * NDSLOT + s] = RHO * P.rr * T;
-        }
-    }
-    __syncthreads();
-
-    // ring-1 cells: VOL/DT, sensors, Laplacians (ghost neighbours read as the cell itself)
-    for (int s = tid; s < NRSLOT; s += NTHREADS) {
-        const int ri = s / RW, rj = s % RW;
-        const int i = i0 - 1 + ri, j = j0 - 1 + rj;
-        if (!(i >= 0 && i < M.ni && j >= 0 && j < M.nj)) continue;
-        const int d = (ri + 1) * DW + (rj + 1);  // same cell in the halo-2 grid
-        int nbs[4] = {d - 1, d + DW, d + 1, d - DW};
-        if (j == 0) nbs[0] = d;
-        if (i == M.ni - 1) nbs[1] = d;
-        if (j == M.nj - 1) nbs[2] = d;
-        if (i == 0) nbs[3] = d;
-        const double* Pp = sd + DP * NDSLOT;
-        const double* C5 = sd + DC4 * NDSLOT;
-        const double PIE = Pp[d], C1I = sd[DC0 * NDSLOT + d], C5I = C5[d];
-        double ANUN = fabs(Pp[nbs[0]] - PIE) + fabs(Pp[nbs[1]] - PIE) + fabs(Pp[nbs[2]] - PIE) +
-                      fabs(Pp[nbs[3]] - PIE);
-        double ANUD = fabs(Pp[nbs[0]] + PIE) + fabs(Pp[nbs[1]] + PIE) + fabs(Pp[nbs[2]] + PIE) +
-                      fabs(Pp[nbs[3]] + PIE);
-        sr[RANU * NRSLOT + s] = ANUN / ANUD;
-        ANUN = fabs(C5[nbs[0]] - C5I) + fabs(C5[nbs[1]] - C5I) + fabs(C5[nbs[2]] - C5I) +
-               fabs(C5[nbs[3]] - C5I);
-        ANUD = fabs(C5[nbs[0]] + C5I) + fabs(C5[nbs[1]] + C5I) + fabs(C5[nbs[2]] + C5I) +
-               fabs(C5[nbs[3]] + C5I);
-        sr[RANURT * NRSLOT + s] = ANUN / dmax1(ANUD, 8.0 * C1I * P.rtol);
-#pragma unroll
-        for (int m = 0; m < 5; m++) {
-            const double* Cm = sd + (DC0 + m) * NDSLOT;
-            sr[(RQ0 + m) * NRSLOT + s] = Cm[nbs[0]] + Cm[nbs[1]] + Cm[nbs[2]] + Cm[nbs[3]] - 4.0 * Cm[d];
-        }
-        // time step and VOL/DT
-        const size_t c = (size_t)i * M.nj + j;
-        double DT;
-        if (P.local) {
-            DT = local_dt(P, sd[DC0 * NDSLOT + d], sd[DC1 * NDSLOT + d], sd[DC2 * NDSLOT + d],
-                          sd[DC3 * NDSLOT + d], M.cfldl[c]);
-            if (ri >= 1 && ri <= TI && rj >= 1 && rj <= TJ) A.dt[c] = (OutT)DT;
-        } else {
-            DT = *A.dtmin;
-        }
-        sr[RVBD * NRSLOT + s] = M.cvol[c] / DT;
-    }
-    __syncthreads();
-
-    const int tj = threadIdx.x, ti = threadIdx.y;
-    const int i = i0 + ti, j = j0 + tj;
-    if (i >= M.ni || j >= M.nj) return;
-    const size_t cell = (size_t)i * M.nj + j;
-    const int r = (ti + 1) * RW + (tj + 1);
-    const int d = (ti + 2) * DW + (tj + 2);
-    const int rn[4] = {r - 1, r + RW, r + 1, r - RW};
-    const int dn[4] = {d - 1, d + DW, d + 1, d - DW};
-    const bool has[4] = {j > 0, i < M.ni - 1, j < M.nj - 1, i > 0};
-    const double VOLBYDT = sr[RVBD * NRSLOT + r];
-    // per-face blend coefficients (identical for the four equations)
-    double D2c[4], D4c[4], D2t[4], D4t[4];
-    const double ANUI = sr[RANU * NRSLOT + r], ANURTI = sr[RANURT * NRSLOT + r];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const double D24N = HALF * (VOLBYDT + sr[RVBD * NRSLOT + rn[k]]);
-        double E2N = C02 * dmax1(ANUI, sr[RANU * NRSLOT + rn[k]]);
-        double E4N = dmax1(0.0, C04 - E2N);
-        D2c[k] = E2N * D24N;
-        D4c[k] = E4N * D24N;
-        E2N = C02 * dmax1(ANURTI, sr[RANURT * NRSLOT + rn[k]]);
-        E4N = dmax1(0.0, C04 - E2N);
-        D2t[k] = E2N * D24N;
-        D4t[k] = E4N * D24N;
-    }
-#pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const double* Cm = sd + (DC0 + m) * NDSLOT;
-        const double* Qm = sr + (RQ0 + m) * NRSLOT;
-        const double CI = Cm[d], D2I = Qm[r];
-        double D2 = 0.0, D4 = 0.0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (!has[k]) continue;  // ghost face: exactly zero contribution
-            const double a2 = (m == 4) ? D2t[k] : D2c[k];
-            const double a4 = (m == 4) ? D4t[k] : D4c[k];
-            D2 = D2 + a2 * (Cm[dn[k]] - CI);
-            D4 = D4 + a4 * (Qm[rn[k]] - D2I);
-        }
-        A.d[m * ncell + cell] = (OutT)(D2 - D4);
-    }
+__device__ __forceinline__ void dissipation_tile_f64(const Params& P, const Mesh& M, const DissArgs<double>& A, int bx,
+                                                     int by) {
+    dissipation_tile(P, M, A, bx, by, [](const double*) {});
 }
 
-template <class OutT>
-__global__ void __launch_bounds__(NTHREADS) k_dissipation(Params P, Mesh M, DissArgs<OutT> A) {
-    dissipation_tile<OutT>(P, M, A, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MINB)) k_dissipation(Params P, Mesh M, DissArgs<double> A) {
+    dissipation_tile_f64(P, M, A, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------- time step min
@@ -896,13 +773,13 @@ void launch_face_states(const Params& P, const Mesh& M, const double* prim, doub
 
 // One launch per kernel advances every active case of a batch; block b works on tile
 // tiles[b] = (case, tile j, tile i) with its case's parameters and buffers.
-__global__ void __launch_bounds__(NTHREADS) k_dissipation_batch(const BatchCase* __restrict__ cases,
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MINB)) k_dissipation_batch(const BatchCase* __restrict__ cases,
                                                                 const int4* __restrict__ tiles,
                                                                 const int* __restrict__ active) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;  // whole block: before any barrier
     const BatchCase& c = cases[t.x];
-    dissipation_tile<double>(c.P, c.M, c.diss, t.y, t.z);
+    dissipation_tile_f64(c.P, c.M, c.diss, t.y, t.z);
 }
 
 __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_BATCH_MINB)) k_viscous_batch(const BatchCase* __restrict__ cases,
@@ -963,7 +840,7 @@ k_batch_persistent(const BatchCase* __restrict__ cases, const int4* __restrict__
                 const int4 t = tiles[w % ntiles];
                 if (active[t.x]) {
                     const BatchCase& c = cases[t.x];
-                    if (ph == 0 && w < ntiles) dissipation_tile<double>(c.P, c.M, c.diss, t.y, t.z);
+                    if (ph == 0 && w < ntiles) dissipation_tile_f64(c.P, c.M, c.diss, t.y, t.z);
                     else if (ph == 0) viscous_tile_f64(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
                     else stage_tile(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
                 }
@@ -1062,10 +939,7 @@ cudaError_t configure_kernels() {
     e = cudaFuncSetAttribute(k_viscous, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)visc_smem_bytes());
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_dissipation<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)diss_smem_bytes());
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_dissipation<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_dissipation, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)diss_smem_bytes());
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_dissipation_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1121,13 +995,7 @@ void launch_batch_f64(const BatchCase* cases, const int4* tiles, const int* acti
 void launch_dissipation(const Params& P, const Mesh& M, const double* q, double* d, double* dt,
                         const double* dtmin, cudaStream_t s) {
     DissArgs<double> A{q, d, dt, dtmin};
-    launch_tile(k_dissipation<double>, tile_grid(M), dim3(TJ, TI), diss_smem_bytes(), s, P, M, A);
-}
-
-void launch_dissipation_mx(const Params& P, const Mesh& M, const double* q, float* d, float* dt,
-                           const double* dtmin, cudaStream_t s) {
-    DissArgs<float> A{q, d, dt, dtmin};
-    launch_tile(k_dissipation<float>, tile_grid(M), dim3(TJ, TI), diss_smem_bytes(), s, P, M, A);
+    launch_tile(k_dissipation, tile_grid(M), dim3(TJ, TI), diss_smem_bytes(), s, P, M, A);
 }
 
 void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, unsigned int* error,

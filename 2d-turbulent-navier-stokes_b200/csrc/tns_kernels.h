@@ -73,8 +73,6 @@ size_t diss_mx_smem_bytes();
 cudaError_t configure_kernels_mx();
 void launch_dissipation_mx(const Params& P, const Mesh& M, const double* q, float* d, float* dt,
                            const double* dtmin, cudaStream_t s);
-void launch_dissipation_mx2(const Params& P, const Mesh& M, const double* q, float* d, float* dt,
-                            const double* dtmin, cudaStream_t s);
 void launch_viscous_mx(const Params& P, const Mesh& M, const double* q, float* vis, unsigned int* error,
                        cudaStream_t s);
 void launch_stage_mx(const Params& P, const Mesh& M, const double* cold, const float* dqin,

@@ -19,6 +19,7 @@
 #include "tns_mx.cuh"
 #include "tns_tile.cuh"
 #include "tns_batch.cuh"
+#include "tns_diss.cuh"
 #include "tns_visc.cuh"
 
 namespace tns {
@@ -388,144 +389,20 @@ k_viscous_mx(Params P, Mesh M, const double* __restrict__ q, float* __restrict__
 
 // ------------------------------------------------------------ dissipation kernel
 
-// JST dissipation (solver_state.f90:70-225) with FP64 state, pressure and every
-// difference of the state, FP32 sensors, Laplacian differences and blend.
-constexpr int DWM = TJ + 4;
-constexpr int NDSLOTM = (TI + 4) * DWM;
-constexpr int RWM = TJ + 2;
-constexpr int NRSLOTM = (TI + 2) * RWM;
-
-struct DissSmemMx {
-    double c[5][NDSLOTM];
-    double p[NDSLOTM];
-    float vbd[NRSLOTM], anu[NRSLOTM], anurt[NRSLOTM], d2q[5][NRSLOTM];
-};
-
-size_t diss_mx_smem_bytes() { return sizeof(DissSmemMx); }
-
-__device__ __forceinline__ double local_dt_mx(const Params& P, double c1, double c2, double c3,
-                                              double c4, double cfldl) {
-    const double rr = 1.0 / c1;
-    const double U = c2 * rr, V = c3 * rr;
-    const double VEL = sqrt(U * U + V * V);
-    const double E = c4 * rr;
-    const double T = (E - 0.5 * (U * U + V * V)) * P.inv_cv;
-    return cfldl / (fabs(VEL) + sqrt(P.gamrr * T));
-}
+size_t diss_mx_smem_bytes() { return sizeof(DissSmem<float>); }
 
 __device__ __forceinline__ void dissipation_mx_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                     float* __restrict__ dout, float* __restrict__ dtout,
                                                     const double* __restrict__ dtmin, int bx, int by) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    DissSmemMx& S = *reinterpret_cast<DissSmemMx*>(smem_raw);
-    const size_t ncell = (size_t)M.ni * M.nj;
-    const int j0 = bx * TJ, i0 = by * TI;
-    const int tid = threadIdx.y * TJ + threadIdx.x;
-    pdl_trigger();
-    pdl_wait();
-    for (int s = tid; s < NDSLOTM; s += NTHREADS) {
-        const int i = i0 - 2 + s / DWM, j = j0 - 2 + s % DWM;
-        if (i >= 0 && i < M.ni && j >= 0 && j < M.nj) {
-            const size_t c = (size_t)i * M.nj + j;
-            double C[5];
-#pragma unroll
-            for (int m = 0; m < 5; m++) {
-                C[m] = q[m * ncell + c];
-                S.c[m][s] = C[m];
-            }
-            const double rr = 1.0 / C[0];
-            const double U = C[1] * rr, V = C[2] * rr;
-            const double T = (C[3] * rr - 0.5 * (U * U + V * V)) * P.inv_cv;
-            S.p[s] = C[0] * P.rr * T;
-        }
-    }
-    __syncthreads();
-    for (int s = tid; s < NRSLOTM; s += NTHREADS) {
-        const int ri = s / RWM, rj = s % RWM;
-        const int i = i0 - 1 + ri, j = j0 - 1 + rj;
-        if (!(i >= 0 && i < M.ni && j >= 0 && j < M.nj)) continue;
-        const int d = (ri + 1) * DWM + (rj + 1);
-        int nbs[4] = {d - 1, d + DWM, d + 1, d - DWM};
-        if (j == 0) nbs[0] = d;
-        if (i == M.ni - 1) nbs[1] = d;
-        if (j == M.nj - 1) nbs[2] = d;
-        if (i == 0) nbs[3] = d;
-        const double PIE = S.p[d], C5I = S.c[4][d];
-        double an = 0.0, ad = 0.0, rn = 0.0, rd = 0.0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            an += fabs(S.p[nbs[k]] - PIE);
-            ad += fabs(S.p[nbs[k]] + PIE);
-            rn += fabs(S.c[4][nbs[k]] - C5I);
-            rd += fabs(S.c[4][nbs[k]] + C5I);
-        }
-        S.anu[s] = (float)an / (float)ad;
-        S.anurt[s] = (float)rn / (float)fmax(rd, 8.0 * S.c[0][d] * P.rtol);
-#pragma unroll
-        for (int m = 0; m < 5; m++)
-            S.d2q[m][s] = (float)(S.c[m][nbs[0]] + S.c[m][nbs[1]] + S.c[m][nbs[2]] + S.c[m][nbs[3]] - 4.0 * S.c[m][d]);
-        const size_t c = (size_t)i * M.nj + j;
-        double DT;
-        if (P.local) {
-            DT = local_dt_mx(P, S.c[0][d], S.c[1][d], S.c[2][d], S.c[3][d], M.cfldl[c]);
-            if (ri >= 1 && ri <= TI && rj >= 1 && rj <= TJ) dtout[c] = (float)DT;
-        } else {
-            DT = *dtmin;
-        }
-        S.vbd[s] = (float)(M.cvol[c] / DT);
-    }
-    if (tid == NTHREADS - 1) {
-        // the tile's reference state for this iteration's stages (its first cell), by the
-        // last warp, which has no second ring slot to wait for
-        const int d0 = 2 * DWM + 2;
-        const double c[5] = {S.c[0][d0], S.c[1][d0], S.c[2][d0], S.c[3][d0], S.c[4][d0]};
+    // with the tile's reference state for this iteration's stages
+    dissipation_tile(P, M, DissArgs<float>{q, dout, dtout, dtmin}, bx, by, [&](const double* c) {
         make_tile_ref(P, c, M.tref[(size_t)by * ((M.nj + TJ - 1) / TJ) + bx]);
-    }
-    __syncthreads();
-    const int tj = threadIdx.x, ti = threadIdx.y;
-    const int i = i0 + ti, j = j0 + tj;
-    if (i >= M.ni || j >= M.nj) return;
-    const size_t cell = (size_t)i * M.nj + j;
-    const int r = (ti + 1) * RWM + (tj + 1);
-    const int d = (ti + 2) * DWM + (tj + 2);
-    const int rn[4] = {r - 1, r + RWM, r + 1, r - RWM};
-    const int dn[4] = {d - 1, d + DWM, d + 1, d - DWM};
-    const bool has[4] = {j > 0, i < M.ni - 1, j < M.nj - 1, i > 0};
-    const float VOLBYDT = S.vbd[r];
-    float D2c[4], D4c[4], D2t[4], D4t[4];
-    const float ANUI = S.anu[r], ANURTI = S.anurt[r];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const float D24N = 0.5f * (VOLBYDT + S.vbd[rn[k]]);
-        float E2N = (float)C02 * fmaxf(ANUI, S.anu[rn[k]]);
-        float E4N = fmaxf(0.0f, (float)C04 - E2N);
-        D2c[k] = E2N * D24N;
-        D4c[k] = E4N * D24N;
-        E2N = (float)C02 * fmaxf(ANURTI, S.anurt[rn[k]]);
-        E4N = fmaxf(0.0f, (float)C04 - E2N);
-        D2t[k] = E2N * D24N;
-        D4t[k] = E4N * D24N;
-    }
-#pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const double CI = S.c[m][d];
-        const float D2I = S.d2q[m][r];
-        float D2 = 0.0f, D4 = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (!has[k]) continue;
-            const float a2 = (m == 4) ? D2t[k] : D2c[k];
-            const float a4 = (m == 4) ? D4t[k] : D4c[k];
-            D2 += a2 * (float)(S.c[m][dn[k]] - CI);
-            D4 += a4 * (S.d2q[m][rn[k]] - D2I);
-        }
-        dout[m * ncell + cell] = D2 - D4;
-    }
+    });
 }
 
-__global__ void __launch_bounds__(NTHREADS) k_dissipation_mx(Params P, Mesh M, const double* __restrict__ q,
-                                                             float* __restrict__ dout, float* __restrict__ dtout,
-                                                             const double* __restrict__ dtmin) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MX_MINB))
+k_dissipation_mx(Params P, Mesh M, const double* __restrict__ q, float* __restrict__ dout, float* __restrict__ dtout,
+                 const double* __restrict__ dtmin) {
     dissipation_mx_tile(P, M, q, dout, dtout, dtmin, blockIdx.x, blockIdx.y);
 }
 
@@ -606,7 +483,7 @@ __global__ void k_prim_out_mx(Params P, Mesh M, const double* __restrict__ cold,
 
 // Mixed-path batch: `parity` selects which of qa / qa2 holds each active case's state
 // (all active cases advance together, so they share it).
-__global__ void __launch_bounds__(NTHREADS) k_dissipation_mx_batch(const BatchCase* __restrict__ cases,
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MX_MINB)) k_dissipation_mx_batch(const BatchCase* __restrict__ cases,
                                                                    const int4* __restrict__ tiles,
                                                                    const int* __restrict__ active, int parity) {
     const int4 t = tiles[blockIdx.x];
@@ -742,7 +619,7 @@ void launch_batch_mx(const BatchCase* cases, const int4* tiles, const int* activ
                     monitor);
 }
 
-void launch_dissipation_mx2(const Params& P, const Mesh& M, const double* q, float* d, float* dt,
+void launch_dissipation_mx(const Params& P, const Mesh& M, const double* q, float* d, float* dt,
                             const double* dtmin, cudaStream_t s) {
     launch_tile(k_dissipation_mx, tile_grid_mx(M), dim3(TJ, TI), diss_mx_smem_bytes(), s, P, M, q, d, dt, dtmin);
 }

@@ -26,6 +26,12 @@ namespace tns {
 #ifndef TNS_VISC_BATCH_MINB
 #define TNS_VISC_BATCH_MINB 1  // descriptor-fed arguments spill at 3 blocks/SM
 #endif
+#ifndef TNS_DISS_MINB
+#define TNS_DISS_MINB 4
+#endif
+#ifndef TNS_DISS_MX_MINB
+#define TNS_DISS_MX_MINB 4
+#endif
 // Resident blocks per SM of a kernel tuned at TI = 8, for the compiled TI: the same
 // threads per SM at every tile height.
 #define TNS_PER_SM(n) ((n) * 8 / TNS_TI > 0 ? (n) * 8 / TNS_TI : 1)
