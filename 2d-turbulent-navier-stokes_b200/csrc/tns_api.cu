@@ -374,6 +374,30 @@ int upload_mesh(tns_handle* h) {
         (rc = up(h->bnode.p, h->hbnode.data(), h->hbnode.size() * 4)))
         return rc;
     // the host copies are not read again
+    // weights of the port sums (boundary.f90:183-214), where there are ports along j or i
+    if (!h->port_ghosts.empty()) {
+        const int ni = h->ni, nj = h->nj;
+        bool along_j = false, along_i = false;
+        for (int g : h->port_ghosts) {
+            const bool row = g < ni || (g >= ni + nj && g < 2 * ni + nj);
+            along_j |= row;
+            along_i |= !row;
+        }
+        std::vector<double> w(ncell);
+        for (int dir = 0; dir < 2; dir++) {
+            if (dir == 0 ? !along_j : !along_i) continue;
+            for (int i = 0; i < ni; i++)
+                for (int j = 0; j < nj; j++) {
+                    const size_t n1 = (size_t)i * (nj + 1) + j;
+                    const double y1 = h->hY[n1], y2 = h->hY[n1 + nj + 1], y3 = h->hY[n1 + nj + 2], y4 = h->hY[n1 + 1];
+                    double v = dir == 0 ? tns::HALF * ((y3 + y4) - (y1 + y2)) : tns::HALF * ((y2 + y3) - (y1 + y4));
+                    if (h->P.iaxis == 1) v = v * ((y1 + y2 + y3 + y4) * 0.25);
+                    w[(size_t)i * nj + j] = v;
+                }
+            DevBuf<double>& d = dir == 0 ? h->wport : h->wport_i;
+            if ((rc = h->cuda(d.alloc(ncell), "cudaMalloc")) || (rc = up(d.p, w.data(), ncell * 8))) return rc;
+        }
+    }
     // static ghost records
     {
         const int ni = h->ni, nj = h->nj;
@@ -400,6 +424,8 @@ int upload_mesh(tns_handle* h) {
     M.ni = h->ni; M.nj = h->nj; M.x = h->x.p; M.y = h->y.p; M.cfldl = h->cfldl.p; M.gtype = h->gtype.p;
     M.grank = h->grank.p; M.gxc = h->gxc.p; M.gyc = h->gyc.p; M.ginj = h->ginj.p;
     M.gport = h->gport.p;
+    M.wport = h->wport.p;
+    M.wport_i = h->wport_i.p;
     M.grec = h->grec.p;
     M.cvol = h->cvol.p;
     M.vcfl = h->vcfl.p;
@@ -1184,7 +1210,7 @@ void tns_destroy(tns_handle* h) {
     h->qa2.release(); h->dqb.release(); h->dqc.release(); h->df.release(); h->visf.release();
     h->dtf.release(); h->tref.release();
     for (auto* b : {&h->x, &h->y, &h->cfldl, &h->gxc, &h->gyc, &h->ginj, &h->gport, &h->qa, &h->qb,
-                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->vcfl, &h->e,
+                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->vcfl, &h->e, &h->wport, &h->wport_i,
                     &h->stile, &h->vtile})
         b->release();
     h->grec.release(); h->bnode.release(); h->gtype.release(); h->grank.release(); h->ports.release();

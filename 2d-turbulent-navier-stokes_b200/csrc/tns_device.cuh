@@ -93,6 +93,9 @@ struct Mesh {
     const GhostRec* grec;   // static geometry per ghost
     const double* ginj;     // type-6 burn-rate multiplier
     const double* gport;    // type-6 port mass flux of the current stage
+    // weights DELY(*YCC) of the port sums per cell (null without such ports): of side 3, along
+    // j, and of side 2, along i
+    const double *wport, *wport_i;
     const double* cvol;     // VOL per cell (geometry.f90:87,98,101)
     const double* vcfl;     // VOL / (CFL*DL) per cell
     const double* stile;    // static data of the stage tiles, one block per tile (tns_tile.cuh)

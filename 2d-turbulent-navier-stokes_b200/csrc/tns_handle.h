@@ -63,7 +63,7 @@ struct tns_handle {
     cudaEvent_t fork = nullptr, join = nullptr;
     // e: the iteration's frozen terms VIS + D, formed by stage 1 (FP64, structured meshes)
     DevBuf<double> x, y, cfldl, gxc, gyc, ginj, gport, qa, qb, qc, d, vis, e, dt, dtmin, partial,
-        primout, cvol, vcfl, stile, vtile;
+        primout, cvol, vcfl, stile, vtile, wport, wport_i;
     // mixed FP32/FP64 path: FP64 state ping-pong (qa, qa2) and FP32 scratch
     int precision = 0;
     int cur = 0;  // mixed: which of qa / qa2 holds the state

@@ -227,7 +227,9 @@ __device__ __forceinline__ void stage_cdiff(const StageArgs& A, const double dv[
 }
 
 // One RK stage (turbnstwod.f90:204-227, boundary.f90:24-48, source_terms.f90:24-104,
-// residual.f90:23-83) on a TI x TJ tile with its halo staged in shared memory.
+// residual.f90:23-83) on a TI x TJ tile with its halo staged in shared memory.  RIM: the block
+// has RIM_ROWS more rows of threads, which evaluate the halo.
+template <bool RIM>
 __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const StageArgs& A, int bx, int by) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StageSmem& S = *reinterpret_cast<StageSmem*>(smem_raw);
@@ -245,15 +247,16 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
     // a tile whose halo holds no ghost (and which is full) needs no classification
     const bool inner = i0 > 0 && j0 > 0 && i0 + TI < M.ni && j0 + TJ < M.nj;
     const int i = i0 + ti, j = j0 + tj;
-    const bool valid = i < M.ni && j < M.nj;
+    const bool valid = (!RIM || ti < TI) && i < M.ni && j < M.nj;
+    const int rt = RIM ? tid - NTHREADS : tid;  // the thread's place on the ring
     // the ring around the tile's cells; a ghost's type and geometry are static too
     const int ri = inner ? TI : min(TI, M.ni - i0), rj = inner ? TJ : min(TJ, M.nj - j0);
     HaloPos h;
     h.kind = -1;
     GhostSite site{0, 0.0, 0.0, 0.0, 0.0};
-    if (tid < 2 * (ri + rj + 2)) {
+    if (rt >= 0 && rt < 2 * (ri + rj + 2)) {
         int li, lj;
-        ring_slot(tid, ri, rj, li, lj);
+        ring_slot(rt, ri, rj, li, lj);
         h = halo_pos(M, inner, i0, j0, li, lj);
         if (h.kind > 0) site = ghost_site(M, h.g);
     }
@@ -298,12 +301,13 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
 }
 
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
-// runs.
-template <int MONITOR>
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MINB)) k_stage(Params P, Mesh M, StageArgs A) {
+// runs, and on the extra rows of threads.
+template <int MONITOR, bool RIM>
+__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), TNS_PER_SM(RIM ? 2 : TNS_STAGE_MINB))
+k_stage(Params P, Mesh M, StageArgs A) {
     StageArgs Ac = A;
     if (!MONITOR) Ac.cdiff = nullptr;
-    stage_tile(P, M, Ac, blockIdx.x, blockIdx.y);
+    stage_tile<RIM>(P, M, Ac, blockIdx.x, blockIdx.y);
 }
 
 // Stages 2-4 of a large mesh, by resident blocks that walk its tiles (tile t, t + grid, ...)
@@ -369,7 +373,6 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
         tensor_copy_3d(W.op[SO_QOLD], &maps.qold, j0, i0, 0, &W.bar_c);
         if (P.local) tensor_copy_3d(W.op[SO_DT], &maps.dt, j0, i0, 0, &W.bar_c);
     };
-    pdl_trigger();
     if (tid == 0) {
         bulk_barrier_init(&W.bar_a);
         bulk_barrier_init(&W.bar_b);
@@ -428,6 +431,9 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
             return;
         }
         const int next = t + gridDim.x;
+        // the next kernel's blocks may start once all of these are on their last tile (asked
+        // for at the start they take an SM's slots early: 0.122 -> 0.125 ms an iteration)
+        if (next >= ntiles) pdl_trigger();
         if (tid == 0 && next < ntiles) fetch_a(next);
         if (valid) {
             double d[5];
@@ -464,16 +470,18 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
 
 size_t visc_smem_bytes() { return sizeof(ViscSmem); }
 
+template <bool RIM>
 __device__ __forceinline__ void viscous_tile_f64(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                  double* __restrict__ vis, unsigned int* error, int bx, int by) {
-    viscous_tile(P, M, q, vis, error, bx, by,
+    viscous_tile<RIM>(P, M, q, vis, error, bx, by,
                  [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
                      double out[4]) { viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
 
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_MINB))
+template <bool RIM>
+__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), TNS_PER_SM(RIM ? 2 : TNS_VISC_MINB))
 k_viscous(Params P, Mesh M, const double* __restrict__ q, double* __restrict__ vis, unsigned int* error) {
-    viscous_tile_f64(P, M, q, vis, error, blockIdx.x, blockIdx.y);
+    viscous_tile_f64<RIM>(P, M, q, vis, error, blockIdx.x, blockIdx.y);
 }
 
 // --------------------------------------------------------- dissipation kernel
@@ -503,75 +511,88 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MINB)) k_dissipa
 
 // ------------------------------------------------------------- time step min
 
-__global__ void __launch_bounds__(256)
-k_dtmin(Params P, Mesh M, const double* __restrict__ q, double* dt, double* partial,
-        unsigned int* counter, double* dtmin) {
-    const size_t ncell = (size_t)M.ni * M.nj;
-    double mn = 100000.0;
-    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < ncell;
-         c += (size_t)gridDim.x * blockDim.x) {
-        const double v = local_dt(P, q[c], q[ncell + c], q[2 * ncell + c], q[3 * ncell + c],
-                                  M.cfldl[c]);
-        mn = dmin1(mn, v);
+// The time step of up to STEP_UNROLL cells a thread, a block apart: all their loads are on
+// their way before the first is used (a grid of one load round at a time was bound by their
+// latency).
+constexpr int STEP_UNROLL = 4;
+template <class Store>
+__device__ __forceinline__ double step_min(const Params& P, const double* __restrict__ q,
+                                           const double* __restrict__ cfldl, long long ncell, long long first,
+                                           long long stride, double mn, Store store) {
+    for (; first < ncell; first += STEP_UNROLL * stride) {
+        double c[STEP_UNROLL][5];
+#pragma unroll
+        for (int k = 0; k < STEP_UNROLL; k++) {
+            const long long i = first + k * stride;
+            if (i < ncell) {
+#pragma unroll
+                for (int m = 0; m < 4; m++) c[k][m] = q[m * ncell + i];
+                c[k][4] = cfldl[i];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < STEP_UNROLL; k++) {
+            const long long i = first + k * stride;
+            if (i < ncell) {
+                const double v = local_dt(P, c[k][0], c[k][1], c[k][2], c[k][3], c[k][4]);
+                store(i, v);
+                mn = dmin1(mn, v);
+            }
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    return mn;
+}
+
+// Minimum over the grid: a partial per block, and the block that finishes last reduces them
+// with all its threads (one thread reading them in turn took most of the kernel: 65 -> 21 us
+// for the time step of 1.57 M cells).  `partial`: one double per block; `counter`: zero on
+// entry, left at zero.
+__device__ __forceinline__ void grid_min(double mn, double* partial, unsigned int* counter, double* dtmin) {
     __shared__ double wmin[8];
     __shared__ bool last;
-    if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = mn;
-    __syncthreads();
+    auto block_min = [&](double v) {
+        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = v;
+        __syncthreads();
+        v = wmin[0];
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) v = fmin(v, wmin[w]);
+        return v;
+    };
+    const double b = block_min(mn);
     if (threadIdx.x == 0) {
-        double b = wmin[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) b = fmin(b, wmin[w]);
         partial[blockIdx.x] = b;
         __threadfence();
-        const unsigned int done = atomicAdd(counter, 1u);
-        last = (done == gridDim.x - 1);
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        double b = 100000.0;
-        for (unsigned int k = 0; k < gridDim.x; k++) b = fmin(b, ((volatile double*)partial)[k]);
-        *dtmin = b;
+    if (!last) return;
+    __threadfence();
+    double v = 100000.0;
+    for (unsigned int k = threadIdx.x; k < gridDim.x; k += blockDim.x) v = fmin(v, ((volatile double*)partial)[k]);
+    v = block_min(v);
+    if (threadIdx.x == 0) {
+        *dtmin = v;
         *counter = 0u;
     }
 }
 
+__global__ void __launch_bounds__(256)
+k_dtmin(Params P, Mesh M, const double* __restrict__ q, double* partial, unsigned int* counter, double* dtmin) {
+    const long long ncell = (long long)M.ni * M.nj;
+    const double mn = step_min(P, q, M.cfldl, ncell, blockIdx.x * 256LL + threadIdx.x, gridDim.x * 256LL, 100000.0,
+                               [](long long, double) {});
+    grid_min(mn, partial, counter, dtmin);
+}
+
 // Variant of k_dtmin for caller-provided device buffers (tns_time_step_noalloc): also
-// stores the per-cell DT, and reduces through the scratch the launcher is handed
-// (`partial`: one double per block, `counter`: zero on entry, left at zero on exit).
+// stores the per-cell DT, and reduces through the scratch the launcher is handed.
 __global__ void __launch_bounds__(256)
 k_time_step_scratch(Params P, const double* __restrict__ q, const double* __restrict__ cfldl,
                     long long ncell, double* __restrict__ dt, double* partial,
                     unsigned int* counter, double* dtmin) {
-    double mn = 100000.0;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncell;
-         c += (long long)gridDim.x * blockDim.x) {
-        const double v = local_dt(P, q[c], q[ncell + c], q[2 * ncell + c], q[3 * ncell + c],
-                                  cfldl[c]);
-        dt[c] = v;
-        mn = dmin1(mn, v);
-    }
-    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    __shared__ double wmin[8];
-    __shared__ bool last;
-    if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = mn;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double b = wmin[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) b = fmin(b, wmin[w]);
-        partial[blockIdx.x] = b;
-        __threadfence();
-        last = (atomicAdd(counter, 1u) == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        double b = 100000.0;
-        for (unsigned int k = 0; k < gridDim.x; k++) b = fmin(b, ((volatile double*)partial)[k]);
-        *dtmin = b;
-        *counter = 0u;
-    }
+    const double mn = step_min(P, q, cfldl, ncell, blockIdx.x * 256LL + threadIdx.x, gridDim.x * 256LL, 100000.0,
+                               [&](long long i, double v) { dt[i] = v; });
+    grid_min(mn, partial, counter, dtmin);
 }
 
 void launch_time_step_scratch(const Params& P, const double* q, const double* cfldl,
@@ -583,50 +604,10 @@ void launch_time_step_scratch(const Params& P, const double* q, const double* cf
 
 // ------------------------------------------------------------ port mass flux
 
-// One block per type-6 ghost: sum of C1*U*DELY(*YCC) along the mesh line through the
-// parent, across to the opposite boundary (the repaired GPORT walk); its threads stride
-// the line, then a warp and block reduction in fixed order.
-__global__ void k_gport(Params P, Mesh M, const double* __restrict__ q, const int* ghosts,
-                        int nport, double* gport) {
-    const int w = blockIdx.x;  // one block per port ghost
-    const int lane = threadIdx.x & 31;
-    if (w >= nport) return;  // whole block
-    const size_t ncell = (size_t)M.ni * M.nj;
-    const int g = ghosts[w];
-    int side, along;
-    if (g < M.ni) { side = 1; along = g; }
-    else if (g < M.ni + M.nj) { side = 2; along = g - M.ni; }
-    else if (g < 2 * M.ni + M.nj) { side = 3; along = g - M.ni - M.nj; }
-    else { side = 4; along = g - 2 * M.ni - M.nj; }
-    const int len = (side == 1 || side == 3) ? M.nj : M.ni;
-    double sum = 0.0;
-    for (int k = threadIdx.x; k < len; k += GP_THREADS) {
-        const int i = (side == 1 || side == 3) ? along : k;
-        const int j = (side == 1 || side == 3) ? k : along;
-        const size_t c = (size_t)i * M.nj + j;
-        const size_t n1 = (size_t)i * (M.nj + 1) + j;
-        const double y1 = M.y[n1], y2 = M.y[n1 + M.nj + 1], y3 = M.y[n1 + M.nj + 2],
-                     y4 = M.y[n1 + 1];
-        double dely;
-        if (side == 1) dely = HALF * ((y1 + y2) - (y3 + y4));
-        else if (side == 2) dely = HALF * ((y2 + y3) - (y1 + y4));
-        else if (side == 3) dely = HALF * ((y3 + y4) - (y1 + y2));
-        else dely = HALF * ((y4 + y1) - (y2 + y3));
-        const double c1 = q[c], u = q[ncell + c] / c1;
-        double term = c1 * u * dely;
-        if (P.iaxis == 1) term = term * ((y1 + y2 + y3 + y4) * 0.25);
-        sum += term;
-    }
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    __shared__ double part[GP_THREADS / 32];
-    if (lane == 0) part[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = part[0];
-#pragma unroll
-        for (int k = 1; k < GP_THREADS / 32; k++) t += part[k];
-        gport[g] = t;
-    }
+// One block per type-6 ghost (port_line, tns_tile.cuh).
+__global__ void __launch_bounds__(GP_THREADS) k_gport(Params P, Mesh M, const double* __restrict__ q,
+                                                      const int* ghosts, double* gport) {
+    port_line(M, StateF64{q, (size_t)M.ni * M.nj}, ghosts, gport);
 }
 
 // ------------------------------------------------------ primitive output
@@ -788,7 +769,7 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_BATCH_MINB)) k_v
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;
     const BatchCase& c = cases[t.x];
-    viscous_tile_f64(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
+    viscous_tile_f64<false>(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
 }
 
 __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_BATCH_MINB)) k_stage_batch(const BatchCase* __restrict__ cases,
@@ -812,9 +793,9 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_BATCH_MINB)) k_
         copy_words(&sA, &c.stage[monitor][stage], sizeof(StageArgs), tid);
         __syncthreads();
     }
-    stage_tile(sP, sM, sA, t.y, t.z);
+    stage_tile<false>(sP, sM, sA, t.y, t.z);
 #else
-    stage_tile(c.P, c.M, c.stage[monitor][stage], t.y, t.z);
+    stage_tile<false>(c.P, c.M, c.stage[monitor][stage], t.y, t.z);
 #endif
 }
 
@@ -841,8 +822,8 @@ k_batch_persistent(const BatchCase* __restrict__ cases, const int4* __restrict__
                 if (active[t.x]) {
                     const BatchCase& c = cases[t.x];
                     if (ph == 0 && w < ntiles) dissipation_tile_f64(c.P, c.M, c.diss, t.y, t.z);
-                    else if (ph == 0) viscous_tile_f64(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
-                    else stage_tile(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
+                    else if (ph == 0) viscous_tile_f64<false>(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
+                    else stage_tile<false>(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
                 }
                 async_proxy_fence();
                 __syncthreads();
@@ -876,7 +857,7 @@ void launch_debug_math(int fn, long long n, const double* a, const double* b, do
 static dim3 tile_grid(const Mesh& M) { return dim3((M.nj + TJ - 1) / TJ, (M.ni + TI - 1) / TI); }
 
 // SMs of the current device, and the pipelined stage's resident blocks on all of them.
-static int sm_count() {
+int sm_count() {
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 148;
@@ -924,21 +905,20 @@ static bool stage_maps(const Params& P, const Mesh& M, const StageArgs& A, Stage
 
 cudaError_t configure_kernels() {
     cudaError_t e;
-    e = cudaFuncSetAttribute(k_stage<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)stage_smem_bytes());
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_stage<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)stage_smem_bytes());
-    if (e != cudaSuccess) return e;
+    for (auto k : {k_stage<0, false>, k_stage<1, false>, k_stage<0, true>, k_stage<1, true>}) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem_bytes());
+        if (e != cudaSuccess) return e;
+    }
     e = cudaFuncSetAttribute(k_stage_pipe<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)PIPE_SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_stage_pipe<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)PIPE_SMEM);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_viscous, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)visc_smem_bytes());
-    if (e != cudaSuccess) return e;
+    for (auto k : {k_viscous<false>, k_viscous<true>}) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)visc_smem_bytes());
+        if (e != cudaSuccess) return e;
+    }
     e = cudaFuncSetAttribute(k_dissipation, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)diss_smem_bytes());
     if (e != cudaSuccess) return e;
@@ -1000,7 +980,14 @@ void launch_dissipation(const Params& P, const Mesh& M, const double* q, double*
 
 void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, unsigned int* error,
                     cudaStream_t s) {
-    launch_tile(k_viscous, tile_grid(M), dim3(TJ, TI), visc_smem_bytes(), s, P, M, q, vis, error);
+    const dim3 grid = tile_grid(M);
+    // the rim rows shorten one tile's chain (115 x 50 nozzle: 22.8 -> 22.2 us an iteration,
+    // 192 x 64: 24.2 -> 22.2) but leave room for two blocks an SM instead of three (400 x 160,
+    // 250 tiles: 28.0 -> 29.9)
+    if ((int)(grid.x * grid.y) <= TNS_VISC_RIM_PER_SM * sm_count())
+        launch_tile(k_viscous<true>, grid, dim3(TJ, TI + RIM_ROWS), visc_smem_bytes(), s, P, M, q, vis, error);
+    else
+        launch_tile(k_viscous<false>, grid, dim3(TJ, TI), visc_smem_bytes(), s, P, M, q, vis, error);
 }
 
 void launch_stage(const Params& P, const Mesh& M, const double* qin, const double* qold,
@@ -1018,7 +1005,13 @@ void launch_stage(const Params& P, const Mesh& M, const double* qin, const doubl
                     maps);
         return;
     }
-    launch_tile(cdiff ? k_stage<1> : k_stage<0>, grid, dim3(TJ, TI), stage_smem_bytes(), s, P, M, A);
+    // the rim rows while every tile has its own resident block of that size: 115 x 50 nozzle,
+    // an iteration, 22.7 -> 22.2 us; 400 x 160 ramp (250 tiles) 31.2 -> 28.0
+    if (ntiles <= TNS_STAGE_RIM_PER_SM * sm_count())
+        launch_tile(cdiff ? k_stage<1, true> : k_stage<0, true>, grid, dim3(TJ, TI + RIM_ROWS), stage_smem_bytes(), s, P,
+                    M, A);
+    else
+        launch_tile(cdiff ? k_stage<1, false> : k_stage<0, false>, grid, dim3(TJ, TI), stage_smem_bytes(), s, P, M, A);
 }
 
 int dtmin_blocks(const Mesh& M) {
@@ -1029,13 +1022,13 @@ int dtmin_blocks(const Mesh& M) {
 
 void launch_dtmin(const Params& P, const Mesh& M, const double* q, double* partial,
                   unsigned int* counter, double* dtmin, cudaStream_t s) {
-    k_dtmin<<<dtmin_blocks(M), 256, 0, s>>>(P, M, q, nullptr, partial, counter, dtmin);
+    k_dtmin<<<dtmin_blocks(M), 256, 0, s>>>(P, M, q, partial, counter, dtmin);
 }
 
 void launch_gport(const Params& P, const Mesh& M, const double* q, const int* ghosts, int nport,
                   double* gport, cudaStream_t s) {
     if (nport <= 0) return;
-    k_gport<<<nport, GP_THREADS, 0, s>>>(P, M, q, ghosts, nport, gport);
+    launch_tile(k_gport, dim3(nport), dim3(GP_THREADS), 0, s, P, M, q, ghosts, gport);
 }
 
 void launch_node_average(const Mesh& M, const double* prim, double* out, cudaStream_t s) {

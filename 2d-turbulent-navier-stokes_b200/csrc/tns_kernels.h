@@ -14,6 +14,7 @@ size_t stage_smem_bytes();
 size_t visc_smem_bytes();
 size_t diss_smem_bytes();
 int dtmin_blocks(const Mesh& M);
+int sm_count();  // SMs of the current device
 
 void launch_dissipation(const Params& P, const Mesh& M, const double* q, double* d, double* dt,
                         const double* dtmin, cudaStream_t s);

@@ -377,7 +377,7 @@ __device__ __forceinline__ void viscous_face_mx(const Params& P, const FaceVals&
 
 __device__ __forceinline__ void viscous_mx_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                 float* __restrict__ vis, unsigned int* error, int bx, int by) {
-    viscous_tile(P, M, q, vis, error, bx, by,
+    viscous_tile<false>(P, M, q, vis, error, bx, by,
                  [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
                      double out[4]) { viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
@@ -408,48 +408,10 @@ k_dissipation_mx(Params P, Mesh M, const double* __restrict__ q, float* __restri
 
 // ------------------------------------------------------------ port mass flux
 
-__global__ void k_gport_mx(Params P, Mesh M, const double* __restrict__ cold,
-                           const float* __restrict__ dq, const int* ghosts, int nport,
-                           double* gport) {
-    const int w = blockIdx.x;  // one block per port ghost
-    const int lane = threadIdx.x & 31;
-    if (w >= nport) return;  // whole block
-    const size_t ncell = (size_t)M.ni * M.nj;
-    const StateMixed st{cold, dq, ncell};
-    const int g = ghosts[w];
-    int side, along;
-    if (g < M.ni) { side = 1; along = g; }
-    else if (g < M.ni + M.nj) { side = 2; along = g - M.ni; }
-    else if (g < 2 * M.ni + M.nj) { side = 3; along = g - M.ni - M.nj; }
-    else { side = 4; along = g - 2 * M.ni - M.nj; }
-    const int len = (side == 1 || side == 3) ? M.nj : M.ni;
-    double sum = 0.0;
-    for (int k = threadIdx.x; k < len; k += GP_THREADS) {
-        const int i = (side == 1 || side == 3) ? along : k;
-        const int j = (side == 1 || side == 3) ? k : along;
-        const size_t c = (size_t)i * M.nj + j;
-        const size_t n1 = (size_t)i * (M.nj + 1) + j;
-        const double y1 = M.y[n1], y2 = M.y[n1 + M.nj + 1], y3 = M.y[n1 + M.nj + 2], y4 = M.y[n1 + 1];
-        double dely;
-        if (side == 1) dely = HALF * ((y1 + y2) - (y3 + y4));
-        else if (side == 2) dely = HALF * ((y2 + y3) - (y1 + y4));
-        else if (side == 3) dely = HALF * ((y3 + y4) - (y1 + y2));
-        else dely = HALF * ((y4 + y1) - (y2 + y3));
-        const double c1 = st.c(0, c), u = st.c(1, c) / c1;
-        double term = c1 * u * dely;
-        if (P.iaxis == 1) term = term * ((y1 + y2 + y3 + y4) * 0.25);
-        sum += term;
-    }
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    __shared__ double part[GP_THREADS / 32];
-    if (lane == 0) part[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = part[0];
-#pragma unroll
-        for (int k = 1; k < GP_THREADS / 32; k++) t += part[k];
-        gport[g] = t;
-    }
+__global__ void __launch_bounds__(GP_THREADS) k_gport_mx(Params P, Mesh M, const double* __restrict__ cold,
+                                                         const float* __restrict__ dq, const int* ghosts,
+                                                         double* gport) {
+    port_line(M, StateMixed{cold, dq, (size_t)M.ni * M.nj}, ghosts, gport);
 }
 
 // ------------------------------------------------------ primitive output
@@ -641,7 +603,7 @@ void launch_stage_mx(const Params& P, const Mesh& M, const double* cold, const f
 void launch_gport_mx(const Params& P, const Mesh& M, const double* cold, const float* dq,
                      const int* ghosts, int nport, double* gport, cudaStream_t s) {
     if (nport <= 0) return;
-    k_gport_mx<<<nport, GP_THREADS, 0, s>>>(P, M, cold, dq, ghosts, nport, gport);
+    launch_tile(k_gport_mx, dim3(nport), dim3(GP_THREADS), 0, s, P, M, cold, dq, ghosts, gport);
 }
 
 void launch_prim_out_mx(const Params& P, const Mesh& M, const double* cold, const float* dq,

@@ -23,6 +23,12 @@ namespace tns {
 #ifndef TNS_VISC_MINB
 #define TNS_VISC_MINB 3  // 80 registers: 3 blocks/SM beat 2 blocks without the cap
 #endif
+#ifndef TNS_STAGE_RIM_PER_SM
+#define TNS_STAGE_RIM_PER_SM 2
+#endif
+#ifndef TNS_VISC_RIM_PER_SM
+#define TNS_VISC_RIM_PER_SM 1
+#endif
 #ifndef TNS_VISC_BATCH_MINB
 #define TNS_VISC_BATCH_MINB 1  // descriptor-fed arguments spill at 3 blocks/SM
 #endif
@@ -61,6 +67,9 @@ __device__ __forceinline__ void ring_slot(int r, int ri, int rj, int& li, int& l
     else if (r < 2 * w + ri) { li = 1 + r - 2 * w; lj = 0; }
     else { li = 1 + r - 2 * w - ri; lj = w - 1; }
 }
+// Rows of threads a block can have on top of one per cell: they take the halo ring (and the
+// other work a tile has on its rim) while the cells' threads evaluate their own.
+constexpr int RIM_ROWS = (NRING + TJ - 1) / TJ;
 constexpr int AW = TJ + 1;  // node-average grid (TI+1) x (TJ+1)
 constexpr int NAVG = (TI + 1) * AW;
 
@@ -327,6 +336,45 @@ __device__ __forceinline__ void ghost_state(const Params& P, const Mesh& M, cons
 __device__ __forceinline__ void ghost_state(const Params& P, const Mesh& M, const double* __restrict__ q,
                                             size_t ncell, int side, int along, Prim& gh) {
     ghost_state(P, M, StateF64{q, ncell}, side, along, gh);
+}
+
+// Port mass flux of type-6 ghost ghosts[blockIdx.x] by one block: the sum of C1*U*DELY(*YCC)
+// along the mesh line through the parent, across to the opposite boundary (the repaired GPORT
+// walk).  C1*U is C2, and DELY(*YCC) is a static weight per cell (M.wport; a line read from
+// the other side has the opposite sign): 16 bytes a cell, several cells of a thread on their
+// way at once, then a reduction in fixed order.  19 -> 9 us at 2048 lines of
+// 768 cells; launched like the tile kernels, so that it and the stage after it start during
+// the tail of the kernel before them.
+template <class St>
+__device__ __forceinline__ void port_line(const Mesh& M, const St& st, const int* ghosts, double* gport) {
+    const int g = ghosts[blockIdx.x];
+    int side, along;
+    if (g < M.ni) { side = 1; along = g; }
+    else if (g < M.ni + M.nj) { side = 2; along = g - M.ni; }
+    else if (g < 2 * M.ni + M.nj) { side = 3; along = g - M.ni - M.nj; }
+    else { side = 4; along = g - 2 * M.ni - M.nj; }
+    const bool row = side == 1 || side == 3;  // a line along j
+    const int len = row ? M.nj : M.ni;
+    const double* w = row ? M.wport : M.wport_i;
+    const size_t first = row ? (size_t)along * M.nj : along, step = row ? 1 : M.nj;
+    pdl_trigger();
+    pdl_wait();
+    double sum = 0.0;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < len; k += GP_THREADS) {
+        const size_t c = first + k * step;
+        sum += st.c(1, c) * w[c];
+    }
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    __shared__ double part[GP_THREADS / 32];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = part[0];
+#pragma unroll
+        for (int k = 1; k < GP_THREADS / 32; k++) t += part[k];
+        gport[g] = side == 1 || side == 4 ? -t : t;
+    }
 }
 
 }  // namespace tns

@@ -44,8 +44,10 @@ __device__ __forceinline__ void face_values(const ViscSmem& S, int sa, int sc, i
 }
 
 // face(FaceVals, sx, sy, ga, gb, gc, gd, ryavg, double out[4]) evaluates one face's flux.
-// error: bit 1 is set when the tile's static copy did not complete.
-template <class OutT, class Face>
+// error: bit 1 is set when the tile's static copy did not complete.  RIM: the block has
+// RIM_ROWS more rows of threads, which take the halo, the nodes and the faces beyond the
+// cells' own.
+template <bool RIM, class OutT, class Face>
 __device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                              OutT* __restrict__ vis, unsigned int* error, int bx, int by, Face face) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -61,24 +63,26 @@ __device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, con
     }
     const bool inner = i0 > 0 && j0 > 0 && i0 + TI < M.ni && j0 + TJ < M.nj;
     const int i = i0 + ti, j = j0 + tj;
-    const bool valid = i < M.ni && j < M.nj;
+    const bool mine = !RIM || ti < TI;  // the thread has a cell's place
+    const bool valid = mine && i < M.ni && j < M.nj;
+    const int rt = RIM ? tid - NTHREADS : tid;  // the thread's place on the rim
     const int ri = inner ? TI : min(TI, M.ni - i0), rj = inner ? TJ : min(TJ, M.nj - j0);
     HaloPos h;
     h.kind = -1;
     GhostSite site{0, 0.0, 0.0, 0.0, 0.0};
-    if (tid < 2 * (ri + rj + 2)) {
+    if (rt >= 0 && rt < 2 * (ri + rj + 2)) {
         int li, lj;
-        ring_slot(tid, ri, rj, li, lj);
+        ring_slot(rt, ri, rj, li, lj);
         h = halo_pos(M, inner, i0, j0, li, lj);
         if (h.kind > 0) site = ghost_site(M, h.g);
     }
     // nodes: the thread's own (ti, tj), and of the last row and column one more for the first
     // threads; the codes of those on the boundary
-    const int xa = tid < AW ? TI : tid - AW, xb = tid < AW ? tid : TJ;
-    const bool extra = tid < AW + TI;
+    const int xa = rt < AW ? TI : rt - AW, xb = rt < AW ? rt : TJ;
+    const bool extra = rt >= 0 && rt < AW + TI;
     int code0 = 0, code1 = 0;
     if (!inner) {
-        code0 = node_code(M, i, j);
+        if (mine) code0 = node_code(M, i, j);
         if (extra) code1 = node_code(M, i0 + xa, j0 + xb);
     }
     pdl_wait();
@@ -175,7 +179,7 @@ __device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, con
         S.atr[s] = make_double2(tr.x * idf, tr.y * idf);
         S.ar[s] = dmax1(P.rtol, rn * idf);
     };
-    if (i <= M.ni && j <= M.nj) node(ti, tj, code0);
+    if (mine && i <= M.ni && j <= M.nj) node(ti, tj, code0);
     if (extra && i0 + xa <= M.ni && j0 + xb <= M.nj) node(xa, xb, code1);
     __syncthreads();
     if (!bulk_wait(&S.bar)) {
@@ -197,14 +201,14 @@ __device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, con
     // a thread's i-face (between cells (i-1, j) and (i, j)), its j-face (between (i, j-1) and
     // (i, j)), then the last row of i-faces and the last column of j-faces
 #pragma unroll 1
-    for (int r = 0; r < 3; r++) {
+    for (int r = mine ? 0 : 2; r < 3; r++) {
         int la = ti, lb = tj;
         bool iface = r == 0;
         if (r == 2) {
-            iface = tid < TJ;
-            la = iface ? TI : tid - TJ;
-            lb = iface ? tid : TJ;
-            if (tid >= TJ + TI) break;
+            iface = rt < TJ;
+            la = iface ? TI : rt - TJ;
+            lb = iface ? rt : TJ;
+            if (rt < 0 || rt >= TJ + TI) break;
         }
         const int fi = i0 + la, fj = j0 + lb;
         if (iface ? fi > M.ni || fj >= M.nj : fi >= M.ni || fj > M.nj) continue;

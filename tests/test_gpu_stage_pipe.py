@@ -70,3 +70,12 @@ def test_large_mesh_equals_batched_tiles_bitwise():
         out.append(s.download())
         s.close()
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("family,ni,nj,local", [
+    ("plume", 200, 250, 1),  # 200 tiles: extra thread rows in the stage kernel alone
+    ("ramp", 395, 255, 0),   # 400 tiles: none, odd rows, last tile short both ways
+    ("port", 60, 40, 1),     # 16 tiles: extra rows in the stage and viscous kernels
+])
+def test_smaller_meshes_of_each_block_shape_match_oracle(family, ni, nj, local):
+    test_large_mesh_matches_oracle(family, ni, nj, local)
