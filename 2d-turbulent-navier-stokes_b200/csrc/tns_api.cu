@@ -716,20 +716,22 @@ void enqueue_iteration(tns_handle* h, bool monitor) {
     }
 }
 
-int capture(tns_handle* h, cudaGraphExec_t* exec, bool mixed, int parity, bool monitor = false) {
+int capture(tns_handle* h, cudaGraphExec_t* exec, bool mixed, int parity, bool monitor = false, int iters = 1) {
     cudaGraph_t g;
     int rc;
     if ((rc = h->cuda(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "capture")))
         return rc;
     const long long before = h->launches;
-    if (mixed) {
-        double* A = parity ? h->qa2.p : h->qa.p;
-        double* B = parity ? h->qa.p : h->qa2.p;
-        enqueue_iteration_mx(h, monitor, A, B);
-    } else {
-        enqueue_iteration_f64(h, monitor);
+    for (int k = 0; k < iters; k++) {
+        if (mixed) {
+            double* A = parity ^ (k & 1) ? h->qa2.p : h->qa.p;
+            double* B = parity ^ (k & 1) ? h->qa.p : h->qa2.p;
+            enqueue_iteration_mx(h, monitor, A, B);
+        } else {
+            enqueue_iteration_f64(h, monitor);
+        }
     }
-    h->per_iter = h->launches - before;
+    h->per_iter = (h->launches - before) / iters;
     h->launches = before;
     if ((rc = h->cuda(cudaStreamEndCapture(h->stream, &g), "capture"))) return rc;
     rc = h->cuda(cudaGraphInstantiate(exec, g, 0), "cudaGraphInstantiate");
@@ -738,16 +740,22 @@ int capture(tns_handle* h, cudaGraphExec_t* exec, bool mixed, int parity, bool m
 }
 
 // Captures one unmonitored iteration as a CUDA graph (once per handle; the mixed path
-// needs one per state-buffer parity).
+// needs one per state-buffer parity), and GRAPH_BLOCK of them as another.
 int ensure_graph(tns_handle* h) {
     int rc;
-    if (h->precision == 1) {
-        for (int par = 0; par < 2; par++)
-            if (!h->graph_mx[par] && (rc = capture(h, &h->graph_mx[par], true, par))) return rc;
-        return TNS_OK;
+    const bool mixed = h->precision == 1;
+    for (int par = 0; par < (mixed ? 2 : 1); par++) {
+        cudaGraphExec_t* g = mixed ? &h->graph_mx[par] : &h->graph;
+        if (!*g && (rc = capture(h, g, mixed, par))) return rc;
     }
-    if (h->graph) return TNS_OK;
-    return capture(h, &h->graph, false, 0);
+    return TNS_OK;
+}
+int ensure_block_graph(tns_handle* h) {
+    const bool mixed = h->precision == 1;
+    int rc;
+    for (int par = 0; par < (mixed ? 2 : 1); par++)
+        if (!h->graph_block[par] && (rc = capture(h, &h->graph_block[par], mixed, par, false, GRAPH_BLOCK))) return rc;
+    return TNS_OK;
 }
 
 // One monitored iteration: a captured graph (memset of the CDIFF slots + the iteration),
@@ -778,7 +786,17 @@ int enqueue_plain(tns_handle* h, int niter) {
         return TNS_OK;
     }
     if ((rc = ensure_graph(h))) return rc;
-    for (int it = 0; it < niter; it++) {
+    int it = 0;
+    if (niter >= GRAPH_BLOCK) {
+        if ((rc = ensure_block_graph(h))) return rc;
+        for (; it + GRAPH_BLOCK <= niter; it += GRAPH_BLOCK) {  // an even number: the parity stays
+            if ((rc = h->cuda(cudaGraphLaunch(h->graph_block[h->precision == 1 ? h->cur : 0], h->stream),
+                              "cudaGraphLaunch")))
+                return rc;
+            h->launches += GRAPH_BLOCK * h->per_iter;
+        }
+    }
+    for (; it < niter; it++) {
         cudaGraphExec_t g = h->precision == 1 ? h->graph_mx[h->cur] : h->graph;
         if ((rc = h->cuda(cudaGraphLaunch(g, h->stream), "cudaGraphLaunch"))) return rc;
         if (h->precision == 1) h->cur ^= 1;
@@ -825,7 +843,7 @@ int tns_prepare(tns_handle* h) {
     if (!h->have_state) return h->fail(TNS_ERR_STATE, "tns_prepare: no state uploaded");
     if (h->profile) return TNS_OK;
     int rc;
-    if ((rc = ensure_graph(h))) return rc;
+    if ((rc = ensure_graph(h)) || (rc = ensure_block_graph(h))) return rc;
     const long long per = h->per_iter;
     const bool mixed = h->precision == 1;
     for (int par = 0; par < (mixed ? 2 : 1); par++) {
@@ -1203,6 +1221,8 @@ void tns_destroy(tns_handle* h) {
     tns_rt::umesh_release(h);
     if (h->graph) cudaGraphExecDestroy(h->graph);
     for (auto g : h->graph_mx)
+        if (g) cudaGraphExecDestroy(g);
+    for (auto g : h->graph_block)
         if (g) cudaGraphExecDestroy(g);
     for (auto g : h->graph_mon_mx)
         if (g) cudaGraphExecDestroy(g);

@@ -19,6 +19,16 @@ using tns::Params;
 
 namespace tns_rt {
 
+// Unmonitored iterations of one captured graph.  Between graph launches a small mesh's GPU is
+// idle for some 3 us, inside a graph its kernels follow one another: 115 x 50 nozzle, an
+// iteration, 25.3 us with one a graph, 22.7 with four, 22.5 with eight; 512 x 192 ramp 39.6,
+// 36.6, 36.0.  Four cost half of eight's capture (0.4 ms a handle).
+#ifndef TNS_GRAPH_BLOCK
+#define TNS_GRAPH_BLOCK 4
+#endif
+constexpr int GRAPH_BLOCK = TNS_GRAPH_BLOCK;
+static_assert(GRAPH_BLOCK % 2 == 0, "the state-buffer parity survives a block");
+
 enum KernelId { K_DISS = 0, K_VISC = 1, K_STAGE = 2, K_DTMIN = 3, K_GPORT = 4, K_NKERNEL = 5 };
 
 template <class T>
@@ -71,6 +81,7 @@ struct tns_handle {
     DevBuf<float> dqb, dqc, df, visf, dtf;
     DevBuf<double> tref;  // per stage tile reference state (TileRefMx words)
     cudaGraphExec_t graph_mx[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph_block[2] = {nullptr, nullptr};  // GRAPH_BLOCK iterations (per parity)
     // monitored iteration (CDIFF reduction in stage 4): FP64, mixed per parity
     cudaGraphExec_t graph_mon = nullptr;
     cudaGraphExec_t graph_mon_mx[2] = {nullptr, nullptr};

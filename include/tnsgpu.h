@@ -89,8 +89,9 @@ int tns_run(tns_handle *h, int niter, int monitor_every, double *cdiff_out, int 
 int tns_enqueue(tns_handle *h, int niter);
 
 /* Captures and instantiates, without running anything, every CUDA graph that tns_run
- * and tns_enqueue launch for this handle (the unmonitored and the monitored iteration;
- * in mixed precision one of each per state-buffer parity).  Otherwise each is captured
+ * and tns_enqueue launch for this handle (the unmonitored iteration, a block of four of
+ * them, and the monitored iteration; in mixed precision one of each per state-buffer
+ * parity).  Otherwise each is captured
  * at its first use, inside whichever call first needs it.  Needs an uploaded state;
  * does nothing while per-kernel profiling is on (those iterations are not graphs). */
 int tns_prepare(tns_handle *h);
