@@ -560,7 +560,7 @@ void enqueue_iteration_f64(tns_handle* h, bool monitor) {
         [&](cudaStream_t s) {
             // the frozen viscous flux of Q_old uses stage 1's boundary state (viscous.f90:29)
             if (np) launch(h, K_GPORT, [&] { tns::launch_gport(P, M, in[0], h->ports.p, np, h->gport.p, s); });
-            launch(h, K_VISC, [&] { tns::launch_viscous(P, M, A, h->vis.p, h->status.p, s); });
+            launch(h, K_VISC, [&] { tns::launch_viscous(P, M, A, h->vis.p, h->status.p, s, h->beside); });
         });
     cudaStream_t s = h->stream;
     if (monitor) cudaMemsetAsync(h->cdiff.p, 0, 5 * sizeof(unsigned long long), s);
@@ -570,7 +570,7 @@ void enqueue_iteration_f64(tns_handle* h, bool monitor) {
         launch(h, K_STAGE, [&] {
             tns::launch_stage(P, M, in[st], A, out[st], h->d.p, h->vis.p, h->dt.p, h->dtmin.p, st, h->e.p,
                               (monitor && st == 3) ? h->cdiff.p : nullptr,
-                              st == 3 ? h->status.p : nullptr, h->status.p, s);
+                              st == 3 ? h->status.p : nullptr, h->status.p, s, h->beside);
         });
     }
 }

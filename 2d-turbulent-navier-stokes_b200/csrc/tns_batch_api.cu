@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -243,6 +244,15 @@ void enqueue_branches(tns_batch* b, int parity, bool monitor, int iters = 1) {
     const int nb = (int)b->branch.size();
     cudaEventRecord(b->fork, b->stream);
     std::vector<char> used(nb, 0);
+    // tiles in flight: every branch has one of its cases (the largest here)
+    std::vector<int> tiles(nb, 0);
+    for (int k = 0; k < n; k++)
+        if (b->active[k] && !b->cases[k]->unstructured) {
+            const tns::Mesh& M = b->cases[k]->M;
+            const int t = ((M.nj + tns::TJ - 1) / tns::TJ) * ((M.ni + tns::TI - 1) / tns::TI);
+            tiles[b->branch_of[k]] = std::max(tiles[b->branch_of[k]], t);
+        }
+    const int all = std::accumulate(tiles.begin(), tiles.end(), 0);
     for (int k = 0; k < n; k++) {
         if (!b->active[k]) continue;
         tns_handle* h = b->cases[k];
@@ -256,6 +266,7 @@ void enqueue_branches(tns_batch* b, int parity, bool monitor, int iters = 1) {
         const long long before = h->launches;
         h->stream = b->branch[bi];
         h->side = nullptr;   // the case's pre-passes in order: the batch is parallel enough
+        h->beside = all - tiles[bi];
         h->profile = false;  // no event synchronisation inside a capture
         for (int i = 0; i < iters; i++) {
             const int par = parity ^ (i & 1);
@@ -269,6 +280,7 @@ void enqueue_branches(tns_batch* b, int parity, bool monitor, int iters = 1) {
         h->launches = before;
         h->stream = keep;
         h->side = keep_side;
+        h->beside = 0;
         h->profile = prof;
     }
     for (int bi = 0; bi < nb; bi++)

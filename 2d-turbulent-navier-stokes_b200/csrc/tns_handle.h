@@ -81,6 +81,7 @@ struct tns_handle {
     DevBuf<float> dqb, dqc, df, visf, dtf;
     DevBuf<double> tref;  // per stage tile reference state (TileRefMx words)
     cudaGraphExec_t graph_mx[2] = {nullptr, nullptr};
+    int beside = 0;  // tiles other cases have in flight beside this one (a batch's branch streams)
     cudaGraphExec_t graph_block[2] = {nullptr, nullptr};  // GRAPH_BLOCK iterations (per parity)
     // monitored iteration (CDIFF reduction in stage 4): FP64, mixed per parity
     cudaGraphExec_t graph_mon = nullptr;

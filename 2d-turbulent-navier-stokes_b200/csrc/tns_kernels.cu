@@ -979,12 +979,12 @@ void launch_dissipation(const Params& P, const Mesh& M, const double* q, double*
 }
 
 void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, unsigned int* error,
-                    cudaStream_t s) {
+                    cudaStream_t s, int beside) {
     const dim3 grid = tile_grid(M);
     // the rim rows shorten one tile's chain (115 x 50 nozzle: 22.8 -> 22.2 us an iteration,
     // 192 x 64: 24.2 -> 22.2) but leave room for two blocks an SM instead of three (400 x 160,
     // 250 tiles: 28.0 -> 29.9)
-    if ((int)(grid.x * grid.y) <= TNS_VISC_RIM_PER_SM * sm_count())
+    if ((int)(grid.x * grid.y) + beside <= TNS_VISC_RIM_PER_SM * sm_count())
         launch_tile(k_viscous<true>, grid, dim3(TJ, TI + RIM_ROWS), visc_smem_bytes(), s, P, M, q, vis, error);
     else
         launch_tile(k_viscous<false>, grid, dim3(TJ, TI), visc_smem_bytes(), s, P, M, q, vis, error);
@@ -993,7 +993,7 @@ void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis
 void launch_stage(const Params& P, const Mesh& M, const double* qin, const double* qold,
                   double* qout, const double* d, const double* vis, const double* dt,
                   const double* dtmin, int stage, double* e, unsigned long long* cdiff,
-                  unsigned int* status, unsigned int* error, cudaStream_t s) {
+                  unsigned int* status, unsigned int* error, cudaStream_t s, int beside) {
     const StageArgs A{qin, qold, qout, d, vis, dt, dtmin, RK_ALPHA[stage], stage ? e : nullptr, stage ? nullptr : e,
                       cdiff, status, error};
     const dim3 grid = tile_grid(M);
@@ -1006,8 +1006,11 @@ void launch_stage(const Params& P, const Mesh& M, const double* qin, const doubl
         return;
     }
     // the rim rows while every tile has its own resident block of that size: 115 x 50 nozzle,
-    // an iteration, 22.7 -> 22.2 us; 400 x 160 ramp (250 tiles) 31.2 -> 28.0
-    if (ntiles <= TNS_STAGE_RIM_PER_SM * sm_count())
+    // an iteration, 22.7 -> 22.2 us; 400 x 160 ramp (250 tiles) 31.2 -> 28.0.  The tiles of
+    // other cases in flight beside this mesh count too: their warps fill the gaps, and the
+    // larger blocks would only displace them (16 ramp cases on branch streams, 20 iterations:
+    // 6.05 ms with the rim rows, 5.28 without; 4 cases 1.63 and 1.50)
+    if (ntiles + beside <= TNS_STAGE_RIM_PER_SM * sm_count())
         launch_tile(cdiff ? k_stage<1, true> : k_stage<0, true>, grid, dim3(TJ, TI + RIM_ROWS), stage_smem_bytes(), s, P,
                     M, A);
     else

@@ -18,15 +18,16 @@ int sm_count();  // SMs of the current device
 
 void launch_dissipation(const Params& P, const Mesh& M, const double* q, double* d, double* dt,
                         const double* dtmin, cudaStream_t s);
+// (beside: tiles of other meshes in flight on other streams at the same time)
 void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis, unsigned int* error,
-                    cudaStream_t s);
+                    cudaStream_t s, int beside = 0);
 // RK stage 0..3 of the iteration; e: [5][ncell] scratch that stage 0 fills with VIS + D and
 // the others read; error: bit 1 is set when a tile's copies did not complete (must not be
 // null)
 void launch_stage(const Params& P, const Mesh& M, const double* qin, const double* qold,
                   double* qout, const double* d, const double* vis, const double* dt,
                   const double* dtmin, int stage, double* e, unsigned long long* cdiff,
-                  unsigned int* status, unsigned int* error, cudaStream_t s);
+                  unsigned int* status, unsigned int* error, cudaStream_t s, int beside = 0);
 void launch_dtmin(const Params& P, const Mesh& M, const double* q, double* partial,
                   unsigned int* counter, double* dtmin, cudaStream_t s);
 void launch_time_step_scratch(const Params& P, const double* q, const double* cfldl,
