@@ -18,6 +18,7 @@
 
 #include "tns_handle.h"
 #include "tns_params.h"
+#include "tns_mx.cuh"
 #include "tns_tile.cuh"
 #include "tns_umesh.h"
 
@@ -241,28 +242,47 @@ void build_geometry(tns_handle* h) {
     const size_t nc = (size_t)ni * nj;
     h->hcvol.assign(nc, 0.0);
     const int ntj = (nj + TJ - 1) / TJ, nti = (ni + TI - 1) / TI;
-    h->hstile.assign((size_t)ntj * nti * STILE, 0.0);
+    const bool mixed = h->precision == 1;  // (its stage has its own static block)
+    const size_t tile = mixed ? MXTILE : STILE;
+    h->hstile.assign((size_t)ntj * nti * tile, 0.0);
     for (int i = 0; i < ni; i++)
         for (int j = 0; j < nj; j++) {
             const size_t k = (size_t)i * nj + j;
-            double* blk = &h->hstile[((size_t)(i / TI) * ntj + j / TJ) * STILE];
-            const int ti = i % TI, tj = j % TJ, gc = 2 * SNN + ti * TJ + tj;
+            double* blk = &h->hstile[((size_t)(i / TI) * ntj + j / TJ) * tile];
+            const int at = i % TI * TJ + j % TJ, gc = 2 * SNN + at;
             double xa, ya, xb, yb, xc, yc, xd, yd;
             centroid(i, j - 1, xa, ya);  // NC1..NC4
             centroid(i + 1, j, xb, yb);
             centroid(i, j + 1, xc, yc);
             centroid(i - 1, j, xd, yd);
-            grad(xa, ya, xb, yb, xc, yc, xd, yd, blk + gc + ST_GA * TI * TJ, (size_t)TI * TJ);
+            double g[4];
+            grad(xa, ya, xb, yb, xc, yc, xd, yd, g, 1);
             const size_t n1 = (size_t)i * (nj + 1) + j;
             const double Xc[4] = {X[n1], X[n1 + nj + 1], X[n1 + nj + 2], X[n1 + 1]};
             const double Yc[4] = {Y[n1], Y[n1 + nj + 1], Y[n1 + nj + 2], Y[n1 + 1]};
             const double ycc = (Yc[0] + Yc[1] + Yc[2] + Yc[3]) * 0.25;
             const double vol = cell_volume(iaxis, Xc, Yc, ycc);
             h->hcvol[k] = vol;
+            if (mixed) {
+                double sx[4], sy[4];
+                for (int f = 0; f < 4; f++) face_vector(iaxis, f + 1, Xc, Yc, sx[f], sy[f]);
+                GeoMx m;
+                geo_mx(iaxis, sx, sy, g, vol, ycc, m);
+                float4* f4 = reinterpret_cast<float4*>(blk) + at;
+                f4[0] = m.s01;
+                f4[TI * TJ] = m.s23;
+                f4[2 * TI * TJ] = m.g;
+                f4[3 * TI * TJ] = m.w;
+                blk[MX_SUMX * TI * TJ + at] = m.sumx;
+                blk[MX_SUMY * TI * TJ + at] = m.sumy;
+                blk[MX_VR * TI * TJ + at] = m.vr;
+                continue;
+            }
+            for (int f = 0; f < 4; f++) blk[gc + (ST_GA + f) * TI * TJ] = g[f];
             blk[gc + ST_RVOL * TI * TJ] = 1.0 / vol;
             blk[gc + ST_RYCC * TI * TJ] = 1.0 / ycc;
         }
-    for (int a = 0; a <= ni; a++)  // nodes of each tile's cells; shared rows go to both tiles
+    for (int a = 0; !mixed && a <= ni; a++)  // nodes of each tile's cells; shared rows go to both tiles
         for (int b = 0; b <= nj; b++)
             for (int bi = std::max(0, (a - 1) / TI); bi <= std::min(nti - 1, a / TI); bi++)
                 for (int bj = std::max(0, (b - 1) / TJ); bj <= std::min(ntj - 1, b / TJ); bj++) {
@@ -442,7 +462,7 @@ int alloc_state(tns_handle* h) {
         if ((rc = h->cuda(h->qa.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->qa2.alloc(5 * nc), "cudaMalloc")) ||
             (rc = h->cuda(h->dqb.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->dqc.alloc(5 * nc), "cudaMalloc")) ||
             (rc = h->cuda(h->df.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->visf.alloc(4 * nc), "cudaMalloc")) ||
-            (rc = h->cuda(h->dtf.alloc(nc), "cudaMalloc")))
+            (rc = h->cuda(h->ef.alloc(4 * nc), "cudaMalloc")) || (rc = h->cuda(h->dtf.alloc(nc), "cudaMalloc")))
             return rc;
         if ((rc = h->cuda(cudaMemset(h->dtf.p, 0, nc * 4), "cudaMemset")) ||
             (rc = h->cuda(cudaMemset(h->visf.p, 0, 4 * nc * 4), "cudaMemset")))
@@ -522,7 +542,7 @@ void enqueue_iteration_mx(tns_handle* h, bool monitor, double* A, double* Aout) 
         },
         [&](cudaStream_t s) {
             if (np) launch(h, K_GPORT, [&] { tns::launch_gport_mx(P, M, A, in[0], h->ports.p, np, h->gport.p, s); });
-            launch(h, K_VISC, [&] { tns::launch_viscous_mx(P, M, A, h->visf.p, h->status.p, s); });
+            launch(h, K_VISC, [&] { tns::launch_viscous_mx(P, M, A, h->visf.p, h->status.p, s, h->beside); });
         });
     cudaStream_t s = h->stream;
     if (monitor) cudaMemsetAsync(h->cdiff.p, 0, 5 * sizeof(unsigned long long), s);
@@ -530,9 +550,9 @@ void enqueue_iteration_mx(tns_handle* h, bool monitor, double* A, double* Aout) 
         if (np && st > 0)
             launch(h, K_GPORT, [&] { tns::launch_gport_mx(P, M, A, in[st], h->ports.p, np, h->gport.p, s); });
         launch(h, K_STAGE, [&] {
-            tns::launch_stage_mx(P, M, A, in[st], out[st], st == 3 ? Aout : nullptr, h->df.p, h->visf.p,
+            tns::launch_stage_mx(P, M, A, in[st], out[st], st == 3 ? Aout : nullptr, h->df.p, h->visf.p, h->ef.p,
                                  h->dtf.p, h->dtmin.p, alpha[st], (monitor && st == 3) ? h->cdiff.p : nullptr,
-                                 st == 3 ? h->status.p : nullptr, h->status.p, s);
+                                 st == 3 ? h->status.p : nullptr, h->status.p, s, h->beside);
         });
     }
 }
@@ -1227,7 +1247,7 @@ void tns_destroy(tns_handle* h) {
     for (auto g : h->graph_mon_mx)
         if (g) cudaGraphExecDestroy(g);
     if (h->graph_mon) cudaGraphExecDestroy(h->graph_mon);
-    h->qa2.release(); h->dqb.release(); h->dqc.release(); h->df.release(); h->visf.release();
+    h->qa2.release(); h->dqb.release(); h->dqc.release(); h->df.release(); h->visf.release(); h->ef.release();
     h->dtf.release(); h->tref.release();
     for (auto* b : {&h->x, &h->y, &h->cfldl, &h->gxc, &h->gyc, &h->ginj, &h->gport, &h->qa, &h->qb,
                     &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->vcfl, &h->e, &h->wport, &h->wport_i,

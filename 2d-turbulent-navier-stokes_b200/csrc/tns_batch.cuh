@@ -45,11 +45,15 @@ struct StageArgsMx {
     const float* dqin;    // stage input increment (null in stage 1)
     float* dqout;         // stage output increment (stages 1-3)
     double* qout;         // new state (stage 4) [5][ncell]
-    const float* d;       // dissipation [5][ncell]
-    const float* vis;     // viscous flux [4][ncell]
+    const float* d;       // dissipation [5][ncell] (all of it in stage 1, then the first)
+    const float* vis;     // viscous flux [4][ncell] (stage 1)
     const float* dt;      // per-cell DT (LOCAL=1)
     const double* dtmin;  // DTMIN (LOCAL=0)
     float alpha;
+    // the frozen terms VIS + D of components 2-5, [4][ncell] (the first has no VIS): stage 1
+    // (e null) forms them and writes them to eout, stages 2-4 read them from e
+    const float* e;
+    float* eout;
     unsigned long long* cdiff;
     unsigned int* status;
     unsigned int* error;  // bit 1: a tile's static-block copy did not complete

@@ -78,7 +78,7 @@ struct tns_handle {
     int precision = 0;
     int cur = 0;  // mixed: which of qa / qa2 holds the state
     DevBuf<double> qa2;
-    DevBuf<float> dqb, dqc, df, visf, dtf;
+    DevBuf<float> dqb, dqc, df, visf, ef, dtf;
     DevBuf<double> tref;  // per stage tile reference state (TileRefMx words)
     cudaGraphExec_t graph_mx[2] = {nullptr, nullptr};
     int beside = 0;  // tiles other cases have in flight beside this one (a batch's branch streams)

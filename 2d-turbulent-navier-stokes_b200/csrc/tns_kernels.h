@@ -76,11 +76,12 @@ cudaError_t configure_kernels_mx();
 void launch_dissipation_mx(const Params& P, const Mesh& M, const double* q, float* d, float* dt,
                            const double* dtmin, cudaStream_t s);
 void launch_viscous_mx(const Params& P, const Mesh& M, const double* q, float* vis, unsigned int* error,
-                       cudaStream_t s);
+                       cudaStream_t s, int beside = 0);
+// e: [4][ncell] scratch that stage 1 (dqin null) fills with VIS + D of components 2-5
 void launch_stage_mx(const Params& P, const Mesh& M, const double* cold, const float* dqin,
-                     float* dqout, double* qout, const float* d, const float* vis, const float* dt,
+                     float* dqout, double* qout, const float* d, const float* vis, float* e, const float* dt,
                      const double* dtmin, double alpha, unsigned long long* cdiff,
-                     unsigned int* status, unsigned int* error, cudaStream_t s);
+                     unsigned int* status, unsigned int* error, cudaStream_t s, int beside = 0);
 void launch_gport_mx(const Params& P, const Mesh& M, const double* cold, const float* dq,
                      const int* ghosts, int nport, double* gport, cudaStream_t s);
 void launch_prim_out_mx(const Params& P, const Mesh& M, const double* cold, const float* dq,

@@ -84,6 +84,12 @@ enum StageTileField { ST_GA, ST_GB, ST_GC, ST_GD, ST_RVOL, ST_RYCC, ST_NF };
 constexpr int STILE = 2 * SNN + ST_NF * TI * TJ;
 static_assert(STILE % 2 == 0, "a stage tile block must be a multiple of 16 bytes");
 
+// The mixed stage's static block of a tile instead (MXTILE doubles a tile): per cell (index
+// ti * TJ + tj) the four 16-byte FP32 words of GeoMx (tns_mx.cuh), a plane each, then the
+// FP64 sums of the face vectors and VOL/YCC; a plane mesh leaves the last one out of the copy.
+enum MixedTilePlane { MX_SUMX = 8, MX_SUMY, MX_VR, MX_N };  // in planes of doubles
+constexpr int MXTILE = MX_N * TI * TJ;
+
 // Faces of a tile: i-faces (between cells (i-1, j) and (i, j)) for i in i0..i0+TI, j-faces
 // (between (i, j-1) and (i, j)) for j in j0..j0+TJ; and the tile's static face geometry
 // (tile (bx, by) at M.vtile + (by * ntiles_j + bx) * VTILE), [FG_N][NVF], i-face (la, lb) at

@@ -40,6 +40,8 @@ struct UMesh {
     const int* nc;        // [4][ne] neighbour slot: a cell 0..ne-1 or a ghost ne+line
     const int* nod;       // [4][ne] 0-based node ids
     const double* cg;     // [UCG_N][ne]
+    const double* gmx;    // mixed stage: GeoMx (tns_mx.cuh) of each cell, its four 16-byte words
+                          // [4][ne], then its doubles [3][ne] (null on FP64 handles)
     const double* fg;     // [UFG_N][4][ne]
     const double* cfldl;  // [ne] CFL*DL
     const int* gpar;      // [ng] parent cell

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "tns_handle.h"
+#include "tns_mx.cuh"
 #include "tns_umesh.h"
 #include "tns_tile.cuh"
 
@@ -569,12 +570,12 @@ struct tns_umesh_state {
     tns::UMesh M{};
     DevBuf<int> nc, nod, gpar, gopp, gtype, gside, nptr, nslot, nreset, pghost, pptr, pcell, fcell, fref, cptr,
         cslot, lnb;
-    DevBuf<double> cg, fg, cfldl, gsx, gsy, gyc, ginj, gport, pdely, W, aux, na, vf;
+    DevBuf<double> cg, gmx, fg, cfldl, gsx, gsy, gyc, ginj, gport, pdely, W, aux, na, vf;
     // host layout, uploaded by umesh_upload
     std::vector<int> hnc, hnod, hgpar, hgopp, hgtype, hgside, hnptr, hnslot, hnreset, hpghost, hpptr, hpcell,
         hfcell, hfref, hcptr, hcslot, hlnb;
     int hmax = 0;
-    std::vector<double> hcg, hfg, hcfldl, hgsx, hgsy, hgyc, hginj, hpdely;
+    std::vector<double> hcg, hgmx, hfg, hcfldl, hgsx, hgsy, hgyc, hginj, hpdely;
 };
 
 namespace tns_rt {
@@ -731,6 +732,7 @@ int umesh_build(tns_handle* h, const tns_mesh* m) {
     u->hnc.assign((size_t)4 * ne, 0);
     u->hnod.assign((size_t)4 * ne, 0);
     u->hcg.assign((size_t)UCG_N * ne, 0.0);
+    if (h->precision == 1) u->hgmx.assign(11 * (size_t)ne, 0.0);
     u->hfg.assign((size_t)UFG_N * 4 * ne, 0.0);
     u->hcfldl.assign(ne, 0.0);
     for (int k = 0; k < ne; k++) {
@@ -751,6 +753,21 @@ int umesh_build(tns_handle* h, const tns_mesh* m) {
         u->hcg[(size_t)UCG_RVOL * ne + k] = 1.0 / vol[c];
         u->hcg[(size_t)UCG_YCC * ne + k] = ycc[c];
         u->hcg[(size_t)UCG_RYCC * ne + k] = 1.0 / ycc[c];
+        if (h->precision == 1) {
+            const double g[4] = {u->hcg[(size_t)UCG_GA * ne + k], u->hcg[(size_t)UCG_GB * ne + k],
+                                 u->hcg[(size_t)UCG_GC * ne + k], u->hcg[(size_t)UCG_GD * ne + k]};
+            GeoMx m;
+            geo_mx(h->P.iaxis, &sx[4 * (size_t)c], &sy[4 * (size_t)c], g, vol[c], ycc[c], m);
+            float4* f4 = reinterpret_cast<float4*>(u->hgmx.data()) + k;
+            f4[0] = m.s01;
+            f4[(size_t)ne] = m.s23;
+            f4[2 * (size_t)ne] = m.g;
+            f4[3 * (size_t)ne] = m.w;
+            double* d = u->hgmx.data() + 8 * (size_t)ne + k;
+            d[0] = m.sumx;
+            d[(size_t)ne] = m.sumy;
+            d[2 * (size_t)ne] = m.vr;
+        }
         u->hcfldl[k] = h->P.cfl * dl[c];
         // faces for the viscous flux: A = the cell, C = NC_f, B = N_f, D = N_f+1
         for (int f = 0; f < 4; f++) {
@@ -935,7 +952,8 @@ int umesh_upload(tns_handle* h) {
         (rc = upi(u->pghost, u->hpghost)) || (rc = upi(u->pptr, u->hpptr)) || (rc = upi(u->pcell, u->hpcell)) ||
         (rc = upi(u->fcell, u->hfcell)) || (rc = upi(u->fref, u->hfref)) ||
         (rc = upi(u->cptr, u->hcptr)) || (rc = upi(u->cslot, u->hcslot)) || (rc = upi(u->lnb, u->hlnb)) ||
-        (rc = upd(u->cg, u->hcg)) || (rc = upd(u->fg, u->hfg)) || (rc = upd(u->cfldl, u->hcfldl)) ||
+        (rc = upd(u->cg, u->hcg)) || (h->precision == 1 && (rc = upd(u->gmx, u->hgmx))) ||
+        (rc = upd(u->fg, u->hfg)) || (rc = upd(u->cfldl, u->hcfldl)) ||
         (rc = upd(u->gsx, u->hgsx)) || (rc = upd(u->gsy, u->hgsy)) || (rc = upd(u->gyc, u->hgyc)) ||
         (rc = upd(u->ginj, u->hginj)) || (rc = upd(u->pdely, u->hpdely)))
         return rc;
@@ -948,7 +966,7 @@ int umesh_upload(tns_handle* h) {
         return rc;
     tns::UMesh& M = u->M;
     M.ne = ne; M.ng = ng; M.nnode = nn; M.nport = (int)u->hpghost.size();
-    M.nc = u->nc.p; M.nod = u->nod.p; M.cg = u->cg.p; M.fg = u->fg.p; M.cfldl = u->cfldl.p;
+    M.nc = u->nc.p; M.nod = u->nod.p; M.cg = u->cg.p; M.gmx = u->gmx.p; M.fg = u->fg.p; M.cfldl = u->cfldl.p;
     M.gpar = u->gpar.p; M.gopp = u->gopp.p; M.gtype = u->gtype.p; M.gside = u->gside.p;
     M.gsx = u->gsx.p; M.gsy = u->gsy.p; M.gyc = u->gyc.p; M.ginj = u->ginj.p; M.gport = u->gport.p;
     M.nptr = u->nptr.p; M.nslot = u->nslot.p; M.nreset = u->nreset.p;
@@ -964,7 +982,7 @@ int umesh_upload(tns_handle* h) {
     for (auto* v : {&u->hnc, &u->hnod, &u->hgpar, &u->hgopp, &u->hgside, &u->hnptr, &u->hnslot, &u->hnreset,
                     &u->hpghost, &u->hpptr, &u->hpcell, &u->hfcell, &u->hfref, &u->hcptr, &u->hcslot, &u->hlnb})
         std::vector<int>().swap(*v);
-    for (auto* v : {&u->hcg, &u->hfg, &u->hcfldl, &u->hgsx, &u->hgsy, &u->hgyc, &u->hpdely})
+    for (auto* v : {&u->hcg, &u->hgmx, &u->hfg, &u->hcfldl, &u->hgsx, &u->hgsy, &u->hgyc, &u->hpdely})
         std::vector<double>().swap(*v);
     return TNS_OK;
 }
@@ -1050,8 +1068,8 @@ void enqueue_iteration_u_mx(tns_handle* h, bool monitor, double* A, double* Aout
             if (fork) cudaStreamWaitEvent(s, h->join, 0);
         }
         tns::StageArgsMx S{A, in[st], out[st], st == 3 ? Aout : nullptr, h->df.p, h->visf.p, h->dtf.p, h->dtmin.p,
-                           (float)alpha[st], (monitor && st == 3) ? h->cdiff.p : nullptr,
-                           st == 3 ? h->status.p : nullptr, h->status.p};
+                           (float)alpha[st], st ? h->ef.p : nullptr, st ? nullptr : h->ef.p,
+                           (monitor && st == 3) ? h->cdiff.p : nullptr, st == 3 ? h->status.p : nullptr, h->status.p};
         launch(h, K_STAGE, [&] { tns::launch_u_stage_chunk_mx(P, M, S, s); });
     }
 }
@@ -1109,7 +1127,7 @@ void umesh_release(tns_handle* h) {
     for (auto* b : {&u->nc, &u->nod, &u->gpar, &u->gopp, &u->gtype, &u->gside, &u->nptr, &u->nslot, &u->nreset,
                     &u->pghost, &u->pptr, &u->pcell, &u->fcell, &u->fref, &u->cptr, &u->cslot, &u->lnb})
         b->release();
-    for (auto* b : {&u->cg, &u->fg, &u->cfldl, &u->gsx, &u->gsy, &u->gyc, &u->ginj, &u->gport, &u->pdely, &u->W,
+    for (auto* b : {&u->cg, &u->gmx, &u->fg, &u->cfldl, &u->gsx, &u->gsy, &u->gyc, &u->ginj, &u->gport, &u->pdely, &u->W,
                     &u->aux, &u->na, &u->vf})
         b->release();
     delete u;
