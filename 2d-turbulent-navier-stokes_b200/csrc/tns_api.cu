@@ -477,7 +477,7 @@ int alloc_state(tns_handle* h) {
     } else if ((rc = h->cuda(h->qa.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->qb.alloc(5 * nc), "cudaMalloc")) ||
                (rc = h->cuda(h->qc.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->d.alloc(5 * nc), "cudaMalloc")) ||
                (rc = h->cuda(h->vis.alloc(4 * nc), "cudaMalloc")) || (rc = h->cuda(h->dt.alloc(nc), "cudaMalloc")) ||
-               (!h->unstructured && (rc = h->cuda(h->e.alloc(5 * nc), "cudaMalloc")))) {
+               (rc = h->cuda(h->e.alloc(5 * nc), "cudaMalloc"))) {
         return rc;
     }
     if ((rc = h->cuda(h->dtmin.alloc(1), "cudaMalloc")) ||

@@ -163,7 +163,12 @@ __device__ __forceinline__ void stage_mx_tile(const Params& P, const Mesh& M, co
         const double* g8 = S.st + tid;
         const GeoMx G{g[0], g[NTHREADS], g[2 * NTHREADS], g[3 * NTHREADS], g8[MX_SUMX * NTHREADS],
                       g8[MX_SUMY * NTHREADS], P.iaxis == 1 ? g8[MX_VR * NTHREADS] : 0.0};
-        stage_cell_mx(P, S.ref, A, ncell, (size_t)i * M.nj + j, W, c, nb, G, own, dv);
+        const size_t cell = (size_t)i * M.nj + j;
+        stage_cell_mx(P, S.ref, A, ncell, cell, W, c, nb, G, own,
+                      [&](float v[4]) {
+#pragma unroll
+                          for (int m = 0; m < 4; m++) v[m] = A.vis[m * ncell + cell];
+                      }, dv);
     }
     if (A.cdiff) stage_cdiff_mx(A, dv);
 }

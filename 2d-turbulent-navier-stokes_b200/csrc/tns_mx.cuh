@@ -133,10 +133,11 @@ inline void geo_mx(int iaxis, const double sx[4], const double sy[4], const doub
 // slot is c and whose neighbours' are nb, as an FP32 increment on the FP64 state.  The flux
 // residual: the cell's own deviation meets the sum of the face vectors and each neighbour's
 // its face vector, in FP32; the reference flux (cancelling over a closed contour) meets the
-// sum in FP64.
+// sum in FP64.  vis(float[4]) gives the cell's viscous flux (stage 1).
+template <class Vis>
 __device__ __forceinline__ void stage_cell_mx(const Params& P, const TileRefMx& R, const StageArgsMx& A, size_t ncell,
                                               size_t cell, const SlotsMx& S, int c, const int nb[4], const GeoMx& G,
-                                              const float3& own, double dv[5]) {
+                                              const float3& own, Vis vis, double dv[5]) {
     float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f, r3 = 0.0f, r4 = 0.0f;
     float4 cn[4];
     auto add = [&](int s, const float4& k, float sx, float sy) {
@@ -212,8 +213,10 @@ __device__ __forceinline__ void stage_cell_mx(const Params& P, const TileRefMx& 
 #pragma unroll
         for (int m = 1; m < 5; m++) e[m] = A.e[(m - 1) * ncell + cell];
     } else {
+        float v[4];
+        vis(v);
 #pragma unroll
-        for (int m = 1; m < 5; m++) e[m] = A.vis[(m - 1) * ncell + cell] + A.d[m * ncell + cell];
+        for (int m = 1; m < 5; m++) e[m] = v[m - 1] + A.d[m * ncell + cell];
 #pragma unroll
         for (int m = 1; m < 5; m++) A.eout[(m - 1) * ncell + cell] = e[m];
     }

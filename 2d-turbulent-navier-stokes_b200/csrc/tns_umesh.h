@@ -29,11 +29,8 @@ enum UCellGeo {
 // A = the cell, C = NC_k, B = node N_k, D = node N_k+1): [UFG_N][4][ne], the
 // diamond-gradient coefficients and 1/YAVG (0 where YAVG is below the axis threshold).
 enum UFaceGeo { UFG_GA, UFG_GB, UFG_GC, UFG_GD, UFG_RYAVG, UFG_N };
-// Per-slot (cells, then ghosts) primitive and flux field set of one stage [UW_N][ne+ng].
-enum USlot {
-    UW_F1, UW_F2, UW_F3, UW_F4, UW_F5, UW_G1, UW_G2, UW_G3, UW_G4, UW_G5,
-    UW_U, UW_V, UW_T, UW_P, UW_RHO, UW_RI, UW_QM, UW_N
-};
+// Per-slot (cells, then ghosts) primitive field set [UW_N][ne+ng].
+enum USlot { UW_U, UW_V, UW_T, UW_P, UW_RHO, UW_RI, UW_N };
 
 struct UMesh {
     int ne, ng, nnode, nport;
@@ -70,7 +67,7 @@ struct UMesh {
     // stage chunks: chunk b holds cells UT b .. UT b + UT - 1 and the halo slots
     // cslot[cptr[b] .. cptr[b+1]) (cells of other chunks and ghosts its cells touch);
     // lnb[k][ne] is the local slot of each cell's face-k neighbour (below UT: a cell of
-    // the chunk, UT + h: halo slot h); hmax the largest halo
+    // the chunk, UT + h: halo slot h; ~(UT + h) where that slot is a ghost); hmax the largest halo
     int nchunk, hmax;
     const int* cptr;
     const int* cslot;
@@ -78,11 +75,30 @@ struct UMesh {
 };
 constexpr int UT = 256;  // threads per block of the general-mesh kernels, cells per stage chunk
 
+// The viscous flux of cell I: its four faces in order, face 1 assigning and the others adding.
+__device__ __forceinline__ void u_gather_faces(const UMesh& M, const double* __restrict__ vf, int I, double v[4]) {
+    const size_t nf = (size_t)M.nface;
+    int r[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) r[k] = M.fref[(size_t)k * M.ne + I];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int e = r[k] >= 0 ? r[k] : ~r[k];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const double w = r[k] >= 0 ? vf[m * nf + e] : -vf[m * nf + e];
+            v[m] = k == 0 ? w : v[m] + w;
+        }
+    }
+}
+
 struct StageArgsU {
     const double* qold;  // [5][ne] state at the start of the iteration
     double* qout;        // [5][ne] stage output (may alias qold: own-cell reads only)
     const double* d;     // [5][ne]
-    const double* vis;   // [4][ne]
+    const double* vf;    // [4][nface] viscous face fluxes (stage 1 gathers them)
+    double* vis;         // [4][ne] viscous flux, written by stage 1
+    double* e;           // [5][ne] frozen terms VIS + D: written by stage 1, read by the others
     const double* dt;    // [ne] (LOCAL=1)
     const double* dtmin; // (LOCAL=0)
     double alpha;
@@ -95,23 +111,24 @@ void launch_u_prim(const Params& P, const UMesh& M, const double* q, double* W, 
 void launch_u_prim_mx(const Params& P, const UMesh& M, const double* cold, const float* dq, double* W,
                       cudaStream_t s);
 void launch_u_gport_mx(const Params& P, const UMesh& M, const double* cold, const float* dq, cudaStream_t s);
-// mixed path: D, DT (dissipation) and VIS (viscous) stored in FP32
+// mixed path: D and DT stored in FP32
 void launch_u_dissipation(const Params& P, const UMesh& M, const double* q, double* aux, float* d, float* dt,
                           const double* dtmin, cudaStream_t s);
-void launch_u_viscous(const Params& P, const UMesh& M, const double* W, double* na, double* vf, float* vis,
-                      cudaStream_t s);
 void launch_u_gport(const Params& P, const UMesh& M, const double* q, cudaStream_t s);
 void launch_u_dissipation(const Params& P, const UMesh& M, const double* q, double* aux, double* d,
                           double* dt, const double* dtmin, cudaStream_t s);
-void launch_u_viscous(const Params& P, const UMesh& M, const double* W, double* na, double* vf, double* vis,
+// the viscous fluxes vf of state q's faces (W, na: field set and node averages, scratch)
+void launch_u_viscous(const Params& P, const UMesh& M, const double* q, double* W, double* na, double* vf,
                       cudaStream_t s);
-// one RK stage on state q, chunk by chunk; configure_u_chunk once per mesh
-void launch_u_stage_chunk(const Params& P, const UMesh& M, const StageArgsU& A, const double* q, cudaStream_t s);
+// one RK stage on state q, chunk by chunk (first: stage 1); configure_u_chunk once per mesh
+void launch_u_stage_chunk(const Params& P, const UMesh& M, const StageArgsU& A, bool first, const double* q,
+                          cudaStream_t s);
 cudaError_t configure_u_chunk(const UMesh& M);
 // the mixed FP32/FP64 stage (tns_unstructured_mx.cu): A.cold + A.dqin in, A.dqout or
-// (stage 4) A.qout out; configure_u_chunk_mx once per mesh
+// (stage 4) A.qout out; stage 1 gathers vf into vis (A.vis); configure_u_chunk_mx once per mesh
 struct StageArgsMx;
-void launch_u_stage_chunk_mx(const Params& P, const UMesh& M, const StageArgsMx& A, cudaStream_t s);
+void launch_u_stage_chunk_mx(const Params& P, const UMesh& M, const StageArgsMx& A, const double* vf, float* vis,
+                             cudaStream_t s);
 cudaError_t configure_u_chunk_mx(const UMesh& M);
 size_t u_chunk_mx_smem_bytes(const UMesh& M);
 size_t u_chunk_smem_bytes(const UMesh& M);

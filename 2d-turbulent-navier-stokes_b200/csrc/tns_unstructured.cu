@@ -5,14 +5,14 @@
 //   [dtmin]            global time step (LOCAL=0)
 //   k_u_diss1/2        DT, sensors and Laplacians, then the JST blend (solver_state.f90:70-225)
 //   [k_u_gport]        type-6 port mass flux of the stage input (boundary.f90:168-223)
-//   k_u_prim           primitives and fluxes of every cell and ghost (turbnstwod.f90:204-227,
-//                      boundary.f90:24-327) into a slot field set W
+//   k_u_prim           primitives of every cell and ghost (turbnstwod.f90:204-227,
+//                      boundary.f90:24-327) into a slot field set W, stage 1
 //   k_u_node_avg       NODAL_AVERAGE with the bc.in-order resets (viscous.f90:40-124), stage 1
-//   k_u_vface/vsum     every face once, then the four faces of every cell in order
-//                      (viscous.f90:62-70,130-217), stage 1
-//   k_u_stage_chunk    per chunk of 256 cells: primitives and fluxes of its cells and halo
-//                      into shared memory, then source, residual and update
-//                      (source_terms.f90:24-104, residual.f90:23-83), each RK stage
+//   k_u_vface          the viscous flux of every face once (viscous.f90:62-70,130-217), stage 1
+//   k_u_stage_chunk    per chunk of 256 cells: primitives of its cells and halo into shared
+//                      memory, then source, residual and update (source_terms.f90:24-104,
+//                      residual.f90:23-83), each RK stage; stage 1 first gathers the four
+//                      faces of every cell in order
 // The host side lays the mesh out: cells in Hilbert-curve order of their centroids
 // (neighbours near in memory, compact chunks), ghosts after them in bc.in order, the
 // static geometry computed once with the reference's formulas (geometry.f90:55-149).
@@ -55,27 +55,24 @@ __device__ __forceinline__ void u_slot_prim(const Params& P, const UMesh& M, con
     }
 }
 
-// Primitive / flux field set of every slot.
-template <class St>
+// Primitive field set of every slot: what the viscous flux reads, and with FULL the pressure
+// too (post-processing).
+template <class St, bool FULL>
 __global__ void __launch_bounds__(UT) k_u_prim(Params P, UMesh M, St st, double* __restrict__ W) {
     const int s = blockIdx.x * UT + threadIdx.x;
     const int ns = M.ne + M.ng;
+    pdl_trigger();
+    pdl_wait();
     if (s >= ns) return;
     Prim p;
     u_slot_prim(P, M, st, s, p);
     const size_t n = (size_t)ns;
-#pragma unroll
-    for (int m = 0; m < 5; m++) {
-        W[(UW_F1 + m) * n + s] = p.f[m];
-        W[(UW_G1 + m) * n + s] = p.g[m];
-    }
     W[UW_U * n + s] = p.u;
     W[UW_V * n + s] = p.v;
     W[UW_T * n + s] = p.t;
-    W[UW_P * n + s] = p.p;
     W[UW_RHO * n + s] = p.rho;
     W[UW_RI * n + s] = p.ri;
-    W[UW_QM * n + s] = p.qm;
+    if (FULL) W[UW_P * n + s] = p.p;
 }
 
 // Port mass flux of each type-6 ghost: the sum of C1*U*DELY (*YCC) along its port line
@@ -211,6 +208,8 @@ __global__ void __launch_bounds__(UT) k_u_diss2(UMesh M, const double* __restric
 __global__ void __launch_bounds__(UT) k_u_node_avg(Params P, UMesh M, const double* __restrict__ W,
                                                    double* __restrict__ na) {
     const int n = blockIdx.x * UT + threadIdx.x;
+    pdl_trigger();
+    pdl_wait();
     if (n >= M.nnode) return;
     const size_t ns = (size_t)M.ne + M.ng;
     double un = 0.0, vn = 0.0, tn = 0.0, rhon = 0.0, rn = 0.0;
@@ -267,21 +266,24 @@ __global__ void __launch_bounds__(UT) k_u_node_avg(Params P, UMesh M, const doub
     na[4 * nn + n] = dmax1(P.rtol, rn * idf);
 }
 
-// COMPUTE_VISCOUS (viscous.f90:62-70, 130-217) in two passes.  k_u_vface evaluates each
-// face once, in the orientation of the cell that owns it (A = that cell, C = its
-// neighbour across face k, B = node k, D = node k+1); in the neighbour's orientation the
-// face has the same gradient and averages and the opposite face vector, so its flux is
-// the negative.  k_u_vsum then gives every cell its four faces in order, face 1
-// assigning and the others adding, as the reference's loop does.
+// COMPUTE_VISCOUS (viscous.f90:62-70, 130-217): each face once, in the orientation of the
+// cell that owns it (A = that cell, C = its neighbour across face k, B = node k, D = node
+// k+1); in the neighbour's orientation the face has the same gradient and averages and the
+// opposite face vector, so its flux is the negative.  Stage 1 gathers them (u_gather_faces).
 __global__ void __launch_bounds__(UT) k_u_vface(Params P, UMesh M, const double* __restrict__ W,
                                                 const double* __restrict__ na, double* __restrict__ vf) {
     const int e = blockIdx.x * UT + threadIdx.x;
-    if (e >= M.nface) return;
+    pdl_trigger();
+    const bool face = e < M.nface;
     const int ne = M.ne;
-    const int I = M.fcell[e] >> 2, k = M.fcell[e] & 3;
     const size_t ns = (size_t)ne + M.ng, nn = (size_t)M.nnode;
+    // (the connectivity is static)
+    const int code = face ? M.fcell[e] : 0;
+    const int I = code >> 2, k = code & 3;
     const int nbn = M.nod[k * ne + I], ndn = M.nod[((k + 1) & 3) * ne + I];
     const int cc = M.nc[k * ne + I];
+    pdl_wait();
+    if (!face) return;
     FaceVals f;
     f.ua = W[UW_U * ns + I]; f.va = W[UW_V * ns + I]; f.ta = W[UW_T * ns + I];
     f.uc = W[UW_U * ns + cc]; f.vc = W[UW_V * ns + cc]; f.tc = W[UW_T * ns + cc];
@@ -301,117 +303,161 @@ __global__ void __launch_bounds__(UT) k_u_vface(Params P, UMesh M, const double*
     for (int m = 0; m < 4; m++) vf[m * nf + e] = out[m];
 }
 
-template <class OutT>
-__global__ void __launch_bounds__(UT) k_u_vsum(UMesh M, const double* __restrict__ vf, OutT* __restrict__ vis) {
-    const int I = blockIdx.x * UT + threadIdx.x;
-    const int ne = M.ne;
-    if (I >= ne) return;
-    const size_t nf = (size_t)M.nface;
-    int r[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) r[k] = M.fref[k * ne + I];
-    double acc[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int e = r[k] >= 0 ? r[k] : ~r[k];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            const double v = r[k] >= 0 ? vf[m * nf + e] : -vf[m * nf + e];
-            acc[m] = k == 0 ? v : acc[m] + v;
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 4; m++) vis[m * ne + I] = (OutT)acc[m];
-}
-
-// One RK stage of one chunk of UT cells (source_terms.f90:24-104, residual.f90:23-83),
-// with the primitives and fluxes of the chunk's cells and halo staged in shared memory
-// instead of a field set in global memory: each thread evaluates its own cell (keeping
-// its T, P, RHO) and the threads then share the halo slots.  (It gives bitwise the
-// results of a slot field set in global memory gathered per cell.)  Shared memory:
-// (UT + hmax) slots of (F_m, G_m) x 5, (U, V), (C5/C1, |V|).
+// One RK stage of one chunk of UT cells (source_terms.f90:24-104, residual.f90:23-83), with the
+// primitives of the chunk's cells and halo in shared memory as the structured kernel keeps them
+// (StageSlots, tns_kernels.cu): per slot (U, V), (RHO, P), (C4 + P, C5/C1) and |V|, from which a
+// face's flux needs its mass flux alone, and per ghost its own flux through the one face it
+// borders.  Each thread evaluates its own cell (keeping its T) and the threads then share the
+// halo.  FIRST: stage 1, which gathers the viscous flux VIS of its cell from the faces (each
+// cell's four in order, face 1 assigning and the others adding, as the reference's loop does)
+// and forms the frozen terms VIS + D that stages 2-4 read.
+// Latency bound: issue 0.43 an SM quarter a cycle, 24 warps an SM.  Slots of 56 bytes instead of
+// 112 and the mass-flux residual took a stage of 512 x 192 cells from 15 to 10 us, with three
+// blocks an SM now the best; the kernel that summed the faces into VIS (7 us) became 4 us more
+// of stage 1, and each kernel of the iteration starts under the tail of the one before it.
+// Renumbered 512 x 192 nozzle-plume, 30 iterations with the transfers: 3.65 -> 3.24 ms.
 #ifndef TNS_U_CHUNK_MINB
-// Blocks per SM the register budget is sized for; measured on a renumbered 1024 x 384
-// nozzle-plume (B200, one FP64 iteration): 2 -> 0.289 ms, 3 -> 0.294 ms, 4 -> 0.313 ms.
-#define TNS_U_CHUNK_MINB 2
+// (with 2 blocks an SM 3.57 ms, with 4 3.48)
+#define TNS_U_CHUNK_MINB 3
 #endif
+template <bool FIRST>
 __global__ void __launch_bounds__(UT, TNS_U_CHUNK_MINB) k_u_stage_chunk(Params P, UMesh M, StageArgsU A,
                                                          const double* __restrict__ q) {
     extern __shared__ double2 usm[];
     const int ns = UT + M.hmax;
-    double2* fg = usm;
-    double2* uv = usm + 5 * ns;
-    double2* rq = uv + ns;
+    double2* uv = usm;
+    double2* rp = uv + ns;
+    double2* hr = rp + ns;
+    double* qm = reinterpret_cast<double*>(hr + ns);
+    double* gf = qm + ns;  // [5][hmax]
     const int ne = M.ne, t = threadIdx.x;
+    const size_t n = (size_t)ne;
     const int c0 = blockIdx.x * UT, I = c0 + t;
     const int h0 = M.cptr[blockIdx.x], nh = M.cptr[blockIdx.x + 1] - h0;
-    auto put = [&](int s, const Prim& p) {
-#pragma unroll
-        for (int m = 0; m < 5; m++) fg[m * ns + s] = make_double2(p.f[m], p.g[m]);
-        uv[s] = make_double2(p.u, p.v);
-        rq[s] = make_double2(p.ri, p.qm);
+    pdl_trigger();
+    // a halo slot's cell, or the ghost's parent
+    int hs = -1, hc = 0;
+    auto halo = [&](int h) {
+        hs = M.cslot[h0 + h];
+        hc = hs < ne ? hs : M.gpar[hs - ne];
     };
-    double own_t = 0.0, own_p = 0.0, own_rho = 0.0;
+    if (t < nh) halo(t);
+    pdl_wait();
+    auto prim = [&](int c, Prim& p) {
+        double s[5];
+#pragma unroll
+        for (int m = 0; m < 5; m++) s[m] = q[m * n + c];
+        primitive(P, s[0], s[1], s[2], s[3], s[4], p);
+        return s[3] + p.p;
+    };
+    auto put = [&](int s, const Prim& p, double h) {
+        uv[s] = make_double2(p.u, p.v);
+        rp[s] = make_double2(p.rho, p.p);
+        hr[s] = make_double2(h, p.ri);
+        qm[s] = p.qm;
+    };
+    double own_t = 0.0;
     if (I < ne) {
         Prim p;
-        u_cell_prim(P, StateF64{q, (size_t)ne}, I, p);
-        put(t, p);
+        const double h = prim(I, p);
+        put(t, p, h);
         own_t = kept(p.t);
-        own_p = kept(p.p);
-        own_rho = kept(p.rho);
     }
     for (int h = t; h < nh; h += UT) {
-        Prim p;
-        u_slot_prim(P, M, StateF64{q, (size_t)ne}, M.cslot[h0 + h], p);
-        put(UT + h, p);
+        if (h != t) halo(h);
+        Prim pa;
+        const double hh = prim(hc, pa);
+        if (hs < ne) {
+            put(UT + h, pa, hh);
+            continue;
+        }
+        const int L = hs - ne, type = M.gtype[L];
+        const double sx = M.gsx[L], sy = M.gsy[L];
+        Prim op = pa, p;
+        if (type == 3) prim(M.gopp[L], op);
+        boundary_ghost(P, type, pa, op, sx, sy, M.gyc[L], M.cg[UCG_YCC * n + hc], type == 6 ? M.gport[L] : 0.0,
+                       M.ginj[L], p);
+        put(UT + h, p, 0.0);
+#pragma unroll
+        for (int m = 0; m < 5; m++) gf[m * M.hmax + h] = p.f[m] * sx + p.g[m] * sy;
+    }
+    // the cell's local slots and face vectors arrive while the halo is formed
+    int nb[4] = {0, 0, 0, 0};
+    double SX[4], SY[4];
+    const double* G = M.cg + I;
+    if (I < ne) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            nb[k] = M.lnb[k * ne + I];
+            SX[k] = G[(UCG_SX1 + k) * n];
+            SY[k] = G[(UCG_SY1 + k) * n];
+        }
     }
     __syncthreads();
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (I < ne) {
-        int nb[4];
+        // inviscid residual, as the structured kernel's
+        double R[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        auto add = [&](int s, double sx, double sy) {
+            const double2 w = uv[s], r = rp[s], h = hr[s];
+            const double vn = w.x * sx + w.y * sy;
+            const double m = r.x * vn;
+            R[0] = R[0] + m;
+            R[1] = fma(m, w.x, fma(r.y, sx, R[1]));
+            R[2] = fma(m, w.y, fma(r.y, sy, R[2]));
+            R[3] = fma(h.x, vn, R[3]);
+            R[4] = fma(m, h.y, R[4]);
+        };
+        add(t, (SX[0] + SX[2]) + (SX[1] + SX[3]), (SY[0] + SY[2]) + (SY[1] + SY[3]));
 #pragma unroll
-        for (int k = 0; k < 4; k++) nb[k] = M.lnb[k * ne + I];
-        const double* G = M.cg + I;
+        for (int k = 0; k < 4; k++) {
+            if (nb[k] < 0) {  // a ghost
+                nb[k] = ~nb[k];
+#pragma unroll
+                for (int m = 0; m < 5; m++) R[m] = R[m] + gf[m * M.hmax + nb[k] - UT];
+            } else {
+                add(nb[k], SX[k], SY[k]);
+            }
+        }
         double src3, src5;
         {
             SrcIn s;
-            s.ga = G[UCG_GA * ne]; s.gb = G[UCG_GB * ne]; s.gc = G[UCG_GC * ne]; s.gd = G[UCG_GD * ne];
+            s.ga = G[UCG_GA * n]; s.gb = G[UCG_GB * n]; s.gc = G[UCG_GC * n]; s.gd = G[UCG_GD * n];
             const double2 ua = uv[nb[0]], ub = uv[nb[1]], uc = uv[nb[2]], ud = uv[nb[3]];
-            const double2 ra = rq[nb[0]], rb = rq[nb[1]], rc = rq[nb[2]], rd = rq[nb[3]];
             s.ua = ua.x; s.ub = ub.x; s.uc = uc.x; s.ud = ud.x;
             s.va = ua.y; s.vb = ub.y; s.vc = uc.y; s.vd = ud.y;
-            s.ra = ra.x; s.rb = rb.x; s.rc = rc.x; s.rd = rd.x;
-            s.qa = ra.y; s.qb = rb.y; s.qc = rc.y; s.qd = rd.y;
-            source_terms(P, s, own_rho, rq[t].x, own_t, own_p, uv[t].y, G[UCG_YCC * ne], G[UCG_RYCC * ne], src3,
-                         src5);
+            s.ra = hr[nb[0]].y; s.rb = hr[nb[1]].y; s.rc = hr[nb[2]].y; s.rd = hr[nb[3]].y;
+            s.qa = qm[nb[0]]; s.qb = qm[nb[1]]; s.qc = qm[nb[2]]; s.qd = qm[nb[3]];
+            source_terms(P, s, rp[t].x, hr[t].y, own_t, rp[t].y, uv[t].y, G[UCG_YCC * n], G[UCG_RYCC * n], src3, src5);
         }
-        double R[5];
+        // update (residual.f90:67-83), the sources per volume
+        double e[5], Cn[5], Co[5];
+        if (FIRST) {
+            double v[4];
+            u_gather_faces(M, A.vf, I, v);
+            e[0] = A.d[I];
 #pragma unroll
-        for (int m = 0; m < 5; m++) {
-            const double2* F = fg + m * ns;
-            const double2 Fi = F[t], a = F[nb[0]], b = F[nb[1]], e = F[nb[2]], d = F[nb[3]];
-            R[m] = HALF * ((Fi.x + a.x) * G[UCG_SX1 * ne] + (Fi.y + a.y) * G[UCG_SY1 * ne] +
-                           (Fi.x + b.x) * G[UCG_SX2 * ne] + (Fi.y + b.y) * G[UCG_SY2 * ne] +
-                           (Fi.x + e.x) * G[UCG_SX3 * ne] + (Fi.y + e.y) * G[UCG_SY3 * ne] +
-                           (Fi.x + d.x) * G[UCG_SX4 * ne] + (Fi.y + d.y) * G[UCG_SY4 * ne]);
+            for (int m = 1; m < 5; m++) e[m] = v[m - 1] + A.d[m * n + I];
+#pragma unroll
+            for (int m = 0; m < 4; m++) A.vis[m * n + I] = v[m];
+#pragma unroll
+            for (int m = 0; m < 5; m++) A.e[m * n + I] = e[m];
+        } else {
+#pragma unroll
+            for (int m = 0; m < 5; m++) e[m] = A.e[m * n + I];
         }
-        const double VOL = G[UCG_VOL * ne];
-        R[4] = R[4] - VOL * src5;
-        if (P.iaxis == 1) R[2] = R[2] - VOL * src3;
-        const double DT = P.local ? A.dt[I] : *A.dtmin;
-        const double DTBYVOL = DT * G[UCG_RVOL * ne];
-        const double al = A.alpha;
-        double Cn[5], Co[5];
 #pragma unroll
-        for (int m = 0; m < 5; m++) Co[m] = A.qold[m * ne + I];
-        Cn[0] = Co[0] - al * DTBYVOL * (R[0] - A.d[I]);
-        Cn[1] = Co[1] - al * DTBYVOL * (R[1] - A.vis[I] - A.d[ne + I]);
-        Cn[2] = Co[2] - al * DTBYVOL * (R[2] - A.vis[ne + I] - A.d[2 * ne + I]);
-        Cn[3] = Co[3] - al * DTBYVOL * (R[3] - A.vis[2 * ne + I] - A.d[3 * ne + I]);
-        Cn[4] = Co[4] - al * DTBYVOL * CFLTURB * (R[4] - A.vis[3 * ne + I] - A.d[4 * ne + I]);
-        Cn[4] = Cn[0] * dmax1(P.rtol, Cn[4] / Cn[0]);
+        for (int m = 0; m < 5; m++) Co[m] = A.qold[m * n + I];
+        const double RVOL = G[UCG_RVOL * n];
+        const double aDT = A.alpha * (P.local ? A.dt[I] : *A.dtmin);
+        Cn[0] = Co[0] - aDT * (RVOL * (HALF * R[0] - e[0]));
+        Cn[1] = Co[1] - aDT * (RVOL * (HALF * R[1] - e[1]));
+        Cn[2] = Co[2] - aDT * fma(RVOL, HALF * R[2] - e[2], -src3);
+        Cn[3] = Co[3] - aDT * (RVOL * (HALF * R[3] - e[3]));
+        Cn[4] = Co[4] - aDT * CFLTURB * fma(RVOL, HALF * R[4] - e[4], -src5);
+        Cn[4] = Cn[0] * dmax1(P.rtol, Cn[4] * recip(Cn[0]));
 #pragma unroll
-        for (int m = 0; m < 5; m++) A.qout[m * ne + I] = Cn[m];
+        for (int m = 0; m < 5; m++) A.qout[m * n + I] = Cn[m];
         if (A.status) {
             bool bad = false;
 #pragma unroll
@@ -431,7 +477,9 @@ __global__ void __launch_bounds__(UT, TNS_U_CHUNK_MINB) k_u_stage_chunk(Params P
     }
 }
 
-size_t u_chunk_smem_bytes(const UMesh& M) { return sizeof(double2) * 7 * ((size_t)UT + M.hmax); }
+size_t u_chunk_smem_bytes(const UMesh& M) {
+    return 7 * sizeof(double) * ((size_t)UT + M.hmax) + 5 * sizeof(double) * (size_t)M.hmax;
+}
 
 // POSTPROCESS node averages (solver_state.f90:237-281): P, U, V, T of the contributions
 // in the same visit order, divided by their count; out [4][nnode].
@@ -507,11 +555,12 @@ __global__ void __launch_bounds__(UT) k_u_bsums(Params P, UMesh M, const double*
 static unsigned blocks(long long n) { return (unsigned)((n + UT - 1) / UT); }
 
 void launch_u_prim(const Params& P, const UMesh& M, const double* q, double* W, cudaStream_t s) {
-    k_u_prim<<<blocks((long long)M.ne + M.ng), UT, 0, s>>>(P, M, StateF64{q, (size_t)M.ne}, W);
+    k_u_prim<StateF64, true><<<blocks((long long)M.ne + M.ng), UT, 0, s>>>(P, M, StateF64{q, (size_t)M.ne}, W);
 }
 void launch_u_prim_mx(const Params& P, const UMesh& M, const double* cold, const float* dq, double* W,
                       cudaStream_t s) {
-    k_u_prim<<<blocks((long long)M.ne + M.ng), UT, 0, s>>>(P, M, StateMixed{cold, dq, (size_t)M.ne}, W);
+    k_u_prim<StateMixed, true>
+        <<<blocks((long long)M.ne + M.ng), UT, 0, s>>>(P, M, StateMixed{cold, dq, (size_t)M.ne}, W);
 }
 void launch_u_gport(const Params& P, const UMesh& M, const double* q, cudaStream_t s) {
     if (M.nport > 0) k_u_gport<<<blocks(M.nport), UT, 0, s>>>(P, M, StateF64{q, (size_t)M.ne});
@@ -529,24 +578,25 @@ void launch_u_dissipation(const Params& P, const UMesh& M, const double* q, doub
     k_u_diss1<<<blocks(M.ne), UT, 0, s>>>(P, M, q, aux, dt, dtmin);
     k_u_diss2<<<blocks(M.ne), UT, 0, s>>>(M, q, aux, d);
 }
-void launch_u_viscous(const Params& P, const UMesh& M, const double* W, double* na, double* vf, double* vis,
+void launch_u_viscous(const Params& P, const UMesh& M, const double* q, double* W, double* na, double* vf,
                       cudaStream_t s) {
-    k_u_node_avg<<<blocks(M.nnode), UT, 0, s>>>(P, M, W, na);
-    k_u_vface<<<blocks(M.nface), UT, 0, s>>>(P, M, W, na, vf);
-    k_u_vsum<<<blocks(M.ne), UT, 0, s>>>(M, vf, vis);
+    const StateF64 st{q, (size_t)M.ne};
+    launch_tile(k_u_prim<StateF64, false>, dim3(blocks((long long)M.ne + M.ng)), dim3(UT), 0, s, P, M, st, W);
+    launch_tile(k_u_node_avg, dim3(blocks(M.nnode)), dim3(UT), 0, s, P, M, (const double*)W, na);
+    launch_tile(k_u_vface, dim3(blocks(M.nface)), dim3(UT), 0, s, P, M, (const double*)W, (const double*)na, vf);
 }
-void launch_u_viscous(const Params& P, const UMesh& M, const double* W, double* na, double* vf, float* vis,
-                      cudaStream_t s) {
-    k_u_node_avg<<<blocks(M.nnode), UT, 0, s>>>(P, M, W, na);
-    k_u_vface<<<blocks(M.nface), UT, 0, s>>>(P, M, W, na, vf);
-    k_u_vsum<<<blocks(M.ne), UT, 0, s>>>(M, vf, vis);
-}
-void launch_u_stage_chunk(const Params& P, const UMesh& M, const StageArgsU& A, const double* q, cudaStream_t s) {
-    k_u_stage_chunk<<<M.nchunk, UT, u_chunk_smem_bytes(M), s>>>(P, M, A, q);
+void launch_u_stage_chunk(const Params& P, const UMesh& M, const StageArgsU& A, bool first, const double* q,
+                          cudaStream_t s) {
+    launch_tile(first ? k_u_stage_chunk<true> : k_u_stage_chunk<false>, dim3(M.nchunk), dim3(UT),
+                u_chunk_smem_bytes(M), s, P, M, A, q);
 }
 cudaError_t configure_u_chunk(const UMesh& M) {
-    return cudaFuncSetAttribute(k_u_stage_chunk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)u_chunk_smem_bytes(M));
+    for (auto k : {k_u_stage_chunk<true>, k_u_stage_chunk<false>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)u_chunk_smem_bytes(M));
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 void launch_u_post_average(const UMesh& M, const double* W, double* out, cudaStream_t s) {
     k_u_post_avg<<<blocks(M.nnode), UT, 0, s>>>(M, W, out);
@@ -832,12 +882,12 @@ int umesh_build(tns_handle* h, const tns_mesh* m) {
                         }
                         l = loc[v];
                     }
-                    u->hlnb[(size_t)f * ne + k] = l;
+                    u->hlnb[(size_t)f * ne + k] = v >= ne ? ~l : l;
                 }
             u->hcptr[b + 1] = (int)u->hcslot.size();
             hmax = std::max(hmax, u->hcptr[b + 1] - u->hcptr[b]);
         }
-        // at most 4 UT halo slots: (UT + hmax) slots of 112 bytes fit a block's shared memory
+        // at most 4 UT halo slots: UT + hmax slots of 56 bytes and 40 a ghost fit a block's shared memory
         u->hmax = hmax;
     }
     // ghosts in bc.in order
@@ -1021,15 +1071,12 @@ void enqueue_iteration_u(tns_handle* h, bool monitor) {
         if (M.nport) launch(h, K_GPORT, [&] { tns::launch_u_gport(P, M, in[st], s); });
         if (st == 0) {
             // stage 1's field set W feeds the viscous flux (the chunked stages need none)
-            launch(h, K_VISC, [&] {
-                tns::launch_u_prim(P, M, in[st], u->W.p, s);
-                tns::launch_u_viscous(P, M, u->W.p, u->na.p, u->vf.p, h->vis.p, s);
-            }, 4);
+            launch(h, K_VISC, [&] { tns::launch_u_viscous(P, M, in[st], u->W.p, u->na.p, u->vf.p, s); }, 3);
             if (fork) cudaStreamWaitEvent(s, h->join, 0);
         }
-        tns::StageArgsU S{A, out[st], h->d.p, h->vis.p, h->dt.p, h->dtmin.p, alpha[st],
+        tns::StageArgsU S{A, out[st], h->d.p, u->vf.p, h->vis.p, h->e.p, h->dt.p, h->dtmin.p, alpha[st],
                           (monitor && st == 3) ? h->cdiff.p : nullptr, st == 3 ? h->status.p : nullptr};
-        launch(h, K_STAGE, [&] { tns::launch_u_stage_chunk(P, M, S, in[st], s); });
+        launch(h, K_STAGE, [&] { tns::launch_u_stage_chunk(P, M, S, st == 0, in[st], s); });
     }
 }
 
@@ -1061,16 +1108,13 @@ void enqueue_iteration_u_mx(tns_handle* h, bool monitor, double* A, double* Aout
     for (int st = 0; st < 4; st++) {
         if (M.nport) launch(h, K_GPORT, [&] { tns::launch_u_gport_mx(P, M, A, in[st], s); });
         if (st == 0) {
-            launch(h, K_VISC, [&] {
-                tns::launch_u_prim(P, M, A, u->W.p, s);
-                tns::launch_u_viscous(P, M, u->W.p, u->na.p, u->vf.p, h->visf.p, s);
-            }, 4);
+            launch(h, K_VISC, [&] { tns::launch_u_viscous(P, M, A, u->W.p, u->na.p, u->vf.p, s); }, 3);
             if (fork) cudaStreamWaitEvent(s, h->join, 0);
         }
         tns::StageArgsMx S{A, in[st], out[st], st == 3 ? Aout : nullptr, h->df.p, h->visf.p, h->dtf.p, h->dtmin.p,
                            (float)alpha[st], st ? h->ef.p : nullptr, st ? nullptr : h->ef.p,
                            (monitor && st == 3) ? h->cdiff.p : nullptr, st == 3 ? h->status.p : nullptr, h->status.p};
-        launch(h, K_STAGE, [&] { tns::launch_u_stage_chunk_mx(P, M, S, s); });
+        launch(h, K_STAGE, [&] { tns::launch_u_stage_chunk_mx(P, M, S, u->vf.p, h->visf.p, s); });
     }
 }
 

@@ -35,7 +35,9 @@ size_t u_chunk_mx_smem_bytes(const UMesh& M) {
 // nozzle-plume (B200, one mixed iteration): 4 -> 0.248 ms, 3 -> 0.264 ms, 5 -> 0.257 ms.
 #define TNS_U_CHUNK_MX_MINB 4
 #endif
-__global__ void __launch_bounds__(UT, TNS_U_CHUNK_MX_MINB) k_u_stage_chunk_mx(Params P, UMesh M, StageArgsMx A) {
+__global__ void __launch_bounds__(UT, TNS_U_CHUNK_MX_MINB) k_u_stage_chunk_mx(Params P, UMesh M, StageArgsMx A,
+                                                                            const double* __restrict__ vf,
+                                                                            float* vis) {
     extern __shared__ __align__(16) unsigned char usm_raw[];
     TileRefMx& R = *reinterpret_cast<TileRefMx*>(usm_raw);
     const int ns = UT + M.hmax;
@@ -113,19 +115,30 @@ __global__ void __launch_bounds__(UT, TNS_U_CHUNK_MX_MINB) k_u_stage_chunk_mx(Pa
     int nb[4];
     if (I < ne) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) nb[k] = M.lnb[k * ne + I];
+        for (int k = 0; k < 4; k++) {
+            const int l = M.lnb[k * ne + I];
+            nb[k] = l < 0 ? ~l : l;
+        }
         const float4* g = reinterpret_cast<const float4*>(M.gmx) + I;
         const double* g8 = M.gmx + 8 * n + I;
         G = GeoMx{g[0], g[n], g[2 * n], g[3 * n], g8[0], g8[n], P.iaxis == 1 ? g8[2 * n] : 0.0};
     }
     __syncthreads();
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (I < ne) stage_cell_mx(P, R, A, n, (size_t)I, W, t, nb, G, own, dv);
+    if (I < ne)
+        stage_cell_mx(P, R, A, n, (size_t)I, W, t, nb, G, own,
+                      [&](float v[4]) {
+                          double s[4];
+                          u_gather_faces(M, vf, I, s);
+#pragma unroll
+                          for (int m = 0; m < 4; m++) vis[m * n + I] = v[m] = (float)s[m];
+                      }, dv);
     if (A.cdiff) stage_cdiff_mx(A, dv);
 }
 
-void launch_u_stage_chunk_mx(const Params& P, const UMesh& M, const StageArgsMx& A, cudaStream_t s) {
-    launch_tile(k_u_stage_chunk_mx, dim3(M.nchunk), dim3(UT), u_chunk_mx_smem_bytes(M), s, P, M, A);
+void launch_u_stage_chunk_mx(const Params& P, const UMesh& M, const StageArgsMx& A, const double* vf, float* vis,
+                             cudaStream_t s) {
+    launch_tile(k_u_stage_chunk_mx, dim3(M.nchunk), dim3(UT), u_chunk_mx_smem_bytes(M), s, P, M, A, vf, vis);
 }
 
 cudaError_t configure_u_chunk_mx(const UMesh& M) {
