@@ -458,6 +458,11 @@ int upload_mesh(tns_handle* h) {
 int alloc_state(tns_handle* h) {
     const size_t nc = h->ncell();
     int rc;
+    if (!h->identity &&
+        ((rc = h->cuda(h->dcell_of.alloc(nc), "cudaMalloc")) || (rc = h->cuda(h->renum.alloc(5 * nc), "cudaMalloc")) ||
+         (rc = h->cuda(cudaMemcpy(h->dcell_of.p, h->cell_of.data(), nc * sizeof(int), cudaMemcpyHostToDevice),
+                       "cudaMemcpy"))))
+        return rc;
     if (h->precision == 1) {
         if ((rc = h->cuda(h->qa.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->qa2.alloc(5 * nc), "cudaMalloc")) ||
             (rc = h->cuda(h->dqb.alloc(5 * nc), "cudaMalloc")) || (rc = h->cuda(h->dqc.alloc(5 * nc), "cudaMalloc")) ||
@@ -695,28 +700,25 @@ int tns_upload_state(tns_handle* h, const double* c1, const double* c2, const do
     const size_t nc = h->ncell();
     const double* src[5] = {c1, c2, c3, c4, c5};
     int rc;
-    bool direct = h->identity;
-    for (int m = 0; m < 5 && direct; m++) {
-        cudaPointerAttributes at;
-        direct = cudaPointerGetAttributes(&at, src[m]) == cudaSuccess && at.type == cudaMemoryTypeHost;
-    }
-    cudaGetLastError();
+    // a state in the caller's own numbering is put in the device's order there
+    double* dst = h->identity ? h->state() : h->renum.p;
+    bool direct = true;
+    for (int m = 0; m < 5 && direct; m++) direct = page_locked(src[m]);
     if (direct) {
         // page-locked caller arrays: one DMA per component, no staging copy
         for (int m = 0; m < 5; m++)
-            if ((rc = h->cuda(cudaMemcpyAsync(h->state() + m * nc, src[m], nc * 8, cudaMemcpyHostToDevice,
-                                              h->stream), "cudaMemcpyAsync")))
+            if ((rc = h->cuda(cudaMemcpyAsync(dst + m * nc, src[m], nc * 8, cudaMemcpyHostToDevice, h->stream),
+                              "cudaMemcpyAsync")))
                 return rc;
     } else {
-        for (int m = 0; m < 5; m++) {
-            double* dst = h->pinned + m * nc;
-            if (h->identity) std::memcpy(dst, src[m], nc * 8);
-            else
-                for (size_t k = 0; k < nc; k++) dst[k] = src[m][h->cell_of[k]];
-        }
-        if ((rc = h->cuda(cudaMemcpyAsync(h->state(), h->pinned, 5 * nc * 8, cudaMemcpyHostToDevice, h->stream),
+        for (int m = 0; m < 5; m++) std::memcpy(h->pinned + m * nc, src[m], nc * 8);
+        if ((rc = h->cuda(cudaMemcpyAsync(dst, h->pinned, 5 * nc * 8, cudaMemcpyHostToDevice, h->stream),
                           "cudaMemcpyAsync")))
             return rc;
+    }
+    if (!h->identity) {
+        tns::launch_renumber(h->dcell_of.p, dst, h->state(), nc, true, h->stream);
+        if ((rc = h->cuda(cudaGetLastError(), "kernel launch"))) return rc;
     }
     rc = h->cuda(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
     if (rc) return rc;
@@ -944,30 +946,26 @@ int tns_download_state(tns_handle* h, double* c1, double* c2, double* c3, double
     if (!h->have_state) return h->fail(TNS_ERR_STATE, "tns_download_state: no state");
     const size_t nc = h->ncell();
     double* dst[5] = {c1, c2, c3, c4, c5};
-    bool direct = h->identity;
-    for (int m = 0; m < 5 && direct; m++) {
-        cudaPointerAttributes at;
-        direct = cudaPointerGetAttributes(&at, dst[m]) == cudaSuccess && at.type == cudaMemoryTypeHost;
-    }
-    cudaGetLastError();
     int rc;
+    const double* src = h->state();
+    if (!h->identity) {
+        tns::launch_renumber(h->dcell_of.p, src, h->renum.p, nc, false, h->stream);
+        if ((rc = h->cuda(cudaGetLastError(), "kernel launch"))) return rc;
+        src = h->renum.p;
+    }
+    bool direct = true;
+    for (int m = 0; m < 5 && direct; m++) direct = page_locked(dst[m]);
     if (direct) {
         // page-locked caller arrays: one DMA per component, no staging copy
         for (int m = 0; m < 5; m++)
-            if ((rc = h->cuda(cudaMemcpyAsync(dst[m], h->state() + m * nc, nc * 8, cudaMemcpyDeviceToHost,
-                                              h->stream), "cudaMemcpyAsync")))
+            if ((rc = h->cuda(cudaMemcpyAsync(dst[m], src + m * nc, nc * 8, cudaMemcpyDeviceToHost, h->stream),
+                              "cudaMemcpyAsync")))
                 return rc;
         return h->cuda(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
     }
-    rc = h->cuda(cudaMemcpyAsync(h->pinned, h->state(), 5 * nc * 8, cudaMemcpyDeviceToHost, h->stream),
-                 "cudaMemcpyAsync");
+    rc = h->cuda(cudaMemcpyAsync(h->pinned, src, 5 * nc * 8, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpyAsync");
     if (rc || (rc = h->cuda(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize"))) return rc;
-    for (int m = 0; m < 5; m++) {
-        const double* src = h->pinned + m * nc;
-        if (h->identity) std::memcpy(dst[m], src, nc * 8);
-        else
-            for (size_t k = 0; k < nc; k++) dst[m][h->cell_of[k]] = src[k];
-    }
+    for (int m = 0; m < 5; m++) std::memcpy(dst[m], h->pinned + m * nc, nc * 8);
     return TNS_OK;
 }
 
@@ -1248,7 +1246,7 @@ void tns_destroy(tns_handle* h) {
         if (g) cudaGraphExecDestroy(g);
     if (h->graph_mon) cudaGraphExecDestroy(h->graph_mon);
     h->qa2.release(); h->dqb.release(); h->dqc.release(); h->df.release(); h->visf.release(); h->ef.release();
-    h->dtf.release(); h->tref.release();
+    h->dtf.release(); h->tref.release(); h->dcell_of.release(); h->renum.release();
     for (auto* b : {&h->x, &h->y, &h->cfldl, &h->gxc, &h->gyc, &h->ginj, &h->gport, &h->qa, &h->qb,
                     &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->vcfl, &h->e, &h->wport, &h->wport_i,
                     &h->stile, &h->vtile})

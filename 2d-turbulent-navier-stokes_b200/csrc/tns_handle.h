@@ -59,6 +59,8 @@ struct tns_handle {
     int ni = 0, nj = 0, neles = 0, nods = 0, nghosts = 0, maxid = 0;
     std::vector<int> cell_of;   // structured index k -> 0-based original cell id
     bool identity = true;
+    DevBuf<int> dcell_of;  // cell_of on the device, and a state in the caller's numbering
+    DevBuf<double> renum;  // (both where identity is false)
     std::vector<int> ghost_line;  // device ghost index -> bc.in line
     std::vector<int> ghost_id;    // bc.in line -> Fortran ghost id
     std::vector<int> port_ghosts;

@@ -972,6 +972,28 @@ void launch_batch_f64(const BatchCase* cases, const int4* tiles, const int* acti
         launch_tile(k_stage_batch, dim3(ntiles), blk, stage_smem_bytes(), s, cases, tiles, active, stage, monitor);
 }
 
+// A state between the caller's numbering and the device's.  The host loop it replaces took a
+// cache miss a value: 98,304 cells up and down, 0.9 ms of a 3.2 ms pass.
+template <bool TO_DEVICE>
+__global__ void __launch_bounds__(256) k_renumber(const int* __restrict__ cell_of, const double* __restrict__ src,
+                                                  double* __restrict__ dst, size_t n) {
+    const size_t k = blockIdx.x * (size_t)256 + threadIdx.x;
+    if (k >= n) return;
+    const size_t c = (size_t)cell_of[k];
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        if (TO_DEVICE) dst[m * n + k] = src[m * n + c];
+        else dst[m * n + c] = src[m * n + k];
+    }
+}
+
+void launch_renumber(const int* cell_of, const double* src, double* dst, size_t ncell, bool to_device,
+                     cudaStream_t s) {
+    const unsigned grid = (unsigned)((ncell + 255) / 256);
+    if (to_device) k_renumber<true><<<grid, 256, 0, s>>>(cell_of, src, dst, ncell);
+    else k_renumber<false><<<grid, 256, 0, s>>>(cell_of, src, dst, ncell);
+}
+
 void launch_dissipation(const Params& P, const Mesh& M, const double* q, double* d, double* dt,
                         const double* dtmin, cudaStream_t s) {
     DissArgs<double> A{q, d, dt, dtmin};

@@ -15,6 +15,9 @@ size_t visc_smem_bytes();
 size_t diss_smem_bytes();
 int dtmin_blocks(const Mesh& M);
 int sm_count();  // SMs of the current device
+// a state's five components between the caller's cell numbering and the device's: cell k of the
+// device order is the caller's cell_of[k]
+void launch_renumber(const int* cell_of, const double* src, double* dst, size_t ncell, bool to_device, cudaStream_t s);
 
 void launch_dissipation(const Params& P, const Mesh& M, const double* q, double* d, double* dt,
                         const double* dtmin, cudaStream_t s);
