@@ -240,7 +240,7 @@ TNS_HD void s0_point(const AdjArgs& a, long long ps) {
 // Reverse of COMPUTE_PRIMITIVE_VARS (turbnstwod.f90:204-227) for one cell: the adjoint
 // of its field-set rows wb -> the adjoint of its conservative state qb (added).
 TNS_HD void prim_adj(const Params& P, const double q[5], const double wb[NWROW], double qb[5]) {
-    const double irho = 1.0 / q[0];
+    const double irho = recip(q[0]);
     const double rho = q[0], u = q[1] * irho, v = q[2] * irho, e = q[3] * irho;
     const double t = (e - 0.5 * (u * u + v * v)) * P.inv_cv;
     const double p = rho * P.rr * t, rt = q[4] * irho;
@@ -469,12 +469,27 @@ TNS_HD void ghost_adj(const Params& P, int type, const double gw[NWROW], const d
 
 // ------------------------------------------------------------------ source terms
 
+// The reverse's arithmetic is the solver's: recip / root and one expm1 a tanh instead of
+// divisions, square roots and tanh calls with slow paths (stage reverse of 512 x 192 cells, with
+// its two evaluations of the sources, 36 -> 30 us; a step 364 -> 334).  The comparisons that
+// select a branch (the C5 and RTOL floors, the sensors' larger side, the signs of pressure
+// differences) keep the divisions they had, so that ties fall as before.
+// tanh(x) for x >= 0 (capped at 20, where it is 1 to double precision), its reciprocal and its
+// derivative 1 - tanh^2 = 4 (E + 1) / (E + 2)^2 from one E = expm1(2x).
+struct TanhWork {
+    double t, inv, d;
+};
+TNS_HD TanhWork tanh_work(double x) {
+    const double E = expm1_nonneg(2.0 * fmin(x, 20.0)), r = recip(E + 2.0);
+    return TanhWork{E * r, (E + 2.0) * recip(E), x < 20.0 ? 4.0 * (E + 1.0) * (r * r) : 0.0};
+}
+
 struct SrcWork {
     double dnr, yBD, yAC, xBD, xAC;
     double da[4], db[4];  // q r u v: A-C and B-D differences
     double ic1[4];        // 1 / C1 of the neighbours
     double GX[4], GY[4];  // DQX DRX DUX DVX / DQY DRY DUY DVY
-    double rho, ri, amu, chi, ta, tb, fmu, sc, t1, t2, fr2, amut, dee, vbyy, divvel, sum, aor, pk, ratio, pw,
+    double rho, ri, amu, chi, dta, dtb, dt1, dt2, fmu, sc, fr2, amut, dee, vbyy, divvel, sum, aor, pk, ratio, pw,
         x, sq, A5, s3, s5, ycc, den, T, idnr, irho, ia, itb, it2, iycc;
     bool pos, near, pkpos, selm;
 };
@@ -485,8 +500,8 @@ TNS_HD void src_forward(const Params& P, const double nb[4][4], const double nx[
                         double c5, double T, double Pc, double Vc, double ycc, SrcWork& s) {
     double f[4][4];  // q r u v per neighbour
     for (int k = 0; k < 4; k++) {
-        f[0][k] = sqrt(nb[k][0] * nb[k][0] + nb[k][1] * nb[k][1]);
-        s.ic1[k] = 1.0 / nb[k][2];
+        f[0][k] = root(nb[k][0] * nb[k][0] + nb[k][1] * nb[k][1]);
+        s.ic1[k] = recip(nb[k][2]);
         f[1][k] = nb[k][3] * s.ic1[k];
         f[2][k] = nb[k][0];
         f[3][k] = nb[k][1];
@@ -496,7 +511,7 @@ TNS_HD void src_forward(const Params& P, const double nb[4][4], const double nx[
     s.xBD = nx[1] - nx[3];
     s.xAC = nx[0] - nx[2];
     s.dnr = s.xAC * s.yBD - s.xBD * s.yAC;
-    s.idnr = 1.0 / s.dnr;
+    s.idnr = recip(s.dnr);
     for (int q = 0; q < 4; q++) {
         s.da[q] = f[q][0] - f[q][2];
         s.db[q] = f[q][1] - f[q][3];
@@ -507,21 +522,23 @@ TNS_HD void src_forward(const Params& P, const double nb[4][4], const double nx[
     const double DQY = s.GY[0], DRY = s.GY[1], DUY = s.GY[2], DVY = s.GY[3];
     s.rho = rho;
     s.T = T;
-    s.irho = 1.0 / rho;
+    s.irho = recip(rho);
     s.ri = c5 * s.irho;
-    s.amu = amu_of(P, T);
-    s.ia = 1.0 / (CMU * s.amu);
+    const FifthRoots tr = fifth_roots(T);
+    s.amu = P.suth_amol * (T * tr.m04);
+    s.ia = P.inv_cmu_suth * tr.m06;
     s.chi = rho * s.ri * s.ia;
     const double X2 = s.chi * s.chi;
-    s.ta = tanh(ALPHA_T * X2);
-    s.tb = tanh(BETA_T * X2);
-    s.itb = 1.0 / s.tb;
-    s.fmu = s.ta * s.itb;
-    s.sc = sqrt(s.chi);
-    s.t1 = tanh(s.sc);
-    s.t2 = tanh(s.chi * P.fr2k);
-    s.it2 = 1.0 / s.t2;
-    s.fr2 = s.t1 * s.it2;
+    s.sc = root(s.chi);
+    {
+        const TanhWork ta = tanh_work(ALPHA_T * X2), tb = tanh_work(BETA_T * X2);
+        const TanhWork t1 = tanh_work(s.sc), t2 = tanh_work(s.chi * P.fr2k);
+        s.dta = ta.d; s.dtb = tb.d; s.dt1 = t1.d; s.dt2 = t2.d;
+        s.itb = tb.inv;
+        s.fmu = ta.t * s.itb;
+        s.it2 = t2.inv;
+        s.fr2 = t1.t * s.it2;
+    }
     s.amut = s.fmu * rho * s.ri;
     const double phi = DQX * DRX + DQY * DRY;
     s.pos = phi > 0.0;
@@ -550,7 +567,7 @@ TNS_HD void src_forward(const Params& P, const double nb[4][4], const double nx[
     s.ratio = s.selm ? 1.0 : s.amut / s.den;  // x / x = 1 exactly
     s.pw = powi(s.ratio, P.npseudo);
     s.x = s.ri * s.pk;
-    s.sq = s.x > 0.0 ? sqrt(s.x) : 0.0;
+    s.sq = s.x > 0.0 ? root(s.x) : 0.0;
     s.A5 = rho * (CONST1 - CONST2 * s.fr2) * s.sq - rho * CONST3 * s.dee;
     s.s5 = s.A5 * s.pw;
     s.s3 = 0.0;
@@ -577,7 +594,7 @@ TNS_HD void src_reverse(const Params& P, const SrcWork& s, const double nb[4][4]
     const double fr2b = -A5b * s.rho * CONST2 * s.sq;
     const double sqb = A5b * s.rho * (CONST1 - CONST2 * s.fr2);
     const double deeb = -A5b * s.rho * CONST3;
-    const double xb = s.x > 0.0 ? sqb / (2.0 * s.sq) : 0.0;
+    const double xb = s.sq > 0.0 ? 0.5 * sqb * recip(s.sq) : 0.0;
     rib += xb * s.pk;
     const double pkb = xb * s.ri;
     if (P.iaxis == 1) {
@@ -629,12 +646,12 @@ TNS_HD void src_reverse(const Params& P, const SrcWork& s, const double nb[4][4]
     const double fmub = amutb * s.rho * s.ri;
     rhob += amutb * s.fmu * s.ri;
     rib += amutb * s.fmu * s.rho;
-    chib += fmub * (ALPHA_T * (1.0 - s.ta * s.ta) - s.fmu * BETA_T * (1.0 - s.tb * s.tb)) * s.itb * 2.0 * s.chi;
-    chib += fr2b * ((1.0 - s.t1 * s.t1) * 0.5 / s.sc - s.fr2 * (1.0 - s.t2 * s.t2) * P.fr2k) * s.it2;
+    chib += fmub * (ALPHA_T * s.dta - s.fmu * BETA_T * s.dtb) * s.itb * 2.0 * s.chi;
+    chib += fr2b * (s.dt1 * 0.5 * recip(s.sc) - s.fr2 * s.dt2 * P.fr2k) * s.it2;
     rhob += chib * s.ri * s.ia;
     rib += chib * s.rho * s.ia;
     amub -= chib * s.chi * s.ia * CMU;
-    b.t = amub * 0.6 * s.amu / s.T;  // AMU = SUTH sqrt(AMOL) T**0.6
+    b.t = amub * 0.6 * s.amu * recip(s.T);  // AMU = SUTH sqrt(AMOL) T**0.6
     b.c5 = rib * s.irho;
     rhob -= rib * s.ri * s.irho;
     b.c1 = rhob;
@@ -773,7 +790,7 @@ TNS_HD void s1_point(const AdjArgs& a, long long cell) {
         }
     }
     const double dtbyvolb = a.alpha * dtvb;
-    const double ivol = 1.0 / g.vol;
+    const double ivol = recip(g.vol);
     const double dtb = dtbyvolb * ivol;
     double volb = -dtb * DT * ivol;
     if (a.first) a.dtbar[cell] = dtb;
@@ -803,8 +820,10 @@ TNS_HD void s1_point(const AdjArgs& a, long long cell) {
     a.wself[4 * a.ncell + cell] = b.c5;
     for (int k = 0; k < 4; k++) {
         for (int q = 0; q < 4; q++) a.srcn[(k * 4 + q) * a.ncell + cell] = b.nb[k][q];
-        a.srcg[(k * 2 + 0) * a.ncell + cell] = b.nx[k];
-        a.srcg[(k * 2 + 1) * a.ncell + cell] = b.ny[k];
+        if (a.geo) {
+            a.srcg[(k * 2 + 0) * a.ncell + cell] = b.nx[k];
+            a.srcg[(k * 2 + 1) * a.ncell + cell] = b.ny[k];
+        }
     }
     if (a.sens) a.rtolc[cell] += rtolb;
     if (a.geo) {  // (the face-vector part of the residual reverse: geo_point)
@@ -872,8 +891,10 @@ TNS_HD void s3_point(const AdjArgs& a, long long cell) {
         wb[WV] += a.srcn[(kk * 4 + 1) * a.ncell + nc];
         wb[WC1] += a.srcn[(kk * 4 + 2) * a.ncell + nc];
         wb[WC5] += a.srcn[(kk * 4 + 3) * a.ncell + nc];
-        xcb += a.srcg[(kk * 2 + 0) * a.ncell + nc];
-        ycb += a.srcg[(kk * 2 + 1) * a.ncell + nc];
+        if (a.geo) {
+            xcb += a.srcg[(kk * 2 + 0) * a.ncell + nc];
+            ycb += a.srcg[(kk * 2 + 1) * a.ncell + nc];
+        }
     }
     wb[WT] += a.wself[0 * a.ncell + cell];
     wb[WP] += a.wself[1 * a.ncell + cell];
@@ -1081,7 +1102,7 @@ TNS_HD void v0_point(const AdjArgs& a, long long node) {
 // the flux it adds to VISU, VISV, VIST, VISR).  out: NVF values (see VF_*).
 TNS_HD void visc_face_adj(const Params& P, const FaceIn& f, const double w[4], double* out, long long stride) {
     const double ybd = f.yb - f.yd, yac = f.ya - f.yc, xbd = f.xb - f.xd, xac = f.xa - f.xc;
-    const double dnr = xac * ybd - xbd * yac, idnr = 1.0 / dnr;
+    const double dnr = xac * ybd - xbd * yac, idnr = recip(dnr);
     const double A[5] = {f.ua, f.va, f.ta, f.rhoa, f.ra}, B[5] = {f.ub, f.vb, f.tb, f.rhob, f.rb};
     const double C[5] = {f.uc, f.vc, f.tc, f.rhoc, f.rc}, D[5] = {f.ud, f.vd, f.td, f.rhod, f.rd};
     double da[5], db[5], GX[5], GY[5];
@@ -1096,23 +1117,25 @@ TNS_HD void visc_face_adj(const Params& P, const FaceIn& f, const double w[4], d
     const double DUX = GX[0], DVX = GX[1], DTX = GX[2], DRX = GX[4];
     const double DUY = GY[0], DVY = GY[1], DTY = GY[2], DRY = GY[4];
     const double UAVG = AV[0], VAVG = AV[1], TAVG = AV[2], RHOAVG = AV[3], RAVG = AV[4];
-    double YAVG = 0.0, VBYY = 0.0, DIVVEL;
+    double RYAVG = 0.0, VBYY = 0.0, DIVVEL;
     bool near = false;
     if (P.iaxis == 1) {
-        YAVG = 0.5 * (f.yb + f.yd);
+        const double YAVG = 0.5 * (f.yb + f.yd);
         near = YAVG < YAXIS_THRESH;
-        VBYY = near ? DVY : VAVG / YAVG;
+        RYAVG = near ? 0.0 : recip(YAVG);
+        VBYY = near ? DVY : VAVG * RYAVG;
         DIVVEL = DUX + DVY + VBYY;
     } else {
         DIVVEL = DUX + DVY;
     }
-    const double AMU = amu_of(P, TAVG);
+    const FifthRoots tr = fifth_roots(TAVG);
+    const double AMU = P.suth_amol * (TAVG * tr.m04);
     const double AK = AMU * P.cp_pr;
-    const double iac = 1.0 / (AMU * CMU);
+    const double iac = P.inv_cmu_suth * tr.m06;
     const double CHI = RHOAVG * RAVG * iac;
     const double X2 = CHI * CHI;
-    const double ta = tanh(ALPHA_T * X2), tb = tanh(BETA_T * X2), itb = 1.0 / tb;
-    const double FMU = ta * itb;
+    const TanhWork ta = tanh_work(ALPHA_T * X2), tb = tanh_work(BETA_T * X2);
+    const double itb = tb.inv, FMU = ta.t * itb;
     const double AMUT = RHOAVG * RAVG * FMU;
     const double AKT = AMUT * P.cp_prt;
     const double AMUEFF = AMU + AMUT, AKEFF = AK + AKT;
@@ -1153,8 +1176,8 @@ TNS_HD void visc_face_adj(const Params& P, const FaceIn& f, const double w[4], d
         if (near) {
             GYb[1] += DIVb;
         } else {
-            AVb[1] += DIVb / YAVG;
-            YAVGb = -DIVb * VBYY / YAVG;
+            AVb[1] += DIVb * RYAVG;
+            YAVGb = -DIVb * VBYY * RYAVG;
         }
     }
     double AMUb = AMUEFFb + AKEFFb * P.cp_pr;
@@ -1162,11 +1185,11 @@ TNS_HD void visc_face_adj(const Params& P, const FaceIn& f, const double w[4], d
     AVb[3] += AMUTb * RAVG * FMU;
     AVb[4] += AMUTb * RHOAVG * FMU;
     const double FMUb = AMUTb * RHOAVG * RAVG;
-    const double CHIb = FMUb * (ALPHA_T * (1.0 - ta * ta) - FMU * BETA_T * (1.0 - tb * tb)) * itb * 2.0 * CHI;
+    const double CHIb = FMUb * (ALPHA_T * ta.d - FMU * BETA_T * tb.d) * itb * 2.0 * CHI;
     AVb[3] += CHIb * RAVG * iac;
     AVb[4] += CHIb * RHOAVG * iac;
     AMUb -= CHIb * CHI * iac * CMU;
-    AVb[2] += AMUb * 0.6 * AMU / TAVG;
+    AVb[2] += AMUb * 0.6 * AMU * recip(TAVG);
     double Ab[5], Bb[5], Cb[5], Db[5];
     for (int q = 0; q < 5; q++) Ab[q] = Bb[q] = Cb[q] = Db[q] = 0.25 * AVb[q];
     double dnrb = 0.0, ybdb = 0.0, yacb = 0.0, xbdb = 0.0, xacb = 0.0;
@@ -1335,12 +1358,12 @@ TNS_HD void v3_point(const AdjArgs& a, long long ps) {
             s[3] += a.nbar[3 * a.nnode + node];
             if (m & 4) s[4] += a.nbar[4 * a.nnode + node];
         }
-    const double c1 = wv(a, WC1, ps), r = wv(a, WC5, ps) / c1;
+    const double ic1 = recip(wv(a, WC1, ps)), r = wv(a, WC5, ps) * ic1;
     a.wvisc[0 * a.npad + ps] = s[0];
     a.wvisc[1 * a.npad + ps] = s[1];
     a.wvisc[2 * a.npad + ps] = s[2];
-    a.wvisc[3 * a.npad + ps] = s[3] - s[4] * r / c1;
-    a.wvisc[4 * a.npad + ps] = s[4] / c1;
+    a.wvisc[3 * a.npad + ps] = s[3] - s[4] * r * ic1;
+    a.wvisc[4 * a.npad + ps] = s[4] * ic1;
     if (a.geo) {
         a.xcbar[ps] += xb;
         a.ycbar[ps] += yb;
@@ -1359,32 +1382,29 @@ TNS_HD double ts_pressure(const Params& P, const double* q, long long n, long lo
 // pressure and dtb of its local time step -> its conservative state and DL.
 TNS_HD void ts_adj(const Params& P, const double q[5], double cfldl, double pb, double dtb, double qb[5],
                    double& dlb) {
-    const double rho = q[0], u = q[1] / rho, v = q[2] / rho, e = q[3] / rho;
-    const double vel = sqrt(u * u + v * v);
-    const double t = (e - 0.5 * (u * u + v * v)) / P.cv;
-    const double sq = sqrt(P.gamrr * t);
-    const double den = fabs(vel) + sq;
-    const double dt = cfldl / den;
-    const double denb = -dtb * dt / den;
-    dlb += dtb * P.cfl / den;
+    const double rho = q[0], ir = recip(rho), u = q[1] * ir, v = q[2] * ir, e = q[3] * ir;
+    const double vel = root(u * u + v * v);
+    const double t = (e - 0.5 * (u * u + v * v)) * P.inv_cv;
+    const double sq = root(P.gamrr * t);
+    const double iden = recip(vel + sq);
+    const double denb = -dtb * cfldl * (iden * iden);
+    dlb += dtb * P.cfl * iden;
     double ub = 0.0, vb = 0.0, rhob = 0.0;
-    double tb = denb * P.gamrr / (2.0 * sq);
+    double tb = 0.5 * denb * P.gamrr * recip(sq);
     if (vel > 0.0) {
-        const double sb = denb / (2.0 * vel);
-        ub += 2.0 * u * sb;
-        vb += 2.0 * v * sb;
+        const double sb = denb * recip(vel);
+        ub += u * sb;
+        vb += v * sb;
     }
     rhob += pb * P.rr * t;
     tb += pb * rho * P.rr;
-    const double eb = tb / P.cv;
-    ub -= tb * u / P.cv;
-    vb -= tb * v / P.cv;
-    qb[3] += eb / rho;
-    rhob -= eb * e / rho;
-    qb[1] += ub / rho;
-    rhob -= ub * u / rho;
-    qb[2] += vb / rho;
-    rhob -= vb * v / rho;
+    const double eb = tb * P.inv_cv;
+    ub -= eb * u;
+    vb -= eb * v;
+    qb[3] += eb * ir;
+    qb[1] += ub * ir;
+    qb[2] += vb * ir;
+    rhob -= (eb * e + ub * u + vb * v) * ir;
     qb[0] += rhob;
 }
 
@@ -1507,10 +1527,10 @@ TNS_HD void d2_point(const AdjArgs& a, long long cell) {
     // this cell's own sensors
     const double sa = dz[DO_SA * n + cell], sr = dz[DO_SR * n + cell];
     const double numa = o[DP_NUMA * n + cell], dena = o[DP_DENA * n + cell];
-    const double Na = sa / dena, Da = -sa * numa / (dena * dena);
+    const double ia = recip(dena), Na = sa * ia, Da = -Na * numa * ia;
     const double numr = o[DP_NUMR * n + cell], denr = o[DP_DENR * n + cell], fl = 8.0 * q[0] * P.rtol;
     const double deff = denr >= fl ? denr : fl;
-    const double Nr = sr / deff, Deff = -sr * numr / (deff * deff);
+    const double ie = recip(deff), Nr = sr * ie, Deff = -Nr * numr * ie;
     const double Dr = denr >= fl ? Deff : 0.0;
     if (!(denr >= fl)) {
         qb[0] += Deff * 8.0 * P.rtol;
@@ -1532,11 +1552,11 @@ TNS_HD void d2_point(const AdjArgs& a, long long cell) {
         // the neighbour's sensors, in which this cell is a neighbour
         const double san = dz[DO_SA * n + nc], srn = dz[DO_SR * n + nc];
         const double numan = o[DP_NUMA * n + nc], denan = o[DP_DENA * n + nc];
-        const double Nan = san / denan, Dan = -san * numan / (denan * denan);
+        const double ian = recip(denan), Nan = san * ian, Dan = -Nan * numan * ian;
         const double numrn = o[DP_NUMR * n + nc], denrn = o[DP_DENR * n + nc];
         const double fln = 8.0 * a.qold[nc] * P.rtol;
         const double deffn = denrn >= fln ? denrn : fln;
-        const double Nrn = srn / deffn, Drn = denrn >= fln ? -srn * numrn / (deffn * deffn) : 0.0;
+        const double ien = recip(deffn), Nrn = srn * ien, Drn = denrn >= fln ? -Nrn * numrn * ien : 0.0;
         pb += Nan * sgn(p - pn) + Dan * sgn(p + pn);
         c5b += Nrn * sgn(c5 - c5n) + Drn * sgn(c5 + c5n);
     }
@@ -1547,8 +1567,8 @@ TNS_HD void d2_point(const AdjArgs& a, long long cell) {
     CellGeo g;
     cell_geo(a, i, j, g);
     const double vbdb = dz[DO_VBD * n + cell];
-    const double volb = vbdb / dt;
-    const double dtb = a.dtbar[cell] - vbdb * g.vol / (dt * dt);
+    const double idt = recip(dt), volb = vbdb * idt;
+    const double dtb = a.dtbar[cell] - volb * g.vol * idt;
     double dlb = 0.0;
     ts_adj(P, q, a.M.cfldl[cell], pb, P.local ? dtb : 0.0, qb, dlb);
     if (!P.local) a.dtbar[cell] = dtb;
