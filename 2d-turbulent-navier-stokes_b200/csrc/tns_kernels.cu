@@ -61,6 +61,15 @@ struct StageSmem {
 
 size_t stage_smem_bytes() { return sizeof(StageSmem); }
 
+// With extra thread rows, the update operands of the tile's cells too: Q_old, DT and VIS + D (in
+// stage 1 D and VIS), a plane of NTHREADS each, asked for with the states: their latency is then
+// no longer the end of the tile's chain (115 x 50 nozzle, an iteration, 22.2 -> 20.6 us; 201 x 67
+// ramp 23.1 -> 21.9; in registers instead 21.6, and 5 % slower at two blocks an SM).  With more
+// tiles the other blocks hide it, and the shared memory is worth more as L1 (384 tiles: 35.7 ->
+// 38.8 us, so those read the operands at the end).
+enum RimOp { RO_QOLD, RO_DT = 5, RO_E = 6, RO_D = 6, RO_VIS = 11, RO_N = 15 };
+constexpr size_t RIM_SMEM = sizeof(StageSmem) + sizeof(double) * RO_N * NTHREADS;
+
 __device__ __forceinline__ void put_slot(StageSlots& S, int s, const Prim& p, double h) {
     S.uv[s] = make_double2(p.u, p.v);
     S.rp[s] = make_double2(p.rho, p.p);
@@ -199,13 +208,14 @@ __device__ __forceinline__ void stage_cell(const Params& P, const Mesh& M, const
     for (int m = 0; m < 5; m++) dv[m] = fabs(Co[m] - Cn[m]);
 }
 
-// The frozen terms VIS + D of a cell, by stage 1.
-__device__ __forceinline__ void frozen_terms(const StageArgs& A, size_t ncell, size_t cell, double e[5]) {
+// The frozen terms VIS + D of a cell, by stage 1; D and VIS read from planes `dst` apart.
+__device__ __forceinline__ void frozen_terms(const StageArgs& A, size_t ncell, size_t cell, const double* dp,
+                                             const double* vp, size_t dst, double e[5]) {
     double d[5], v[4];
 #pragma unroll
-    for (int m = 0; m < 5; m++) d[m] = A.d[m * ncell + cell];
+    for (int m = 0; m < 5; m++) d[m] = dp[m * dst];
 #pragma unroll
-    for (int m = 0; m < 4; m++) v[m] = A.vis[m * ncell + cell];
+    for (int m = 0; m < 4; m++) v[m] = vp[m * dst];
     e[0] = d[0];
 #pragma unroll
     for (int m = 1; m < 5; m++) e[m] = v[m - 1] + d[m];
@@ -271,6 +281,22 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
     double qo[5], qr[5], own_t = 0.0;
     if (valid) load(i, j, qo);
     if (h.kind >= 0) load(h.ci, h.cj, qr);
+    double* op = reinterpret_cast<double*>(smem_raw + sizeof(StageSmem)) + tid;
+    if (RIM && valid) {
+        const size_t cell = (size_t)i * M.nj + j;
+        auto fetch = [&](int at, int n, const double* src) {
+#pragma unroll
+            for (int m = 0; m < n; m++) copy_async(op + (at + m) * NTHREADS, src + m * ncell + cell);
+        };
+        fetch(RO_QOLD, 5, A.qold);
+        if (P.local) fetch(RO_DT, 1, A.dt);
+        if (A.e) {
+            fetch(RO_E, 5, A.e);
+        } else {
+            fetch(RO_D, 5, A.d);
+            fetch(RO_VIS, 4, A.vis);
+        }
+    }
     if (valid) own_t = put_cell_slot(P, S.w, (ti + 1) * SW + tj + 1, qo);
     if (h.kind >= 0) put_halo_slot(P, M, S.w, h, site, qr, [&](double c[5]) { load(h.ci + h.oi, h.cj + h.oj, c); });
     __syncthreads();
@@ -279,6 +305,7 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
         // this block's shared memory) and leave the tile
         if (tid == 0) atomicOr(A.error, 2u);
         bulk_wait(&S.bar);
+        if (RIM) copies_wait();
         return;
     }
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -286,14 +313,18 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
         const size_t cell = (size_t)i * M.nj + j;
         stage_cell(P, M, A, S.w, S.st, S.st + 2 * SNN, inner, i, j, own_t,
                    [&](StageOps& o) {
+                       if (RIM) copies_wait();
 #pragma unroll
-                       for (int m = 0; m < 5; m++) o.qold[m] = A.qold[m * ncell + cell];
-                       o.dt = P.local ? A.dt[cell] : *A.dtmin;
+                       for (int m = 0; m < 5; m++)
+                           o.qold[m] = RIM ? op[(RO_QOLD + m) * NTHREADS] : A.qold[m * ncell + cell];
+                       o.dt = !P.local ? *A.dtmin : RIM ? op[RO_DT * NTHREADS] : A.dt[cell];
                        if (A.e) {
 #pragma unroll
-                           for (int m = 0; m < 5; m++) o.e[m] = A.e[m * ncell + cell];
+                           for (int m = 0; m < 5; m++) o.e[m] = RIM ? op[(RO_E + m) * NTHREADS] : A.e[m * ncell + cell];
+                       } else if (RIM) {
+                           frozen_terms(A, ncell, cell, op + RO_D * NTHREADS, op + RO_VIS * NTHREADS, NTHREADS, o.e);
                        } else {
-                           frozen_terms(A, ncell, cell, o.e);
+                           frozen_terms(A, ncell, cell, A.d + cell, A.vis + cell, ncell, o.e);
                        }
                    }, dv);
     }
@@ -906,7 +937,7 @@ static bool stage_maps(const Params& P, const Mesh& M, const StageArgs& A, Stage
 cudaError_t configure_kernels() {
     cudaError_t e;
     for (auto k : {k_stage<0, false>, k_stage<1, false>, k_stage<0, true>, k_stage<1, true>}) {
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem_bytes());
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RIM_SMEM);
         if (e != cudaSuccess) return e;
     }
     e = cudaFuncSetAttribute(k_stage_pipe<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1028,13 +1059,13 @@ void launch_stage(const Params& P, const Mesh& M, const double* qin, const doubl
         return;
     }
     // the rim rows while every tile has its own resident block of that size: 115 x 50 nozzle,
-    // an iteration, 22.7 -> 22.2 us; 400 x 160 ramp (250 tiles) 31.2 -> 28.0.  The tiles of
+    // an iteration, 22.7 -> 22.2 us (20.6 with the operands fetched early); 400 x 160 ramp (250
+    // tiles) 31.2 -> 28.0.  The tiles of
     // other cases in flight beside this mesh count too: their warps fill the gaps, and the
     // larger blocks would only displace them (16 ramp cases on branch streams, 20 iterations:
     // 6.05 ms with the rim rows, 5.28 without; 4 cases 1.63 and 1.50)
     if (ntiles + beside <= TNS_STAGE_RIM_PER_SM * sm_count())
-        launch_tile(cdiff ? k_stage<1, true> : k_stage<0, true>, grid, dim3(TJ, TI + RIM_ROWS), stage_smem_bytes(), s, P,
-                    M, A);
+        launch_tile(cdiff ? k_stage<1, true> : k_stage<0, true>, grid, dim3(TJ, TI + RIM_ROWS), RIM_SMEM, s, P, M, A);
     else
         launch_tile(cdiff ? k_stage<1, false> : k_stage<0, false>, grid, dim3(TJ, TI), stage_smem_bytes(), s, P, M, A);
 }

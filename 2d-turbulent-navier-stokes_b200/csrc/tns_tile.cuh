@@ -131,6 +131,15 @@ __device__ __forceinline__ void bulk_barrier_init(unsigned long long* bar) {
     // initialised yet, and the wait never ends
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// Per-thread copies of 4 or 8 bytes global -> shared that need no registers on the way; the
+// thread that issued them waits for all of its own (copies_wait).
+template <class T>
+__device__ __forceinline__ void copy_async(T* dst, const T* src) {
+    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "sizes cp.async takes");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"((int)sizeof(T)) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // barrier_expect: the phase completes when `bytes` of copies have arrived.
 __device__ __forceinline__ void barrier_expect(unsigned long long* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;"
