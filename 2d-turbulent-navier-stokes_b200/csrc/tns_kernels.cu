@@ -4,10 +4,11 @@
 //   [k_dtmin]      global time step (LOCAL=0 only): per-cell DT and a grid-wide min
 //   k_dissipation  DT (LOCAL=1) and the frozen JST dissipation D of Q_old
 //                  (solver_state.f90:70-225), radius-2 shared-memory tile
-//   k_stage<1>     primitives + ghost BCs + nodal averages + viscous flux (frozen VIS)
-//                  + source + residual + update with alpha=1/4
-//   k_stage<0> x3  primitives + ghost BCs + source + residual + update (alpha 1/3,1/2,1);
-//                  the last one also reduces CDIFF and checks the state is finite.
+//   k_viscous      nodal averages and the frozen viscous flux VIS of Q_old, each face once
+//   k_stage        primitives + ghost BCs + source + residual + update, four times (alpha 1/4,
+//                  1/3, 1/2, 1); the first writes VIS + D for the others, the last one also
+//                  reduces CDIFF and checks the state is finite; k_stage_pipe is its form for
+//                  stages 2-4 of large meshes
 //   [k_gport]      type-6 port mass flux of the stage input (only if such ghosts exist)
 // Ghost cells are never stored: each tile evaluates the BC of the ghosts in its halo
 // from the parent and the parent's opposite neighbour, both already in the tile.

@@ -33,18 +33,20 @@ for _p in (ROOT, PKG):
 METRIC = "RK4 cell-iters/s on 1 B200, FP32 vs FP64 at equal residual; adjoint/primal time"
 UNIT = "cell-iter/s"
 # Compulsory DRAM bytes per cell for one launch of each kernel (FP64, 8 B words):
-#   dissipation: Q_old 5 + nodes 2 + CFL*DL 1 in, D 5 + DT 1 out                = 14 words
-#   viscous    : Q_old 5 + nodes 2 in, VIS 4 out                                = 11 words
-#   stage      : Q_in 5 + Q_old 5 + D 5 + VIS 4 + DT 1 + nodes 2 in, Q 5 out    = 27 words
-#                (stage 1 reads Q_in = Q_old once: 22 words; mean of the 4 = 25.75)
-KERNEL_BYTES_PER_CELL = {"dissipation": 112, "viscous": 88, "stage": 206}
-KERNEL_NAMES = {"dissipation": "k_dissipation", "viscous": "k_viscous", "stage": "k_stage"}
+# (the tiles' static blocks are not counted)
+#   dissipation: Q_old 5 + CFL*DL 1 + VOL/(CFL*DL) 1 in, D 5 + DT 1 out         = 13 words
+#   viscous    : Q_old 5 in, VIS 4 out                                          = 9 words
+#   stage      : Q_in 5 + Q_old 5 + (VIS + D) 5 + DT 1 in, Q 5 out              = 21 words
+#                (stage 1: Q_old 5 + D 5 + VIS 4 + DT 1 in, Q 5 + (VIS + D) 5 out: 25 words;
+#                mean of the 4 = 22)
+KERNEL_BYTES_PER_CELL = {"dissipation": 104, "viscous": 72, "stage": 176}
+KERNEL_NAMES = {"dissipation": "k_dissipation", "viscous": "k_viscous", "stage": "k_stage / k_stage_pipe"}
 # Mixed FP32/FP64 path: D, VIS, DT and the stage increments dQ are FP32 (4 B words):
-#   dissipation: Q_old 40 + nodes 16 + CFL*DL 8 in, D 20 + DT 4 out              = 88
-#   viscous    : Q_old 40 + nodes 16 in, VIS 16 out                              = 72
-#   stage      : Q_old 40 + dQ_in 20 + D 20 + VIS 16 + DT 4 + nodes 16 in,
-#                dQ_out 20 out (stage 4: Q_new 40); stage 1 reads no dQ_in        -> mean 143
-KERNEL_BYTES_PER_CELL_MX = {"dissipation": 88, "viscous": 72, "stage": 143}
+#   dissipation: Q_old 40 + CFL*DL 8 + VOL/(CFL*DL) 8 in, D 20 + DT 4 out        = 80
+#   viscous    : Q_old 40 in, VIS 16 out                                         = 56
+#   stage      : Q_old 40 + dQ_in 20 + (VIS + D) 20 + DT 4 in, dQ_out 20 out (stage 4: Q_new
+#                40); stage 1: Q_old 40 + D 20 + VIS 16 + DT 4 in, dQ_out 20 + 16 out -> mean 112
+KERNEL_BYTES_PER_CELL_MX = {"dissipation": 80, "viscous": 56, "stage": 112}
 KERNEL_NAMES_MX = {"dissipation": "k_dissipation_mx", "viscous": "k_viscous_mx", "stage": "k_stage_mx"}
 
 
