@@ -8,7 +8,7 @@
 //   k_stage        primitives + ghost BCs + source + residual + update, four times (alpha 1/4,
 //                  1/3, 1/2, 1); the first writes VIS + D for the others, the last one also
 //                  reduces CDIFF and checks the state is finite; k_stage_pipe is its form for
-//                  stages 2-4 of large meshes
+//                  large meshes
 //   [k_gport]      type-6 port mass flux of the stage input (only if such ghosts exist)
 // Ghost cells are never stored: each tile evaluates the BC of the ghosts in its halo
 // from the parent and the parent's opposite neighbour, both already in the tile.
@@ -342,28 +342,30 @@ k_stage(Params P, Mesh M, StageArgs A) {
     stage_tile<RIM>(P, M, Ac, blockIdx.x, blockIdx.y);
 }
 
-// Stages 2-4 of a large mesh, by resident blocks that walk its tiles (tile t, t + grid, ...)
+// A stage of a large mesh, by resident blocks that walk its tiles (tile t, t + grid, ...)
 // with the data of the next tile on its way through the TMA engine while they compute:
 //   a: the stage input's halo box (rows i0-1 .. i0+TI, columns j0-2 .. j0+TJ+1: one column
 //      early so that the box starts at a multiple of 16 bytes; positions outside the mesh
 //      arrive as zeros), asked for as soon as the tile before has formed its slots;
 //   b: the tile's static block, and
-//   c: Q_old, the frozen terms and DT of its cells, asked for when the tile before is done
-//      and needed when this one's slots are formed, and at its very end.
+//   c: Q_old, the frozen terms and DT of its cells (FIRST: D, VIS and DT), asked for when the
+//      tile before is done and needed when this one's slots are formed, and at its very end.
 // The copies take the global-load latency (4.7 of 11.6 stall cycles an instruction in the
 // kernel above, half of its time) out of the warps; a tile's buffers fit three times into an
-// SM because VIS + D is one array, so 24 warps stay resident at 80 registers (with D and VIS
+// SM because VIS + D is one array (and stage 1's Q_old is its input, read again from global
+// memory), so 24 warps stay resident at 80 registers (with D and VIS
 // apart and two blocks a SM it was no faster than the plain kernel).  What bounds it now:
 // issue (0.5 an SM quarter a cycle under 24 warps) and the launch.  1024 x 384 nozzle-plume,
 // a FP64 iteration: 0.153 ms with the plain kernel in all stages, 0.138 ms with this one;
-// 2048 x 768 port 0.647 -> 0.565 ms.  It needs more tiles than the plain kernel has resident
+// 2048 x 768 port 0.647 -> 0.565 ms; stage 1 by it as well 0.1179 -> 0.1161 ms.  It needs more tiles than the plain kernel has resident
 // blocks (at 384 tiles the two take the same 42 us an iteration) and rows and arrays that
 // TMA can address.
 constexpr int QH = TI + 2, QW = TJ + 4;  // halo box
 static_assert(QW % 2 == 0 && STILE % 2 == 0, "box rows and static blocks are multiples of 16 bytes");
 
 // Planes of the update operands
-enum StageOp { SO_QOLD, SO_E = 5, SO_DT = 10, SO_N };
+// (stage 1: VIS, D and DT; its Q_old is its input, and read again from global memory)
+enum StageOp { SO_QOLD, SO_VIS = 0, SO_E = 5, SO_DT = 10, SO_N };
 
 struct StagePipeSmem {
     // (128-byte aligned destinations first)
@@ -378,7 +380,7 @@ struct StageMaps {
     CUtensorMap q, qold, e, dt;
 };
 
-template <int MONITOR>
+template <int MONITOR, bool FIRST>
 __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MINB))
 k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ StageMaps maps) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -400,7 +402,7 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
     };
     auto fetch_c = [&](int t) {
         const int j0 = col_of(t) * TJ, i0 = row_of(t) * TI;
-        barrier_expect(&W.bar_c, sizeof(double) * (P.local ? SO_N : SO_DT) * NTHREADS);
+        barrier_expect(&W.bar_c, sizeof(double) * ((FIRST ? 9 : 10) + (P.local ? 1 : 0)) * NTHREADS);
         tensor_copy_3d(W.op[SO_E], &maps.e, j0, i0, 0, &W.bar_c);
         tensor_copy_3d(W.op[SO_QOLD], &maps.qold, j0, i0, 0, &W.bar_c);
         if (P.local) tensor_copy_3d(W.op[SO_DT], &maps.dt, j0, i0, 0, &W.bar_c);
@@ -472,10 +474,15 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
             stage_cell(P, M, A, S, W.st, W.st + 2 * SNN, inner, i, j, own_t,
                        [&](StageOps& o) {
                            ok = bulk_wait(&W.bar_c, parity) && ok;
+                           const size_t cell = (size_t)i * M.nj + j, ncell = (size_t)M.ni * M.nj;
 #pragma unroll
-                           for (int m = 0; m < 5; m++) {
-                               o.qold[m] = W.op[SO_QOLD + m][tid];
-                               o.e[m] = W.op[SO_E + m][tid];
+                           for (int m = 0; m < 5; m++)
+                               o.qold[m] = FIRST ? A.qold[m * ncell + cell] : W.op[SO_QOLD + m][tid];
+                           if (FIRST) {
+                               frozen_terms(A, ncell, cell, &W.op[SO_E][tid], &W.op[SO_VIS][tid], NTHREADS, o.e);
+                           } else {
+#pragma unroll
+                               for (int m = 0; m < 5; m++) o.e[m] = W.op[SO_E + m][tid];
                            }
                            o.dt = P.local ? W.op[SO_DT][tid] : *A.dtmin;
                        }, d);
@@ -898,7 +905,7 @@ int sm_count() {
 constexpr size_t PIPE_SMEM = sizeof(StagePipeSmem) + 128;  // (the kernel aligns its boxes to 128 bytes)
 static int pipe_grid() {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pipe<0>, NTHREADS, PIPE_SMEM) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pipe<0, false>, NTHREADS, PIPE_SMEM) != cudaSuccess)
         return 0;
     return per_sm * sm_count();
 }
@@ -931,8 +938,11 @@ static bool plane_map(const Mesh& M, const double* a, int planes, int rows, int 
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 static bool stage_maps(const Params& P, const Mesh& M, const StageArgs& A, StageMaps* m) {
-    return plane_map(M, A.qin, 5, QH, QW, &m->q) && plane_map(M, A.qold, 5, TI, TJ, &m->qold) &&
-           plane_map(M, A.e, 5, TI, TJ, &m->e) && plane_map(M, P.local ? A.dt : A.e, 1, TI, TJ, &m->dt);
+    const bool first = !A.e;
+    const double* e = first ? A.d : A.e;
+    return plane_map(M, A.qin, 5, QH, QW, &m->q) &&
+           (first ? plane_map(M, A.vis, 4, TI, TJ, &m->qold) : plane_map(M, A.qold, 5, TI, TJ, &m->qold)) &&
+           plane_map(M, e, 5, TI, TJ, &m->e) && plane_map(M, P.local ? A.dt : e, 1, TI, TJ, &m->dt);
 }
 
 cudaError_t configure_kernels() {
@@ -941,12 +951,10 @@ cudaError_t configure_kernels() {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RIM_SMEM);
         if (e != cudaSuccess) return e;
     }
-    e = cudaFuncSetAttribute(k_stage_pipe<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)PIPE_SMEM);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_stage_pipe<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)PIPE_SMEM);
-    if (e != cudaSuccess) return e;
+    for (auto k : {k_stage_pipe<0, false>, k_stage_pipe<1, false>, k_stage_pipe<0, true>}) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PIPE_SMEM);
+        if (e != cudaSuccess) return e;
+    }
     for (auto k : {k_viscous<false>, k_viscous<true>}) {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)visc_smem_bytes());
         if (e != cudaSuccess) return e;
@@ -1053,9 +1061,9 @@ void launch_stage(const Params& P, const Mesh& M, const double* qin, const doubl
     const dim3 grid = tile_grid(M);
     const int ntiles = grid.x * grid.y;
     StageMaps maps;
-    const int pipe = A.e && ntiles > TNS_PER_SM(TNS_STAGE_MINB) * sm_count() ? pipe_grid() : 0;
+    const int pipe = (A.e || !cdiff) && ntiles > TNS_PER_SM(TNS_STAGE_MINB) * sm_count() ? pipe_grid() : 0;
     if (pipe > 0 && pipe <= ntiles && stage_maps(P, M, A, &maps)) {
-        launch_tile(cdiff ? k_stage_pipe<1> : k_stage_pipe<0>, dim3(pipe), dim3(TJ, TI), PIPE_SMEM, s, P, M, A, ntiles,
+        launch_tile(!A.e ? k_stage_pipe<0, true> : cdiff ? k_stage_pipe<1, false> : k_stage_pipe<0, false>, dim3(pipe), dim3(TJ, TI), PIPE_SMEM, s, P, M, A, ntiles,
                     maps);
         return;
     }
