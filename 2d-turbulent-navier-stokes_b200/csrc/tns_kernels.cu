@@ -239,9 +239,10 @@ __device__ __forceinline__ void stage_cdiff(const StageArgs& A, const double dv[
 
 // One RK stage (turbnstwod.f90:204-227, boundary.f90:24-48, source_terms.f90:24-104,
 // residual.f90:23-83) on a TI x TJ tile with its halo staged in shared memory.  RIM: the block
-// has RIM_ROWS more rows of threads, which evaluate the halo.
+// has RIM_ROWS more rows of threads, which evaluate the halo.  False (for the whole block) where
+// the static block did not arrive: the block then leaves the kernel.
 template <bool RIM>
-__device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const StageArgs& A, int bx, int by) {
+__device__ __forceinline__ bool stage_tile(const Params& P, const Mesh& M, const StageArgs& A, int bx, int by) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StageSmem& S = *reinterpret_cast<StageSmem*>(smem_raw);
     const size_t ncell = (size_t)M.ni * M.nj;
@@ -300,14 +301,9 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
     }
     if (valid) own_t = put_cell_slot(P, S.w, (ti + 1) * SW + tj + 1, qo);
     if (h.kind >= 0) put_halo_slot(P, M, S.w, h, site, qr, [&](double c[5]) { load(h.ci + h.oi, h.cj + h.oj, c); });
-    __syncthreads();
-    if (!bulk_wait(&S.bar)) {
-        // the copy did not complete: report it, give it one more bounded wait (it writes
-        // this block's shared memory) and leave the tile
-        if (tid == 0) atomicOr(A.error, 2u);
-        bulk_wait(&S.bar);
+    if (!bulk_wait_block(&S.bar, A.error)) {
         if (RIM) copies_wait();
-        return;
+        return false;
     }
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid) {
@@ -330,6 +326,7 @@ __device__ __forceinline__ void stage_tile(const Params& P, const Mesh& M, const
                    }, dv);
     }
     if (A.cdiff) stage_cdiff(A, dv);
+    return true;
 }
 
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
@@ -510,11 +507,11 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
 size_t visc_smem_bytes() { return sizeof(ViscSmem); }
 
 template <bool RIM>
-__device__ __forceinline__ void viscous_tile_f64(const Params& P, const Mesh& M, const double* __restrict__ q,
+__device__ __forceinline__ bool viscous_tile_f64(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                  double* __restrict__ vis, unsigned int* error, int bx, int by) {
-    viscous_tile<RIM>(P, M, q, vis, error, bx, by,
-                 [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
-                     double out[4]) { viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
+    return viscous_tile<RIM>(P, M, q, vis, error, bx, by,
+                             [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd,
+                                 double ry, double out[4]) { viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
 
 template <bool RIM>
@@ -844,7 +841,8 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_BATCH_MINB)) k_
 // write disjoint arrays), then the four stages -- with a grid barrier between phases
 // (bounded waits: a barrier that gives up sets error bit 2 and the kernel returns).  A
 // block that finishes a tile synchronises before the next, whose static-block copy
-// reuses the tile's shared memory and barrier.  Cases need LOCAL=1 and no type-6 port
+// reuses the tile's shared memory and barrier; one whose copy did not arrive leaves (the
+// others then give up at the grid barrier).  Cases need LOCAL=1 and no type-6 port
 // (those add per-case reductions between the phases).
 #ifndef TNS_PERSIST_MINB
 #define TNS_PERSIST_MINB 3
@@ -858,12 +856,14 @@ k_batch_persistent(const BatchCase* __restrict__ cases, const int4* __restrict__
             const int nwork = ph == 0 ? 2 * ntiles : ntiles;
             for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
                 const int4 t = tiles[w % ntiles];
+                bool ok = true;
                 if (active[t.x]) {
                     const BatchCase& c = cases[t.x];
                     if (ph == 0 && w < ntiles) dissipation_tile_f64(c.P, c.M, c.diss, t.y, t.z);
-                    else if (ph == 0) viscous_tile_f64<false>(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
-                    else stage_tile<false>(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
+                    else if (ph == 0) ok = viscous_tile_f64<false>(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
+                    else ok = stage_tile<false>(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
                 }
+                if (!ok) return;  // the whole block
                 async_proxy_fence();
                 __syncthreads();
             }

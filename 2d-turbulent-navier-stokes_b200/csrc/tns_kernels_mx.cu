@@ -63,9 +63,10 @@ size_t stage_mx_smem_bytes() { return sizeof(StageSmemMx); }
 #define TNS_VISC_MX_BATCH_MINB 4
 #endif
 // One stage on tile (bx, by) of a mesh; the single-case and the batched kernels wrap it.
-// RIM: the block has RIM_ROWS more rows of threads, which form the halo.
+// RIM: the block has RIM_ROWS more rows of threads, which form the halo.  False (for the whole
+// block) where the static block did not arrive: the block then leaves the kernel.
 template <bool RIM>
-__device__ __forceinline__ void stage_mx_tile(const Params& P, const Mesh& M, const StageArgsMx& A,
+__device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, const StageArgsMx& A,
                                               int bx, int by) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StageSmemMx& S = *reinterpret_cast<StageSmemMx*>(smem_raw);
@@ -147,14 +148,7 @@ __device__ __forceinline__ void stage_mx_tile(const Params& P, const Mesh& M, co
         slot_ghost_mx(S.ref, gh, o);
         W.put(h.li * SW + h.lj, o);
     }
-    __syncthreads();
-    if (!bulk_wait(&S.bar)) {
-        // the copy did not complete: report it, give it one more bounded wait (it writes
-        // this block's shared memory) and leave the tile
-        if (tid == 0) atomicOr(A.error, 2u);
-        bulk_wait(&S.bar);
-        return;
-    }
+    if (!bulk_wait_block(&S.bar, A.error)) return false;
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid) {
         const int c = (ti + 1) * SW + (tj + 1);
@@ -171,6 +165,7 @@ __device__ __forceinline__ void stage_mx_tile(const Params& P, const Mesh& M, co
                       }, dv);
     }
     if (A.cdiff) stage_cdiff_mx(A, dv);
+    return true;
 }
 
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
@@ -235,11 +230,11 @@ __device__ __forceinline__ void viscous_face_mx(const Params& P, const FaceVals&
 }
 
 template <bool RIM>
-__device__ __forceinline__ void viscous_mx_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
+__device__ __forceinline__ bool viscous_mx_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                 float* __restrict__ vis, unsigned int* error, int bx, int by) {
-    viscous_tile<RIM>(P, M, q, vis, error, bx, by,
-                 [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
-                     double out[4]) { viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
+    return viscous_tile<RIM>(P, M, q, vis, error, bx, by,
+                             [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd,
+                                 double ry, double out[4]) { viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
 
 template <bool RIM>
@@ -327,7 +322,7 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_MX_BATCH_MINB)) 
 
 // A stage on a tile of a batch's case, its arguments in shared memory: constant-address loads
 // instead of loads through a descriptor pointer held in registers.
-__device__ __forceinline__ void stage_mx_batch_tile(const BatchCase& c, const StageArgsMx& args, int bx, int by) {
+__device__ __forceinline__ bool stage_mx_batch_tile(const BatchCase& c, const StageArgsMx& args, int bx, int by) {
 #if TNS_BATCH_SMEM_ARGS
     // (raw storage: the structs are copied in, never constructed)
     __shared__ __align__(16) unsigned char sargs[sizeof(Params) + sizeof(Mesh) + sizeof(StageArgsMx)];
@@ -339,9 +334,9 @@ __device__ __forceinline__ void stage_mx_batch_tile(const BatchCase& c, const St
     copy_words(&sM, &c.M, sizeof(Mesh), tid);
     copy_words(&sA, &args, sizeof(StageArgsMx), tid);
     __syncthreads();
-    stage_mx_tile<false>(sP, sM, sA, bx, by);
+    return stage_mx_tile<false>(sP, sM, sA, bx, by);
 #else
-    stage_mx_tile<false>(c.P, c.M, args, bx, by);
+    return stage_mx_tile<false>(c.P, c.M, args, bx, by);
 #endif
 }
 
@@ -370,15 +365,18 @@ k_batch_persistent_mx(const BatchCase* __restrict__ cases, const int4* __restric
             const int nwork = ph == 0 ? 2 * ntiles : ntiles;
             for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
                 const int4 t = tiles[w % ntiles];
+                bool ok = true;
                 if (active[t.x]) {
                     const BatchCase& c = cases[t.x];
                     if (ph == 0 && w < ntiles)
                         dissipation_mx_tile(c.P, c.M, c.qmx[parity], c.df, c.dtf, c.dtmin, t.y, t.z);
                     else if (ph == 0)
-                        viscous_mx_tile<false>(c.P, c.M, c.qmx[parity], c.visf, c.stage_mx[0][0][0].error, t.y, t.z);
+                        ok = viscous_mx_tile<false>(c.P, c.M, c.qmx[parity], c.visf, c.stage_mx[0][0][0].error, t.y,
+                                                    t.z);
                     else
-                        stage_mx_batch_tile(c, c.stage_mx[parity][0][ph - 1], t.y, t.z);
+                        ok = stage_mx_batch_tile(c, c.stage_mx[parity][0][ph - 1], t.y, t.z);
                 }
+                if (!ok) return;  // the whole block
                 async_proxy_fence();
                 __syncthreads();
             }

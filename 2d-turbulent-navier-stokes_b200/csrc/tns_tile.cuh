@@ -184,6 +184,22 @@ __device__ __forceinline__ bool bulk_wait(unsigned long long* bar, unsigned pari
     return false;
 }
 
+// Waits for the block's one-shot copy, and is the block barrier its threads would need there
+// anyway: the block goes on or gives up as one.  (Each thread counts its own polls, so around the
+// limit some see the copy and some do not; were each to leave by itself, those would miss the
+// block's later barriers, and in a kernel that loops over tiles run one barrier ahead of the
+// others into the next tile's buffers.)  On false the copy did not complete: that is reported
+// (bit 1 of *error), the copy, which writes this block's shared memory, had one more bounded wait,
+// and the caller leaves the kernel.
+__device__ __forceinline__ bool bulk_wait_block(unsigned long long* bar, unsigned int* error) {
+    if (__syncthreads_and(bulk_wait(bar))) return true;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        atomicOr(error, 2u);
+        bulk_wait(bar);
+    }
+    return false;
+}
+
 // Orders this thread's shared-memory accesses before later bulk copies into them (issued after
 // a block barrier), for kernels whose tiles reuse one buffer.
 __device__ __forceinline__ void async_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

@@ -44,11 +44,12 @@ __device__ __forceinline__ void face_values(const ViscSmem& S, int sa, int sc, i
 }
 
 // face(FaceVals, sx, sy, ga, gb, gc, gd, ryavg, double out[4]) evaluates one face's flux.
-// error: bit 1 is set when the tile's static copy did not complete.  RIM: the block has
+// False (for the whole block; bit 1 of *error set) where the tile's static copy did not complete:
+// the block then leaves the kernel.  RIM: the block has
 // RIM_ROWS more rows of threads, which take the halo, the nodes and the faces beyond the
 // cells' own.
 template <bool RIM, class OutT, class Face>
-__device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
+__device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                              OutT* __restrict__ vis, unsigned int* error, int bx, int by, Face face) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ViscSmem& S = *reinterpret_cast<ViscSmem*>(smem_raw);
@@ -181,14 +182,7 @@ __device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, con
     };
     if (mine && i <= M.ni && j <= M.nj) node(ti, tj, code0);
     if (extra && i0 + xa <= M.ni && j0 + xb <= M.nj) node(xa, xb, code1);
-    __syncthreads();
-    if (!bulk_wait(&S.bar)) {
-        // the copy did not complete: report it, give it one more bounded wait (it writes
-        // this block's shared memory) and leave the tile
-        if (tid == 0) atomicOr(error, 2u);
-        bulk_wait(&S.bar);
-        return;
-    }
+    if (!bulk_wait_block(&S.bar, error)) return false;
     auto eval = [&](int f, int sa, int sc, int ab, int ad) {
         FaceVals v;
         face_values(S, sa, sc, ab, ad, v);
@@ -221,7 +215,7 @@ __device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, con
         eval(iface ? la * TJ + lb : NIF + la * AW + lb, flip ? s : sb, flip ? sb : s, rev ? nb : n, rev ? n : nb);
     }
     __syncthreads();
-    if (!valid) return;
+    if (!valid) return true;
     const size_t cell = (size_t)i * M.nj + j;
     const int f1 = NIF + ti * AW + tj, f4 = ti * TJ + tj;  // j-face j, i-face i
     const double s1 = (j == 0) ? 1.0 : -1.0, s4 = (i == 0) ? 1.0 : -1.0;
@@ -229,6 +223,7 @@ __device__ __forceinline__ void viscous_tile(const Params& P, const Mesh& M, con
     for (int k = 0; k < 4; k++)
         vis[k * ncell + cell] =
             (OutT)(((s1 * S.fg[k][f1] + S.fg[k][f4 + TJ]) + S.fg[k][f1 + 1]) + s4 * S.fg[k][f4]);
+    return true;
 }
 
 }  // namespace tns

@@ -1,0 +1,53 @@
+"""How the tile kernels end a bounded wait for a bulk copy, read off their source.
+
+A wait that gives up is counted by each thread for itself, so threads of one block can
+disagree about it.  A thread that left a tile by its own count would miss the block's later
+barriers (and, in the persistent kernels, run a barrier ahead of the others into the next
+tile's buffers).  So a wait decides only through a block-wide vote, the tile functions
+report the verdict, and the persistent kernels leave on it.  What would happen otherwise is
+not run on a GPU; this reads the code instead."""
+import glob
+import os
+import re
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "2d-turbulent-navier-stokes_b200", "csrc")
+
+
+def _code(path):
+    """The source without comments."""
+    with open(path) as f:
+        s = f.read()
+    return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", s, flags=re.S))
+
+
+SOURCES = {os.path.basename(p): _code(p) for p in glob.glob(os.path.join(CSRC, "*.cu*"))}
+
+
+def _body(code, head):
+    """The braces that follow the first match of `head`."""
+    at = code.index("{", re.search(head, code).end())
+    depth, end = 0, at
+    for end in range(at, len(code)):
+        depth += {"{": 1, "}": -1}.get(code[end], 0)
+        if depth == 0:
+            break
+    return code[at:end + 1]
+
+
+def test_no_thread_leaves_a_wait_by_its_own_count():
+    assert any("bulk_wait(" in c for c in SOURCES.values())
+    for name, code in SOURCES.items():
+        assert not re.search(r"(if|while)\s*\(\s*!?\s*bulk_wait\(", code), name
+    vote = _body(SOURCES["tns_tile.cuh"], r"bool bulk_wait_block\(")
+    assert "__syncthreads_and(bulk_wait(" in vote
+
+
+def test_tiles_report_the_vote_and_persistent_kernels_leave_on_it():
+    for name, head in (("tns_kernels.cu", r"bool stage_tile\("), ("tns_kernels_mx.cu", r"bool stage_mx_tile\("),
+                       ("tns_visc.cuh", r"bool viscous_tile\(")):
+        body = _body(SOURCES[name], head)
+        assert re.search(r"if \(!bulk_wait_block\([^)]*\)\)\s*(\{[^}]*)?return false;", body), name
+    for name, head in (("tns_kernels.cu", r"k_batch_persistent\("), ("tns_kernels_mx.cu", r"k_batch_persistent_mx\(")):
+        body = _body(SOURCES[name], head)
+        assert body.count("ok = ") == 3 and "if (!ok) return;" in body, name
