@@ -131,6 +131,11 @@ __device__ __forceinline__ void bulk_barrier_init(unsigned long long* bar) {
     // initialised yet, and the wait never ends
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// Its shared memory is ordinary memory again.  One thread, when no thread and no copy uses the
+// barrier any more.
+__device__ __forceinline__ void bulk_barrier_end(unsigned long long* bar) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"((unsigned)__cvta_generic_to_shared(bar)) : "memory");
+}
 // Per-thread copies of 4 or 8 bytes global -> shared that need no registers on the way; the
 // thread that issued them waits for all of its own (copies_wait).
 template <class T>
@@ -190,10 +195,16 @@ __device__ __forceinline__ bool bulk_wait(unsigned long long* bar, unsigned pari
 // block's later barriers, and in a kernel that loops over tiles run one barrier ahead of the
 // others into the next tile's buffers.)  On false the copy did not complete: that is reported
 // (bit 1 of *error), the copy, which writes this block's shared memory, had one more bounded wait,
-// and the caller leaves the kernel.
+// and the caller leaves the kernel.  On true no thread looks at the barrier any more, and it is
+// taken down: a kernel that loops over tiles writes other data over its place and sets one up
+// there again, neither of which a live barrier allows.
 __device__ __forceinline__ bool bulk_wait_block(unsigned long long* bar, unsigned int* error) {
-    if (__syncthreads_and(bulk_wait(bar))) return true;
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
+    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+    if (__syncthreads_and(bulk_wait(bar))) {
+        if (first) bulk_barrier_end(bar);
+        return true;
+    }
+    if (first) {
         atomicOr(error, 2u);
         bulk_wait(bar);
     }

@@ -51,3 +51,16 @@ def test_tiles_report_the_vote_and_persistent_kernels_leave_on_it():
     for name, head in (("tns_kernels.cu", r"k_batch_persistent\("), ("tns_kernels_mx.cu", r"k_batch_persistent_mx\(")):
         body = _body(SOURCES[name], head)
         assert body.count("ok = ") == 3 and "if (!ok) return;" in body, name
+
+
+def test_a_tile_takes_its_barrier_down_before_the_next_sets_one_up():
+    """A loop over tiles puts other data where a tile's barrier was and initialises one there
+    again; PTX defines neither while the barrier is live."""
+    vote = _body(SOURCES["tns_tile.cuh"], r"bool bulk_wait_block\(")
+    assert re.search(r"if \(__syncthreads_and\(bulk_wait\(bar\)\)\)\s*\{\s*if \(first\) bulk_barrier_end\(bar\);", vote)
+    assert "mbarrier.inval" in _body(SOURCES["tns_tile.cuh"], r"void bulk_barrier_end\(")
+    # every barrier a tile function sets up is one it waits for through the vote
+    for name, head in (("tns_kernels.cu", r"bool stage_tile\("), ("tns_kernels_mx.cu", r"bool stage_mx_tile\("),
+                       ("tns_visc.cuh", r"bool viscous_tile\(")):
+        body = _body(SOURCES[name], head)
+        assert body.count("bulk_barrier_init(&S.bar)") == 1 == body.count("bulk_wait_block(&S.bar"), name
