@@ -473,7 +473,8 @@ TNS_HD void ghost_adj(const Params& P, int type, const double gw[NWROW], const d
 // divisions, square roots and tanh calls with slow paths (stage reverse of 512 x 192 cells, with
 // its two evaluations of the sources, 36 -> 30 us; a step 364 -> 334).  The comparisons that
 // select a branch (the C5 and RTOL floors, the sensors' larger side, the signs of pressure
-// differences) keep the divisions they had, so that ties fall as before.
+// differences) divide; the one that must meet a value of the solver's bit for bit (DTMIN) takes
+// that value from the solver's function.
 // tanh(x) for x >= 0 (capped at 20, where it is 1 to double precision), its reciprocal and its
 // derivative 1 - tanh^2 = 4 (E + 1) / (E + 2)^2 from one E = expm1(2x).
 struct TanhWork {
@@ -1587,10 +1588,7 @@ TNS_HD void dtmin_point(const AdjArgs& a, long long cell) {
     const long long n = a.ncell;
     double q[5];
     for (int m = 0; m < 5; m++) q[m] = a.qold[m * n + cell];
-    const double rho = q[0], u = q[1] / rho, v = q[2] / rho;
-    const double vel = sqrt(u * u + v * v);
-    const double t = (q[3] / rho - 0.5 * (u * u + v * v)) / P.cv;
-    const double dtl = a.M.cfldl[cell] / (fabs(vel) + sqrt(P.gamrr * t));
+    const double dtl = local_dt(P, q[0], q[1], q[2], q[3], a.M.cfldl[cell]);  // as the solver formed DTMIN
     if (!(dtl == *a.dtmin) || dtl >= 100000.0) return;
     double qb[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, dlb = 0.0;
     ts_adj(P, q, a.M.cfldl[cell], 0.0, *a.dtsum, qb, dlb);

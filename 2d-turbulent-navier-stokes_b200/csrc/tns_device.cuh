@@ -405,6 +405,24 @@ TNS_HD double inlet_density(const Params& P, double T) {
     return pow(P.s0 / (P.rr * T), P.inv1mg);
 }
 
+// DT of one cell (turbnstwod.f90:97-108).  The reverse of a global time step finds the cell
+// that DTMIN came from by comparing this value, so no two kernels may round it differently:
+// each product that meets a sum does so in a named fused multiply-add, and the compiler has no
+// choice left.  (On the host, as a program that divides computes it.)
+TNS_HD double local_dt(const Params& P, double c1, double c2, double c3, double c4, double cfldl) {
+#ifdef __CUDA_ARCH__
+    const double rr = 1.0 / c1;
+    const double U = c2 * rr, V = c3 * rr;
+    const double q2 = fma(U, U, V * V);
+    const double T = fma(-0.5, q2, c4 * rr) * P.inv_cv;
+    return cfldl / (sqrt(q2) + sqrt(P.gamrr * T));
+#else
+    const double U = c2 / c1, V = c3 / c1;
+    const double T = (c4 / c1 - 0.5 * (U * U + V * V)) / P.cv;
+    return cfldl / (sqrt(U * U + V * V) + sqrt(P.gamrr * T));
+#endif
+}
+
 // Ghost state from its parent (and the parent's opposite neighbour) for BC types 2..7
 // (boundary.f90:53-327; type 6 with the port flux supplied by the caller).
 // par: parent cell, opp: parent's neighbour across the face opposite the ghost.

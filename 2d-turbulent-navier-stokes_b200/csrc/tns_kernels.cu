@@ -524,18 +524,6 @@ k_viscous(Params P, Mesh M, const double* __restrict__ q, double* __restrict__ v
 
 size_t diss_smem_bytes() { return sizeof(DissSmem<double>); }
 
-__device__ __forceinline__ double local_dt(const Params& P, double c1, double c2, double c3,
-                                           double c4, double cfldl) {
-    // turbnstwod.f90:97-108
-    const double RHO = c1;
-    const double rr = 1.0 / RHO;
-    const double U = c2 * rr, V = c3 * rr;
-    const double VEL = sqrt(U * U + V * V);
-    const double E = c4 * rr;
-    const double T = (E - 0.5 * (U * U + V * V)) * P.inv_cv;
-    return cfldl / (fabs(VEL) + sqrt(P.gamrr * T));
-}
-
 __device__ __forceinline__ void dissipation_tile_f64(const Params& P, const Mesh& M, const DissArgs<double>& A, int bx,
                                                      int by) {
     dissipation_tile(P, M, A, bx, by, [](const double*) {});
