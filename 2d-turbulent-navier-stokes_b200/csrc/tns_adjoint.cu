@@ -70,13 +70,19 @@ TNS_ADJ_KERNEL(k_adj_geo, geo_point, 1)
 TNS_ADJ_KERNEL(k_adj_port, port_point, 1)
 TNS_ADJ_KERNEL(k_adj_port_nodes, port_node_point, 1)
 
-// LOCAL = 0: sum of the per-cell dt adjoints (block sums, one atomic per block).
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_dtsum(const double* __restrict__ v, long long n,
-                                                           double* __restrict__ out) {
+// LOCAL = 0: sum of the per-cell dt adjoints (block sums, one atomic per block), and the number
+// of cells whose step is DTMIN.
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_dtsum(const AdjArgs a, double* __restrict__ out,
+                                                           double* __restrict__ ties) {
     __shared__ double red[ADJ_THREADS / 32];
     double s = 0.0;
-    for (long long i = (long long)blockIdx.x * ADJ_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * ADJ_THREADS)
-        s += v[i];
+    int hit = 0;
+    for (long long i = (long long)blockIdx.x * ADJ_THREADS + threadIdx.x; i < a.ncell;
+         i += (long long)gridDim.x * ADJ_THREADS) {
+        s += a.dtbar[i];
+        hit += has_dtmin(a, i) ? 1 : 0;
+    }
+    if (hit) atomicAdd(ties, (double)hit);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
@@ -195,6 +201,7 @@ AdjArgs base_args(tns_handle* h, tns_adjoint_state* s, int set, int geo) {
     a.vfi = s->vfi.p;
     a.vfj = s->vfj.p;
     a.dtsum = s->dtsum.p;
+    a.dtties = s->dtsum.p + 1;
     a.sens = geo >= 1;  // geo: 0 none, 1 scalars (RTOLERANCE, T0, S0), 2 everything
     a.geo = geo >= 2;
     double* sp = s->sens.p;
@@ -317,8 +324,8 @@ long long enqueue_reverse(tns_handle* h, tns_adjoint_state* s, int set, int geo,
             launch_points(k_adj_diss_gather, a, a.ncell, s->side[0]);
             nl += 2;
             if (!P.local) {
-                cudaMemsetAsync(s->dtsum.p, 0, sizeof(double), s->side[0]);
-                k_adj_dtsum<<<148, ADJ_THREADS, 0, s->side[0]>>>(s->dtbar.p, a.ncell, s->dtsum.p);
+                cudaMemsetAsync(s->dtsum.p, 0, 2 * sizeof(double), s->side[0]);
+                k_adj_dtsum<<<148, ADJ_THREADS, 0, s->side[0]>>>(a, s->dtsum.p, s->dtsum.p + 1);
                 launch_points(k_adj_dtmin, a, a.ncell, s->side[0]);
                 nl += 2;
             }
@@ -445,7 +452,7 @@ int tns_adjoint_enable(tns_handle* h) {
                              {&s->lamg, 5 * n}, {&s->lamd, 5 * n}, {&s->gbar, 4 * 5 * npad}, {&s->srcn, 16 * n},
                              {&s->srcg, 8 * n}, {&s->wself, 5 * n}, {&s->wvisc, 5 * npad}, {&s->dbar, 5 * n},
                              {&s->visbar, 4 * n}, {&s->dtbar, n}, {&s->dout, NDOUT * n}, {&s->nbar, 5 * nnode},
-                             {&s->vfi, NVF * nif}, {&s->vfj, NVF * njf}, {&s->dtsum, 1}, {&s->sens, s->nsens},
+                             {&s->vfi, NVF * nif}, {&s->vfj, NVF * njf}, {&s->dtsum, 2}, {&s->sens, s->nsens},
                              {&s->xcs, npad}, {&s->ycs, npad}, {&s->gportb, 4 * (2 * (h->ni + h->nj))},
                              {&s->portacc, 3 * (2 * (h->ni + h->nj))}};
     for (auto& f : s->set)

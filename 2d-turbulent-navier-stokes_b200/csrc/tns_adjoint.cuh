@@ -93,6 +93,7 @@ struct AdjArgs {
     double* vfi;           // i-face adjoints [NVF][nif]
     double* vfj;           // j-face adjoints [NVF][njf]
     double* dtsum;         // LOCAL = 0: sum of the dt adjoints [1]
+    const double* dtties;  // LOCAL = 0: number of cells whose step is DTMIN [1] (null: one)
     // type-6 port ghosts
     const double* gport;   // port mass flux of this stage's input [nghost]
     double* gportb;        // its adjoint [nghost] (this stage)
@@ -1581,17 +1582,25 @@ TNS_HD void d2_point(const AdjArgs& a, long long cell) {
     }
 }
 
-// LOCAL = 0: the global step DTMIN = min(1e5, min DT) hands the summed dt adjoint to the
-// cell(s) whose local step is the minimum.
+// LOCAL = 0: whether the cell's step is the global one, DTMIN = min(1e5, min DT), formed as the
+// solver formed it.
+TNS_HD bool has_dtmin(const AdjArgs& a, long long cell) {
+    const long long n = a.ncell;
+    const double dtl = local_dt(a.P, a.qold[cell], a.qold[n + cell], a.qold[2 * n + cell], a.qold[3 * n + cell],
+                                a.M.cfldl[cell]);
+    return dtl == *a.dtmin && dtl < 100000.0;
+}
+
+// LOCAL = 0: the summed dt adjoint goes to the cell whose step is DTMIN, in equal parts where
+// several share it (a uniform state on equal cells).
 TNS_HD void dtmin_point(const AdjArgs& a, long long cell) {
     const Params& P = a.P;
     const long long n = a.ncell;
+    if (!has_dtmin(a, cell)) return;
     double q[5];
     for (int m = 0; m < 5; m++) q[m] = a.qold[m * n + cell];
-    const double dtl = local_dt(P, q[0], q[1], q[2], q[3], a.M.cfldl[cell]);  // as the solver formed DTMIN
-    if (!(dtl == *a.dtmin) || dtl >= 100000.0) return;
     double qb[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, dlb = 0.0;
-    ts_adj(P, q, a.M.cfldl[cell], 0.0, *a.dtsum, qb, dlb);
+    ts_adj(P, q, a.M.cfldl[cell], 0.0, a.dtties ? *a.dtsum / *a.dtties : *a.dtsum, qb, dlb);
     for (int m = 0; m < 5; m++) a.lamd[m * n + cell] += qb[m];
     if (a.geo) a.dlbar[cell] += dlb;
 }

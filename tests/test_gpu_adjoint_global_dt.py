@@ -64,3 +64,15 @@ def test_global_time_step_reverse_on_many_states(family, seed):
             C = sch.iteration(C, geo0, prm0)
     lam = torch.tensor(rng.normal(size=(5,) + mesh.shape), device="cuda")
     _compare(mesh, flow, sch, C, lam)
+
+
+def test_global_time_step_reverse_where_cells_share_the_minimum():
+    """A uniform state on a flat wall: every cell of the first row has the same step, and each
+    gets an equal part of DTMIN's adjoint."""
+    mesh, base = cases.ramp_mesh(40, 16, 0.0), cases.ramp_flow()
+    flow = formats.Flow(**{**base.__dict__, "local": 0})
+    sch = RestatedScheme(mesh, flow, device="cuda", rinit=formats.rinit_cold(flow))
+    c0 = formats.cold_state(flow, mesh.neles, formats.rinit_cold(flow))
+    C = torch.tensor(c0.reshape(5, *mesh.shape), device="cuda")
+    lam = torch.tensor(np.random.default_rng(7).normal(size=(5,) + mesh.shape), device="cuda")
+    _compare(mesh, flow, sch, C, lam)
