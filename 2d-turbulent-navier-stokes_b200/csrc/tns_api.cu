@@ -309,10 +309,17 @@ void build_geometry(tns_handle* h) {
         const double yavg = HALF * (yb + yd);
         fg[FG_RYAVG] = (iaxis == 1 && !(yavg < YAXIS_THRESH)) ? 1.0 / yavg : 0.0;
     };
-    h->hvtile.assign((size_t)ntj * nti * VTILE, 0.0);
+    const size_t vt = mixed ? VTILE_MX : VTILE;
+    h->hvtile.assign((size_t)ntj * nti * vt, 0.0);
     auto store = [&](const double* fg, int bi, int bj, int f) {
-        double* blk = &h->hvtile[((size_t)bi * ntj + bj) * VTILE + f];
-        for (int k = 0; k < FG_N; k++) blk[(size_t)k * NVF] = fg[k];
+        double* blk = &h->hvtile[((size_t)bi * ntj + bj) * vt];
+        if (mixed) {
+            float* b4 = reinterpret_cast<float*>(blk);
+            for (int k = 0; k < FG_RYAVG; k++) b4[(size_t)k * NVF + f] = (float)fg[k];
+            blk[(size_t)FG_RYAVG * NVF / 2 + f] = fg[FG_RYAVG];
+            return;
+        }
+        for (int k = 0; k < FG_N; k++) blk[(size_t)k * NVF + f] = fg[k];
     };
     double fg[FG_N];
     for (int i = 0; i <= ni; i++)

@@ -504,14 +504,14 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
 
 // ---------------------------------------------------------------- viscous kernel
 
-size_t visc_smem_bytes() { return sizeof(ViscSmem); }
+size_t visc_smem_bytes() { return sizeof(ViscSmem<double>); }
 
 template <bool RIM>
 __device__ __forceinline__ bool viscous_tile_f64(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                  double* __restrict__ vis, unsigned int* error, int bx, int by) {
-    return viscous_tile<RIM>(P, M, q, vis, error, bx, by,
-                             [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd,
-                                 double ry, double out[4]) { viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
+    return viscous_tile<RIM, double>(
+        P, M, q, vis, error, bx, by, [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
+                                      double out[4]) { viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
 
 template <bool RIM>

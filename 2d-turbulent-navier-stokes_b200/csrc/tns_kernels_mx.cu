@@ -2,18 +2,23 @@
 //
 // What stays FP64: the state Q (and every stage state COLD + dQ), each stage tile's
 // reference state with its primitives and fluxes, ghost states, the viscous and
-// dissipation kernels' primitives, geometry (node coordinates, surface vectors,
-// volumes, centroids), the differences of nearly equal quantities in the viscous and
-// dissipation kernels (gradient stencils, node averages), the part of the flux residual
-// that cancels (the reference flux times the closed-contour sum of S), the state
-// accumulation and the residual monitor.  What is FP32: the stage increments dQ, the
-// dissipation D, the viscous flux VIS and DT as stored, the stage slots as deviations
-// from the tile reference (primitives, fluxes and the source stencils), and the
-// source / viscous arithmetic with its transcendentals (T**0.6, tanh, sqrt).
+// dissipation kernels' primitives and pressures, the differences of nearly equal
+// quantities there (gradient stencils, node averages, sensors, Laplacians, VOL/DT until
+// each is rounded once), the part of the flux residual that cancels (the reference flux
+// times the closed-contour sum of S, and VOL/YCC times the reference pressure), the sums
+// of a cell's viscous face fluxes, 1/YAVG, the state accumulation and the residual
+// monitor.  The geometry is computed in FP64 on the host; face vectors, gradient
+// coefficients, 1/VOL, VOL and 1/YCC are rounded once from there.  What is FP32: the
+// stage increments dQ, the dissipation D, the viscous flux VIS, VIS + D and DT as stored,
+// the stage slots as deviations from the tile reference (primitives, fluxes and the
+// source stencils), and the source / viscous arithmetic with its transcendentals
+// (T**0.6, tanh, sqrt).
 //
 // Working with deviations instead of values keeps the FP32 rounding of the residual
 // proportional to the flow's variation inside a tile rather than to the pressure and
 // total-enthalpy levels, so the iteration can still converge by RTRED=1e-5 and more.
+#include <algorithm>
+
 #include "tns_device.cuh"
 #include "tns_kernels.h"
 #include "tns_mx.cuh"
@@ -180,13 +185,14 @@ k_stage_mx(Params P, Mesh M, StageArgsMx A) {
 
 // ---------------------------------------------------------------- viscous kernel
 
-size_t visc_mx_smem_bytes() { return sizeof(ViscSmem); }
+size_t visc_mx_smem_bytes() { return sizeof(ViscSmem<float>); }
+// (four blocks of the largest phase leave the persistent kernel a fifth of an SM's 228 KB as L1)
+static_assert(TI != 8 || 4 * std::max(sizeof(ViscSmem<float>), sizeof(StageSmemMx)) <= 183 * 1024,
+              "shared memory of a mixed tile");
 
 // One face of viscous.f90:130-217: FP64 stencil differences, FP32 rest.
-__device__ __forceinline__ void viscous_face_mx(const Params& P, const FaceVals& f, double dsx, double dsy, double dga,
-                                                double dgb, double dgc, double dgd, double ryavg, double out[4]) {
-    const float sx = (float)dsx, sy = (float)dsy;
-    const float ga = (float)dga, gb = (float)dgb, gc = (float)dgc, gd = (float)dgd;
+__device__ __forceinline__ void viscous_face_mx(const Params& P, const FaceVals& f, float sx, float sy, float ga,
+                                                float gb, float gc, float gd, double ryavg, float out[4]) {
     const float duac = (float)(f.ua - f.uc), dubd = (float)(f.ub - f.ud);
     const float dvac = (float)(f.va - f.vc), dvbd = (float)(f.vb - f.vd);
     const float dtac = (float)(f.ta - f.tc), dtbd = (float)(f.tb - f.td);
@@ -232,9 +238,9 @@ __device__ __forceinline__ void viscous_face_mx(const Params& P, const FaceVals&
 template <bool RIM>
 __device__ __forceinline__ bool viscous_mx_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                 float* __restrict__ vis, unsigned int* error, int bx, int by) {
-    return viscous_tile<RIM>(P, M, q, vis, error, bx, by,
-                             [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd,
-                                 double ry, double out[4]) { viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
+    return viscous_tile<RIM, float>(
+        P, M, q, vis, error, bx, by, [&](const FaceVals& f, float sx, float sy, float ga, float gb, float gc, float gd,
+                                      double ry, float out[4]) { viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
 }
 
 template <bool RIM>

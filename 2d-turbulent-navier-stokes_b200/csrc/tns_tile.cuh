@@ -93,12 +93,15 @@ constexpr int MXTILE = MX_N * TI * TJ;
 // Faces of a tile: i-faces (between cells (i-1, j) and (i, j)) for i in i0..i0+TI, j-faces
 // (between (i, j-1) and (i, j)) for j in j0..j0+TJ; and the tile's static face geometry
 // (tile (bx, by) at M.vtile + (by * ntiles_j + bx) * VTILE), [FG_N][NVF], i-face (la, lb) at
-// la * TJ + lb, j-face (la, lb) at NIF + la * (TJ + 1) + lb.
+// la * TJ + lb, j-face (la, lb) at NIF + la * (TJ + 1) + lb.  On mixed-precision handles (VTILE_MX
+// doubles a tile) the face vectors and gradient coefficients are floats, rounded on the host as
+// the kernel would at their use, and the last row, 1/YAVG, doubles.
 constexpr int NIF = (TI + 1) * TJ;
 constexpr int NJF = TI * (TJ + 1);
 constexpr int NVF = NIF + NJF;
 constexpr int VTILE = FG_N * NVF;
-static_assert(NVF % 2 == 0, "rows of the face geometry are multiples of 16 bytes");
+constexpr int VTILE_MX = FG_RYAVG * NVF / 2 + NVF;
+static_assert(NVF % 4 == 0, "rows of the face geometry are multiples of 16 bytes");
 
 // Programmatic dependent launch: a tile kernel lets the next kernel in the stream start
 // as soon as all its blocks are running (pdl_trigger), and waits for the previous one

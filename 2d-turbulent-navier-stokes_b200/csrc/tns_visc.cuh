@@ -19,9 +19,16 @@
 
 namespace tns {
 
-// One tile's shared memory.
+// One tile's shared memory; G: type of the face vectors, gradient coefficients and face fluxes.
+// On the mixed path that is float, 43 KB a tile instead of 56: the persistent batch kernel has four
+// blocks an SM with its largest phase's shared memory, and lives on the L1 that is left (with 56 KB
+// a block in place of 36 an earlier form of it went from 20.1 to 23.4 ms; 64 ramp cases, 20
+// iterations).  Those 64 cases: 21.3 -> 19.2 ms, by tile-table launches 17.0 -> 15.2, on branch
+// streams 14.3 -> 13.0.
+template <class G>
 struct ViscSmem {
-    double fg[FG_N][NVF];                  // face geometry, then the fluxes of VIS 0..3
+    G fg[FG_RYAVG][NVF];                   // face geometry, then the fluxes of VIS 0..3
+    double ry[NVF];                        // 1/YAVG (axisymmetric meshes)
     double2 uv[NSLOT], tr[NSLOT];          // slots: (U, V), (T, RHO)
     double2 auv[NAVG + 1], atr[NAVG + 1];  // nodal averages
     double ri[NSLOT], ar[NAVG + 1];        // C5/C1 of both
@@ -30,7 +37,8 @@ struct ViscSmem {
 
 // The values of one face's four points: A = the cell (slot sa), C = its neighbour (slot sc),
 // B, D = the face's nodes ab, ad.
-__device__ __forceinline__ void face_values(const ViscSmem& S, int sa, int sc, int ab, int ad, FaceVals& f) {
+template <class G>
+__device__ __forceinline__ void face_values(const ViscSmem<G>& S, int sa, int sc, int ab, int ad, FaceVals& f) {
     double2 v;
     v = S.uv[sa]; f.ua = v.x; f.va = v.y;
     v = S.uv[sc]; f.uc = v.x; f.vc = v.y;
@@ -43,16 +51,17 @@ __device__ __forceinline__ void face_values(const ViscSmem& S, int sa, int sc, i
     f.ra = S.ri[sa]; f.rc = S.ri[sc]; f.rb = S.ar[ab]; f.rd = S.ar[ad];
 }
 
-// face(FaceVals, sx, sy, ga, gb, gc, gd, ryavg, double out[4]) evaluates one face's flux.
+// face(FaceVals, G sx, sy, ga, gb, gc, gd, double ryavg, G out[4]) evaluates one face's flux.
 // False (for the whole block; bit 1 of *error set) where the tile's static copy did not complete:
 // the block then leaves the kernel.  RIM: the block has
 // RIM_ROWS more rows of threads, which take the halo, the nodes and the faces beyond the
 // cells' own.
-template <bool RIM, class OutT, class Face>
+template <bool RIM, class G, class OutT, class Face>
 __device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                              OutT* __restrict__ vis, unsigned int* error, int bx, int by, Face face) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ViscSmem& S = *reinterpret_cast<ViscSmem*>(smem_raw);
+    ViscSmem<G>& S = *reinterpret_cast<ViscSmem<G>*>(smem_raw);
+    constexpr int BLOCK = sizeof(G) == sizeof(double) ? VTILE : VTILE_MX;
     const size_t ncell = (size_t)M.ni * M.nj;
     const int j0 = bx * TJ, i0 = by * TI;
     const int tj = threadIdx.x, ti = threadIdx.y, tid = ti * TJ + tj;
@@ -60,7 +69,7 @@ __device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, con
     if (tid == 0) {
         bulk_barrier_init(&S.bar);
         const size_t tile = (size_t)by * ((M.nj + TJ - 1) / TJ) + bx;
-        bulk_copy_start(S.fg, M.vtile + tile * VTILE, sizeof(double) * (P.iaxis == 1 ? FG_N : FG_RYAVG) * NVF, &S.bar);
+        bulk_copy_start(S.fg, M.vtile + tile * BLOCK, sizeof(S.fg) + (P.iaxis == 1 ? sizeof(S.ry) : 0), &S.bar);
     }
     const bool inner = i0 > 0 && j0 > 0 && i0 + TI < M.ni && j0 + TJ < M.nj;
     const int i = i0 + ti, j = j0 + tj;
@@ -186,9 +195,9 @@ __device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, con
     auto eval = [&](int f, int sa, int sc, int ab, int ad) {
         FaceVals v;
         face_values(S, sa, sc, ab, ad, v);
-        double out[4];
+        G out[4];
         face(v, S.fg[FG_SX][f], S.fg[FG_SY][f], S.fg[FG_GA][f], S.fg[FG_GB][f], S.fg[FG_GC][f], S.fg[FG_GD][f],
-             P.iaxis == 1 ? S.fg[FG_RYAVG][f] : 0.0, out);
+             P.iaxis == 1 ? S.ry[f] : 0.0, out);
 #pragma unroll
         for (int k = 0; k < 4; k++) S.fg[k][f] = out[k];
     };
@@ -222,7 +231,8 @@ __device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, con
 #pragma unroll
     for (int k = 0; k < 4; k++)
         vis[k * ncell + cell] =
-            (OutT)(((s1 * S.fg[k][f1] + S.fg[k][f4 + TJ]) + S.fg[k][f1 + 1]) + s4 * S.fg[k][f4]);
+            (OutT)(((s1 * (double)S.fg[k][f1] + (double)S.fg[k][f4 + TJ]) + (double)S.fg[k][f1 + 1]) +
+                   s4 * (double)S.fg[k][f4]);
     return true;
 }
 
