@@ -60,7 +60,6 @@ struct tns_batch {
     int mode = 0;
     bool general = false;  // a case is a general mesh: per-case schedules (1, 2) only
     static constexpr int PERSIST = 256;
-    int persist_grid = 0;               // resident blocks of the persistent kernel
     DevBuf<unsigned int> d_bar;         // its grid barrier: arrival counter, generation
     DevBuf<unsigned int> d_error;       // bit 2: a grid barrier gave up
     unsigned int* h_error = nullptr;    // pinned
@@ -504,10 +503,9 @@ int tns_batch_run(tns_batch* b, int niter, int monitor_every, double stop_ratio,
             // the run of unmonitored iterations from here, in one persistent launch
             step = 1;
             while (step < tns_batch::PERSIST && it + step <= niter && !monitored(it + step)) step++;
-            const int grid = std::min(b->persist_grid, 2 * b->ntiles);
             if ((rc = b->cuda(cudaMemsetAsync(b->d_bar.p, 0, 2 * sizeof(unsigned int), b->stream), "cudaMemsetAsync")) ||
                 (rc = b->cuda(tns::launch_persistent(b->precision == 1, b->d_desc.p, b->d_tiles.p, b->d_active.p,
-                                                     b->ntiles, step, parity, grid, b->d_bar.p, b->d_error.p,
+                                                     b->ntiles, step, parity, b->d_bar.p, b->d_error.p,
                                                      b->stream), "persistent launch")))
                 return rc;
             b->launches++;
@@ -597,8 +595,7 @@ int tns_batch_set_schedule(tns_batch* b, int schedule) {
         if ((rc = b->cuda(cudaGetDevice(&dev), "cudaGetDevice")) ||
             (rc = b->cuda(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev), "cudaDeviceGetAttribute")))
             return rc;
-        b->persist_grid = coop ? tns::persistent_grid(b->precision == 1) : 0;
-        if (b->persist_grid <= 0)
+        if (!coop || tns::persistent_grid(b->precision == 1, 1) <= 0)
             return b->fail(TNS_ERR_UNSUPPORTED, "schedule 3 needs a cooperative launch of the persistent kernel");
         if (!b->d_bar.p && ((rc = b->cuda(b->d_bar.alloc(2), "cudaMalloc")) ||
                             (rc = b->cuda(b->d_error.alloc(1), "cudaMalloc")) ||

@@ -968,25 +968,33 @@ size_t persistent_smem_bytes(bool mixed) {
     return std::max(stage_smem_bytes(), std::max(visc_smem_bytes(), diss_smem_bytes()));
 }
 
-int persistent_grid(bool mixed) {
-    int per_sm = 0, dev = 0, sms = 0;
-    const void* k = mixed ? persistent_kernel_mx() : (const void*)k_batch_persistent;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NTHREADS, persistent_smem_bytes(mixed)) !=
-            cudaSuccess)
+int persistent_grid(bool mixed, int ntiles) {
+    int per_sm = 0, grid = 0;
+    if (mixed) {
+        persistent_kernel_mx(ntiles, &grid);
+        return grid;
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_persistent, NTHREADS,
+                                                      persistent_smem_bytes(mixed)) != cudaSuccess)
         return 0;
-    return per_sm * sms;
+    return per_sm * sm_count();
 }
 
 cudaError_t launch_persistent(bool mixed, const BatchCase* cases, const int4* tiles, const int* active,
-                              int ntiles, int iters, int parity, int grid, unsigned int* bar,
-                              unsigned int* error, cudaStream_t s) {
-    if (mixed) return launch_persistent_mx(cases, tiles, active, ntiles, iters, parity, grid, bar, error, s);
+                              int ntiles, int iters, int parity, unsigned int* bar, unsigned int* error,
+                              cudaStream_t s) {
+    int grid = 0;
+    const void* k = mixed ? persistent_kernel_mx(ntiles, &grid) : (const void*)k_batch_persistent;
+    grid = std::min(mixed ? grid : persistent_grid(false, ntiles), 2 * ntiles);
+    const dim3 blk(TJ, TI);
+    if (mixed) {  // (its tile table holds active cases alone)
+        void* args[] = {(void*)&cases, (void*)&tiles,  (void*)&ntiles, (void*)&iters,
+                        (void*)&parity, (void*)&bar, (void*)&error};
+        return cudaLaunchCooperativeKernel(k, dim3(grid), blk, args, persistent_smem_bytes(true), s);
+    }
     void* args[] = {(void*)&cases, (void*)&tiles, (void*)&active, (void*)&ntiles, (void*)&iters, (void*)&bar,
                     (void*)&error};
-    return cudaLaunchCooperativeKernel((const void*)k_batch_persistent, dim3(grid), dim3(TJ, TI), args,
-                                       persistent_smem_bytes(false), s);
+    return cudaLaunchCooperativeKernel(k, dim3(grid), blk, args, persistent_smem_bytes(false), s);
 }
 
 void launch_batch_f64(const BatchCase* cases, const int4* tiles, const int* active, int ntiles,

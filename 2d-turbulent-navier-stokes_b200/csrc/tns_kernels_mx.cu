@@ -68,9 +68,10 @@ size_t stage_mx_smem_bytes() { return sizeof(StageSmemMx); }
 #define TNS_VISC_MX_BATCH_MINB 4
 #endif
 // One stage on tile (bx, by) of a mesh; the single-case and the batched kernels wrap it.
-// RIM: the block has RIM_ROWS more rows of threads, which form the halo.  False (for the whole
+// RIM: the block has RIM_ROWS more rows of threads, which form the halo.  LATE: the halo's places
+// are looked up after the own slots (they cost registers until then).  False (for the whole
 // block) where the static block did not arrive: the block then leaves the kernel.
-template <bool RIM>
+template <bool RIM, bool LATE = false>
 __device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, const StageArgsMx& A,
                                               int bx, int by) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -96,12 +97,15 @@ __device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, co
     GhostSite site{0, 0.0, 0.0, 0.0, 0.0};
     const int rt = RIM ? tid - NTHREADS : tid;  // the thread's place on the ring
     const int ri = inner ? TI : min(TI, M.ni - i0), rj = inner ? TJ : min(TJ, M.nj - j0);
-    if (rt >= 0 && rt < 2 * (ri + rj + 2)) {
-        int li, lj;
-        ring_slot(rt, ri, rj, li, lj);
-        h = halo_pos(M, inner, i0, j0, li, lj);
-        if (h.kind > 0) site = ghost_site(M, h.g);
-    }
+    auto place = [&]() {
+        if (rt >= 0 && rt < 2 * (ri + rj + 2)) {
+            int li, lj;
+            ring_slot(rt, ri, rj, li, lj);
+            h = halo_pos(M, inner, i0, j0, li, lj);
+            if (h.kind > 0) site = ghost_site(M, h.g);
+        }
+    };
+    if (!LATE) place();
     pdl_wait();
     // a cell's COLD and stage increment
     auto load = [&](int ci, int cj, double q[5], float d[5]) {
@@ -132,6 +136,7 @@ __device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, co
         cell_slot((ti + 1) * SW + tj + 1, qo, dqo, o);
         own = o.own;
     }
+    if (LATE) place();
     if (!RIM && h.kind >= 0) load(h.ci, h.cj, qr, dqr);
     if (h.kind == 0) {
         SlotMx o;
@@ -357,31 +362,56 @@ __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MX_BATCH_MINB))
 }
 
 // Persistent batched iterations of the mixed path (schedule 3), as k_batch_persistent:
-// the state parity alternates from `parity` with every iteration.
-#ifndef TNS_PERSIST_MX_MINB
-#define TNS_PERSIST_MX_MINB 4
-#endif
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_PERSIST_MX_MINB))
-k_batch_persistent_mx(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles,
-                      const int* __restrict__ active, int ntiles, int iters, int parity0, unsigned int* bar,
-                      unsigned int* error) {
+// the state parity alternates from `parity` with every iteration.  A case's arguments stay in
+// shared memory until a tile of another case comes.  The two pre-passes of a tile follow one
+// another in one block, which finds the state in L1, where every block gets a tile that way.
+// Two register budgets, PER_SM blocks of eight rows an SM: a tile's chain is shorter with 80
+// registers, and with 64 more tiles are under way; the launcher takes the first where it needs no
+// more rounds over the tiles (692 tiles, 20 iterations: 2.36 -> 1.93 ms; 9500 tiles, which it takes
+// at 64, 19.2 with 64 and 20.8 with 80).  Arguments copied for every stage tile, and all
+// dissipation tiles before the first viscous one: 1.34 ms for 1 case of 224 tiles, 19.4 for 64
+// cases; now 1.15 and 18.5.
+template <int PER_SM>
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(PER_SM))
+k_batch_persistent_mx(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles, int ntiles, int iters,
+                      int parity0, unsigned int* bar, unsigned int* error) {
+    // (raw storage: the structs are copied in, never constructed)
+    __shared__ __align__(16) unsigned char sargs[sizeof(Params) + sizeof(Mesh) + sizeof(StageArgsMx)];
+    Params& sP = *reinterpret_cast<Params*>(sargs);
+    Mesh& sM = *reinterpret_cast<Mesh*>(sargs + sizeof(Params));
+    StageArgsMx& sA = *reinterpret_cast<StageArgsMx*>(sargs + sizeof(Params) + sizeof(Mesh));
+    const bool pairs = ntiles >= (int)gridDim.x;
+    int held = -1;  // the case whose Params and Mesh are in shared memory
     for (int it = 0; it < iters; it++) {
         const int parity = parity0 ^ (it & 1);
         for (int ph = 0; ph < 5; ph++) {
+            // pre-passes (ph 0): dissipation of tile k is item 2 k, its viscous flux 2 k + 1, taken
+            // in pairs, or apart (the viscous tiles then go to other blocks than the dissipation's)
+            const bool two = ph == 0 && pairs;
             const int nwork = ph == 0 ? 2 * ntiles : ntiles;
-            for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-                const int4 t = tiles[w % ntiles];
-                bool ok = true;
-                if (active[t.x]) {
-                    const BatchCase& c = cases[t.x];
-                    if (ph == 0 && w < ntiles)
-                        dissipation_mx_tile(c.P, c.M, c.qmx[parity], c.df, c.dtf, c.dtmin, t.y, t.z);
-                    else if (ph == 0)
-                        ok = viscous_mx_tile<false>(c.P, c.M, c.qmx[parity], c.visf, c.stage_mx[0][0][0].error, t.y,
-                                                    t.z);
-                    else
-                        ok = stage_mx_batch_tile(c, c.stage_mx[parity][0][ph - 1], t.y, t.z);
+            int args = -1;  // the case whose stage arguments are
+            for (int w = two ? 2 * blockIdx.x : blockIdx.x; w < nwork;
+                 w += !two ? gridDim.x : w & 1 ? 2 * gridDim.x - 1 : 1) {
+                const int4 t = tiles[two ? w >> 1 : w < ntiles ? w : w - ntiles];
+                const BatchCase& c = cases[t.x];
+                if (t.x != args) {
+                    const int tid = threadIdx.y * TJ + threadIdx.x;
+                    if (t.x != held) {
+                        copy_words(&sP, &c.P, sizeof(Params), tid);
+                        copy_words(&sM, &c.M, sizeof(Mesh), tid);
+                        held = t.x;
+                    }
+                    if (ph) copy_words(&sA, &c.stage_mx[parity][0][ph - 1], sizeof(StageArgsMx), tid);
+                    args = t.x;
+                    __syncthreads();
                 }
+                bool ok = true;
+                if (ph)
+                    ok = stage_mx_tile<false, true>(sP, sM, sA, t.y, t.z);
+                else if (two ? w & 1 : w >= ntiles)
+                    ok = viscous_mx_tile<false>(sP, sM, c.qmx[parity], c.visf, c.stage_mx[0][0][0].error, t.y, t.z);
+                else
+                    dissipation_mx_tile(sP, sM, c.qmx[parity], c.df, c.dtf, c.dtmin, t.y, t.z);
                 if (!ok) return;  // the whole block
                 async_proxy_fence();
                 __syncthreads();
@@ -394,15 +424,20 @@ k_batch_persistent_mx(const BatchCase* __restrict__ cases, const int4* __restric
     }
 }
 
-const void* persistent_kernel_mx() { return (const void*)k_batch_persistent_mx; }
-
-cudaError_t launch_persistent_mx(const BatchCase* cases, const int4* tiles, const int* active, int ntiles,
-                                 int iters, int parity, int grid, unsigned int* bar, unsigned int* error,
-                                 cudaStream_t s) {
-    void* args[] = {(void*)&cases, (void*)&tiles, (void*)&active, (void*)&ntiles, (void*)&iters,
-                    (void*)&parity, (void*)&bar, (void*)&error};
-    return cudaLaunchCooperativeKernel((const void*)k_batch_persistent_mx, dim3(grid), dim3(TJ, TI), args,
-                                       persistent_smem_bytes(true), s);
+// The kernel for a batch of ntiles tiles, and its resident blocks on the device (0: none).
+const void* persistent_kernel_mx(int ntiles, int* grid) {
+    const void* k[2] = {(const void*)k_batch_persistent_mx<3>, (const void*)k_batch_persistent_mx<4>};
+    int g[2];
+    for (int v = 0; v < 2; v++) {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k[v], NTHREADS, persistent_smem_bytes(true)) !=
+            cudaSuccess)
+            per_sm = 0;
+        g[v] = per_sm * sm_count();
+    }
+    const int v = g[0] > 0 && (g[1] <= 0 || (ntiles + g[0] - 1) / g[0] <= (ntiles + g[1] - 1) / g[1]) ? 0 : 1;
+    *grid = g[v];
+    return k[v];
 }
 
 // ------------------------------------------------------------------ launchers
@@ -428,9 +463,10 @@ cudaError_t configure_kernels_mx() {
     e = cudaFuncSetAttribute(k_viscous_mx_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)visc_mx_smem_bytes());
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_batch_persistent_mx, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)persistent_smem_bytes(true));
-    if (e != cudaSuccess) return e;
+    for (auto k : {k_batch_persistent_mx<3>, k_batch_persistent_mx<4>}) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)persistent_smem_bytes(true));
+        if (e != cudaSuccess) return e;
+    }
     return cudaFuncSetAttribute(k_stage_mx_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)stage_mx_smem_bytes());
 }
