@@ -414,7 +414,7 @@ TNS_HD double local_dt(const Params& P, double c1, double c2, double c3, double 
     const double rr = 1.0 / c1;
     const double U = c2 * rr, V = c3 * rr;
     const double q2 = fma(U, U, V * V);
-    const double T = fma(-0.5, q2, c4 * rr) * P.inv_cv;
+    const double T = fma(c4, rr, -0.5 * q2) * P.inv_cv;
     return cfldl / (sqrt(q2) + sqrt(P.gamrr * T));
 #else
     const double U = c2 / c1, V = c3 / c1;
