@@ -163,6 +163,18 @@ TNS_HD double root(double x) {
 #endif
 }
 
+// a/b by recip and one correction of the quotient (Markstein, IBM J. Res. Dev. 34(1), 1990): the
+// correctly rounded quotient but for rare cases, where a product with the reciprocal is rounded
+// twice.  For quotients that become part of the state.
+TNS_HD double quot(double a, double b) {
+#ifdef __CUDA_ARCH__
+    const double r = recip(b), q = a * r;
+    return fma(fma(-q, b, a), r, q);
+#else
+    return a / b;
+#endif
+}
+
 // T**-0.4 and T**-0.6 for T > 0: a single-precision estimate y = exp2(-0.2 log2 T) of
 // T**(-1/5) (about 1e-7 relative) and one cubically convergent step for the inverse fifth
 // root,

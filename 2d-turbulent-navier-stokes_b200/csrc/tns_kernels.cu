@@ -196,7 +196,7 @@ __device__ __forceinline__ void stage_cell(const Params& P, const Mesh& M, const
     Cn[2] = Co[2] - aDT * fma(RVOL, HALF * R[2] - o.e[2], -src3);
     Cn[3] = Co[3] - aDT * (RVOL * (HALF * R[3] - o.e[3]));
     Cn[4] = Co[4] - aDT * CFLTURB * fma(RVOL, HALF * R[4] - o.e[4], -src5);
-    Cn[4] = Cn[0] * dmax1(P.rtol, Cn[4] * recip(Cn[0]));
+    Cn[4] = Cn[0] * dmax1(P.rtol, quot(Cn[4], Cn[0]));
 #pragma unroll
     for (int m = 0; m < 5; m++) A.qout[m * ncell + cell] = Cn[m];
     if (A.status) {

@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(UT, TNS_U_CHUNK_MINB) k_u_stage_chunk(Params P
         Cn[2] = Co[2] - aDT * fma(RVOL, HALF * R[2] - e[2], -src3);
         Cn[3] = Co[3] - aDT * (RVOL * (HALF * R[3] - e[3]));
         Cn[4] = Co[4] - aDT * CFLTURB * fma(RVOL, HALF * R[4] - e[4], -src5);
-        Cn[4] = Cn[0] * dmax1(P.rtol, Cn[4] * recip(Cn[0]));
+        Cn[4] = Cn[0] * dmax1(P.rtol, quot(Cn[4], Cn[0]));
 #pragma unroll
         for (int m = 0; m < 5; m++) A.qout[m * n + I] = Cn[m];
         if (A.status) {
