@@ -259,6 +259,27 @@ TNS_HD double tanh_ratio(double a, double b) {
     return r.num / r.den;
 }
 
+// The damping ratios of the turbulence model at CHI = RHO nu~ / (CMU AMU):
+// FMU = tanh(ALPHA_T CHI^2) / tanh(BETA_T CHI^2) and FR2 = tanh(sqrt CHI) / tanh(FR2K CHI), the
+// sources' two by one reciprocal.  The scale, an exact factor of both parts of FR2, keeps the
+// product of the denominators, some CHI^3 for small CHI, from underflowing before CHI^2 does.
+TNS_HD double damping_fmu(double chi) {
+    const double chi2 = chi * chi;
+    const Ratio m = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
+    return m.num * recip(m.den);
+}
+struct Damping {
+    double fmu, fr2;
+};
+TNS_HD Damping damping(double chi, double fr2k) {
+    const double chi2 = chi * chi;
+    const Ratio m = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
+    const Ratio r = tanh_ratio_parts(root(chi), chi * fr2k);
+    const double num = r.num * 0x1p700, den = r.den * 0x1p700;
+    const double inv = recip(m.den * den);
+    return Damping{m.num * den * inv, num * m.den * inv};
+}
+
 // Sutherland-type molecular viscosity SUTH_COEF*DSQRT(AMOL)*T**0.6 (viscous.f90:188).
 TNS_HD double amu_of(const Params& P, double T) {
     return P.suth_amol * pow06(T);
@@ -578,12 +599,8 @@ __device__ __forceinline__ void source_terms(const Params& P, const SrcIn& s, do
     const FifthRoots tr = fifth_roots(TI);
     const double AMU = P.suth_amol * (TI * tr.m04);
     const double CHI = RHO * RI * (P.inv_cmu_suth * tr.m06);
-    const double chi2 = CHI * CHI;
-    const Ratio fm = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
-    const Ratio fr = tanh_ratio_parts(root(CHI), CHI * P.fr2k);
-    const double inv = recip(fm.den * fr.den);
-    const double FMU = fm.num * fr.den * inv;
-    const double FR2 = fr.num * fm.den * inv;
+    const Damping damp = damping(CHI, P.fr2k);
+    const double FMU = damp.fmu, FR2 = damp.fr2;
     const double AMUT = FMU * RHO * RI;
     const double PHI = DQX * DRX + DQY * DRY;
     double DEE = 0.0;
@@ -679,9 +696,7 @@ __device__ __forceinline__ void viscous_face(const Params& P, const FaceVals& f,
     const double AMU = P.suth_amol * (TAVG * tr.m04);
     const double AK = AMU * P.cp_pr;
     const double CHI = RHOAVG * RAVG * (P.inv_cmu_suth * tr.m06);
-    const double chi2 = CHI * CHI;
-    const Ratio fm = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
-    const double FMU = fm.num * recip(fm.den);
+    const double FMU = damping_fmu(CHI);
     const double AMUT = RHOAVG * RAVG * FMU;
     const double AKT = AMUT * P.cp_prt;
     const double AMUEFF = AMU + AMUT;
