@@ -1231,9 +1231,13 @@ int tns_time_step_noalloc(const double* d_q, const double* d_cfldl, long long nc
     unsigned int* counter =
         reinterpret_cast<unsigned int*>(static_cast<unsigned char*>(base) + TNS_NOALLOC_MAX_BLOCKS * sizeof(double));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const Params P = make_params(*params);
+    if (ncell <= tns::STEP_CLUSTER_CELLS) {  // (after the set-up, which a later call may rely on)
+        tns::launch_time_step_cluster(P, d_q, d_cfldl, ncell, d_dt, d_dtmin, s);
+        return cudaGetLastError() == cudaSuccess ? TNS_OK : TNS_ERR_CUDA;
+    }
     // the array keeps whatever the previous call left: the counter must start at zero
     if (cudaMemsetAsync(counter, 0, sizeof(unsigned int), s) != cudaSuccess) return TNS_ERR_CUDA;
-    const Params P = make_params(*params);
     tns::launch_time_step_scratch(P, d_q, d_cfldl, ncell, d_dt, partial, counter, d_dtmin,
                                   (int)nblocks, s);
     return cudaGetLastError() == cudaSuccess ? TNS_OK : TNS_ERR_CUDA;

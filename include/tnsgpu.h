@@ -199,15 +199,17 @@ const char *tns_last_error(tns_handle *h);
  *   d_dtmin  device, one double out: DTMIN (the LOCAL=0 step)
  *   stream   cudaStream_t as void* (NULL = the legacy default stream)
  *
- * Its reduction scratch is a fixed array inside the library (one partial minimum per
+ * Up to 32768 cells one cluster of blocks computes it without scratch.  Beyond, its
+ * reduction scratch is a fixed array inside the library (one partial minimum per
  * block of TNS_NOALLOC_CELLS_PER_THREAD*256 cells, at most TNS_NOALLOC_MAX_BLOCKS
  * blocks: 64 KiB), so ncell is limited to TNS_NOALLOC_MAX_CELLS; larger problems get
- * TNS_ERR_TOO_LARGE.  It calls no cudaMalloc / cudaFree.  The first call on each device
- * looks up the array's device address (cudaGetSymbolAddress), so make that first call
- * before any stream capture starts.  The address is kept until the process exits; after
- * cudaDeviceReset on that device it no longer names the array, so do not call this entry
- * point on a device that has been reset.  All calls share the one array, so calls that
- * may overlap on the GPU (different streams without ordering) race; serialise them.
+ * TNS_ERR_TOO_LARGE.  It calls no cudaMalloc / cudaFree.  The first call on each device,
+ * of any size, looks up the array's device address (cudaGetSymbolAddress), so make that
+ * first call before any stream capture starts.  The address is kept until the process
+ * exits; after cudaDeviceReset on that device it no longer names the array, so do not
+ * call this entry point on a device that has been reset.  All calls share the one array,
+ * so calls that may overlap on the GPU (different streams without ordering) race;
+ * serialise them.
  * The call is asynchronous on `stream`. */
 #define TNS_NOALLOC_MAX_BLOCKS 8192
 #define TNS_NOALLOC_CELLS_PER_THREAD 4
