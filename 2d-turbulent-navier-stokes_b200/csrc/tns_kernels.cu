@@ -333,7 +333,7 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const Mesh& M, const
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
 // runs, and on the extra rows of threads.
 template <int MONITOR, bool RIM>
-__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), TNS_PER_SM(RIM ? 2 : TNS_STAGE_MINB))
+__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), RIM ? RIM_MINB : TNS_PER_SM(TNS_STAGE_MINB))
 k_stage(Params P, Mesh M, StageArgs A) {
     StageArgs Ac = A;
     if (!MONITOR) Ac.cdiff = nullptr;
@@ -516,7 +516,7 @@ __device__ __forceinline__ bool viscous_tile_f64(const Params& P, const Mesh& M,
 }
 
 template <bool RIM>
-__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), TNS_PER_SM(RIM ? 2 : TNS_VISC_MINB))
+__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), RIM ? RIM_MINB : TNS_PER_SM(TNS_VISC_MINB))
 k_viscous(Params P, Mesh M, const double* __restrict__ q, double* __restrict__ vis, unsigned int* error) {
     viscous_tile_f64<RIM>(P, M, q, vis, error, blockIdx.x, blockIdx.y);
 }
@@ -1075,7 +1075,7 @@ void launch_viscous(const Params& P, const Mesh& M, const double* q, double* vis
     // the rim rows shorten one tile's chain (115 x 50 nozzle: 22.8 -> 22.2 us an iteration,
     // 192 x 64: 24.2 -> 22.2) but leave room for two blocks an SM instead of three (400 x 160,
     // 250 tiles: 28.0 -> 29.9)
-    if ((int)(grid.x * grid.y) + beside <= TNS_VISC_RIM_PER_SM * sm_count())
+    if ((int)(grid.x * grid.y) + beside <= VISC_RIM_PER_SM * sm_count())
         launch_tile(k_viscous<true>, grid, dim3(TJ, TI + RIM_ROWS), visc_smem_bytes(), s, P, M, q, vis, error);
     else
         launch_tile(k_viscous<false>, grid, dim3(TJ, TI), visc_smem_bytes(), s, P, M, q, vis, error);
@@ -1096,13 +1096,14 @@ void launch_stage(const Params& P, const Mesh& M, const double* qin, const doubl
                     maps);
         return;
     }
-    // the rim rows while every tile has its own resident block of that size: 115 x 50 nozzle,
+    // the rim rows while every tile has its own resident block of that size (at 8 rows a tile; for
+    // other heights see tns_tile.cuh): 115 x 50 nozzle,
     // an iteration, 22.7 -> 22.2 us (20.6 with the operands fetched early); 400 x 160 ramp (250
     // tiles) 31.2 -> 28.0.  The tiles of
     // other cases in flight beside this mesh count too: their warps fill the gaps, and the
     // larger blocks would only displace them (16 ramp cases on branch streams, 20 iterations:
     // 6.05 ms with the rim rows, 5.28 without; 4 cases 1.63 and 1.50)
-    if (ntiles + beside <= TNS_STAGE_RIM_PER_SM * sm_count())
+    if (ntiles + beside <= STAGE_RIM_PER_SM * sm_count())
         launch_tile(cdiff ? k_stage<1, true> : k_stage<0, true>, grid, dim3(TJ, TI + RIM_ROWS), RIM_SMEM, s, P, M, A);
     else
         launch_tile(cdiff ? k_stage<1, false> : k_stage<0, false>, grid, dim3(TJ, TI), stage_smem_bytes(), s, P, M, A);

@@ -181,7 +181,7 @@ __device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, co
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
 // runs, and on the extra rows of threads.
 template <int MONITOR, bool RIM>
-__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), TNS_PER_SM(RIM ? 2 : TNS_STAGE_MX_MINB))
+__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), RIM ? RIM_MINB : TNS_PER_SM(TNS_STAGE_MX_MINB))
 k_stage_mx(Params P, Mesh M, StageArgsMx A) {
     StageArgsMx Ac = A;
     if (!MONITOR) Ac.cdiff = nullptr;
@@ -249,7 +249,7 @@ __device__ __forceinline__ bool viscous_mx_tile(const Params& P, const Mesh& M, 
 }
 
 template <bool RIM>
-__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), TNS_PER_SM(RIM ? 2 : TNS_VISC_MX_MINB))
+__global__ void __launch_bounds__(NTHREADS + (RIM ? TJ * RIM_ROWS : 0), RIM ? RIM_MINB : TNS_PER_SM(TNS_VISC_MX_MINB))
 k_viscous_mx(Params P, Mesh M, const double* __restrict__ q, float* __restrict__ vis, unsigned int* error) {
     viscous_mx_tile<RIM>(P, M, q, vis, error, blockIdx.x, blockIdx.y);
 }
@@ -493,7 +493,7 @@ void launch_viscous_mx(const Params& P, const Mesh& M, const double* q, float* v
                        cudaStream_t s, int beside) {
     const dim3 grid = tile_grid_mx(M);
     // the rim rows by the FP64 kernel's rule
-    if ((int)(grid.x * grid.y) + beside <= TNS_VISC_RIM_PER_SM * sm_count())
+    if ((int)(grid.x * grid.y) + beside <= VISC_RIM_PER_SM * sm_count())
         launch_tile(k_viscous_mx<true>, grid, dim3(TJ, TI + RIM_ROWS), visc_mx_smem_bytes(), s, P, M, q, vis, error);
     else
         launch_tile(k_viscous_mx<false>, grid, dim3(TJ, TI), visc_mx_smem_bytes(), s, P, M, q, vis, error);
@@ -506,8 +506,8 @@ void launch_stage_mx(const Params& P, const Mesh& M, const double* cold, const f
     const StageArgsMx A{cold, dqin, dqout, qout, d, vis, dt, dtmin, (float)alpha, dqin ? e : nullptr,
                         dqin ? nullptr : e, cdiff, status, error};
     const dim3 grid = tile_grid_mx(M);
-    // the rim rows by the FP64 stage's rule
-    if ((int)(grid.x * grid.y) + beside <= TNS_STAGE_RIM_PER_SM * sm_count())
+    // the rim rows by the FP64 stage's rule, which here follows the tile height (tns_tile.cuh)
+    if ((int)(grid.x * grid.y) + beside <= STAGE_MX_RIM_PER_SM * sm_count())
         launch_tile(cdiff ? k_stage_mx<1, true> : k_stage_mx<0, true>, grid, dim3(TJ, TI + RIM_ROWS),
                     stage_mx_smem_bytes(), s, P, M, A);
     else

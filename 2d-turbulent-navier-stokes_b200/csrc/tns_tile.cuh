@@ -45,6 +45,17 @@ constexpr int TJ = 32;      // tile extent along j (contiguous in memory)
 constexpr int GP_THREADS = 128;  // threads per port line of the type-6 port-flux kernels
 constexpr int TI = TNS_TI;  // tile extent along i
 constexpr int NTHREADS = TJ * TI;
+// Tiles an SM, in all meshes in flight, up to which the stage and viscous kernels take blocks with
+// extra rows of threads for a tile's rim (RIM_ROWS), at 8 rows a tile see launch_stage and
+// launch_viscous.  The mixed stage's line moves with the tile height, as its blocks' residency
+// does (16 rows, 200 tiles: 44.1 us an iteration with the extra rows, 38.5 without; 4 rows, 560
+// tiles: 28.3 with, 31.6 without).  The others' does not: the FP64 stage's early operands outweigh
+// a second round of blocks (16 rows, 200 tiles: 48.4 with, 50.8 without), and the viscous blocks
+// soon lack shared memory (4 rows, 280 tiles: 31.5 with, 27.2 without).
+constexpr int STAGE_RIM_PER_SM = TNS_STAGE_RIM_PER_SM;
+constexpr int STAGE_MX_RIM_PER_SM = TNS_PER_SM(TNS_STAGE_RIM_PER_SM);
+constexpr int VISC_RIM_PER_SM = TNS_VISC_RIM_PER_SM;
+constexpr int RIM_MINB = TNS_PER_SM(2);  // resident blocks an SM the register budget of such a kernel is for
 // Halo-1 slot grid (TI+2) x (TJ+2).
 constexpr int SW = TJ + 2;
 constexpr int NSLOT = (TI + 2) * SW;
