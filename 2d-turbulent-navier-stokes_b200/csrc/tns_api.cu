@@ -1259,8 +1259,8 @@ void tns_destroy(tns_handle* h) {
     h->qa2.release(); h->dqb.release(); h->dqc.release(); h->df.release(); h->visf.release(); h->ef.release();
     h->dtf.release(); h->tref.release(); h->dcell_of.release(); h->renum.release();
     for (auto* b : {&h->x, &h->y, &h->cfldl, &h->gxc, &h->gyc, &h->ginj, &h->gport, &h->qa, &h->qb,
-                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->vcfl, &h->e, &h->wport, &h->wport_i,
-                    &h->stile, &h->vtile})
+                    &h->qc, &h->d, &h->vis, &h->dt, &h->dtmin, &h->partial, &h->primout, &h->cvol, &h->vcfl, &h->e,
+                    &h->wport, &h->wport_i, &h->stile, &h->vtile})
         b->release();
     h->grec.release(); h->bnode.release(); h->gtype.release(); h->grank.release(); h->ports.release();
     h->counter.release(); h->status.release(); h->cdiff.release();

@@ -136,8 +136,9 @@ TNS_HD double powi(double x, int n) {
 // temperatures, squared speeds -- never need.  The kernels are bound by instruction issue and
 // dependent FP64 latency: with these, the cubic T**-1/5 step, the shorter expm1 and the skipped
 // denominators below, a FP64 iteration of the 1024 x 384 nozzle-plume went 0.180 -> 0.160 ms
-// (0.041 -> 0.0375 ms on the 115 x 50 nozzle), its error against a FP64 restatement unchanged.  recip(0), recip(inf) and root(inf) are NaN: a
-// state that holds them is non-finite either way.  root() takes a subnormal for zero.
+// (0.041 -> 0.0375 ms on the 115 x 50 nozzle).  A product with recip() is rounded twice: where it
+// becomes part of the state, use quot().  recip(0), recip(inf) and root(inf) are NaN: a state that
+// holds them is non-finite either way.  root() takes a subnormal for zero.
 TNS_HD double recip(double x) {
 #ifdef __CUDA_ARCH__
     double r;

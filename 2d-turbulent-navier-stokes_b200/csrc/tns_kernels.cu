@@ -351,13 +351,13 @@ k_stage(Params P, Mesh M, StageArgs A) {
 // The copies take the global-load latency (4.7 of 11.6 stall cycles an instruction in the
 // kernel above, half of its time) out of the warps; a tile's buffers fit three times into an
 // SM because VIS + D is one array (and stage 1's Q_old is its input, read again from global
-// memory), so 24 warps stay resident at 80 registers (with D and VIS
-// apart and two blocks a SM it was no faster than the plain kernel).  What bounds it now:
-// issue (0.5 an SM quarter a cycle under 24 warps) and the launch.  1024 x 384 nozzle-plume,
-// a FP64 iteration: 0.153 ms with the plain kernel in all stages, 0.138 ms with this one;
-// 2048 x 768 port 0.647 -> 0.565 ms; stage 1 by it as well 0.1179 -> 0.1161 ms.  It needs more tiles than the plain kernel has resident
-// blocks (at 384 tiles the two take the same 42 us an iteration) and rows and arrays that
-// TMA can address.
+// memory), so 24 warps stay resident at 80 registers (with D and VIS apart and two blocks an SM
+// it was no faster than the plain kernel).  What bounds it now: issue (0.5 an SM quarter a cycle
+// under 24 warps) and the launch.  1024 x 384 nozzle-plume, a FP64 iteration: 0.153 ms with the
+// plain kernel in all stages, 0.138 ms with this one; 2048 x 768 port 0.647 -> 0.565 ms; stage 1
+// by it as well 0.1179 -> 0.1161 ms.  It needs more tiles than the plain kernel has resident
+// blocks (at 384 tiles the two take the same 42 us an iteration) and rows and arrays that TMA can
+// address.
 constexpr int QH = TI + 2, QW = TJ + 4;  // halo box
 static_assert(QW % 2 == 0 && STILE % 2 == 0, "box rows and static blocks are multiples of 16 bytes");
 
@@ -382,8 +382,8 @@ template <int MONITOR, bool FIRST>
 __global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MINB))
 k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ StageMaps maps) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    StagePipeSmem& W =
-        *reinterpret_cast<StagePipeSmem*>(smem_raw + ((128u - ((unsigned)__cvta_generic_to_shared(smem_raw) & 127u)) & 127u));
+    const unsigned skew = (128u - ((unsigned)__cvta_generic_to_shared(smem_raw) & 127u)) & 127u;
+    StagePipeSmem& W = *reinterpret_cast<StagePipeSmem*>(smem_raw + skew);
     StageSlots& S = W.w;
     const int ntj = (M.nj + TJ - 1) / TJ;
     const int tj = threadIdx.x, ti = threadIdx.y, tid = ti * TJ + tj;
@@ -396,7 +396,8 @@ k_stage_pipe(Params P, Mesh M, StageArgs A, int ntiles, const __grid_constant__ 
         tensor_copy_3d(W.q, &maps.q, col_of(t) * TJ - 2, row_of(t) * TI - 1, 0, &W.bar_a);
     };
     auto fetch_b = [&](int t) {
-        bulk_copy_start(W.st, M.stile + ((size_t)row_of(t) * ntj + col_of(t)) * STILE, sizeof(double) * STILE, &W.bar_b);
+        const size_t tile = (size_t)row_of(t) * ntj + col_of(t);
+        bulk_copy_start(W.st, M.stile + tile * STILE, sizeof(double) * STILE, &W.bar_b);
     };
     auto fetch_c = [&](int t) {
         const int j0 = col_of(t) * TJ, i0 = row_of(t) * TI;
@@ -510,9 +511,11 @@ size_t visc_smem_bytes() { return sizeof(ViscSmem<double>); }
 template <bool RIM>
 __device__ __forceinline__ bool viscous_tile_f64(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                  double* __restrict__ vis, unsigned int* error, int bx, int by) {
-    return viscous_tile<RIM, double>(
-        P, M, q, vis, error, bx, by, [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc, double gd, double ry,
-                                      double out[4]) { viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
+    return viscous_tile<RIM, double>(P, M, q, vis, error, bx, by,
+                                     [&](const FaceVals& f, double sx, double sy, double ga, double gb, double gc,
+                                         double gd, double ry, double out[4]) {
+                                         viscous_face(P, f, sx, sy, ga, gb, gc, gd, ry, out);
+                                     });
 }
 
 template <bool RIM>
@@ -530,7 +533,8 @@ __device__ __forceinline__ void dissipation_tile_f64(const Params& P, const Mesh
     dissipation_tile(P, M, A, bx, by, [](const double*) {});
 }
 
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MINB)) k_dissipation(Params P, Mesh M, DissArgs<double> A) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MINB))
+k_dissipation(Params P, Mesh M, DissArgs<double> A) {
     dissipation_tile_f64(P, M, A, blockIdx.x, blockIdx.y);
 }
 
@@ -811,28 +815,26 @@ void launch_face_states(const Params& P, const Mesh& M, const double* prim, doub
 
 // One launch per kernel advances every active case of a batch; block b works on tile
 // tiles[b] = (case, tile j, tile i) with its case's parameters and buffers.
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MINB)) k_dissipation_batch(const BatchCase* __restrict__ cases,
-                                                                const int4* __restrict__ tiles,
-                                                                const int* __restrict__ active) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MINB))
+k_dissipation_batch(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles,
+                    const int* __restrict__ active) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;  // whole block: before any barrier
     const BatchCase& c = cases[t.x];
     dissipation_tile_f64(c.P, c.M, c.diss, t.y, t.z);
 }
 
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_BATCH_MINB)) k_viscous_batch(const BatchCase* __restrict__ cases,
-                                                                          const int4* __restrict__ tiles,
-                                                                          const int* __restrict__ active) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_BATCH_MINB))
+k_viscous_batch(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles, const int* __restrict__ active) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;
     const BatchCase& c = cases[t.x];
     viscous_tile_f64<false>(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
 }
 
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_BATCH_MINB)) k_stage_batch(const BatchCase* __restrict__ cases,
-                                                                         const int4* __restrict__ tiles,
-                                                                         const int* __restrict__ active,
-                                                                         int stage, int monitor) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_BATCH_MINB))
+k_stage_batch(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles, const int* __restrict__ active,
+              int stage, int monitor) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;
     const BatchCase& c = cases[t.x];
@@ -919,14 +921,16 @@ static dim3 tile_grid(const Mesh& M) { return dim3((M.nj + TJ - 1) / TJ, (M.ni +
 // SMs of the current device, and the pipelined stage's resident blocks on all of them.
 int sm_count() {
     int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 148;
     return n;
 }
 constexpr size_t PIPE_SMEM = sizeof(StagePipeSmem) + 128;  // (the kernel aligns its boxes to 128 bytes)
 static int pipe_grid() {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pipe<0, false>, NTHREADS, PIPE_SMEM) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pipe<0, false>, NTHREADS, PIPE_SMEM) !=
+        cudaSuccess)
         return 0;
     return per_sm * sm_count();
 }
@@ -1092,8 +1096,8 @@ void launch_stage(const Params& P, const Mesh& M, const double* qin, const doubl
     StageMaps maps;
     const int pipe = (A.e || !cdiff) && ntiles > TNS_PER_SM(TNS_STAGE_MINB) * sm_count() ? pipe_grid() : 0;
     if (pipe > 0 && pipe <= ntiles && stage_maps(P, M, A, &maps)) {
-        launch_tile(!A.e ? k_stage_pipe<0, true> : cdiff ? k_stage_pipe<1, false> : k_stage_pipe<0, false>, dim3(pipe), dim3(TJ, TI), PIPE_SMEM, s, P, M, A, ntiles,
-                    maps);
+        launch_tile(!A.e ? k_stage_pipe<0, true> : cdiff ? k_stage_pipe<1, false> : k_stage_pipe<0, false>, dim3(pipe),
+                    dim3(TJ, TI), PIPE_SMEM, s, P, M, A, ntiles, maps);
         return;
     }
     // the rim rows while every tile has its own resident block of that size (at 8 rows a tile; for

@@ -243,9 +243,11 @@ __device__ __forceinline__ void viscous_face_mx(const Params& P, const FaceVals&
 template <bool RIM>
 __device__ __forceinline__ bool viscous_mx_tile(const Params& P, const Mesh& M, const double* __restrict__ q,
                                                 float* __restrict__ vis, unsigned int* error, int bx, int by) {
-    return viscous_tile<RIM, float>(
-        P, M, q, vis, error, bx, by, [&](const FaceVals& f, float sx, float sy, float ga, float gb, float gc, float gd,
-                                      double ry, float out[4]) { viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out); });
+    return viscous_tile<RIM, float>(P, M, q, vis, error, bx, by,
+                                    [&](const FaceVals& f, float sx, float sy, float ga, float gb, float gc, float gd,
+                                        double ry, float out[4]) {
+                                        viscous_face_mx(P, f, sx, sy, ga, gb, gc, gd, ry, out);
+                                    });
 }
 
 template <bool RIM>
@@ -312,19 +314,18 @@ __global__ void k_prim_out_mx(Params P, Mesh M, const double* __restrict__ cold,
 
 // Mixed-path batch: `parity` selects which of qa / qa2 holds each active case's state
 // (all active cases advance together, so they share it).
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MX_MINB)) k_dissipation_mx_batch(const BatchCase* __restrict__ cases,
-                                                                   const int4* __restrict__ tiles,
-                                                                   const int* __restrict__ active, int parity) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_DISS_MX_MINB))
+k_dissipation_mx_batch(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles,
+                       const int* __restrict__ active, int parity) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;  // whole block: before any barrier
     const BatchCase& c = cases[t.x];
     dissipation_mx_tile(c.P, c.M, c.qmx[parity], c.df, c.dtf, c.dtmin, t.y, t.z);
 }
 
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_MX_BATCH_MINB)) k_viscous_mx_batch(const BatchCase* __restrict__ cases,
-                                                                                const int4* __restrict__ tiles,
-                                                                                const int* __restrict__ active,
-                                                                                int parity) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_VISC_MX_BATCH_MINB))
+k_viscous_mx_batch(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles,
+                   const int* __restrict__ active, int parity) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;
     const BatchCase& c = cases[t.x];
@@ -351,10 +352,9 @@ __device__ __forceinline__ bool stage_mx_batch_tile(const BatchCase& c, const St
 #endif
 }
 
-__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MX_BATCH_MINB)) k_stage_mx_batch(const BatchCase* __restrict__ cases,
-                                                                               const int4* __restrict__ tiles,
-                                                                               const int* __restrict__ active,
-                                                                               int parity, int stage, int monitor) {
+__global__ void __launch_bounds__(NTHREADS, TNS_PER_SM(TNS_STAGE_MX_BATCH_MINB))
+k_stage_mx_batch(const BatchCase* __restrict__ cases, const int4* __restrict__ tiles, const int* __restrict__ active,
+                 int parity, int stage, int monitor) {
     const int4 t = tiles[blockIdx.x];
     if (!active[t.x]) return;
     const BatchCase& c = cases[t.x];

@@ -1,6 +1,7 @@
 // tns_tile.cuh -- tile geometry and the helpers every tile kernel shares: bulk copies,
-// programmatic dependent launch, halo classification, primitive variables of a cell, and the ghost state of a halo
-// position (BC of boundary.f90:24-327 from the parent and its opposite neighbour).
+// programmatic dependent launch, halo classification, primitive variables of a cell, and the
+// ghost state of a halo position (BC of boundary.f90:24-327 from the parent and its opposite
+// neighbour).
 #pragma once
 
 #include <utility>

@@ -3,7 +3,7 @@
 // its ghosts), the nodal averages, then each face once; a cell adds its four faces in order
 // 1..4, negating the two that were evaluated in the neighbour's orientation.
 //
-// The face geometry (vector, diamond-gradient coefficients, 1/YAVG: 31 KB a tile) is static:
+// The face geometry (vector, diamond-gradient coefficients, 1/YAVG: 31 KB a tile, mixed 18) is static:
 // one bulk copy per tile, started before the previous kernel has ended.  Each face's flux
 // then takes the place of its own geometry, which only the thread that evaluates it reads.
 // Boundary nodes find the visit order and the types of their two ghosts in a static code
