@@ -240,8 +240,7 @@ __device__ __forceinline__ void stage_cdiff(const StageArgs& A, const double dv[
 
 // One RK stage (turbnstwod.f90:204-227, boundary.f90:24-48, source_terms.f90:24-104,
 // residual.f90:23-83) on a TI x TJ tile with its halo staged in shared memory.  RIM: the block
-// has RIM_ROWS more rows of threads, which evaluate the halo.  False (for the whole block) where
-// the static block did not arrive: the block then leaves the kernel.
+// has RIM_ROWS more rows of threads, which evaluate the halo.  The result: tile_copy_wait.
 template <bool RIM>
 __device__ __forceinline__ bool stage_tile(const Params& P, const Mesh& M, const StageArgs& A, int bx, int by) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -302,10 +301,7 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const Mesh& M, const
     }
     if (valid) own_t = put_cell_slot(P, S.w, (ti + 1) * SW + tj + 1, qo);
     if (h.kind >= 0) put_halo_slot(P, M, S.w, h, site, qr, [&](double c[5]) { load(h.ci + h.oi, h.cj + h.oj, c); });
-    if (!bulk_wait_block(&S.bar, A.error)) {
-        if (RIM) copies_wait();
-        return false;
-    }
+    const bool arrived = tile_copy_wait(&S.bar, A.error);
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid) {
         const size_t cell = (size_t)i * M.nj + j;
@@ -327,7 +323,7 @@ __device__ __forceinline__ bool stage_tile(const Params& P, const Mesh& M, const
                    }, dv);
     }
     if (A.cdiff) stage_cdiff(A, dv);
-    return true;
+    return arrived;
 }
 
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
@@ -886,9 +882,8 @@ k_batch_persistent(const BatchCase* __restrict__ cases, const int4* __restrict__
                     else if (ph == 0) ok = viscous_tile_f64<false>(c.P, c.M, c.q, c.vis, c.stage[0][0].error, t.y, t.z);
                     else ok = stage_tile<false>(c.P, c.M, c.stage[0][ph - 1], t.y, t.z);
                 }
-                if (!ok) return;  // the whole block
                 async_proxy_fence();
-                __syncthreads();
+                if (!__syncthreads_and(ok)) return;  // the whole block
             }
             if (!grid_barrier(bar, bar + 1)) {
                 if (threadIdx.x == 0 && threadIdx.y == 0) atomicOr(error, 4u);

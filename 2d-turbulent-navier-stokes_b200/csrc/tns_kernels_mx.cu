@@ -69,8 +69,7 @@ size_t stage_mx_smem_bytes() { return sizeof(StageSmemMx); }
 #endif
 // One stage on tile (bx, by) of a mesh; the single-case and the batched kernels wrap it.
 // RIM: the block has RIM_ROWS more rows of threads, which form the halo.  LATE: the halo's places
-// are looked up after the own slots (they cost registers until then).  False (for the whole
-// block) where the static block did not arrive: the block then leaves the kernel.
+// are looked up after the own slots (they cost registers until then).  The result: tile_copy_wait.
 template <bool RIM, bool LATE = false>
 __device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, const StageArgsMx& A,
                                               int bx, int by) {
@@ -158,7 +157,7 @@ __device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, co
         slot_ghost_mx(S.ref, gh, o);
         W.put(h.li * SW + h.lj, o);
     }
-    if (!bulk_wait_block(&S.bar, A.error)) return false;
+    const bool arrived = tile_copy_wait(&S.bar, A.error);
     double dv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid) {
         const int c = (ti + 1) * SW + (tj + 1);
@@ -175,7 +174,7 @@ __device__ __forceinline__ bool stage_mx_tile(const Params& P, const Mesh& M, co
                       }, dv);
     }
     if (A.cdiff) stage_cdiff_mx(A, dv);
-    return true;
+    return arrived;
 }
 
 // Specialised on the residual monitor, so the CDIFF reduction is compiled only where it
@@ -412,9 +411,8 @@ k_batch_persistent_mx(const BatchCase* __restrict__ cases, const int4* __restric
                     ok = viscous_mx_tile<false>(sP, sM, c.qmx[parity], c.visf, c.stage_mx[0][0][0].error, t.y, t.z);
                 else
                     dissipation_mx_tile(sP, sM, c.qmx[parity], c.df, c.dtf, c.dtmin, t.y, t.z);
-                if (!ok) return;  // the whole block
                 async_proxy_fence();
-                __syncthreads();
+                if (!__syncthreads_and(ok)) return;  // the whole block
             }
             if (!grid_barrier(bar, bar + 1)) {
                 if (threadIdx.x == 0 && threadIdx.y == 0) atomicOr(error, 4u);

@@ -204,26 +204,26 @@ __device__ __forceinline__ bool bulk_wait(unsigned long long* bar, unsigned pari
     return false;
 }
 
-// Waits for the block's one-shot copy, and is the block barrier its threads would need there
-// anyway: the block goes on or gives up as one.  (Each thread counts its own polls, so around the
-// limit some see the copy and some do not; were each to leave by itself, those would miss the
-// block's later barriers, and in a kernel that loops over tiles run one barrier ahead of the
-// others into the next tile's buffers.)  On false the copy did not complete: that is reported
-// (bit 1 of *error), the copy, which writes this block's shared memory, had one more bounded wait,
-// and the caller leaves the kernel.  On true no thread looks at the barrier any more, and it is
-// taken down: a kernel that loops over tiles writes other data over its place and sets one up
-// there again, neither of which a live barrier allows.
-__device__ __forceinline__ bool bulk_wait_block(unsigned long long* bar, unsigned int* error) {
-    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
-    if (__syncthreads_and(bulk_wait(bar))) {
-        if (first) bulk_barrier_end(bar);
-        return true;
-    }
-    if (first) {
+// A tile's wait for its static copy, and the block barrier its threads need there anyway.  Each
+// thread counts its own polls, so around the limit some see the copy and some do not.  None
+// leaves by itself (it would miss the block's later barriers, and in a kernel that loops over
+// tiles run one barrier ahead of the others into the next tile's buffers): a thread that gives up
+// reports it (bit 1 of *error, which ends the run with an error), gives the copy, which writes this
+// block's shared memory, one more bounded wait, and goes through the tile with what is there --
+// geometry, no indices.  The result says whether the copy arrived; a kernel that loops over tiles
+// votes on it before the next.  After the barrier no thread looks at the copy's barrier any more
+// and it is taken down: such a kernel writes other data over its place and sets one up there
+// again, neither of which a live barrier allows.  (A vote in place of this barrier cost 1 % of an
+// iteration on small meshes.)
+__device__ __forceinline__ bool tile_copy_wait(unsigned long long* bar, unsigned int* error) {
+    bool arrived = bulk_wait(bar);
+    if (!arrived) {
         atomicOr(error, 2u);
-        bulk_wait(bar);
+        arrived = bulk_wait(bar);
     }
-    return false;
+    __syncthreads();
+    if (arrived && threadIdx.x == 0 && threadIdx.y == 0) bulk_barrier_end(bar);
+    return arrived;
 }
 
 // Orders this thread's shared-memory accesses before later bulk copies into them (issued after

@@ -52,8 +52,7 @@ __device__ __forceinline__ void face_values(const ViscSmem<G>& S, int sa, int sc
 }
 
 // face(FaceVals, G sx, sy, ga, gb, gc, gd, double ryavg, G out[4]) evaluates one face's flux.
-// False (for the whole block; bit 1 of *error set) where the tile's static copy did not complete:
-// the block then leaves the kernel.  RIM: the block has
+// The result: tile_copy_wait.  RIM: the block has
 // RIM_ROWS more rows of threads, which take the halo, the nodes and the faces beyond the
 // cells' own.
 template <bool RIM, class G, class OutT, class Face>
@@ -191,7 +190,7 @@ __device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, con
     };
     if (mine && i <= M.ni && j <= M.nj) node(ti, tj, code0);
     if (extra && i0 + xa <= M.ni && j0 + xb <= M.nj) node(xa, xb, code1);
-    if (!bulk_wait_block(&S.bar, error)) return false;
+    const bool arrived = tile_copy_wait(&S.bar, error);
     auto eval = [&](int f, int sa, int sc, int ab, int ad) {
         FaceVals v;
         face_values(S, sa, sc, ab, ad, v);
@@ -224,7 +223,7 @@ __device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, con
         eval(iface ? la * TJ + lb : NIF + la * AW + lb, flip ? s : sb, flip ? sb : s, rev ? nb : n, rev ? n : nb);
     }
     __syncthreads();
-    if (!valid) return true;
+    if (!valid) return arrived;
     const size_t cell = (size_t)i * M.nj + j;
     const int f1 = NIF + ti * AW + tj, f4 = ti * TJ + tj;  // j-face j, i-face i
     const double s1 = (j == 0) ? 1.0 : -1.0, s4 = (i == 0) ? 1.0 : -1.0;
@@ -233,7 +232,7 @@ __device__ __forceinline__ bool viscous_tile(const Params& P, const Mesh& M, con
         vis[k * ncell + cell] =
             (OutT)(((s1 * (double)S.fg[k][f1] + (double)S.fg[k][f4 + TJ]) + (double)S.fg[k][f1 + 1]) +
                    s4 * (double)S.fg[k][f4]);
-    return true;
+    return arrived;
 }
 
 }  // namespace tns
