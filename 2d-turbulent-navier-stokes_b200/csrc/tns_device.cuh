@@ -164,12 +164,16 @@ TNS_HD double root(double x) {
 #endif
 }
 
-// a/b by recip and one correction of the quotient (Markstein, IBM J. Res. Dev. 34(1), 1990): the
-// correctly rounded quotient but for rare cases, where a product with the reciprocal is rounded
-// twice.  For quotients that become part of the state.
+// a/b as recip's estimate after its first step (2^-40), the product with it and one correction of
+// the quotient (Markstein, IBM J. Res. Dev. 34(1), 1990), which leaves 2^-80 before the last
+// rounding: the correctly rounded quotient but for rare cases, in as many operations as a product
+// with recip(), which is rounded twice.  For quotients that become part of the state.
 TNS_HD double quot(double a, double b) {
 #ifdef __CUDA_ARCH__
-    const double r = recip(b), q = a * r;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    r = fma(r, fma(-b, r, 1.0), r);
+    const double q = a * r;
     return fma(fma(-q, b, a), r, q);
 #else
     return a / b;
