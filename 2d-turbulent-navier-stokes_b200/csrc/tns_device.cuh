@@ -276,10 +276,10 @@ TNS_HD double damping_fmu(double chi) {
 struct Damping {
     double fmu, fr2;
 };
-TNS_HD Damping damping(double chi, double fr2k) {
+TNS_HD Damping damping(const Params& P, double chi) {  // (P by reference: FR2K is loaded at its use)
     const double chi2 = chi * chi;
     const Ratio m = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
-    const Ratio r = tanh_ratio_parts(root(chi), chi * fr2k);
+    const Ratio r = tanh_ratio_parts(root(chi), chi * P.fr2k);
     const double num = r.num * 0x1p700, den = r.den * 0x1p700;
     const double inv = recip(m.den * den);
     return Damping{m.num * den * inv, num * m.den * inv};
@@ -604,7 +604,7 @@ __device__ __forceinline__ void source_terms(const Params& P, const SrcIn& s, do
     const FifthRoots tr = fifth_roots(TI);
     const double AMU = P.suth_amol * (TI * tr.m04);
     const double CHI = RHO * RI * (P.inv_cmu_suth * tr.m06);
-    const Damping damp = damping(CHI, P.fr2k);
+    const Damping damp = damping(P, CHI);
     const double FMU = damp.fmu, FR2 = damp.fr2;
     const double AMUT = FMU * RHO * RI;
     const double PHI = DQX * DRX + DQY * DRY;

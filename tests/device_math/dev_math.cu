@@ -17,8 +17,8 @@ __global__ void k_eval(int fn, Params P, long long n, const double* a, const dou
         case 2: r = quot(x, y); break;
         case 3: r = fifth_roots(x).m04; break;
         case 4: r = fifth_roots(x).m06; break;
-        case 5: r = damping(x, P.fr2k).fmu; break;
-        case 6: r = damping(x, P.fr2k).fr2; break;
+        case 5: r = damping(P, x).fmu; break;
+        case 6: r = damping(P, x).fr2; break;
         case 7: r = damping_fmu(x); break;
         case 8: r = adj::tanh_work(x).t; break;
         case 9: r = adj::tanh_work(x).inv; break;
