@@ -261,7 +261,7 @@ TNS_HD Ratio tanh_ratio_parts(double a, double b) {
 }
 TNS_HD double tanh_ratio(double a, double b) {
     const Ratio r = tanh_ratio_parts(a, b);
-    return r.num / r.den;
+    return r.num * recip(r.den);
 }
 
 // The damping ratios of the turbulence model at CHI = RHO nu~ / (CMU AMU):
@@ -270,8 +270,7 @@ TNS_HD double tanh_ratio(double a, double b) {
 // product of the denominators, some CHI^3 for small CHI, from underflowing before CHI^2 does.
 TNS_HD double damping_fmu(double chi) {
     const double chi2 = chi * chi;
-    const Ratio m = tanh_ratio_parts(ALPHA_T * chi2, BETA_T * chi2);
-    return m.num * recip(m.den);
+    return tanh_ratio(ALPHA_T * chi2, BETA_T * chi2);
 }
 struct Damping {
     double fmu, fr2;
